@@ -9,13 +9,18 @@
 // on its 4 neighbours, handled breadth first with multiplicity merging 1 - (1 - p)^m before the next photon; trap
 // afterpulses are scheduled per firing and fired after all photons in time order.
 //
-// GPU mapping: one warp per SiPM.  The warp stages the SiPM's photons in shared memory, sorts them by
-// (time, draw key) with a bitonic network, and keeps the pixel state (last-discharge time per pixel + a fired
-// bitmap) in shared memory.  Photons are evaluated 32 at a time, one per lane, against the state at the start of the
-// batch; the batch commits up to the first lane whose result could depend on an earlier lane of the same batch (same
-// pixel as an earlier lane) or that starts a cross-talk cascade (then the cascade runs, generation by generation,
-// with the frontier spread over the lanes).  Keyed draws make every lane's random numbers independent of the
-// processing order, so the result is exactly the serial one.
+// GPU mapping: one warp per SiPM.  The warp draws every photon's pixel and fire uniform as it loads it and keeps only
+// those that can fire (4 in 10), in time order, in shared memory beside the pixel state (last-discharge time per pixel +
+// a fired bitmap); it then steps through them with their first-generation cross-talk, one touch of a pixel per lane
+// (simulate_sipm).  Keyed draws make every lane's random numbers independent of the processing order, so the result is
+// exactly the serial one.
+//
+// What bounds the SiPM kernel: instruction issue and instruction fetch.  All warps are at different places of one large
+// loop body; DRAM traffic is 2 % of the peak.  Measured on 65,536 workload events (7.8 M SiPMs of 85 photons, FP32):
+// evaluating all 85 photons in the serial step 79.3 ms; only those that can fire, with their first generation in the
+// step, all inlined (98 KB of code, 59 % of the fetches hit) 79.7 ms; photons and nodes in one lane order (62 KB)
+// 42.0 ms; rare paths as calls with one copy of Philox (51 KB) 36.0 ms; all first-pass draws as calls, 20 warps instead
+// of 16 per SM 33.0 ms.  FP64, 1,500 events: 14.4 -> 4.3 ms (draws decided on integers, most photons never reach FP64).
 #pragma once
 #include "crv_device.cuh"
 #include "crv_scan.cuh"
@@ -325,7 +330,6 @@ __global__ void k_photon_emit(CrvParams p, CrvEvents ev, CrvSteps st, CrvBars ba
 // scheduled afterpulses per SiPM: a SiPM of at most 256 photons fires at most a few hundred pixels, with trap-0
 // probabilities of a few percent; beyond the queue the SiPM reports CRV_ST_LIMIT
 __host__ __device__ constexpr int sipm_tcap(int cap) { return cap <= 256 ? 32 : 128; }
-constexpr int SIPM_WARPS = 8;    // warps per block
 
 struct SipmGroups {
   const long long* n;            // device: number of groups
@@ -352,86 +356,115 @@ struct SipmOut {
   int32_t* fired;                // pixels that fired at least once
 };
 
-template <typename R>
+// The staged photons are those that can fire (see k_sipm_sim): time, draw key, and the pixel with a flag.
+constexpr uint32_t PH_PIX = 0x7FFu;      // pixel id (below 1,681)
+constexpr uint32_t PH_FIRES = 0x8000u;   // its fire uniform is below the firing probability at full overvoltage
+
+// A warp's shared memory: CAP photons; LOC: the photons' positions in the group are kept (ph_loc), for per-photon ids
+// (photon_id); without them a warp needs 4 bytes less per photon and more warps fit an SM.  One byte offset and
+// compile-time offsets from it, so the layout costs one register, passes to the called functions as it is, and every
+// access is a shared-memory one there too.
+extern __shared__ __align__(16) char sipm_smem[];
+template <typename R, int CAP, bool LOC>
 struct SipmShared {
-  R* ph_t;
-  uint32_t* ph_key;
-  uint32_t* ph_loc;
-  R* last;
-  uint32_t* bm;
-  R* tr_t;
-  R* tr_uf;
-  long long* tr_id;
-  uint16_t* tr_pix;
-  uint16_t* fr_pix;
-  uint16_t* fr_m;
-  uint16_t* cand;
-  int* misc;                     // [0] n candidates
-  int tcap;                      // afterpulse queue length
+  static constexpr int TCAP = sipm_tcap(CAP);                      // afterpulse queue length
+  static constexpr int O_T = NPS_ALLOC * int(sizeof(R)), O_TRT = O_T + CAP * int(sizeof(R)),
+                       O_TRU = O_TRT + TCAP * int(sizeof(R)), O_TRI = O_TRU + TCAP * int(sizeof(R)),
+                       O_KEY = O_TRI + TCAP * 8, O_LOC = O_KEY + CAP * 4, O_BM = O_LOC + (LOC ? CAP * 4 : 0),
+                       O_MISC = O_BM + 64 * 4, O_CAND = O_MISC + 16, O_TRP = O_CAND + 256 * 2,
+                       O_FRP = O_TRP + TCAP * 2, O_FRM = O_FRP + 64 * 2, O_PIX = O_FRM + 64 * 2,
+                       BYTES = (O_PIX + CAP * 2 + 15) / 16 * 16;
+  static_assert(O_TRI % 8 == 0, "afterpulse ids on 8 bytes");
+  int base;
+  template <typename T>
+  __device__ __forceinline__ T* at(int off) const { return reinterpret_cast<T*>(sipm_smem + base + off); }
+  __device__ __forceinline__ R* last() const { return at<R>(0); }
+  __device__ __forceinline__ R* ph_t() const { return at<R>(O_T); }
+  __device__ __forceinline__ uint32_t* ph_key() const { return at<uint32_t>(O_KEY); }
+  __device__ __forceinline__ uint32_t* ph_loc() const { return at<uint32_t>(O_LOC); }
+  __device__ __forceinline__ uint16_t* ph_pix() const { return at<uint16_t>(O_PIX); }   // PH_PIX | PH_FIRES
+  __device__ __forceinline__ uint32_t* bm() const { return at<uint32_t>(O_BM); }
+  __device__ __forceinline__ R* tr_t() const { return at<R>(O_TRT); }
+  __device__ __forceinline__ R* tr_uf() const { return at<R>(O_TRU); }
+  __device__ __forceinline__ long long* tr_id() const { return at<long long>(O_TRI); }
+  __device__ __forceinline__ uint16_t* tr_pix() const { return at<uint16_t>(O_TRP); }
+  __device__ __forceinline__ uint16_t* fr_pix() const { return at<uint16_t>(O_FRP); }
+  __device__ __forceinline__ uint16_t* fr_m() const { return at<uint16_t>(O_FRM); }
+  // 256 cross-talk candidates; also the photon step's 32 node words
+  __device__ __forceinline__ uint16_t* cand() const { return at<uint16_t>(O_CAND); }
+  __device__ __forceinline__ uint32_t* nodes() const { return at<uint32_t>(O_CAND); }
+  __device__ __forceinline__ int* misc() const { return at<int>(O_MISC); }   // [0..3] run_cascade's results
 };
-
-// loc: the photons' positions in the group are kept (ph_loc), for per-photon ids (photon_id); without them a warp
-// needs 4 bytes less per photon and more warps fit an SM
-template <typename R>
-__host__ __device__ inline size_t sipm_smem_per_warp(int cap, bool loc = true) {
-  size_t b = 0;
-  b += size_t(cap) * (sizeof(R) + (loc ? 8 : 4));   // ph_t, ph_key, ph_loc
-  b += NPS_ALLOC * sizeof(R);                  // last
-  b += 64 * 4;                                 // bm (53 used)
-  b += size_t(sipm_tcap(cap)) * (2 * sizeof(R) + 8 + 2);   // traps
-  b += 64 * 2 + 64 * 2 + 256 * 2 + 16;         // frontier, candidates, misc
-  return (b + 15) & ~size_t(15);
-}
-
-template <typename R>
-__device__ SipmShared<R> carve(char* base, int cap, bool loc) {
-  SipmShared<R> S;
-  char* q = base;
-  S.last = reinterpret_cast<R*>(q); q += NPS_ALLOC * sizeof(R);
-  S.ph_t = reinterpret_cast<R*>(q); q += size_t(cap) * sizeof(R);
-  const int tcap = sipm_tcap(cap);
-  S.tcap = tcap;
-  S.tr_t = reinterpret_cast<R*>(q); q += tcap * sizeof(R);
-  S.tr_uf = reinterpret_cast<R*>(q); q += tcap * sizeof(R);
-  S.tr_id = reinterpret_cast<long long*>(q); q += tcap * 8;
-  S.ph_key = reinterpret_cast<uint32_t*>(q); q += size_t(cap) * 4;
-  S.ph_loc = loc ? reinterpret_cast<uint32_t*>(q) : nullptr;
-  if (loc) q += size_t(cap) * 4;
-  S.bm = reinterpret_cast<uint32_t*>(q); q += 64 * 4;
-  S.misc = reinterpret_cast<int*>(q); q += 16;
-  S.tr_pix = reinterpret_cast<uint16_t*>(q); q += tcap * 2;
-  S.fr_pix = reinterpret_cast<uint16_t*>(q); q += 64 * 2;
-  S.fr_m = reinterpret_cast<uint16_t*>(q); q += 64 * 2;
-  S.cand = reinterpret_cast<uint16_t*>(q); q += 256 * 2;
-  return S;
-}
 
 __device__ __forceinline__ bool bm_test(const uint32_t* bm, int p) { return (bm[p >> 5] >> (p & 31)) & 1u; }
 __device__ __forceinline__ void bm_set(uint32_t* bm, int p) { atomicOr(&bm[p >> 5], 1u << (p & 31)); }
 
+// The integer a uniform is made of (uni = bits * 2^-53 in FP64, * 2^-24 in FP32, both exact) and the threshold T of a
+// probability q with bits < T exactly when uni < q: a draw is then decided by one integer compare, without building
+// the uniform (in FP64 two conversions, a multiplication and a compare on the FP64 pipe).
+template <typename R> struct UniBits;
+template <> struct UniBits<double> {
+  using T = unsigned long long;
+  static __device__ __forceinline__ T of(const U4& w, int h) { return h ? bits53(w.z, w.w) : bits53(w.x, w.y); }
+  static __device__ __forceinline__ T below(double q) {
+    const double x = q * 0x1p53;
+    if (!(x > 0.0)) return 0ull;
+    if (x >= 0x1p53) return 1ull << 53;
+    const T k = (T)x;
+    return k + (double(k) < x ? 1ull : 0ull);
+  }
+};
+template <> struct UniBits<float> {
+  using T = uint32_t;
+  static __device__ __forceinline__ T of(const U4& w, int h) { return (h ? w.z : w.x) >> 8; }
+  static __device__ __forceinline__ T below(float q) {
+    const float x = q * 0x1p24f;
+    if (!(x > 0.0f)) return 0u;
+    if (x >= 0x1p24f) return 1u << 24;
+    const T k = (T)x;
+    return k + (float(k) < x ? 1u : 0u);
+  }
+};
+
+// floor(u * 1600) of the pixel draw.  FP64: u = k 2^-53, so the exact product is m 2^-47 with m = 25 k; the FP64
+// product rounds it to 53 bits, which reaches the next integer exactly when the fraction lies within half a unit of
+// it (at the half the even neighbour is that integer).  Integer instructions, the FP64 product's result.
+__device__ __forceinline__ int map_bin(double, unsigned long long k) {
+  const unsigned long long m = k * 25ull;
+  int b = int(m >> 47);
+  const int s = 11 - __clzll((long long)m);      // bits the product is rounded by
+  if (s > 0 && (m & ((1ull << 47) - 1ull)) >= (1ull << 47) - (1ull << (s - 1))) ++b;
+  return b;
+}
+__device__ __forceinline__ int map_bin(float, uint32_t k) {
+  return int(floorf(float(k) * 0x1p-24f * float(NPX)));
+}
+
 // Photon-map bin by the CDF (GetRandom2), then the pixel id of the point: "truncate" keeps the bin, "lrint" rounds
 // the point, i.e. moves to the next pixel in x and in y each with probability 1/2 (crv/crvfastsim/response/sipm.py:
 // 80-91).  The two halves are bits 0 and 1 of the draw word whose low bits the bin uniform does not use.
+static __device__ __noinline__ int map_search(const double* cum, double u) {
+  const double v = u * cum[NPX - 1];
+  int lo = 0, hi = NPX;
+#pragma unroll 1
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (cum[mid] <= v) lo = mid + 1; else hi = mid;
+  }
+  return lo;
+}
 template <typename R>
-__device__ __forceinline__ int draw_pixel(const CrvParams& p, const CrvPixels& px, const uint32_t* dead, R u,
-                                          uint32_t half) {
+__device__ __forceinline__ int draw_pixel(const CrvParams& p, const CrvPixels& px, const uint32_t* dead, const U4& w) {
   int b;
   if (p.uniform_map) {
-    b = int(floor(u * R(NPX)));
+    b = map_bin(R(0), UniBits<R>::of(w, 0));
   } else {
-    double v = double(u) * px.cum[NPX - 1];
-    int lo = 0, hi = NPX;
-    while (lo < hi) {
-      int mid = (lo + hi) >> 1;
-      if (px.cum[mid] <= v) lo = mid + 1; else hi = mid;
-    }
-    b = lo;
+    b = map_search(px.cum, double(Math<R>::uni(w, 0)));
   }
   if (b > NPX - 1) b = NPX - 1;
   if (b < 0) b = 0;
-  int x = b / 40, y = b - 40 * (b / 40);
-  if (p.pixel_lrint) { x += int(half & 1u); y += int((half >> 1) & 1u); }
-  const int q = x * PXS + y;
+  int q = b + b / 40;                            // x * 41 + y of x = b / 40, y = b % 40
+  if (p.pixel_lrint) q += PXS * int(w.y & 1u) + int((w.y >> 1) & 1u);
   return ((dead[q >> 5] >> (q & 31)) & 1u) ? -1 : q;
 }
 
@@ -439,30 +472,13 @@ __device__ __forceinline__ int draw_pixel(const CrvParams& p, const CrvPixels& p
 // conversion from the FP64 parameters inside the per-photon code would issue on the narrow FP64 pipe every time)
 template <typename R>
 struct SipmK {
-  R vov, tau, p1, p2, q_ct, q_t0, q_t1, life0, life1, t_end;
+  R vov, tau, p1, p2, life0, life1, t_end;
+  typename UniBits<R>::T t_ct, t_t0, t_t1;       // cross-talk and trap draws
+  typename UniBits<R>::T t_fire;                 // a pixel at full overvoltage fires
+  typename UniBits<R>::T t_cand;                 // a photon at or above it fires on no pixel, whatever its state
   float t_end_dn;                // largest float <= t_end: float times compare with it exactly as with t_end
   int ct_on, t0_on, t1_on, npx, npy;
 };
-
-template <typename R>
-__device__ __forceinline__ SipmK<R> sipm_consts(const CrvParams& p) {
-  SipmK<R> K;
-  K.vov = R(p.overvoltage); K.tau = R(p.time_constant); K.p1 = R(p.p1); K.p2 = R(p.p2);
-  K.q_ct = R(p.q_ct); K.q_t0 = R(p.q_t0); K.q_t1 = R(p.q_t1);
-  K.life0 = R(p.trap0_lifetime); K.life1 = R(p.trap1_lifetime); K.t_end = R(p.t_end);
-  K.t_end_dn = __double2float_rd(p.t_end);
-  K.ct_on = p.q_ct > 0.0; K.t0_on = p.q_t0 > 0.0; K.t1_on = p.q_t1 > 0.0;
-  K.npx = p.n_pixels_x; K.npy = p.n_pixels_y;
-  return K;
-}
-
-// recovered overvoltage of pixel q at time t (Vov if it never fired)
-template <typename R>
-__device__ __forceinline__ R recovered(const SipmK<R>& K, const SipmShared<R>& S, int q, R t) {
-  using M = Math<R>;
-  if (!bm_test(S.bm, q)) return K.vov;
-  return K.vov * (R(1) - M::exp(-(t - S.last[q]) / K.tau));
-}
 
 template <typename R>
 __device__ __forceinline__ R pfire(const SipmK<R>& K, R v) {
@@ -475,8 +491,41 @@ template <typename R>
 __device__ __forceinline__ R pfire_m(const SipmK<R>& K, R v, int m) {
   R q = R(1) - pfire<R>(K, v);
   R qm = q;
+#pragma unroll 1
   for (int i = 1; i < m; ++i) qm = qm * q;
   return R(1) - qm;
+}
+
+template <typename R>
+__device__ __forceinline__ SipmK<R> sipm_consts(const CrvParams& p) {
+  SipmK<R> K;
+  K.vov = R(p.overvoltage); K.tau = R(p.time_constant); K.p1 = R(p.p1); K.p2 = R(p.p2);
+  K.life0 = R(p.trap0_lifetime); K.life1 = R(p.trap1_lifetime); K.t_end = R(p.t_end);
+  K.t_end_dn = __double2float_rd(p.t_end);
+  K.ct_on = p.q_ct > 0.0; K.t0_on = p.q_t0 > 0.0; K.t1_on = p.q_t1 > 0.0;
+  K.t_ct = UniBits<R>::below(R(p.q_ct)); K.t_t0 = UniBits<R>::below(R(p.q_t0)); K.t_t1 = UniBits<R>::below(R(p.q_t1));
+  K.npx = p.n_pixels_x; K.npy = p.n_pixels_y;
+  const R pm = pfire_m<R>(K, K.vov, 1);
+  K.t_fire = UniBits<R>::below(pm);
+  // A recovering pixel has 0 <= v <= overvoltage (photons come in time order), and pfire grows with v, so no state
+  // fires a photon that a full pixel would not; 1e-6 covers the rounding of the exponentials many times over.  With
+  // constants of other signs every photon on a live pixel is kept.
+  const bool grows = K.vov >= R(0) && K.tau > R(0) && K.p1 >= R(0) && K.p2 > R(0);
+  K.t_cand = grows ? UniBits<R>::below(pm + R(1e-6)) : UniBits<R>::below(R(2));
+  return K;
+}
+
+// recovered overvoltage at time t of a pixel that fired last at t0
+template <typename R>
+__device__ __forceinline__ R recovered_from(const SipmK<R>& K, R t, R t0) {
+  using M = Math<R>;
+  return K.vov * (R(1) - M::exp(-(t - t0) / K.tau));
+}
+// recovered overvoltage of pixel q at time t (Vov if it never fired)
+template <typename R, int CAP, bool LOC>
+__device__ __forceinline__ R recovered(const SipmK<R>& K, const SipmShared<R, CAP, LOC>& S, int q, R t) {
+  if (!bm_test(S.bm(), q)) return K.vov;
+  return recovered_from<R>(K, t, S.last()[q]);
 }
 
 // Per SiPM context while simulating.
@@ -490,52 +539,90 @@ struct SipmCtx {
   int limit;               // a key/capacity limit was hit
 };
 
-// Schedule the afterpulses of a fired node (trap0: call 1 (u, u_time), call 4 word 0-1 (u_fire);
-// trap1: call 4 word 2-3 (u), call 5 (u_time, u_fire)).  Returns how many were scheduled into (t, uf).
-template <typename R>
-__device__ __forceinline__ int node_traps(const CrvParams& p, const SipmK<R>& K, const SipmCtx& C, uint32_t gen,
-                                          uint32_t idx, uint32_t key, R t, R* tt, R* uf) {
-  using M = Math<R>;
-  if (!K.t0_on && !K.t1_on) return 0;
-  U4 a = keyed(p.seed, C.ek, w2_of(ST_SIPM, gen, idx, 1, C.chan), key);
-  const bool trap0 = K.t0_on && M::uni(a, 0) < K.q_t0;
-  if (!trap0 && !K.t1_on) return 0;              // call 4 is only read by a trap-0 afterpulse or the trap-1 draw
-  U4 b = keyed(p.seed, C.ek, w2_of(ST_SIPM, gen, idx, 4, C.chan), key);
-  int n = 0;
-  if (trap0) {
-    tt[n] = t - K.life0 * M::log(M::uni_open(a, 1));
-    uf[n] = M::uni(b, 0);
-    ++n;
-  }
-  if (K.t1_on && M::uni(b, 1) < K.q_t1) {
-    U4 c = keyed(p.seed, C.ek, w2_of(ST_SIPM, gen, idx, 5, C.chan), key);
-    tt[n] = t - K.life1 * M::log(M::uni_open(c, 0));
-    uf[n] = M::uni(c, 1);
-    ++n;
-  }
-  return n;
+// A draw as a call: the kernel's warps are all at different places of a large loop body, so its speed hangs on how much
+// of that body the instruction cache holds (with everything inlined 98 KB of code, half of the fetches missed).
+static __device__ __noinline__ U4 keyed_call(uint32_t seed, EvKey ek, uint32_t w2, uint32_t w3) {
+  return keyed(seed, ek, w2, w3);
 }
 
-// cross-talk candidates of a fired node: bit q set for neighbour q (x-1, x+1, y-1, y+1) when it is drawn
+// The photon step's draws: called in the first pass; inlined in the others, whose few warps per SM wait for their own
+// instructions' results more than for the cache.
+template <int CAP>
+__device__ __forceinline__ U4 draw(uint32_t seed, const EvKey& ek, uint32_t w2, uint32_t w3) {
+  if constexpr (CAP <= 256) return keyed_call(seed, ek, w2, w3);
+  else return keyed(seed, ek, w2, w3);
+}
+
+// Schedule the afterpulses of a fired node (trap0: call 1 (u, u_time), call 4 word 0-1 (u_fire);
+// trap1: call 4 word 2-3 (u), call 5 (u_time, u_fire)) from its call-1 draw a.  Returns how many were scheduled into
+// (t, uf).
 template <typename R>
-__device__ __forceinline__ unsigned node_crosstalk(const CrvParams& p, const SipmK<R>& K, const SipmCtx& C,
-                                                   uint32_t gen, uint32_t idx, uint32_t key, int pix) {
+struct Traps {
+  R t[2], uf[2];
+  int n;
+};
+template <typename R>
+__device__ __noinline__ Traps<R> schedule_traps(uint32_t seed, const SipmK<R>& K, EvKey ek, uint32_t w2, uint32_t key,
+                                                R t, U4 a, bool trap0) {
   using M = Math<R>;
-  if (!K.ct_on) return 0;
-  U4 a = keyed(p.seed, C.ek, w2_of(ST_SIPM, gen, idx, 2, C.chan), key);
-  U4 b = keyed(p.seed, C.ek, w2_of(ST_SIPM, gen, idx, 3, C.chan), key);
-  int x = pix / PXS, y = pix - PXS * (pix / PXS);
-  const R q = K.q_ct;
+  Traps<R> o;
+  o.t[0] = o.t[1] = o.uf[0] = o.uf[1] = R(0);
+  o.n = 0;
+  const U4 b = keyed_call(seed, ek, w2 | (4u << 15), key);
+  if (trap0) {
+    o.t[0] = t - K.life0 * M::log(M::uni_open(a, 1));
+    o.uf[0] = M::uni(b, 0);
+    o.n = 1;
+  }
+  if (K.t1_on && UniBits<R>::of(b, 1) < K.t_t1) {
+    const U4 c = keyed_call(seed, ek, w2 | (5u << 15), key);
+    const R t1 = t - K.life1 * M::log(M::uni_open(c, 0)), u1 = M::uni(c, 1);
+    if (o.n) { o.t[1] = t1; o.uf[1] = u1; }
+    else { o.t[0] = t1; o.uf[0] = u1; }
+    ++o.n;
+  }
+  return o;
+}
+template <typename R>
+__device__ __forceinline__ int node_traps(uint32_t seed, const SipmK<R>& K, const SipmCtx& C, uint32_t gen,
+                                          uint32_t idx, uint32_t key, R t, const U4& a, R* tt, R* uf) {
+  const bool trap0 = K.t0_on && UniBits<R>::of(a, 0) < K.t_t0;
+  if (!trap0 && !K.t1_on) return 0;              // call 4 is only read by a trap-0 afterpulse or the trap-1 draw
+  const Traps<R> o = schedule_traps<R>(seed, K, C.ek, w2_of(ST_SIPM, gen, idx, 0, C.chan), key, t, a, trap0);
+  tt[0] = o.t[0]; tt[1] = o.t[1];
+  uf[0] = o.uf[0]; uf[1] = o.uf[1];
+  return o.n;
+}
+
+// Neighbours of a pixel in increasing pixel order: bit 0 x - 1, bit 1 y - 1, bit 2 y + 1, bit 3 x + 1.
+__device__ __forceinline__ int neighbour(int pix, int q) {
+  return pix + (q == 0 ? -PXS : (q == 1 ? -1 : (q == 2 ? 1 : PXS)));
+}
+
+// cross-talk candidates of a fired node among the neighbours inside the grid, from its draws: xa / xb bit 0 and bit 1
+// set for call 2's (x - 1, x + 1) and call 3's (y - 1, y + 1) uniforms below the cross-talk probability
+template <typename R>
+__device__ __forceinline__ unsigned crosstalk_mask(const SipmK<R>& K, unsigned xa, unsigned xb, int pix) {
+  const int x = pix / PXS, y = pix - PXS * x;
   unsigned m = 0;
-  if (x > 0 && M::uni(a, 0) < q) m |= 1u;
-  if (x + 1 < K.npx && M::uni(a, 1) < q) m |= 2u;
-  if (y > 0 && M::uni(b, 0) < q) m |= 4u;
-  if (y + 1 < K.npy && M::uni(b, 1) < q) m |= 8u;
+  if (x > 0) m |= xa & 1u;
+  if (y > 0) m |= (xb & 1u) << 1;
+  if (y + 1 < K.npy) m |= (xb & 2u) << 1;
+  if (x + 1 < K.npx) m |= (xa & 2u) << 2;
   return m;
 }
 
-__device__ __forceinline__ int neighbour(int pix, int q) {
-  return q == 0 ? pix - PXS : (q == 1 ? pix + PXS : (q == 2 ? pix - 1 : pix + 1));
+template <typename R>
+__device__ __forceinline__ unsigned node_crosstalk(uint32_t seed, const SipmK<R>& K, const SipmCtx& C,
+                                                   uint32_t gen, uint32_t idx, uint32_t key, int pix) {
+  using B = UniBits<R>;
+  if (!K.ct_on) return 0;
+  U4 a = keyed_call(seed, C.ek, w2_of(ST_SIPM, gen, idx, 2, C.chan), key);
+  U4 b = keyed_call(seed, C.ek, w2_of(ST_SIPM, gen, idx, 3, C.chan), key);
+  const unsigned xa = unsigned(B::of(a, 0) < K.t_ct) | (unsigned(B::of(a, 1) < K.t_ct) << 1);
+  const unsigned xb = unsigned(B::of(b, 0) < K.t_ct) | (unsigned(B::of(b, 1) < K.t_ct) << 1);
+  if ((xa | xb) == 0u) return 0;
+  return crosstalk_mask<R>(K, xa, xb, pix);
 }
 
 // Append a charge record (lane-ordered position pos relative to C.nq) if it fits.
@@ -554,67 +641,88 @@ __device__ __forceinline__ void put_charge(const SipmOut& O, const SipmCtx& C, i
   }
 }
 
+// Queue a lane's n (0..2) scheduled afterpulses at position pos of the queue.
+template <typename R, int CAP, bool LOC>
+__device__ __forceinline__ void put_traps(const SipmShared<R, CAP, LOC>& S, int pos, int n, const R* tt, const R* uf, int pix,
+                                          long long id) {
+#pragma unroll
+  for (int a = 0; a < 2; ++a) {
+    if (a >= n) break;
+    const int k = pos + a;
+    if (k < S.TCAP) { S.tr_t()[k] = tt[a]; S.tr_uf()[k] = uf[a]; S.tr_pix()[k] = uint16_t(pix); S.tr_id()[k] = id; }
+  }
+}
+
 // Build the next frontier from the candidate list (lane 0): sort, unique with multiplicity, drop dead.
-template <typename R>
-__device__ __forceinline__ int make_frontier(const SipmShared<R>& S, int nc, const uint32_t* dead, int* limit) {
+template <typename R, int CAP, bool LOC>
+__device__ __forceinline__ int make_frontier(const SipmShared<R, CAP, LOC>& S, int nc, const uint32_t* dead, int* limit) {
   int nf = 0;
   if (lane_id() == 0) {
+#pragma unroll 1
     for (int a = 1; a < nc; ++a) {           // insertion sort (tiny lists)
-      uint16_t x = S.cand[a];
+      uint16_t x = S.cand()[a];
       int b = a - 1;
-      while (b >= 0 && S.cand[b] > x) { S.cand[b + 1] = S.cand[b]; --b; }
-      S.cand[b + 1] = x;
+#pragma unroll 1
+      while (b >= 0 && S.cand()[b] > x) { S.cand()[b + 1] = S.cand()[b]; --b; }
+      S.cand()[b + 1] = x;
     }
+#pragma unroll 1
     for (int a = 0; a < nc;) {
       int b = a;
-      while (b < nc && S.cand[b] == S.cand[a]) ++b;
-      int q = S.cand[a];
+#pragma unroll 1
+      while (b < nc && S.cand()[b] == S.cand()[a]) ++b;
+      int q = S.cand()[a];
       if (!((dead[q >> 5] >> (q & 31)) & 1u)) {
         if (nf > MAX_IDX) { *limit = 1; break; }
-        S.fr_pix[nf] = uint16_t(q);
-        S.fr_m[nf] = uint16_t(b - a);
+        S.fr_pix()[nf] = uint16_t(q);
+        S.fr_m()[nf] = uint16_t(b - a);
         ++nf;
       }
       a = b;
     }
-    S.misc[1] = nf;
+    S.misc()[3] = nf;
   }
   __syncwarp();
-  nf = S.misc[1];
+  nf = S.misc()[3];
   __syncwarp();
   return nf;
 }
 
-// Cross-talk cascade of one fired primary (generation 1 onwards), frontier spread over the lanes.
-template <typename R>
-__device__ void run_cascade(const CrvParams& p, const SipmK<R>& K, const SipmShared<R>& S, const uint32_t* dead,
-                            SipmCtx& C, const SipmOut& O, unsigned cand0, int pix0, R t, uint32_t key, long long id) {
-  // generation-1 candidates from the primary
-  int nc = 0;
-  if (lane_id() == 0) {
-    for (int q = 0; q < 4; ++q)
-      if (cand0 & (1u << q)) S.cand[nc++] = uint16_t(neighbour(pix0, q));
-  }
-  nc = __shfl_sync(FULL, nc, 0);
+// Cross-talk cascade of one photon from generation 2 on; the frontier is spread over the lanes.  ct: the lane's drawn
+// neighbours of its pixel pix (0: none, or a node of another photon).  Generation 1 is part of the photon step (simulate_sipm), so this runs for the few photons whose
+// cascade goes further; called, not inlined, to keep the photon step's code and registers small.  C.nq, C.ntr and
+// C.limit come back in S.misc()[0..2].
+template <typename R, int CAP, bool LOC>
+__device__ __noinline__ void run_cascade(uint32_t seed, const SipmK<R>& K, SipmShared<R, CAP, LOC> S,
+                                         const uint32_t* dead, SipmCtx C, const SipmOut& O, unsigned ct, int pix, int src,
+                                         R t, uint32_t key, long long id) {
+  t = __shfl_sync(FULL, t, src);
+  key = __shfl_sync(FULL, key, src);
+  id = __shfl_sync(FULL, id, src);
+  int nc, at = warp_excl(__popc(ct), &nc);
+#pragma unroll 1
+  for (unsigned m = ct; m; m &= m - 1u) S.cand()[at++] = uint16_t(neighbour(pix, __ffs(m) - 1));
   __syncwarp();
+  uint32_t gen = 2;
   int lim = 0;
-  int nf = make_frontier<R>(S, nc, dead, &lim);
-  lim = __shfl_sync(FULL, lim, 0);
-  if (lim) nf = 0;
-  uint32_t gen = 1;
-  while (nf > 0) {
+#pragma unroll 1
+  while (true) {
+    const int nf = make_frontier(S, nc, dead, &lim);
+    lim = __shfl_sync(FULL, lim, 0);
+    if (lim || nf == 0) break;
     if (gen > MAX_GEN) { lim = 1; break; }
     int ncand = 0;
+#pragma unroll 1
     for (int base = 0; base < nf; base += 32) {
       int i = base + lane_id();
       bool act = i < nf;
-      int q = act ? S.fr_pix[i] : 0;
+      int q = act ? S.fr_pix()[i] : 0;
       R v = R(0);
       bool fire = false;
       if (act) {
-        v = recovered<R>(K, S, q, t);
-        R pm = pfire_m<R>(K, v, S.fr_m[i]);
-        U4 w = keyed(p.seed, C.ek, w2_of(ST_SIPM, gen, uint32_t(i), 0, C.chan), key);
+        v = recovered(K, S, q, t);
+        R pm = pfire_m<R>(K, v, S.fr_m()[i]);
+        U4 w = keyed_call(seed, C.ek, w2_of(ST_SIPM, gen, uint32_t(i), 0, C.chan), key);
         fire = Math<R>::uni(w, 1) < pm;
       }
       unsigned fm = __ballot_sync(FULL, fire);
@@ -624,141 +732,257 @@ __device__ void run_cascade(const CrvParams& p, const SipmK<R>& K, const SipmSha
       unsigned ct = 0;
       if (fire) {
         put_charge<R>(O, C, pos, t, v, id);
-        S.last[q] = t;
-        bm_set(S.bm, q);
-        ntr = node_traps<R>(p, K, C, gen, uint32_t(i), key, t, tt, uf);
-        ct = node_crosstalk<R>(p, K, C, gen, uint32_t(i), key, q);
+        S.last()[q] = t;
+        bm_set(S.bm(), q);
+        if (K.t0_on || K.t1_on) {
+          const U4 a = keyed_call(seed, C.ek, w2_of(ST_SIPM, gen, uint32_t(i), 1, C.chan), key);
+          ntr = node_traps<R>(seed, K, C, gen, uint32_t(i), key, t, a, tt, uf);
+        }
+        ct = node_crosstalk<R>(seed, K, C, gen, uint32_t(i), key, q);
       }
       C.nq += __popc(fm);
       // traps in node order
       int tot;
       int tpos = warp_excl(ntr, &tot);
-      for (int a = 0; a < ntr; ++a) {
-        int k = C.ntr + tpos + a;
-        if (k < S.tcap) { S.tr_t[k] = tt[a]; S.tr_uf[k] = uf[a]; S.tr_pix[k] = uint16_t(q); S.tr_id[k] = id; }
-      }
+      put_traps(S, C.ntr + tpos, ntr, tt, uf, q, id);
       C.ntr += tot;
       // candidates
       int nct = __popc(ct);
       int cpos = warp_excl(nct, &tot);
       int a = 0;
-      for (int qq = 0; qq < 4; ++qq)
-        if (ct & (1u << qq)) {
-          int k = ncand + cpos + a++;
-          if (k < 256) S.cand[k] = uint16_t(neighbour(q, qq));
-        }
+#pragma unroll 1
+      for (unsigned m = ct; m; m &= m - 1u) {
+        int k = ncand + cpos + a++;
+        if (k < 256) S.cand()[k] = uint16_t(neighbour(q, __ffs(m) - 1));
+      }
       ncand += tot;
       __syncwarp();
     }
     if (ncand > 256) { lim = 1; break; }
     ++gen;
-    nf = make_frontier<R>(S, ncand, dead, &lim);
-    lim = __shfl_sync(FULL, lim, 0);
-    if (lim) break;
+    nc = ncand;
   }
-  if (__any_sync(FULL, lim)) C.limit = 1;
+  lim = __any_sync(FULL, lim) || C.limit;
+  if (lane_id() == 0) { S.misc()[0] = C.nq; S.misc()[1] = C.ntr; S.misc()[2] = lim; }
+  __syncwarp();
 }
 
-// Serial-semantics simulation of one SiPM whose sorted photons (n <= cap) sit in S.ph_*.
+// A touch at time t of a pixel that fired last at t0, with fire draw fb: recovered overvoltage and whether it fires.
+// Called: few touches meet a pixel that has fired.
 template <typename R>
-__device__ void simulate_sipm(const CrvParams& p, const SipmK<R>& K, const CrvPixels& px, const SipmShared<R>& S,
-                              const uint32_t* dead, SipmCtx& C, const SipmOut& O, int n, const long long* photon_id,
-                              long long gstart, long long id_base) {
-  using M = Math<R>;
-  for (int w = lane_id(); w < 64; w += 32) S.bm[w] = 0u;
-  __syncwarp();
+struct Touch {
+  R v;
+  bool fire;
+};
+template <typename R>
+__device__ __noinline__ Touch<R> touch_again(const SipmK<R>& K, R t, R t0, typename UniBits<R>::T fb) {
+  Touch<R> o;
+  o.v = recovered_from<R>(K, t, t0);
+  o.fire = fb < UniBits<R>::below(pfire_m<R>(K, o.v, 1));
+  return o;
+}
+
+// Serial-semantics simulation of one SiPM whose n staged photons (those that can fire, in time order) sit in S.ph_*.
+//
+// The serial order of events is: photon, its first-generation cross-talk nodes in pixel order, the rest of its cascade,
+// next photon.  A step takes the next photons and their first-generation nodes (about one photon in eight has any), as
+// many as fit a warp, one touch per lane in that order.  All draws are keyed, so the step has them before anything is
+// decided.  A touch whose pixel no earlier touch of the step names is decided at once, against the state the step
+// starts from; the others (one step in four has one) are decided one at a time in order, each against the last touch
+// before it that fired.  A node fires only if its photon did.  The step then commits everything, or, when a fired node
+// starts a second generation, everything up to that photon, whose cascade continues in run_cascade.
+template <typename R, int CAP, bool LOC>
+__device__ __forceinline__ void simulate_sipm(const CrvParams& p, const SipmK<R>& K,
+                                              const SipmShared<R, CAP, LOC>& S, const uint32_t* dead, SipmCtx& C,
+                                              const SipmOut& O, int n, const long long* photon_id, long long gstart,
+                                              long long id_base) {
+  using B = UniBits<R>;
+  const int lane = lane_id();
+  const unsigned lt = lanemask_lt();
   int k = 0;
+#pragma unroll 1
   while (k < n) {
-    int i = k + lane_id();
-    bool has = i < n;
-    R t = has ? S.ph_t[i] : R(0);
-    uint32_t key = has ? S.ph_key[i] : 0u;
-    int pix = -1;
-    U4 w0{0, 0, 0, 0};
-    if (has) {
-      w0 = keyed(p.seed, C.ek, w2_of(ST_SIPM, 0, 0, 0, C.chan), key);
-      pix = draw_pixel<R>(p, px, dead, M::uni(w0, 0), w0.y);
+    // photons, one per lane: their cross-talk draws (calls 2 and 3) give the first-generation nodes, the drawn
+    // neighbours on live pixels in pixel order
+    bool has = k + lane < n;
+    const uint32_t pkey = has ? S.ph_key()[k + lane] : 0u;
+    const uint32_t ppix = has ? uint32_t(S.ph_pix()[k + lane]) : 0u;
+    unsigned live = 0;
+    if (K.ct_on) {
+      unsigned xy = 0;
+#pragma unroll 1
+      for (uint32_t call = 2; call < 4; ++call) {
+        const U4 w = draw<CAP>(p.seed, C.ek, w2_of(ST_SIPM, 0, 0, call, C.chan), pkey);
+        xy = (xy >> 2) | (unsigned(B::of(w, 0) < K.t_ct) << 2) | (unsigned(B::of(w, 1) < K.t_ct) << 3);
+      }
+      if (has && xy) {
+        const int pix = int(ppix & PH_PIX);
+#pragma unroll 1
+        for (unsigned m = crosstalk_mask<R>(K, xy & 3u, xy >> 2, pix); m; m &= m - 1u) {
+          const int q = __ffs(m) - 1, np = neighbour(pix, q);
+          if (!((dead[np >> 5] >> (np & 31)) & 1u)) live |= 1u << q;
+        }
+      }
     }
-    bool live = pix >= 0;
-    unsigned same = __match_any_sync(FULL, live ? pix : -1 - lane_id());
-    bool collide = live && (same & lanemask_lt()) != 0u;
-    bool fire = false;
-    unsigned ct = 0;
-    R v = R(0);
-    if (live && !collide) {
-      v = recovered<R>(K, S, pix, t);
-      R pm = pfire_m<R>(K, v, 1);
-      fire = M::uni(w0, 1) < pm;
-      if (fire) ct = node_crosstalk<R>(p, K, C, 0, 0, key, pix);
+    // the step's touches in serial order: pixel, node flag, index in the generation, photon's lane above, photon's touch
+    int take = min(n - k, 32), total = take;
+    {
+      const int c = has ? 1 + __popc(live) : 0;
+      const unsigned b0 = __ballot_sync(FULL, c & 1), b1 = __ballot_sync(FULL, c & 2), b2 = __ballot_sync(FULL, c & 4);
+      const int base = __popc(b0 & lt) + 2 * __popc(b1 & lt) + 4 * __popc(b2 & lt);
+      has = has && base + c <= 32;
+      take = __popc(__ballot_sync(FULL, has));
+      total = __shfl_sync(FULL, base + c, take - 1);
+      __syncwarp();
+      if (has) {
+        const uint32_t who = (uint32_t(lane) << 19) | (uint32_t(base) << 24);
+        S.nodes()[base] = ppix | who;
+        uint32_t at = uint32_t(base), idx = 0;
+#pragma unroll 1
+        for (unsigned m = live; m; m &= m - 1u, ++idx)
+          S.nodes()[++at] = uint32_t(neighbour(int(ppix & PH_PIX), __ffs(m) - 1)) | (1u << 16) | (idx << 17) | who;
+      }
+      __syncwarp();
     }
-    int nv = min(n - k, 32);
-    unsigned cm = __ballot_sync(FULL, collide);
-    unsigned sm = __ballot_sync(FULL, ct != 0u);
-    int f = cm ? __ffs(cm) - 1 : 32;
-    int g = sm ? __ffs(sm) - 1 : 32;
-    int ncommit = (g < f) ? g + 1 : min(f, nv);
-    bool commit = lane_id() < ncommit && fire;
+    const bool act = lane < total;
+    const uint32_t w = act ? S.nodes()[lane] : 0u;
+    const int pix = int(w & PH_PIX), pl = int((w >> 19) & 31u), par = int(w >> 24);
+    const uint32_t node = (w >> 16) & 1u, idx = (w >> 17) & 3u;
+    const uint32_t key = __shfl_sync(FULL, pkey, pl);
+    const R t = act ? S.ph_t()[k + pl] : R(0);
+    const unsigned same = __match_any_sync(FULL, act ? pix : -1 - lane);
+    const bool set = act && bm_test(S.bm(), pix);
+    bool dirty = act && (same & lt) != 0u;
+    // decisions
+    R v = K.vov;
+    bool fire = (w & PH_FIRES) != 0u;
+    if (__any_sync(FULL, node || set || dirty)) {
+      const U4 w0 = draw<CAP>(p.seed, C.ek, w2_of(ST_SIPM, node, idx, 0, C.chan), key);
+      const typename B::T fb = B::of(w0, 1);
+      if (node) fire = fb < K.t_fire;
+      if (set) {
+        const Touch<R> o = touch_again<R>(K, t, S.last()[pix], fb);
+        v = o.v;
+        fire = o.fire;
+      }
+      unsigned dm = __ballot_sync(FULL, dirty);
+      dirty = dirty || (node && ((dm >> par) & 1u));
+      dm = __ballot_sync(FULL, dirty);
+      const bool pfire0 = __shfl_sync(FULL, int(fire && !dirty), par) != 0;
+      fire = fire && !dirty && (!node || pfire0);
+#pragma unroll 1
+      while (dm) {                                 // in serial order
+        const int d = __ffs(dm) - 1;
+        const int x = __shfl_sync(FULL, pix, d);
+        const unsigned m = __ballot_sync(FULL, fire && pix == x) & ((1u << d) - 1u);
+        const R tl = __shfl_sync(FULL, t, m ? 31 - __clz(m) : 0);
+        const bool pf = __shfl_sync(FULL, int(fire), par) != 0;
+        if (lane == d) {
+          v = K.vov;
+          fire = fb < K.t_fire;
+          if (m || set) {
+            const Touch<R> o = touch_again<R>(K, t, m ? tl : S.last()[pix], fb);
+            v = o.v;
+            fire = o.fire;
+          }
+          fire = fire && (!node || pf);
+        }
+        dm &= dm - 1u;
+      }
+    }
+    // the fired nodes' cross-talk draws, calls 2 and 3 of sixteen nodes per Philox evaluation; the step ends with the
+    // first photon that has a node with cross-talk of its own
+    unsigned nct = 0;
+    int cut = 32;
+    const unsigned nfm = __ballot_sync(FULL, fire && node);
+    if (nfm && K.ct_on) {
+      const bool mine = fire && node;
+      const int rank = __popc(nfm & lt), cnt = __popc(nfm);
+      if (mine) S.fr_pix()[rank] = uint16_t(lane);
+      __syncwarp();
+#pragma unroll 1
+      for (int g = 0; g < cnt; g += 16) {
+        const int j = g + (lane & 15);
+        const int src = j < cnt ? S.fr_pix()[j] : 0;
+        const uint32_t kk = __shfl_sync(FULL, key, src), ii = __shfl_sync(FULL, idx, src);
+        const U4 a = draw<CAP>(p.seed, C.ek, w2_of(ST_SIPM, 1, ii, 2u + uint32_t(lane >> 4), C.chan), kk);
+        const unsigned x = unsigned(B::of(a, 0) < K.t_ct) | (unsigned(B::of(a, 1) < K.t_ct) << 1);
+        const unsigned xa = __shfl_sync(FULL, x, rank & 15), xb = __shfl_sync(FULL, x, 16 + (rank & 15));
+        if (mine && (rank >> 4) == (g >> 4) && (xa | xb)) nct = crosstalk_mask<R>(K, xa, xb, pix);
+      }
+      const unsigned m2 = __ballot_sync(FULL, nct != 0u);
+      if (m2) {
+        cut = __shfl_sync(FULL, par, __ffs(m2) - 1);
+        fire = fire && par <= cut;
+      }
+    }
+    // commit: charges in serial order, pixel state (the last touch of a pixel stays), afterpulses
+    const unsigned fm = __ballot_sync(FULL, fire);
     long long id = 0;
-    if (commit) id = photon_id ? photon_id[gstart + S.ph_loc[i]] : id_base + (long long)(key >> 16);
-    unsigned fm = __ballot_sync(FULL, commit);
-    R tt[2], uf[2];
+    if (act) id = LOC ? photon_id[gstart + S.ph_loc()[k + pl]] : id_base + (long long)(key >> 16);
     int ntr = 0;
-    if (commit) {
-      put_charge<R>(O, C, __popc(fm & lanemask_lt()), t, v, id);
-      S.last[pix] = t;
-      bm_set(S.bm, pix);
-      ntr = node_traps<R>(p, K, C, 0, 0, key, t, tt, uf);
+    R tt[2], uf[2];
+    if (fire) {
+      put_charge<R>(O, C, __popc(fm & lt), t, v, id);
+      bm_set(S.bm(), pix);
+      if ((same & fm & ~lt) == (1u << lane)) S.last()[pix] = t;
+      if (K.t0_on || K.t1_on) {
+        const U4 a = draw<CAP>(p.seed, C.ek, w2_of(ST_SIPM, node, idx, 1, C.chan), key);
+        ntr = node_traps<R>(p.seed, K, C, node, idx, key, t, a, tt, uf);
+      }
     }
     C.nq += __popc(fm);
-    int tot;
-    int tpos = warp_excl(ntr, &tot);
-    for (int a = 0; a < ntr; ++a) {
-      int kk = C.ntr + tpos + a;
-      if (kk < S.tcap) { S.tr_t[kk] = tt[a]; S.tr_uf[kk] = uf[a]; S.tr_pix[kk] = uint16_t(pix); S.tr_id[kk] = id; }
+    const unsigned a1 = __ballot_sync(FULL, ntr > 0);
+    if (a1) {
+      const unsigned a2 = __ballot_sync(FULL, ntr > 1);
+      put_traps(S, C.ntr + __popc(a1 & lt) + __popc(a2 & lt), ntr, tt, uf, pix, id);
+      C.ntr += __popc(a1) + __popc(a2);
     }
-    C.ntr += tot;
     __syncwarp();
-    if (g < f) {
-      unsigned c0 = __shfl_sync(FULL, ct, g);
-      int p0 = __shfl_sync(FULL, pix, g);
-      R tg = __shfl_sync(FULL, t, g);
-      uint32_t kg = __shfl_sync(FULL, key, g);
-      long long idg = __shfl_sync(FULL, id, g);
-      run_cascade<R>(p, K, S, dead, C, O, c0, p0, tg, kg, idg);
+    if (cut < 32) {
+      take = __shfl_sync(FULL, pl, cut) + 1;
+      run_cascade(p.seed, K, S, dead, C, O, par == cut ? nct : 0u, pix, cut, t, key, id);
+      C.nq = S.misc()[0];
+      C.ntr = S.misc()[1];
+      C.limit = S.misc()[2];
+      __syncwarp();
     }
-    k += ncommit;
+    k += take;
   }
-  if (C.ntr > S.tcap) C.limit = 1;
+  if (C.ntr > S.TCAP) C.limit = 1;
 }
 
 // Afterpulses after all photons, in (time, schedule order); stored after the main records.  Returns the count.
-template <typename R>
-__device__ int run_afterpulses(const SipmK<R>& K, const SipmShared<R>& S, SipmCtx& C, const SipmOut& O) {
-  int ntr = min(C.ntr, S.tcap);
+template <typename R, int CAP, bool LOC>
+__device__ __noinline__ int run_afterpulses(const SipmK<R>& K, SipmShared<R, CAP, LOC> S, SipmCtx C, const SipmOut& O) {
+  int ntr = min(C.ntr, S.TCAP);
   int nap = 0;
   if (lane_id() == 0 && ntr > 0) {
     // insertion sort by time (stable: equal times keep schedule order)
+#pragma unroll 1
     for (int a = 1; a < ntr; ++a) {
-      R x = S.tr_t[a], xu = S.tr_uf[a];
-      uint16_t xp = S.tr_pix[a];
-      long long xi = S.tr_id[a];
+      R x = S.tr_t()[a], xu = S.tr_uf()[a];
+      uint16_t xp = S.tr_pix()[a];
+      long long xi = S.tr_id()[a];
       int b = a - 1;
-      while (b >= 0 && S.tr_t[b] > x) {
-        S.tr_t[b + 1] = S.tr_t[b]; S.tr_uf[b + 1] = S.tr_uf[b]; S.tr_pix[b + 1] = S.tr_pix[b];
-        S.tr_id[b + 1] = S.tr_id[b];
+#pragma unroll 1
+      while (b >= 0 && S.tr_t()[b] > x) {
+        S.tr_t()[b + 1] = S.tr_t()[b]; S.tr_uf()[b + 1] = S.tr_uf()[b]; S.tr_pix()[b + 1] = S.tr_pix()[b];
+        S.tr_id()[b + 1] = S.tr_id()[b];
         --b;
       }
-      S.tr_t[b + 1] = x; S.tr_uf[b + 1] = xu; S.tr_pix[b + 1] = xp; S.tr_id[b + 1] = xi;
+      S.tr_t()[b + 1] = x; S.tr_uf()[b + 1] = xu; S.tr_pix()[b + 1] = xp; S.tr_id()[b + 1] = xi;
     }
+#pragma unroll 1
     for (int a = 0; a < ntr; ++a) {
-      R t1 = S.tr_t[a];
+      R t1 = S.tr_t()[a];
       if (t1 > K.t_end) continue;
-      int q = S.tr_pix[a];
-      R v = recovered<R>(K, S, q, t1);
-      if (S.tr_uf[a] < pfire<R>(K, v)) {
-        S.last[q] = t1;
-        S.bm[q >> 5] |= 1u << (q & 31);
-        long long id = S.tr_id[a];
+      int q = S.tr_pix()[a];
+      R v = recovered(K, S, q, t1);
+      if (S.tr_uf()[a] < pfire<R>(K, v)) {
+        S.last()[q] = t1;
+        S.bm()[q >> 5] |= 1u << (q & 31);
+        long long id = S.tr_id()[a];
         int kk = C.nq + nap;
         if (kk < C.cap) {
           long long o = C.slot + kk;
@@ -793,30 +1017,37 @@ __device__ __forceinline__ bool after(double ta, uint32_t ka, double tb, uint32_
 }
 
 // sort the staged photons by (time, key) (warp bitonic over the next power of two)
-template <typename R>
-__device__ void sort_photons(const SipmShared<R>& S, int n) {
+template <typename R, int CAP, bool LOC>
+__device__ __noinline__ void sort_photons(SipmShared<R, CAP, LOC> S, int n) {
   int P = 1;
   while (P < n) P <<= 1;
+#pragma unroll 1
   for (int i = n + lane_id(); i < P; i += 32) {
-    S.ph_t[i] = R(INFINITY);
-    S.ph_key[i] = 0xFFFFFFFFu;
-    if (S.ph_loc) S.ph_loc[i] = 0xFFFFFFFFu;
+    S.ph_t()[i] = R(INFINITY);
+    S.ph_key()[i] = 0xFFFFFFFFu;
+    S.ph_pix()[i] = 0;
+    if (LOC) S.ph_loc()[i] = 0xFFFFFFFFu;
   }
   __syncwarp();
+#pragma unroll 1
   for (int size = 2; size <= P; size <<= 1) {
+#pragma unroll 1
     for (int stride = size >> 1; stride > 0; stride >>= 1) {
+#pragma unroll 1
       for (int q = lane_id(); q < (P >> 1); q += 32) {
         const int lo = ((q & ~(stride - 1)) << 1) | (q & (stride - 1));   // stride is a power of two
         const int hi = lo + stride;
         const bool up = (lo & size) == 0;
-        const R ta = S.ph_t[lo], tb = S.ph_t[hi];
-        const uint32_t ka = S.ph_key[lo], kb = S.ph_key[hi];
+        const R ta = S.ph_t()[lo], tb = S.ph_t()[hi];
+        const uint32_t ka = S.ph_key()[lo], kb = S.ph_key()[hi];
         if (after(ta, ka, tb, kb) == up) {
-          S.ph_t[lo] = tb; S.ph_t[hi] = ta;
-          S.ph_key[lo] = kb; S.ph_key[hi] = ka;
-          if (S.ph_loc) {
-            uint32_t la = S.ph_loc[lo];
-            S.ph_loc[lo] = S.ph_loc[hi]; S.ph_loc[hi] = la;
+          S.ph_t()[lo] = tb; S.ph_t()[hi] = ta;
+          S.ph_key()[lo] = kb; S.ph_key()[hi] = ka;
+          const uint16_t xa = S.ph_pix()[lo];
+          S.ph_pix()[lo] = S.ph_pix()[hi]; S.ph_pix()[hi] = xa;
+          if (LOC) {
+            uint32_t la = S.ph_loc()[lo];
+            S.ph_loc()[lo] = S.ph_loc()[hi]; S.ph_loc()[hi] = la;
           }
         }
       }
@@ -825,19 +1056,27 @@ __device__ void sort_photons(const SipmShared<R>& S, int n) {
   }
 }
 
+// Warps per block.  20 warps of the first pass (11 KB of shared memory each, FP32) fit an SM, as two blocks of 102
+// registers a thread; the later passes have room for 11 warps or fewer, in one block.
+__host__ __device__ constexpr int sipm_block_warps(int cap) { return cap <= 256 ? 10 : 16; }
+
+// draw key of photon i of a group that starts at row a
+__device__ __forceinline__ uint32_t draw_key(const SipmGroups& G, long long a, int i) {
+  return G.key32 ? G.key32[a + i] : G.key64 ? uint32_t(G.key64[a + i]) : uint32_t(i);
+}
+
 // SiPM stage over photon groups (PT: storage type of the photon times)
-template <typename R, typename PT>
-__global__ void __launch_bounds__(512) k_sipm_sim(CrvParams p, CrvPixels px, SipmGroups G,
-                                                 const PT* __restrict__ ph_time, int lo, int cap, int last_pass,
-                                                 SipmOut O, Status* status) {
-  extern __shared__ __align__(16) char smem[];
+template <typename R, typename PT, int CAP, bool LOC>
+__global__ void __launch_bounds__(sipm_block_warps(CAP) * 32, CAP <= 256 ? 2 : 1) k_sipm_sim(const __grid_constant__ CrvParams p, CrvPixels px, SipmGroups G,
+                                                 const PT* __restrict__ ph_time, int lo, int last_pass,
+                                                 const __grid_constant__ SipmOut O, Status* status) {
+  constexpr int cap = CAP;
   __shared__ uint32_t dead[64];
   __shared__ SipmK<R> K;
   for (int i = threadIdx.x; i < 64; i += blockDim.x) dead[i] = i < DEAD_WORDS ? px.dead_bits[i] : 0u;
   if (threadIdx.x == 0) K = sipm_consts<R>(p);
   __syncthreads();
-  const bool loc = G.photon_id != nullptr;
-  SipmShared<R> S = carve<R>(smem + size_t(warp_in_block()) * sipm_smem_per_warp<R>(cap, loc), cap, loc);
+  const SipmShared<R, CAP, LOC> S{warp_in_block() * SipmShared<R, CAP, LOC>::BYTES};
   for (int q = 0; q < 2; ++q)
     if (G.guard[q] && *G.guard[q] > G.guard_cap[q]) return;
   const long long ngroups = *G.n;
@@ -873,45 +1112,58 @@ __global__ void __launch_bounds__(512) k_sipm_sim(CrvParams p, CrvPixels px, Sip
       }
       continue;
     }
-    // stage photons with t <= t_end, four chunks of 32 per step (their loads in flight together)
+    // Stage the photons with t <= t_end that can fire: on a live pixel, with a fire uniform below t_cand (4 in 10 of
+    // them; the others change nothing).  The next 32 photons are loaded while these are drawn; one copy of the draw
+    // in the code (four chunks per step unrolled took 20 KB more of it than the instruction cache has room for).
     int n = 0;
-    for (int base = 0; base < cnt; base += 128) {
-      PT tv[4];
-      uint32_t kv[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int i = base + 32 * u + lane_id();
-        tv[u] = i < cnt ? ph_time[a + i] : PT(0);
-        kv[u] = i < cnt ? (G.key32 ? G.key32[a + i] : G.key64 ? uint32_t(G.key64[a + i]) : uint32_t(i)) : 0u;
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int i = base + 32 * u + lane_id();
-        bool keep;
-        if constexpr (sizeof(PT) == 4) keep = i < cnt && (float(tv[u]) <= K.t_end_dn);
-        else keep = i < cnt && (double(tv[u]) <= p.t_end);
-        const unsigned km = __ballot_sync(FULL, keep);
-        if (keep) {
-          const int o = n + __popc(km & lanemask_lt());
-          S.ph_t[o] = R(tv[u]);
-          S.ph_key[o] = kv[u];
-          if (loc) S.ph_loc[o] = uint32_t(i);
-        }
-        n += __popc(km);
-      }
+    PT tn = PT(0);
+    uint32_t kn = 0;
+    if (lane_id() < cnt) {
+      tn = ph_time[a + lane_id()];
+      kn = draw_key(G, a, lane_id());
     }
+#pragma unroll 1
+    for (int base = 0; base < cnt; base += 32) {
+      const int i = base + lane_id();
+      const PT tv = tn;
+      const uint32_t kv = kn;
+      if (i + 32 < cnt) {
+        tn = ph_time[a + i + 32];
+        kn = draw_key(G, a, i + 32);
+      }
+      bool keep;
+      if constexpr (sizeof(PT) == 4) keep = i < cnt && (float(tv) <= K.t_end_dn);
+      else keep = i < cnt && (double(tv) <= p.t_end);
+      const U4 w = draw<CAP>(p.seed, C.ek, w2_of(ST_SIPM, 0, 0, 0, C.chan), kv);
+      const typename UniBits<R>::T fb = UniBits<R>::of(w, 1);
+      keep = keep && fb < K.t_cand;
+      int pix = -1;
+      if (keep) pix = draw_pixel<R>(p, px, dead, w);
+      keep = pix >= 0;
+      const unsigned km = __ballot_sync(FULL, keep);
+      if (keep) {
+        const int o = n + __popc(km & lanemask_lt());
+        S.ph_t()[o] = R(tv);
+        S.ph_key()[o] = kv;
+        S.ph_pix()[o] = uint16_t(uint32_t(pix) | (fb < K.t_fire ? PH_FIRES : 0u));
+        if (LOC) S.ph_loc()[o] = uint32_t(i);
+      }
+      n += __popc(km);
+    }
+    for (int w = lane_id(); w < 64; w += 32) S.bm()[w] = 0u;
     __syncwarp();
     // the photons of one (step, SiPM) row come out of the photon stage in (time, key) order, so a SiPM hit by one
     // step needs no sort: check the order, sort only when it is broken
     bool ordered = true;
+#pragma unroll 1
     for (int i = lane_id(); i + 1 < n; i += 32)
-      ordered = ordered && !after(S.ph_t[i], S.ph_key[i], S.ph_t[i + 1], S.ph_key[i + 1]);
-    if (!__all_sync(FULL, ordered)) sort_photons<R>(S, n);
+      ordered = ordered && !after(S.ph_t()[i], S.ph_key()[i], S.ph_t()[i + 1], S.ph_key()[i + 1]);
+    if (!__all_sync(FULL, ordered)) sort_photons(S, n);
     const long long idb = G.id_base ? G.id_base[g] : 0;
-    simulate_sipm<R>(p, K, px, S, dead, C, O, n, G.photon_id, a, idb);
-    int nap = run_afterpulses<R>(K, S, C, O);
+    simulate_sipm(p, K, S, dead, C, O, n, G.photon_id, a, idb);
+    const int nap = C.ntr ? run_afterpulses(K, S, C, O) : 0;
     int fired = 0;
-    for (int w = lane_id(); w < DEAD_WORDS; w += 32) fired += __popc(S.bm[w]);
+    for (int w = lane_id(); w < DEAD_WORDS; w += 32) fired += __popc(S.bm()[w]);
     fired = warp_sum(fired);
     if (lane_id() == 0) {
       O.nmain[g] = C.nq;
