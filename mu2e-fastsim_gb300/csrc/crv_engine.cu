@@ -1137,30 +1137,25 @@ static int coinc_run(const CrvParams* p, const CrvFinderGeom* g, int64_t nevents
   CoincIn I{nevents, nev_dev, reinterpret_cast<const long long*>(ev_start), ev_count, bar, sipm, seq, time, pe, status};
   CoincOut O{w.rec, w.mem_idx, w.ncl, w.nmem};
   const DeviceInfo& di = device_info();
-  // events up to 192 hits (nearly all) at one warp per block (~11 resident warps per SM); the larger ones in a pass
-  // with their lists in global memory (many warps per SM, where a 1024-hit shared-memory pass fits two)
-  struct Pass { int hcap, warps; } passes[3] = {{192, 1}, {1024, 1}, {0, 1}};
-  for (int k = 0; k < 3; ++k) {
-    if (k == 1) continue;
-    size_t per = k < 2 ? coinc_smem_per_warp(passes[k].hcap) + coinc_work_per_warp(passes[k].hcap) : 0;
-    size_t smem = per * passes[k].warps;
-    if (smem > di.smem_optin - 1024) return CRV_ERR_CUDA;
-    long long blocks = (nevents + passes[k].warps - 1) / passes[k].warps;
-    // the global pass (118 registers: 16 one-warp blocks per SM) sees the few large events of a batch, or every event
-    // at full scale (~11,000 hits each)
-    long long maxb = (long long)di.sms * (k == 0 ? 16 : (k == 1 ? 2 : 16));
-    const unsigned grid = (unsigned)(blocks < maxb ? blocks : maxb);
-    if (k < 2) {
-      CK(allow_dynamic_smem(k_coinc<false>));
-      crv::Mark mark_("k_coinc", s);
-      k_coinc<false><<<grid, passes[k].warps * 32, smem, s>>>(*p, G, I, passes[k].hcap, k, O, w.deferred, w.gscratch,
-                                                             S);
-    } else {
-      crv::Mark mark_("k_coinc_global", s);
-      k_coinc<true><<<grid, passes[k].warps * 32, 0, s>>>(*p, G, I, 0, k, O, w.deferred, w.gscratch, S);
-    }
-    CK(cudaGetLastError());
+  // events up to COINC_HCAP hits (nearly all) at one warp per block (~11 resident warps per SM), then the larger ones, a
+  // block each with its lists in global memory: the few large events of a batch, or every event at full scale
+  if (g->ntypes > 255) return CRV_ERR_ARG;
+  const size_t smem = coinc_smem_per_warp(COINC_HCAP) + coinc_work_per_warp(COINC_HCAP);
+  if (smem > di.smem_optin - 1024) return CRV_ERR_CUDA;
+  CK(allow_dynamic_smem(k_coinc));
+  {
+    const long long maxb = (long long)di.sms * 16;
+    crv::Mark mark_("k_coinc", s);
+    k_coinc<<<(unsigned)(nevents < maxb ? nevents : maxb), 32, smem, s>>>(*p, G, I, O, w.deferred);
   }
+  CK(cudaGetLastError());
+  {
+    const long long maxb = (long long)di.sms * 3;
+    crv::Mark mark_("k_coinc_global", s);
+    k_coinc_global<<<(unsigned)(nevents < maxb ? nevents : maxb), CO_GWARPS * 32, 0, s>>>(*p, G, I, O, w.deferred,
+                                                                                         w.gscratch, S);
+  }
+  CK(cudaGetLastError());
   CK(exclusive_scan(w.ncl, nevents, Identity(), w.cl_off, &w.totals[0], w.parts, s, nev_dev));
   CK(exclusive_scan(w.nmem, nevents, Identity(), w.mem_off, &w.totals[1], w.parts, s, nev_dev));
   {
