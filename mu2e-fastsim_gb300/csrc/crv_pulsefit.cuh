@@ -46,73 +46,67 @@ __device__ __forceinline__ double round_half_away(double x) {
   return x < 0.0 ? -a : (x > 0.0 ? a : 0.0 * x);
 }
 
+// |x| as an integer in the order of |x|
+__device__ __forceinline__ unsigned long long abs_bits(double x) {
+  return (unsigned long long)__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFull;
+}
+// Correctly rounded a / b from y = 1 / b rounded to nearest (Markstein, "Computation of elementary functions on the IBM
+// RISC System/6000 processor", 1990): a quotient within an ulp, its exact remainder, one correction; the first
+// correction makes sure of the ulp.  Five FP64 instructions instead of a division's dozen.  Operands outside
+// 2^-500 .. 2^500 (quotient and remainder could leave the normal range; zero) take the division.
+__device__ __forceinline__ double div_by(double a, double b, double y) {
+  const int ea = int((abs_bits(a) >> 52)), eb = int((abs_bits(b) >> 52));
+  if (unsigned(eb - 523) > 1000u || unsigned(ea - 523) > 1000u) return a / b;
+  double q = a * y;
+  q = __fma_rn(__fma_rn(-q, b, a), y, q);
+  return __fma_rn(__fma_rn(-q, b, a), y, q);
+}
+
+// whether |x| > |y| (false with a NaN, as the floating-point compare)
+__device__ __forceinline__ bool abs_greater(double x, double y) {
+  return abs_bits(x) > abs_bits(y) && abs_bits(x) <= 0x7FF0000000000000ull;
+}
+
 // LU with partial pivoting (largest |a| in the column, first on ties), then substitution.  Returns false on a zero
-// pivot (singular).
+// pivot (singular).  The pivots' reciprocals serve the substitution's divisions too, and the comparisons are integer
+// ones: of the solve's FP64 instructions a third.
 static __device__ __noinline__ bool solve3(const double M[3][3], const double r[3], double x[3]) {
-  double a[3][3], b[3];
+  double a[3][3], b[3], inv[3];
   for (int i = 0; i < 3; ++i) {
     b[i] = r[i];
     for (int j = 0; j < 3; ++j) a[i][j] = M[i][j];
   }
+#pragma unroll
   for (int k = 0; k < 3; ++k) {
     int piv = k;
-    double mx = fabs(a[k][k]);
+    double mx = a[k][k];
+#pragma unroll
     for (int i = k + 1; i < 3; ++i)
-      if (fabs(a[i][k]) > mx) { mx = fabs(a[i][k]); piv = i; }
-    if (a[piv][k] == 0.0) return false;
-    if (piv != k) {
-      for (int j = 0; j < 3; ++j) { double tmp = a[k][j]; a[k][j] = a[piv][j]; a[piv][j] = tmp; }
-      double tb = b[k]; b[k] = b[piv]; b[piv] = tb;
-    }
-    double inv = 1.0 / a[k][k];
+      if (abs_greater(a[i][k], mx)) { mx = a[i][k]; piv = i; }
+    if (abs_bits(mx) == 0ull) return false;
+#pragma unroll
+    for (int i = k + 1; i < 3; ++i)
+      if (piv == i) {
+        for (int j = 0; j < 3; ++j) { double tmp = a[k][j]; a[k][j] = a[i][j]; a[i][j] = tmp; }
+        double tb = b[k]; b[k] = b[i]; b[i] = tb;
+      }
+    inv[k] = 1.0 / a[k][k];
+#pragma unroll
     for (int i = k + 1; i < 3; ++i) {
-      double l = a[i][k] * inv;
+      double l = a[i][k] * inv[k];
       a[i][k] = l;
       for (int j = k + 1; j < 3; ++j) a[i][j] -= l * a[k][j];
       b[i] -= l * b[k];
     }
   }
+#pragma unroll
   for (int i = 2; i >= 0; --i) {
     double s = b[i];
+#pragma unroll
     for (int j = i + 1; j < 3; ++j) s -= a[i][j] * x[j];
-    x[i] = s / a[i][i];
+    x[i] = div_by(s, a[i][i], inv[i]);
   }
   return true;
-}
-
-// FP64 reciprocal from an FP32 seed and two Newton steps (24 -> 48 -> 96 bits): one FP32 MUFU op and four FP64
-// FMAs instead of an FP64 division
-__device__ __forceinline__ double rcp64(double d) {
-  double r = double(__frcp_rn(float(d)));
-  if (!(fabs(r) < 1e300) || r == 0.0) return 1.0 / d;       // outside the FP32 range: plain division
-  r = r * (2.0 - d * r);
-  r = r * (2.0 - d * r);
-  return r;
-}
-
-// 3x3 solve by the adjugate (FP32-mixed fits): one reciprocal of the determinant
-__device__ __forceinline__ bool solve3_adj(const double M[3][3], const double b[3], double x[3]) {
-  double c00 = M[1][1] * M[2][2] - M[1][2] * M[2][1];
-  double c01 = M[1][2] * M[2][0] - M[1][0] * M[2][2];
-  double c02 = M[1][0] * M[2][1] - M[1][1] * M[2][0];
-  double det = M[0][0] * c00 + M[0][1] * c01 + M[0][2] * c02;
-  if (det == 0.0 || !isfinite(det)) return false;
-  double c10 = M[0][2] * M[2][1] - M[0][1] * M[2][2];
-  double c11 = M[0][0] * M[2][2] - M[0][2] * M[2][0];
-  double c12 = M[0][1] * M[2][0] - M[0][0] * M[2][1];
-  double c20 = M[0][1] * M[1][2] - M[0][2] * M[1][1];
-  double c21 = M[0][2] * M[1][0] - M[0][0] * M[1][2];
-  double c22 = M[0][0] * M[1][1] - M[0][1] * M[1][0];
-  double inv = rcp64(det);
-  x[0] = (c00 * b[0] + c10 * b[1] + c20 * b[2]) * inv;
-  x[1] = (c01 * b[0] + c11 * b[1] + c21 * b[2]) * inv;
-  x[2] = (c02 * b[0] + c12 * b[1] + c22 * b[2]) * inv;
-  return true;
-}
-
-template <typename R>
-__device__ __forceinline__ bool solve3_p(const double M[3][3], const double b[3], double x[3]) {
-  return sizeof(R) == 8 ? solve3(M, b, x) : solve3_adj(M, b, x);
 }
 
 // eigenvalues of a symmetric 3x3 matrix (cyclic Jacobi), ascending
@@ -151,54 +145,67 @@ static __device__ __noinline__ void eig3(const double M[3][3], double e[3]) {
 
 struct Fit3 {
   double lo[3], hi[3], half[3];
-  double t0;                 // time origin of the FP32 evaluation (first window sample)
 };
 
-// One lane's fit: residuals / normal equations at internal parameters u over the window points yw[0..P), times
-// (tdc_fs + i) * period.  Sums are sequential over the points (the reference's contractions are sequential).
-// R = double: every operation in FP64; R = float: mapping, residuals and sums in FP32 relative to the window start.
-template <typename R>
-static __device__ __noinline__ void eval_lane(const Fit3& F, const double u[3], const R* yw, long long tdc_fs,
-                                              double period, int P, double* chi2, double H[6], double g[3]) {
-  R A, mu, b, d0, d1, d2;
-  if (sizeof(R) == 8) {
-    double p0 = F.lo[0] + (F.hi[0] - F.lo[0]) * (sin(u[0]) + 1.0) * 0.5;
-    double p1 = F.lo[1] + (F.hi[1] - F.lo[1]) * (sin(u[1]) + 1.0) * 0.5;
-    double p2 = F.lo[2] + (F.hi[2] - F.lo[2]) * (sin(u[2]) + 1.0) * 0.5;
-    A = R(p0); mu = R(p1); b = R(p2);
-    d0 = R(F.half[0] * cos(u[0])); d1 = R(F.half[1] * cos(u[1])); d2 = R(F.half[2] * cos(u[2]));
-  } else {
-    float s0, c0, s1, c1, s2, c2;
-    sincosf(float(u[0]), &s0, &c0);
-    sincosf(float(u[1]), &s1, &c1);
-    sincosf(float(u[2]), &s2, &c2);
-    A = R(F.lo[0]) + R(F.hi[0] - F.lo[0]) * (s0 + 1.0f) * 0.5f;
-    mu = R(F.lo[1] - F.t0) + R(F.hi[1] - F.lo[1]) * (s1 + 1.0f) * 0.5f;
-    b = R(F.lo[2]) + R(F.hi[2] - F.lo[2]) * (s2 + 1.0f) * 0.5f;
-    d0 = R(F.half[0]) * c0; d1 = R(F.half[1]) * c1; d2 = R(F.half[2]) * c2;
-  }
-  R c = 0, h00 = 0, h01 = 0, h02 = 0, h11 = 0, h12 = 0, h22 = 0, g0 = 0, g1 = 0, g2 = 0;
+constexpr int FIT_KEEP = 16;   // window points whose time the fit, and whose exponentials an evaluation, keeps
+
+// FP64 evaluation of one lane at internal parameters u over the window points yw[0..P), times (tdc_fs + i) * period (the first FIT_KEEP of them in tw):
+// chi2, and when it is below `bound` (or always: `first`) the normal equations too (a rejected step does not need them).
+// Returns whether it is below.  Sums are sequential over the points (the reference's contractions are sequential); every operation rounds as
+// written (no contraction).
+static __device__ __noinline__ bool eval_f64(const Fit3& F, const double u[3], const double* yw, const double* tw,
+                                             long long tdc_fs, double period, int P, bool first, double bound, double* chi2, double H[6],
+                                             double g[3]) {
+  double s0, c0, s1, c1, s2, c2;
+  sincos(u[0], &s0, &c0);
+  sincos(u[1], &s1, &c1);
+  sincos(u[2], &s2, &c2);
+  const double A = F.lo[0] + (F.hi[0] - F.lo[0]) * (s0 + 1.0) * 0.5;
+  const double mu = F.lo[1] + (F.hi[1] - F.lo[1]) * (s1 + 1.0) * 0.5;
+  const double b = F.lo[2] + (F.hi[2] - F.lo[2]) * (s2 + 1.0) * 0.5;
+  const double y = 1.0 / b;
+  double ez_[FIT_KEEP], gg_[FIT_KEEP], z_[FIT_KEEP];
+  double c = 0.0;
+#pragma unroll 1
   for (int i = 0; i < P; ++i) {
-    R t = sizeof(R) == 8 ? R(double(tdc_fs + i) * period) : R(float(i) * float(period));
-    R z = (t - mu) / b;
-    R ez, gg;
-    if (sizeof(R) == 8) { ez = R(exp(double(-z))); gg = R(exp(double(-z - ez))); }
-    else { ez = R(__expf(float(-z))); gg = R(__expf(float(-z - ez))); }
-    R f = A * gg;
-    R r = R(yw[i]) - f;
-    R fz = f * (ez - R(1));
-    R j0 = gg * d0;
-    R j1 = fz * (R(-1) / b) * d1;
-    R j2 = fz * (-z / b) * d2;
+    const double t = i < FIT_KEEP ? tw[i] : double(tdc_fs + i) * period;
+    const double z = div_by(t - mu, b, y);
+    const double ez = exp(-z);
+    const double gg = exp(-z - ez);
+    if (i < FIT_KEEP) { z_[i] = z; ez_[i] = ez; gg_[i] = gg; }
+    const double r = yw[i] - A * gg;
     c += r * r;
+  }
+  *chi2 = c;
+  const bool below = c < bound;
+  if (!below && !first) return false;
+  const double d0 = F.half[0] * c0, d1 = F.half[1] * c1, d2 = F.half[2] * c2;
+  const double nb = -1.0 / b;
+  double h00 = 0, h01 = 0, h02 = 0, h11 = 0, h12 = 0, h22 = 0, g0 = 0, g1 = 0, g2 = 0;
+#pragma unroll 1
+  for (int i = 0; i < P; ++i) {
+    double z, ez, gg;
+    if (i < FIT_KEEP) {
+      z = z_[i]; ez = ez_[i]; gg = gg_[i];
+    } else {
+      const double t = double(tdc_fs + i) * period;
+      z = div_by(t - mu, b, y);
+      ez = exp(-z);
+      gg = exp(-z - ez);
+    }
+    const double f = A * gg;
+    const double r = yw[i] - f;
+    const double fz = f * (ez - 1.0);
+    const double j0 = gg * d0;
+    const double j1 = fz * nb * d1;
+    const double j2 = fz * div_by(-z, b, y) * d2;
     h00 += j0 * j0; h01 += j0 * j1; h02 += j0 * j2;
     h11 += j1 * j1; h12 += j1 * j2; h22 += j2 * j2;
     g0 += j0 * r; g1 += j1 * r; g2 += j2 * r;
   }
-  *chi2 = double(c);
-  H[0] = double(h00); H[1] = double(h01); H[2] = double(h02); H[3] = double(h11); H[4] = double(h12);
-  H[5] = double(h22);
-  g[0] = double(g0); g[1] = double(g1); g[2] = double(g2);
+  H[0] = h00; H[1] = h01; H[2] = h02; H[3] = h11; H[4] = h12; H[5] = h22;
+  g[0] = g0; g[1] = g1; g[2] = g2;
+  return below;
 }
 
 __device__ __forceinline__ void sym3(const double H[6], double M[3][3]) {
@@ -206,55 +213,98 @@ __device__ __forceinline__ void sym3(const double H[6], double M[3][3]) {
   M[1][1] = H[3]; M[1][2] = M[2][1] = H[4]; M[2][2] = H[5];
 }
 
-// bounded Gumbel fit of one lane (40 LM steps, 8 Gauss-Newton steps with halving, EDM + Hessian checks)
-template <typename R>
-__device__ void fit_lane(const Fit3& F, const double p0[3], const R* yw, long long tdc_fs, double period, int P,
-                         int iters, double par[3], double* chi2_out, bool* conv, bool* hok) {
+// Whether the smallest eigenvalue of H exceeds 1e-12 of the largest.  A matrix far inside (positive leading minors and
+// 4 det / trace^2, a lower bound of the smallest eigenvalue, above 1e-9 of the trace, where the minors' rounding of a
+// few 1e-16 of trace^3 does not matter) is told without the eigenvalues.
+static __device__ __noinline__ bool hessian_ok64(const double H[6]) {
+  const double tr = H[0] + H[3] + H[5];
+  const double m2 = H[0] * H[3] - H[1] * H[1];
+  const double det = H[0] * (H[3] * H[5] - H[4] * H[4]) - H[1] * (H[1] * H[5] - H[4] * H[2]) +
+                     H[2] * (H[1] * H[4] - H[3] * H[2]);
+  if (tr > 1e-90 && tr < 1e90 && H[0] > 0.0 && m2 > 1e-9 * tr * tr && 4.0 * det > 1e-9 * tr * tr * tr) return true;
+  double M[3][3], e[3];
+  sym3(H, M);
+  eig3(M, e);
+  return e[0] > 1e-12 * fmax(e[2], 1e-300);
+}
+
+// the same bits (integer compares; equal values of other bits, a signed zero, only cost an evaluation)
+__device__ __forceinline__ bool same3(const double a[3], const double b[3]) {
+  return __double_as_longlong(a[0]) == __double_as_longlong(b[0]) &&
+         __double_as_longlong(a[1]) == __double_as_longlong(b[1]) &&
+         __double_as_longlong(a[2]) == __double_as_longlong(b[2]);
+}
+
+// What bounds the FP64 fit: the FP64 pipe, which takes 64 cycles of a scheduler (19 of an SM with four warps busy) per
+// warp instruction whatever the number of active lanes; four fifths of an evaluation's instructions are its exponentials.
+// Hence: divisions from a reciprocal, sincos for the sine and cosine of a parameter, the derivatives only for accepted
+// steps, no evaluation whose outcome is known, comparisons on integers, small batches spread over every scheduler.
+// Measured: 10,007 uneven waveforms 17.9 -> 11.4 ms, 204,000 waveforms of 12 samples 17.0 -> 11.1 ms, same bits.
+// FP64 bounded Gumbel fit of one lane: the reference's schedule (40 LM steps, 8 Gauss-Newton steps with halving, EDM +
+// Hessian checks), step for step.  Work whose outcome is known is left out, which changes no result: a step that leaves
+// the parameters as they are has the same chi2 and is rejected, and so is the point rejected last (while the damping is
+// small it changes the step by less than the parameters' last bit); a rejected step at the clamped damping, and a
+// Gauss-Newton step that no scale improves, leave the state as it was, so the rest of their loops would repeat them.
+__device__ inline void fit_lane(const Fit3& F, const double p0[3], const double* yw, long long tdc_fs, double period,
+                                int P, int iters, double par[3], double* chi2_out, bool* conv, bool* hok) {
   double u[3];
   for (int k = 0; k < 3; ++k) {
     double c = 2.0 * (p0[k] - F.lo[k]) / (F.hi[k] - F.lo[k]) - 1.0;
     u[k] = asin(fmin(fmax(c, -1.0), 1.0));
   }
+  double tw[FIT_KEEP];
+  for (int i = 0; i < FIT_KEEP && i < P; ++i) tw[i] = double(tdc_fs + i) * period;
   double chi2, H[6], g[3];
-  eval_lane<R>(F, u, yw, tdc_fs, period, P, &chi2, H, g);
+  eval_f64(F, u, yw, tw, tdc_fs, period, P, true, INFINITY, &chi2, H, g);
   double lam = 1e-3;
+  double rej[3] = {NAN, NAN, NAN};       // the last point whose chi2 was not below chi2 (which only falls)
+#pragma unroll 1
   for (int it = 0; it < iters; ++it) {
     double M[3][3];
     sym3(H, M);
     for (int i = 0; i < 3; ++i) M[i][i] = M[i][i] + lam * (M[i][i] + 1e-12);
     double du[3];
-    if (!solve3_p<R>(M, g, du)) du[0] = du[1] = du[2] = 0.0;
+    if (!solve3(M, g, du)) du[0] = du[1] = du[2] = 0.0;
     double un[3] = {u[0] + du[0], u[1] + du[1], u[2] + du[2]};
-    double c2, Hn[6], gn[3];
-    eval_lane<R>(F, un, yw, tdc_fs, period, P, &c2, Hn, gn);
-    bool better = c2 < chi2;
-    if (better) {
-      for (int k = 0; k < 3; ++k) { u[k] = un[k]; g[k] = gn[k]; }
-      for (int k = 0; k < 6; ++k) H[k] = Hn[k];
-      chi2 = c2;
+    bool better = false;
+    if (!same3(un, u) && !same3(un, rej)) {
+      double c2, Hn[6], gn[3];
+      better = eval_f64(F, un, yw, tw, tdc_fs, period, P, false, chi2, &c2, Hn, gn);
+      if (better) {
+        for (int k = 0; k < 3; ++k) { u[k] = un[k]; g[k] = gn[k]; }
+        for (int k = 0; k < 6; ++k) H[k] = Hn[k];
+        chi2 = c2;
+      } else {
+        for (int k = 0; k < 3; ++k) rej[k] = un[k];
+      }
     }
-    lam = fmin(fmax(better ? lam * 0.3 : lam * 10.0, 1e-9), 1e9);
+    const double ln = fmin(fmax(better ? lam * 0.3 : lam * 10.0, 1e-9), 1e9);
+    if (!better && ln == lam) break;
+    lam = ln;
   }
+#pragma unroll 1
   for (int it = 0; it < 8; ++it) {
     double M[3][3];
     sym3(H, M);
     for (int i = 0; i < 3; ++i) M[i][i] += 1e-12;
     double du[3];
-    if (!solve3_p<R>(M, g, du)) break;
+    if (!solve3(M, g, du)) break;
     for (int k = 0; k < 3; ++k)
       if (!isfinite(du[k])) du[k] = 0.0;
     bool moved = false;
-    for (int sc = 0; sc < 4; ++sc) {
+#pragma unroll 1
+    for (int sc = 0; sc < 4 && !moved; ++sc) {
       double s = sc == 0 ? 1.0 : (sc == 1 ? 0.5 : (sc == 2 ? 0.25 : 0.125));
       double un[3] = {u[0] + s * du[0], u[1] + s * du[1], u[2] + s * du[2]};
+      if (same3(un, u) || same3(un, rej)) continue;
       double c2, Hn[6], gn[3];
-      eval_lane<R>(F, un, yw, tdc_fs, period, P, &c2, Hn, gn);
-      if (c2 < chi2) {
+      if (eval_f64(F, un, yw, tw, tdc_fs, period, P, false, chi2, &c2, Hn, gn)) {
         for (int k = 0; k < 3; ++k) { u[k] = un[k]; g[k] = gn[k]; }
         for (int k = 0; k < 6; ++k) H[k] = Hn[k];
         chi2 = c2;
-        moved = true;
-        break;                 // the accepted step zeroes du: later scales would re-evaluate the same point
+        moved = true;            // the accepted step zeroes du: later scales would re-evaluate the same point
+      } else {
+        for (int k = 0; k < 3; ++k) rej[k] = un[k];
       }
     }
     if (!moved) break;         // state unchanged: every remaining Gauss-Newton step would repeat this one exactly
@@ -265,12 +315,9 @@ __device__ void fit_lane(const Fit3& F, const double p0[3], const R* yw, long lo
   double st[3];
   double edm;
   bool okh;
-  if (solve3_p<R>(M, g, st)) {
+  if (solve3(M, g, st)) {
     edm = 0.5 * (g[0] * st[0] + g[1] * st[1] + g[2] * st[2]);
-    double Hm[3][3], e[3];
-    sym3(H, Hm);
-    eig3(Hm, e);
-    okh = e[0] > 1e-12 * fmax(e[2], 1e-300);
+    okh = hessian_ok64(H);
   } else {
     edm = INFINITY;
     okh = false;
@@ -786,11 +833,10 @@ __device__ __forceinline__ bool pf_step(const CrvParams& p, const WaveIn& W, dou
     F.lo[1] = t_ps - p.max_time_difference; F.hi[1] = t_pe + p.max_time_difference;
     F.lo[2] = p.min_beta; F.hi[2] = p.max_beta;
     for (int k = 0; k < 3; ++k) F.half[k] = (F.hi[k] - F.lo[k]) * 0.5;
-    F.t0 = double(st_tdc + fs) * p.period;
     const double p0[3] = {yps * E, t_peak, p.default_beta};
     double par[3], chi2;
     bool conv, hok;
-    fit_lane<R>(F, p0, y + fs, st_tdc + fs, p.period, P, p.lm_iterations, par, &chi2, &conv, &hok);
+    fit_lane(F, p0, reinterpret_cast<const double*>(y + fs), st_tdc + fs, p.period, P, p.lm_iterations, par, &chi2, &conv, &hok);
     const int ndf = P - 3;
     bool nearlim = false;
     for (int k = 0; k < 3; ++k) {
