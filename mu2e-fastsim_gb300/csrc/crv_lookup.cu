@@ -4,6 +4,12 @@
 // Built with -fmad=false (FP64 throughout): every operation rounds as written, so the CPU oracle
 // (oracle/crv_oracle.c, orc_substep_photons) reproduces the photons bit for bit.
 //
+// What bounds it: FP64, the FP64 pipe (19 cycles of an SM per warp instruction, conversions and comparisons included), so
+// everything that need not be FP64 arithmetic is integer or certain FP32 work: bins and box tests compare ordered bits,
+// the binomial draws are decided in FP32 where that is certain, uniforms become integer thresholds (20,011 rows of 137
+// photons: count 2.9 -> 0.33 ms, emit 8.1 -> 1.9 ms, of which the fibre-decay logarithms are most).  FP32-mixed:
+// instruction issue (200,000 rows: count 1.33 -> 1.16 ms, emit 6.8 -> 2.7 ms).
+//
 // Layout: a warp per row, lanes over its substeps (a 20 mm crossing has 200).  Pass 1 counts the arrivals of every
 // row, an exclusive scan turns the counts into output offsets, pass 2 repeats the draws (keyed: the same numbers) and
 // writes the photons in (row, substep, table, arrival) order, each lane at its offset from a warp scan.
@@ -29,9 +35,26 @@ __device__ __forceinline__ U4 sub_block(uint32_t seed, long long step, long long
   return philox(uint32_t(step), uint32_t((unsigned long long)step >> 32), w2, w3, seed, 0u);
 }
 
+// FP64 values without FP64 instructions.  This GPU's FP64 pipe takes a warp instruction of any number of active lanes for
+// 19 cycles of the whole SM, conversions and comparisons included; integer and FP32 instructions cost a hundredth.
+__device__ __forceinline__ double i2d(unsigned long long v) {       // exact below 2^53
+  if (v == 0ull) return 0.0;
+  const int lz = __clzll((long long)v);
+  const unsigned long long m = v << lz;                              // leading bit at 63
+  return __longlong_as_double((long long)(((unsigned long long)(1086 - lz) << 52) + ((m << 1) >> 12)));
+}
+// integers in the order of the doubles (-0 as +0); NaNs order beyond the infinities of their sign
+__device__ __forceinline__ long long ord64(double x) {
+  const long long b = __double_as_longlong(x);
+  return b >= 0 ? b : (long long)(0x8000000000000000ull - (unsigned long long)b);
+}
+__device__ __forceinline__ bool is_nan(double x) {
+  return ((unsigned long long)__double_as_longlong(x) << 1) > 0xFFE0000000000000ull;
+}
+
 // Binomial(n, p): inversion (Kachitvichyanukul & Schmeiser's BINV) on min(p, 1 - p) while the mean is at most 256,
 // else the normal approximation rint(mean + sqrt(mean (1 - q)) z) clipped to [0, n]
-__device__ __forceinline__ long long binomial(long long n, double p, const U4& w) {
+__device__ __noinline__ long long binomial_64(long long n, double p, const U4 w) {
   if (n <= 0 || !(p > 0.0)) return 0;
   if (p >= 1.0) return n;
   const bool flip = p > 0.5;
@@ -58,93 +81,215 @@ __device__ __forceinline__ long long binomial(long long n, double p, const U4& w
   return flip ? n - k : k;
 }
 
+// The same draw, decided in FP32 where that is certain.  The inversion only compares u with the running terms r, so an
+// FP32 run of it gives the FP64 count whenever every comparison's two sides lie further apart than the sum of the
+// errors: of r, relative er: its argument n log(1 - q) (q truncated to 2^-23, log1pf and expf within 2 ulp, a product)
+// is within 6e-7 relative, so r within 6e-7 |arg| + 4e-7, taken as 1e-6 (|arg| + 1); each step multiplies by a / k - s,
+// whose terms are within 6e-7 and at least a factor 2 apart while k <= n / 2, taken as 4e-6 a step; of u, absolute eu:
+// 2^-24 of its truncation and a rounding and r's error per subtraction.  FP64's own errors (1e-14) vanish in these.  A
+// comparison that is not certain (about one draw in 2,000), a mean above 128 or k above n / 2 takes the FP64 form.  A
+// draw costs ~80 FP64 instructions there and none here.
+__device__ __forceinline__ long long binomial(long long n, double p, const U4& w) {
+  const float pf = d2f_trunc(p);
+  if (n > 0 && n < 1000000 && pf > 1e-30f && pf < 0.49f) {
+    const int ni = int(n);
+    const float arg = float(ni) * log1pf(-pf);
+    if (arg > -80.0f && float(ni) * pf < 128.0f) {
+      float u = f01(w.x), eu = 6e-8f;
+      const float s = __fdividef(pf, 1.0f - pf), a = float(ni + 1) * s;
+      float r = expf(arg), er = 1e-6f * (1.0f - arg);
+      int k = 0;
+      while (2 * k <= ni) {
+        const float tol = eu + (er + 2e-7f) * r;
+        if (u < r - tol) return k;
+        if (!(u > r + tol)) break;                 // not certain
+        u = u - r;
+        eu = tol + 1.2e-7f;
+        ++k;
+        r = r * (__fdividef(a, float(k)) - s);
+        er = er + 4e-6f;
+      }
+    }
+  }
+  return binomial_64(n, p, w);
+}
+
 // numpy-style findBin: bin i with e[i] <= v <= e[i+1] (the lower bin on an inner edge), -1 outside
 __device__ __forceinline__ int find_bin(const double* __restrict__ e, int ne, double v) {
-  if (!(v >= e[0]) || !(v <= e[ne - 1])) return -1;
-  if (v == e[0]) return 0;
+  const long long x = ord64(v);
+  if (is_nan(v) || x < ord64(e[0]) || x > ord64(e[ne - 1])) return -1;
+  if (x == ord64(e[0])) return 0;
   int lo = 0, hi = ne;
   while (lo < hi) {
     int mid = (lo + hi) >> 1;
-    if (e[mid] < v) lo = mid + 1; else hi = mid;
+    if (ord64(e[mid]) < x) lo = mid + 1; else hi = mid;
   }
   return lo - 1;
 }
 
 // the same bins for phi given c = cos phi and ce[j] = cos(phi edge j) (descending): phi > edge j <=> c < ce[j]
 __device__ __forceinline__ int find_bin_cos(const double* __restrict__ ce, int ne, double c) {
-  if (!(c <= ce[0]) || !(c >= ce[ne - 1])) return -1;
-  if (c == ce[0]) return 0;
+  const long long x = ord64(c);
+  if (is_nan(c) || x > ord64(ce[0]) || x < ord64(ce[ne - 1])) return -1;
+  if (x == ord64(ce[0])) return 0;
   int lo = 0, hi = ne;
   while (lo < hi) {
     int mid = (lo + hi) >> 1;
-    if (ce[mid] > c) lo = mid + 1; else hi = mid;
+    if (ord64(ce[mid]) > x) lo = mid + 1; else hi = mid;
   }
   return lo - 1;
 }
 
-// first index j whose running sum of the uint8 weights reaches thr (the number of running sums below thr)
-__device__ __forceinline__ int first_reaching(const uint8_t* __restrict__ wts, int n, double thr) {
-  int cum = 0;
-  for (int j = 0; j < n; ++j) {
-    cum += wts[j];
-    if (!(double(cum) < thr)) return j;
+// First index j whose running sum of the row's n uint8 weights reaches thr (the number of running sums below thr), n when
+// none does.  tab: the table's [nrow][n] weights.  The sums are integers, so sum < thr is sum < ceil(thr), and the row
+// is read in aligned 16-byte loads that do not depend on each other, four weights per dp4a, instead of byte by byte with
+// a floating-point compare each (two FP64 instructions a weight in the FP64 kernel): emit of 200,000 FP32 rows of 137
+// photons and 150 weights 6.8 -> 3.5 ms, of 20,011 FP64 rows 8.1 -> 5.3 ms.  Weights outside the row are masked; a
+// load that would leave the table (its ends are rarely aligned) is put together from bytes.
+__device__ __forceinline__ uint32_t keep_bytes(uint32_t w, int lo, int hi) {   // bytes [lo, hi) of a word
+  lo = min(max(lo, 0), 4);
+  hi = min(max(hi, 0), 4);
+  if (hi <= lo) return 0u;
+  return w & (0xFFFFFFFFu >> (8 * (4 - hi))) & (0xFFFFFFFFu << (8 * lo));
+}
+__device__ __noinline__ uint4 edge_words(const uint8_t* q, const uint8_t* row, int n) {
+  uint32_t v[4] = {0u, 0u, 0u, 0u};
+  for (int b = 0; b < 16; ++b)
+    if (q + b >= row && q + b < row + n) v[b >> 2] |= uint32_t(q[b]) << (8 * (b & 3));
+  return make_uint4(v[0], v[1], v[2], v[3]);
+}
+__device__ __forceinline__ int first_reaching(const uint8_t* __restrict__ tab, int nrow, int bin, int n, int thr) {
+  if (thr <= 0) return 0;
+  const uint8_t* row = tab + (long long)bin * n;
+  const uint8_t* end = tab + (long long)nrow * n;
+  const int head = int(reinterpret_cast<uintptr_t>(row) & 15u);
+  uint32_t cum = 0;
+#pragma unroll 1
+  for (int p0 = -head; p0 < n; p0 += 64) {
+    uint4 v[4];                                    // four loads in flight
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+      const int pos = p0 + 16 * b;
+      const uint8_t* q = row + pos;
+      v[b] = make_uint4(0u, 0u, 0u, 0u);
+      if (pos < n) {
+        if (q >= tab && q + 16 <= end) v[b] = __ldg(reinterpret_cast<const uint4*>(q));
+        else v[b] = edge_words(q, row, n);
+      }
+    }
+    if (p0 < 0) {                                  // the weights before the row
+      v[0].x = keep_bytes(v[0].x, -p0, 4);
+      v[0].y = keep_bytes(v[0].y, -p0 - 4, 4);
+      v[0].z = keep_bytes(v[0].z, -p0 - 8, 4);
+      v[0].w = keep_bytes(v[0].w, -p0 - 12, 4);
+    }
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+      const int pos = p0 + 16 * b;
+      const uint32_t s0 = __dp4a(v[b].x, 0x01010101u, cum), s1 = __dp4a(v[b].y, 0x01010101u, s0);
+      const uint32_t s2 = __dp4a(v[b].z, 0x01010101u, s1), s3 = __dp4a(v[b].w, 0x01010101u, s2);
+      if (s3 >= uint32_t(thr)) {                   // the word, then the byte; the weights after the row count as n
+        const bool x = s0 >= uint32_t(thr), y = s1 >= uint32_t(thr), z = s2 >= uint32_t(thr);
+        const uint32_t w = x ? v[b].x : y ? v[b].y : z ? v[b].z : v[b].w;
+        uint32_t t = (x ? cum : y ? s0 : z ? s1 : s2) + (w & 0xFFu);
+        int j = pos + (x ? 0 : y ? 4 : z ? 8 : 12);
+        if (t < uint32_t(thr)) {
+          ++j;
+          t += (w >> 8) & 0xFFu;
+          if (t < uint32_t(thr)) {
+            ++j;
+            t += (w >> 16) & 0xFFu;
+            j += t < uint32_t(thr);
+          }
+        }
+        return min(j, n);
+      }
+      cum = s3;
+    }
   }
   return n;
 }
+// smallest integer not below thr (at most 2^31 - 1): the threshold on integer sums
+__device__ __forceinline__ int sum_threshold(float thr) { return thr < 2147483520.0f ? int(ceilf(thr)) : 2147483647; }
 
 struct SubBins {
   int bin[3];
-  double t, z;
+  double frac, z;
 };
 
-// geometry and bins of substep k of row r (photons.py:139-196)
-__device__ __forceinline__ SubBins substep_bins(const CrvLookup& L, const CrvSubstepRows& R, long long r, long long k,
-                                                long long nsub, int bb, int bth) {
-  const double frac = (double(k) + 0.5) / double(nsub);
-  const double x = R.s[3 * r] + R.d[3 * r] * frac;
-  const double y = R.s[3 * r + 1] + R.d[3 * r + 1] * frac;
-  const double z = R.s[3 * r + 2] + R.d[3 * r + 2] * frac;
-  const double t = R.t0[r] + (R.t1[r] - R.t0[r]) * frac;
+// per-row constants of the substep geometry
+struct SubRow {
+  double s[3], d[3];
+  double nsub, inv_nsub;       // inv_nsub: 1 / nsub rounded
+  int bb, bth;
+};
+
+// correctly rounded a / b from y = 1 / b rounded, operands far from the ends of the exponent range (Markstein's corrections,
+// see div_by in crv_pulsefit.cuh)
+__device__ __forceinline__ double quotient(double a, double b, double y) {
+  double q = a * y;
+  q = __fma_rn(__fma_rn(-q, b, a), y, q);
+  return __fma_rn(__fma_rn(-q, b, a), y, q);
+}
+
+// Geometry and bins of substep k of a row (photons.py:139-196).  The scintillator's hole and the fibres are tested only
+// inside their bounding boxes: outside, ex or ey is at least 1 and so is ex^2 + ey^2, and a radius is at least the
+// larger of its two distances, in rounded arithmetic too (rounding is monotone).
+__device__ __forceinline__ SubBins substep_bins(const CrvLookup& L, const SubRow& w, long long k) {
+  const double k_half = __longlong_as_double(__double_as_longlong(i2d((unsigned long long)(2 * k + 1))) - (1ll << 52));
+  const double frac = quotient(k_half, w.nsub, w.inv_nsub);      // (k + 1/2) / nsub
+  const double x = w.s[0] + w.d[0] * frac;
+  const double y = w.s[1] + w.d[1] * frac;
+  const double z = w.s[2] + w.d[2] * frac;
   const double half_sep = L.fiber_separation / 2.0;
+  const double ax = fabs(x), ay = fabs(y), az = fabs(z);
+  const long long oax = ord64(ax), oay = ord64(ay);
+  const bool inz = ord64(az) < ord64(L.half_length) && !is_nan(az);
   // inside the scintillator: box, outside the elliptic fibre hole, not in a rounded corner
-  const double ax = fabs(x), ay = fabs(y);
-  bool insc = ax < L.half_thickness && ay < L.half_width && fabs(z) < L.half_length;
-  const double ex = ax / L.hole_radius_x, ey = (ay - half_sep) / L.hole_radius_y;
-  insc = insc && (ex * ex + ey * ey >= 1.0);
+  bool insc = oax < ord64(L.half_thickness) && oay < ord64(L.half_width) && inz && !is_nan(ax) && !is_nan(ay);
+  const double hy = ay - half_sep;
+  const bool hole = L.hole_radius_x > 0.0 && L.hole_radius_y > 0.0;
+  if (insc && !(hole && (oax >= ord64(L.hole_radius_x) || ord64(fabs(hy)) >= ord64(L.hole_radius_y)))) {
+    const double ex = ax / L.hole_radius_x, ey = hy / L.hole_radius_y;
+    insc = ex * ex + ey * ey >= 1.0;
+  }
   const double cx = L.half_thickness - L.corner_radius, cy = L.half_width - L.corner_radius;
-  if (ax > cx && ay > cy) {
+  if (insc && oax > ord64(cx) && oay > ord64(cy)) {
     const double qx = ax - cx, qy = ay - cy;
     if (sqrt(qx * qx + qy * qy) > L.corner_radius) insc = false;
   }
+  const int ny = L.nedges[1] - 1, nz = L.nedges[2] - 1, nb = L.nedges[3] - 1;
+  const int nth = L.nedges[4] - 1, nph = L.nedges[5] - 1, nr = L.nedges[6] - 1;
+  SubBins S;
+  S.frac = frac;
+  S.z = z;
+  S.bin[0] = S.bin[1] = S.bin[2] = -1;
+  const int bz = find_bin(L.edges[2], L.nedges[2], z);
+  if (insc && bz >= 0) {
+    const int bx = find_bin(L.edges[0], L.nedges[0], ax), by = find_bin(L.edges[1], L.nedges[1], y);
+    if (bx >= 0 && by >= 0) {
+      S.bin[0] = bz + by * nz + bx * ny * nz;
+      if (w.bb >= 0) S.bin[1] = w.bb + bz * nb + by * nz * nb + bx * ny * nz * nb;
+    }
+  }
   // inside a fibre: radius from the nearer fibre axis and the angle of the step direction to it
   const double y0 = y + half_sep, y1 = y - half_sep;
-  const double r0 = sqrt(x * x + y0 * y0), r1 = sqrt(x * x + y1 * y1);
-  const bool in0 = r0 <= L.fiber_radius, in1 = r1 <= L.fiber_radius;
-  const double ry = in1 ? y1 : y0, rr = in1 ? r1 : r0;
-  const double dx = R.d[3 * r], dy = R.d[3 * r + 1];
-  const double norm = sqrt(dx * dx + dy * dy) * rr;
-  double c = 1.0;
-  if (norm > 0.0) {
-    c = (dx * x + dy * ry) / norm;
-    c = c < -1.0 ? -1.0 : (c > 1.0 ? 1.0 : c);
-  }
-  const bool infb = fabs(z) < L.half_length && (in0 || in1) && !insc;
-  const int nx = L.nedges[0] - 1, ny = L.nedges[1] - 1, nz = L.nedges[2] - 1, nb = L.nedges[3] - 1;
-  const int nth = L.nedges[4] - 1, nph = L.nedges[5] - 1, nr = L.nedges[6] - 1;
-  (void)nx;
-  const int bx = find_bin(L.edges[0], L.nedges[0], ax), by = find_bin(L.edges[1], L.nedges[1], y);
-  const int bz = find_bin(L.edges[2], L.nedges[2], z);
-  const bool geo = bx >= 0 && by >= 0 && bz >= 0;
-  SubBins S;
-  S.t = t;
-  S.z = z;
-  S.bin[0] = (insc && geo) ? bz + by * nz + bx * ny * nz : -1;
-  S.bin[1] = (insc && geo && bb >= 0) ? bb + bz * nb + by * nz * nb + bx * ny * nz * nb : -1;
-  S.bin[2] = -1;
-  if (infb && bb >= 0 && bth >= 0 && bz >= 0) {
-    const int bph = find_bin_cos(L.cos_phi_edges, L.nedges[5], c), br = find_bin(L.edges[6], L.nedges[6], rr);
-    if (bph >= 0 && br >= 0)
-      S.bin[2] = bz + br * nz + bph * nr * nz + bth * nph * nr * nz + bb * nth * nph * nr * nz;
+  const long long ofr = ord64(L.fiber_radius);
+  if (inz && !insc && oax <= ofr && (ord64(fabs(y0)) <= ofr || ord64(fabs(y1)) <= ofr)) {
+    const double r0 = sqrt(x * x + y0 * y0), r1 = sqrt(x * x + y1 * y1);
+    const bool in0 = r0 <= L.fiber_radius, in1 = r1 <= L.fiber_radius;
+    if ((in0 || in1) && w.bb >= 0 && w.bth >= 0 && bz >= 0) {
+      const double ry = in1 ? y1 : y0, rr = in1 ? r1 : r0;
+      const double norm = sqrt(w.d[0] * w.d[0] + w.d[1] * w.d[1]) * rr;
+      double c = 1.0;
+      if (norm > 0.0) {
+        c = (w.d[0] * x + w.d[1] * ry) / norm;
+        c = c < -1.0 ? -1.0 : (c > 1.0 ? 1.0 : c);
+      }
+      const int bph = find_bin_cos(L.cos_phi_edges, L.nedges[5], c), br = find_bin(L.edges[6], L.nedges[6], rr);
+      if (bph >= 0 && br >= 0)
+        S.bin[2] = bz + br * nz + bph * nr * nz + w.bth * nph * nr * nz + w.bb * nth * nph * nr * nz;
+    }
   }
   return S;
 }
@@ -156,22 +301,47 @@ __device__ __forceinline__ long long photons_per_substep(const CrvSubstepRows& R
 // arrivals of table tb at a substep (bin >= 0)
 __device__ __forceinline__ long long arrivals(const CrvLookup& L, const CrvSubstepRows& R, uint32_t seed, long long r,
                                               long long step, long long chan, long long k, int tb, int bin, double z) {
-  double pr = double(L.table[tb].prob[bin]) * R.dev[r];
-  if (R.mu) pr = pr * dexp(-R.mu[r] * z);
-  pr = pr < 1.0 ? pr : 1.0;
+  double pr = f2d(L.table[tb].prob[bin]) * R.dev[r];
+  if (R.mu) {
+    const double mu = R.mu[r];
+    if (ord64(mu) != 0) pr = pr * dexp(-mu * z);   // dexp(0) is 1
+  }
+  if (!is_nan(pr) && ord64(pr) >= ord64(1.0)) pr = 1.0;
   return binomial(photons_per_substep(R, tb, r), pr, sub_block(seed, step, chan, tb, SUB_CALL_BINOMIAL, 0, k, 0));
 }
 
-// arrival time of arrival j (photons.py:128-137, :214-218)
+// ceil(u * sum) of a 53-bit uniform u = k 2^-53 and an integer sum, u * sum rounded to FP64 first: the threshold
+// first_reaching compares integer running sums with.  The product k * sum is exact in 84 bits; rounding to 53 of them
+// (to nearest, ties to even) and the ceiling are integer work.
+__device__ __forceinline__ int ceil_uniform(unsigned long long k, int sum) {
+  if (sum <= 0 || k == 0ull) return 0;
+  const unsigned long long m = (unsigned long long)(uint32_t)sum;
+  unsigned long long hi = __umul64hi(k, m), lo = k * m;
+  const int bits = hi ? 128 - __clzll((long long)hi) : 64 - __clzll((long long)lo);
+  if (bits > 53) {                                 // round off the lowest `s` bits
+    const int s = bits - 53;                       // at most 31
+    const unsigned long long rest = lo & ((1ull << s) - 1ull), half = 1ull << (s - 1);
+    lo -= rest;
+    if (rest > half || (rest == half && ((lo >> s) & 1ull))) {
+      const unsigned long long t = lo + (1ull << s);
+      hi += t < lo;
+      lo = t;
+    }
+  }
+  const unsigned long long q = (hi << 11) | (lo >> 53);
+  return int(q) + ((lo & ((1ull << 53) - 1ull)) != 0ull);
+}
+
+// arrival time of arrival j at a substep of time t (photons.py:128-137, :214-218)
 __device__ __forceinline__ double arrival_time(const CrvLookup& L, uint32_t seed, long long step, long long chan,
                                                long long k, int tb, int bin, int j, double t, Status* status) {
   const CrvLookupTable& T = L.table[tb];
   const U4 w = sub_block(seed, step, chan, tb, SUB_CALL_PHOTON, 0, k, j);
-  const double thr = u01(w.x, w.y) * double(T.delay_sum[bin]);
-  double tt = t + double(first_reaching(T.delays + (long long)bin * T.ndelay, T.ndelay, thr));
+  const int thr = ceil_uniform(bits53(w.x, w.y), T.delay_sum[bin]);
+  double tt = t + i2d((unsigned long long)first_reaching(T.delays, T.nbins, bin, T.ndelay, thr));
   if (L.fiber_decay_time > 0.0) {
-    const double thr2 = u01(w.z, w.w) * double(T.emis_sum[bin]);
-    const int ne = first_reaching(T.emis + (long long)bin * T.nemis, T.nemis, thr2);
+    const int thr2 = ceil_uniform(bits53(w.z, w.w), T.emis_sum[bin]);
+    const int ne = first_reaching(T.emis, T.nbins, bin, T.nemis, thr2);
     if (ne > SUB_MAX_EMISSIONS) {
       set_flag(status, CRV_ST_LIMIT);
     } else if (ne > 0) {
@@ -191,6 +361,16 @@ __device__ __forceinline__ double arrival_time(const CrvLookup& L, uint32_t seed
 __device__ __forceinline__ int theta_bin(const CrvLookup& L, const CrvSubstepRows& R, long long r) {
   return R.theta ? find_bin(L.edges[4], L.nedges[4], R.theta[r])
                  : find_bin_cos(L.cos_theta_edges, L.nedges[4], R.cos_theta[r]);
+}
+
+__device__ __forceinline__ SubRow sub_row(const CrvLookup& L, const CrvSubstepRows& R, long long r, long long nsub) {
+  SubRow w;
+  for (int x = 0; x < 3; ++x) { w.s[x] = R.s[3 * r + x]; w.d[x] = R.d[3 * r + x]; }
+  w.nsub = i2d((unsigned long long)nsub);
+  w.inv_nsub = 1.0 / w.nsub;
+  w.bb = find_bin(L.edges[3], L.nedges[3], R.beta[r]);
+  w.bth = theta_bin(L, R, r);
+  return w;
 }
 
 __device__ __forceinline__ bool row_ok(const CrvSubstepRows& R, long long r, long long* nsub, Status* status) {
@@ -233,10 +413,10 @@ __global__ void __launch_bounds__(SUB_ROWS_PER_BLOCK * 32) k_substep_count(CrvLo
     long long tot = 0;
     if (row_ok(R, r, &nsub, status)) {
       const long long step = R.step[r], chan = R.chan[r];
-      const int bb = find_bin(L.edges[3], L.nedges[3], R.beta[r]);
-      const int bth = theta_bin(L, R, r);
+      const SubRow w = sub_row(L, R, r, nsub);
       for (long long k = lane_id(); k < nsub; k += 32) {
-        const SubBins S = substep_bins(L, R, r, k, nsub, bb, bth);
+        const SubBins S = substep_bins(L, w, k);
+#pragma unroll 1
         for (int tb = 0; tb < 3; ++tb)
           if (S.bin[tb] >= 0) {
             long long a = arrivals(L, R, seed, r, step, chan, k, tb, S.bin[tb], S.z);
@@ -250,6 +430,66 @@ __global__ void __launch_bounds__(SUB_ROWS_PER_BLOCK * 32) k_substep_count(CrvLo
   }
 }
 
+// The arrivals of a warp's row wait in a shared queue, in (substep, table, arrival) order, until 32 of them can be emitted
+// together: a 32-substep chunk has 12 to 22 arrivals, so emitting chunk by chunk left half of the lanes idle (emit
+// of 200,000 FP32 rows of 137 photons 3.5 -> 3.3 ms, of 326,000 rows of 78 photons 5.1 -> 4.2 ms).
+constexpr int SUB_QUEUE = 96;
+template <typename T>
+struct SubQueue {
+  uint32_t key[SUB_QUEUE];       // substep << 12 | arrival
+  int bin[SUB_QUEUE];
+  T at[SUB_QUEUE];               // substep time (FP64) or its fraction of the row (FP32)
+  uint8_t table[SUB_QUEUE];
+};
+
+// Queue one chunk's arrivals (a[tb] of the lane's substep k) and call emit(slot, lane's output row) for every 32 queued,
+// after the row's last chunk for what is left too.  c: queued, o: output row of the queue's front.
+template <typename T, typename Emit>
+__device__ __forceinline__ void queue_chunk(SubQueue<T>& Q, int& c, long long& o, const int a[3], const int bin[3],
+                                            uint32_t k, T at, bool last, Emit emit) {
+  const int lane = lane_id();
+  const int n = a[0] + a[1] + a[2];
+  int sum;
+  const int pre = warp_excl(n, &sum);
+  int off = 0;
+  do {
+    const int m = min(SUB_QUEUE - c, sum - off);
+#pragma unroll 1
+    for (int e = max(off - pre, 0); e < n && pre + e < off + m; ++e) {
+      const int q = c + pre + e - off;
+      const int tb = e < a[0] ? 0 : e < a[0] + a[1] ? 1 : 2;
+      const int j = e - (tb > 0 ? a[0] : 0) - (tb > 1 ? a[1] : 0);
+      Q.key[q] = (k << 12) | uint32_t(j);
+      Q.bin[q] = tb == 0 ? bin[0] : tb == 1 ? bin[1] : bin[2];
+      Q.at[q] = at;
+      Q.table[q] = uint8_t(tb);
+    }
+    __syncwarp();
+    c += m;
+    off += m;
+    const bool flush = last && off == sum;
+    int b = 0;
+#pragma unroll 1
+    for (; b + 32 <= c || (flush && b < c); b += 32) {
+      if (b + lane < c) emit(b + lane, o + lane);
+      o += 32;
+    }
+    __syncwarp();
+    if (b) {                                       // the rest moves to the front
+      const int rest = max(c - b, 0);
+      uint32_t key = 0;
+      int bn = 0;
+      T t = T(0);
+      uint8_t tb = 0;
+      if (lane < rest) { key = Q.key[b + lane]; bn = Q.bin[b + lane]; t = Q.at[b + lane]; tb = Q.table[b + lane]; }
+      __syncwarp();
+      if (lane < rest) { Q.key[lane] = key; Q.bin[lane] = bn; Q.at[lane] = t; Q.table[lane] = tb; }
+      c = rest;
+      __syncwarp();
+    }
+  } while (off < sum);
+}
+
 // o_chan may be null (not written); a row whose offset is negative has no place in the output and is skipped
 __global__ void __launch_bounds__(SUB_ROWS_PER_BLOCK * 32) k_substep_emit(CrvLookup L, CrvSubstepRows R, uint32_t seed,
                                                                           long long nrows, RowSel sel,
@@ -259,6 +499,8 @@ __global__ void __launch_bounds__(SUB_ROWS_PER_BLOCK * 32) k_substep_emit(CrvLoo
                                                                           int64_t* __restrict__ o_chan,
                                                                           double* __restrict__ o_time,
                                                                           Status* status) {
+  __shared__ SubQueue<double> queue[SUB_ROWS_PER_BLOCK];
+  SubQueue<double>& Q = queue[warp_in_block()];
   if (*total > cap) return;                                    // reported by the capacity check
   seed = sel_seed(sel, seed);
   nrows = sel_nrows(sel, nrows);
@@ -268,50 +510,33 @@ __global__ void __launch_bounds__(SUB_ROWS_PER_BLOCK * 32) k_substep_emit(CrvLoo
     long long nsub;
     if (!row_ok(R, r, &nsub, status)) continue;               // warp-uniform
     const long long step = R.step[r], chan = R.chan[r];
-    const int bb = find_bin(L.edges[3], L.nedges[3], R.beta[r]);
-    const int bth = theta_bin(L, R, r);
+    const SubRow w = sub_row(L, R, r, nsub);
+    const double t0 = R.t0[r], dt = R.t1[r] - t0;
+    auto emit = [&](int q, long long o) {
+      o_step[o] = step;
+      if (o_chan) o_chan[o] = chan;
+      const uint32_t key = Q.key[q];
+      o_time[o] = arrival_time(L, seed, step, chan, (long long)(key >> 12), Q.table[q], Q.bin[q], int(key & 0xFFFu),
+                               Q.at[q], status);
+    };
     long long o = offset[r];
+    int c = 0;
     for (long long k0 = 0; k0 < nsub; k0 += 32) {
       const long long k = k0 + lane_id();
       SubBins S;
       S.bin[0] = S.bin[1] = S.bin[2] = -1;
-      S.t = 0.0;
+      S.frac = 0.0;
       int a[3] = {0, 0, 0};
       if (k < nsub) {
-        S = substep_bins(L, R, r, k, nsub, bb, bth);
+        S = substep_bins(L, w, k);
+#pragma unroll
         for (int tb = 0; tb < 3; ++tb)
           if (S.bin[tb] >= 0) {
             long long x = arrivals(L, R, seed, r, step, chan, k, tb, S.bin[tb], S.z);
             a[tb] = x >= SUB_MAX_ARRIVALS ? 0 : int(x);
           }
       }
-      // arrivals spread over the lanes in (substep, table, arrival) order, as in the FP32-mixed pass
-      int sum;
-      const int pre = warp_excl(a[0] + a[1] + a[2], &sum);
-      for (int base = 0; base < sum; base += 32) {
-        const int p = base + lane_id();
-        int owner = 0;
-#pragma unroll
-        for (int step_ = 16; step_ > 0; step_ >>= 1) {
-          const int cand = owner + step_;
-          const int pc = __shfl_sync(0xffffffffu, pre, cand);
-          if (pc <= p) owner = cand;
-        }
-        const int opre = __shfl_sync(0xffffffffu, pre, owner);
-        const int a0 = __shfl_sync(0xffffffffu, a[0], owner), a1 = __shfl_sync(0xffffffffu, a[1], owner);
-        const int b0 = __shfl_sync(0xffffffffu, S.bin[0], owner), b1 = __shfl_sync(0xffffffffu, S.bin[1], owner);
-        const int b2 = __shfl_sync(0xffffffffu, S.bin[2], owner);
-        const double ot = __shfl_sync(0xffffffffu, S.t, owner);
-        if (p < sum) {
-          int j = p - opre, tb = 0, bn = b0;
-          if (j >= a0) { j -= a0; tb = 1; bn = b1; if (j >= a1) { j -= a1; tb = 2; bn = b2; } }
-          const long long q = o + p;
-          o_step[q] = step;
-          if (o_chan) o_chan[q] = chan;
-          o_time[q] = arrival_time(L, seed, step, chan, k0 + owner, tb, bn, j, ot, status);
-        }
-      }
-      o += sum;
+      queue_chunk(Q, c, o, a, S.bin, uint32_t(k), t0 + dt * S.frac, k0 + 32 >= nsub, emit);
     }
   }
 }
@@ -402,6 +627,7 @@ struct RowF {
   double t0;
   long long step, chan;
   int nsub, bb, bth, n[3];
+  int cy, cz;                  // y and z bin of every substep when the row's ends share one, else -2
 };
 
 // double -> float on the integer pipe (truncating; zeros by their bits): every lane of the warp converts the same
@@ -428,6 +654,12 @@ __device__ __forceinline__ RowF load_row_f(const CrvSubstepRows& R, const EdgesF
   w.chan = R.chan[r];
   const long long n3[3] = {R.n_scint[r], R.n_ck_s[r], R.n_ck_f[r]};
   for (int t = 0; t < 3; ++t) w.n[t] = n3[t] < 0 ? 0 : (n3[t] > 0x7FFFFFFFll ? 0x7FFFFFFF : int(n3[t]));
+  // a coordinate runs from one end to the other without leaving their interval (rounding is monotone), and the bins do
+  // not decrease along it
+  const int y0 = find_bin_f(E.e[1], E.n[1], w.s[1]), y1 = find_bin_f(E.e[1], E.n[1], w.s[1] + w.d[1]);
+  const int z0 = find_bin_f(E.e[2], E.n[2], w.s[2]), z1 = find_bin_f(E.e[2], E.n[2], w.s[2] + w.d[2]);
+  w.cy = y0 == y1 && y0 >= 0 ? y0 : -2;
+  w.cz = z0 == z1 && z0 >= 0 ? z0 : -2;
   w.bb = find_bin_f(E.e[3], E.n[3], to_f(R.beta[r]));
   w.bth = R.theta ? find_bin_f(E.e[4], E.n[4], to_f(R.theta[r])) : find_bin_cos_f(E.cth, E.n[4], to_f(R.cos_theta[r]));
   return w;
@@ -447,31 +679,41 @@ __device__ __forceinline__ void substep_bins_f(const GeoF& g, const EdgesF& E, c
   const float frac = (float(k) + 0.5f) * w.inv_nsub;
   const float x = fmaf(w.d[0], frac, w.s[0]), y = fmaf(w.d[1], frac, w.s[1]), z = fmaf(w.d[2], frac, w.s[2]);
   const float ax = fabsf(x), ay = fabsf(y);
-  bool insc = ax < g.ht && ay < g.hw && fabsf(z) < g.hl;
-  const float ex = ax / g.hrx, ey = (ay - g.half_sep) / g.hry;
-  insc = insc && (ex * ex + ey * ey >= 1.f);
+  const bool inz = fabsf(z) < g.hl;
+  bool insc = ax < g.ht && ay < g.hw && inz;
+  // hole and fibres only inside their bounding boxes, as in substep_bins
+  const float hy = ay - g.half_sep;
+  if (insc && !(g.hrx > 0.f && g.hry > 0.f && (ax >= g.hrx || fabsf(hy) >= g.hry))) {
+    const float ex = ax / g.hrx, ey = hy / g.hry;
+    insc = ex * ex + ey * ey >= 1.f;
+  }
   const float cx = g.ht - g.cr, cy = g.hw - g.cr;
-  if (ax > cx && ay > cy) {
+  if (insc && ax > cx && ay > cy) {
     const float qx = ax - cx, qy = ay - cy;
     if (sqrtf(qx * qx + qy * qy) > g.cr) insc = false;
   }
-  const float y0 = y + g.half_sep, y1 = y - g.half_sep;
-  const float r0 = sqrtf(x * x + y0 * y0), r1 = sqrtf(x * x + y1 * y1);
-  const bool in0 = r0 <= g.fr, in1 = r1 <= g.fr;
-  const float ry = in1 ? y1 : y0, rr = in1 ? r1 : r0;
-  const float norm = sqrtf(w.d[0] * w.d[0] + w.d[1] * w.d[1]) * rr;
-  float c = 1.f;
-  if (norm > 0.f) c = fminf(1.f, fmaxf(-1.f, (w.d[0] * x + w.d[1] * ry) / norm));
-  const bool infb = fabsf(z) < g.hl && (in0 || in1) && !insc;
   const int ny = E.n[1] - 1, nz = E.n[2] - 1, nb = E.n[3] - 1, nth = E.n[4] - 1, nph = E.n[5] - 1, nr = E.n[6] - 1;
-  const int bx = find_bin_f(E.e[0], E.n[0], ax), by = find_bin_f(E.e[1], E.n[1], y), bz = find_bin_f(E.e[2], E.n[2], z);
-  const bool geo = bx >= 0 && by >= 0 && bz >= 0;
-  bin[0] = (insc && geo) ? bz + by * nz + bx * ny * nz : -1;
-  bin[1] = (insc && geo && w.bb >= 0) ? w.bb + bz * nb + by * nz * nb + bx * ny * nz * nb : -1;
-  bin[2] = -1;
-  if (infb && w.bb >= 0 && w.bth >= 0 && bz >= 0) {
-    const int bph = find_bin_cos_f(E.cphi, E.n[5], c), br = find_bin_f(E.e[6], E.n[6], rr);
-    if (bph >= 0 && br >= 0) bin[2] = bz + br * nz + bph * nr * nz + w.bth * nph * nr * nz + w.bb * nth * nph * nr * nz;
+  bin[0] = bin[1] = bin[2] = -1;
+  const int bz = w.cz > -2 ? w.cz : find_bin_f(E.e[2], E.n[2], z);
+  if (insc && bz >= 0) {
+    const int bx = find_bin_f(E.e[0], E.n[0], ax), by = w.cy > -2 ? w.cy : find_bin_f(E.e[1], E.n[1], y);
+    if (bx >= 0 && by >= 0) {
+      bin[0] = bz + by * nz + bx * ny * nz;
+      if (w.bb >= 0) bin[1] = w.bb + bz * nb + by * nz * nb + bx * ny * nz * nb;
+    }
+  }
+  const float y0 = y + g.half_sep, y1 = y - g.half_sep;
+  if (inz && !insc && ax <= g.fr && (fabsf(y0) <= g.fr || fabsf(y1) <= g.fr)) {
+    const float r0 = sqrtf(x * x + y0 * y0), r1 = sqrtf(x * x + y1 * y1);
+    const bool in0 = r0 <= g.fr, in1 = r1 <= g.fr;
+    if ((in0 || in1) && w.bb >= 0 && w.bth >= 0 && bz >= 0) {
+      const float ry = in1 ? y1 : y0, rr = in1 ? r1 : r0;
+      const float norm = sqrtf(w.d[0] * w.d[0] + w.d[1] * w.d[1]) * rr;
+      float c = 1.f;
+      if (norm > 0.f) c = fminf(1.f, fmaxf(-1.f, (w.d[0] * x + w.d[1] * ry) / norm));
+      const int bph = find_bin_cos_f(E.cphi, E.n[5], c), br = find_bin_f(E.e[6], E.n[6], rr);
+      if (bph >= 0 && br >= 0) bin[2] = bz + br * nz + bph * nr * nz + w.bth * nph * nr * nz + w.bb * nth * nph * nr * nz;
+    }
   }
   *z_out = z;
   *frac_out = frac;
@@ -485,24 +727,15 @@ __device__ __forceinline__ int arrivals_f(const CrvLookup& L, const CrvSubstepRo
   return binomial_f(w.n[tb], pr, sub_block(seed, w.step, w.chan, tb, SUB_CALL_BINOMIAL, 0, k, 0));
 }
 
-__device__ __forceinline__ int first_reaching_f(const uint8_t* __restrict__ wts, int n, float thr) {
-  int cum = 0;
-  for (int j = 0; j < n; ++j) {
-    cum += wts[j];
-    if (!(float(cum) < thr)) return j;
-  }
-  return n;
-}
-
 // offset of arrival j from the row start time (FP32: substep time, delay, fibre decay)
 __device__ __forceinline__ float arrival_offset_f(const CrvLookup& L, float decay, uint32_t seed, const RowF& w,
                                                   int k, int tb, int bin, int j, float frac, Status* status) {
   const CrvLookupTable& T = L.table[tb];
   const U4 v = sub_block(seed, w.step, w.chan, tb, SUB_CALL_PHOTON, 0, k, j);
-  float off = w.dt * frac + float(first_reaching_f(T.delays + (long long)bin * T.ndelay, T.ndelay,
-                                                   f01(v.x) * float(T.delay_sum[bin])));
+  float off = w.dt * frac + float(first_reaching(T.delays, T.nbins, bin, T.ndelay,
+                                                 sum_threshold(f01(v.x) * float(T.delay_sum[bin]))));
   if (decay > 0.f) {
-    const int ne = first_reaching_f(T.emis + (long long)bin * T.nemis, T.nemis, f01(v.z) * float(T.emis_sum[bin]));
+    const int ne = first_reaching(T.emis, T.nbins, bin, T.nemis, sum_threshold(f01(v.z) * float(T.emis_sum[bin])));
     if (ne > SUB_MAX_EMISSIONS) {
       set_flag(status, CRV_ST_LIMIT);
     } else if (ne > 0) {
@@ -565,6 +798,8 @@ __global__ void __launch_bounds__(SUB_ROWS_PER_BLOCK * 32) k_substep_emit_f32(Cr
                                                                               double* __restrict__ o_time,
                                                                               Status* status) {
   extern __shared__ float edges_sm[];
+  __shared__ SubQueue<float> queue[SUB_ROWS_PER_BLOCK];
+  SubQueue<float>& Q = queue[warp_in_block()];
   if (*total > cap) return;                                    // block-uniform, before the staging barrier
   const EdgesF E = stage_edges_f(L, edges_sm);
   const GeoF g = geo_f(L);
@@ -577,7 +812,15 @@ __global__ void __launch_bounds__(SUB_ROWS_PER_BLOCK * 32) k_substep_emit_f32(Cr
     long long nsub;
     if (!row_ok(R, r, &nsub, status)) continue;
     const RowF w = load_row_f(R, E, r);
+    auto emit = [&](int q, long long o) {
+      o_step[o] = w.step;
+      if (o_chan) o_chan[o] = w.chan;
+      const uint32_t key = Q.key[q];
+      o_time[o] = w.t0 + f2d(arrival_offset_f(L, decay, seed, w, int(key >> 12), Q.table[q], Q.bin[q], int(key & 0xFFFu),
+                                              Q.at[q], status));
+    };
     long long o = offset[r];
+    int c = 0;
     for (int k0 = 0; k0 < w.nsub; k0 += 32) {
       const int k = k0 + lane_id();
       int bin[3] = {-1, -1, -1};
@@ -585,40 +828,14 @@ __global__ void __launch_bounds__(SUB_ROWS_PER_BLOCK * 32) k_substep_emit_f32(Cr
       int a[3] = {0, 0, 0};
       if (k < w.nsub) {
         substep_bins_f(g, E, w, k, bin, &z, &frac);
+#pragma unroll
         for (int tb = 0; tb < 3; ++tb)
           if (bin[tb] >= 0) {
             a[tb] = arrivals_f(L, R, w, seed, k, tb, bin[tb], z);
             if (a[tb] >= SUB_MAX_ARRIVALS) a[tb] = 0;
           }
       }
-      // the chunk's arrivals in (substep, table, arrival) order, spread over the lanes: arrival p belongs to the last
-      // lane whose prefix is at most p (found by a shuffle binary search), so every lane has work
-      int sum;
-      const int pre = warp_excl(a[0] + a[1] + a[2], &sum);
-      for (int base = 0; base < sum; base += 32) {
-        const int p = base + lane_id();
-        int owner = 0;
-#pragma unroll
-        for (int step = 16; step > 0; step >>= 1) {
-          const int cand = owner + step;
-          const int pc = __shfl_sync(0xffffffffu, pre, cand);
-          if (pc <= p) owner = cand;
-        }
-        const int opre = __shfl_sync(0xffffffffu, pre, owner);
-        const int a0 = __shfl_sync(0xffffffffu, a[0], owner), a1 = __shfl_sync(0xffffffffu, a[1], owner);
-        const int b0 = __shfl_sync(0xffffffffu, bin[0], owner), b1 = __shfl_sync(0xffffffffu, bin[1], owner);
-        const int b2 = __shfl_sync(0xffffffffu, bin[2], owner);
-        const float ofrac = __shfl_sync(0xffffffffu, frac, owner);
-        if (p < sum) {
-          int j = p - opre, tb = 0, bn = b0;
-          if (j >= a0) { j -= a0; tb = 1; bn = b1; if (j >= a1) { j -= a1; tb = 2; bn = b2; } }
-          const long long q = o + p;
-          o_step[q] = w.step;
-          if (o_chan) o_chan[q] = w.chan;
-          o_time[q] = w.t0 + double(arrival_offset_f(L, decay, seed, w, k0 + owner, tb, bn, j, ofrac, status));
-        }
-      }
-      o += sum;
+      queue_chunk(Q, c, o, a, bin, uint32_t(k), frac, k0 + 32 >= w.nsub, emit);
     }
   }
 }
