@@ -249,6 +249,14 @@ __device__ __forceinline__ long long bounded_count(long long n, const long long*
   return m < n ? m : n;
 }
 
+// Items (SiPMs) a warp takes at a time when one coalesced load fetches their entries: 32, or fewer when that would leave
+// warps without work or with one tile more than others (eight tiles a warp).  16 events (1,900 SiPMs on 3,040 warps)
+// took 392 us in the SiPM kernel with tiles of 32, 13 us a SiPM on one warp in fifty.
+__device__ __forceinline__ int tile_size(long long n, long long warps) {
+  const long long t = n / (8 * warps);
+  return t < 1 ? 1 : t > 32 ? 32 : int(t);
+}
+
 __device__ __forceinline__ int lane_id() { return threadIdx.x & 31; }
 __device__ __forceinline__ int warp_in_block() { return threadIdx.x >> 5; }
 

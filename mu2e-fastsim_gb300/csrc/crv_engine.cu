@@ -763,10 +763,10 @@ static int digis_run(const CrvParams* p, const CrvChannels* ch, int64_t ncharges
   WfGroups G{&w.totals[0], w.gstart, w.gcount, w.glabel, w.grun};
   if (p->precision == 1)
     CK(launch_wf_prepass<float>(*p, *ch, G, ncharges, time, tmpl, tlen, tdc0_rows, w.g_tdc0, w.g_bound,
-                                w.g_maxlen, w.g_nkept, w.cl, w.head, S, s));
+                                w.g_maxlen, w.g_nkept, w.cl, S, s));
   else
     CK(launch_wf_prepass<double>(*p, *ch, G, ncharges, time, tmpl, tlen, tdc0_rows, w.g_tdc0, w.g_bound,
-                                 w.g_maxlen, w.g_nkept, w.cl, w.head, S, s));
+                                 w.g_maxlen, w.g_nkept, w.cl, S, s));
   CK(exclusive_scan(w.g_bound, ncharges, Identity(), w.slot_off, &w.totals[1], w.parts, s, &w.totals[0]));
   {
     crv::Mark mark_("k_check_caps", s);

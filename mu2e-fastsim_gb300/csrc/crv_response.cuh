@@ -1081,13 +1081,15 @@ __global__ void __launch_bounds__(sipm_block_warps(CAP) * 32, CAP <= 256 ? 2 : 1
     if (G.guard[q] && *G.guard[q] > G.guard_cap[q]) return;
   const long long ngroups = *G.n;
   const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
-  // groups in tiles of 32 per warp: one coalesced load of their counts and a ballot pick the groups of this pass (a
+  // groups in tiles per warp: one coalesced load of their counts and a ballot pick the groups of this pass (a
   // later pass, which holds few groups, does not walk every group with a dependent load)
-  for (long long g0 = (blockIdx.x * (long long)(blockDim.x >> 5) + warp_in_block()) * 32; g0 < ngroups;
-       g0 += warps * 32) {
+  const int tile = tile_size(ngroups, warps);
+  for (long long g0 = (blockIdx.x * (long long)(blockDim.x >> 5) + warp_in_block()) * tile; g0 < ngroups;
+       g0 += warps * tile) {
    const long long gl = g0 + lane_id();
-   const int cl = gl < ngroups ? G.count[gl] : 0;
-   unsigned todo = __ballot_sync(FULL, gl < ngroups && cl > lo);
+   const bool in = lane_id() < tile && gl < ngroups;
+   const int cl = in ? G.count[gl] : 0;
+   unsigned todo = __ballot_sync(FULL, in && cl > lo);
    while (todo) {
     const int bsel = __ffs(todo) - 1;
     todo &= todo - 1;
@@ -1194,14 +1196,15 @@ __global__ void k_charge_compact(const long long* __restrict__ ngroups_dev, cons
   const float cap_f = float(capacitance), inv_vov_f = 1.0f / float(overvoltage);
   long long ngroups = *ngroups_dev;
   long long warps = (long long)gridDim.x * (blockDim.x >> 5);
-  // groups in tiles of 32 per warp: one coalesced load of their sizes and offsets, then the non-empty ones in order
-  for (long long g0 = (blockIdx.x * (long long)(blockDim.x >> 5) + warp_in_block()) * 32; g0 < ngroups;
-       g0 += warps * 32) {
+  // groups in tiles per warp: one coalesced load of their sizes and offsets, then the non-empty ones in order
+  const int tile = tile_size(ngroups, warps);
+  for (long long g0 = (blockIdx.x * (long long)(blockDim.x >> 5) + warp_in_block()) * tile; g0 < ngroups;
+       g0 += warps * tile) {
    const long long gl = g0 + lane_id();
    int nm_l = 0, na_l = 0;
    long long s0_l = 0, o0_l = 0, lab_l = 0;
    bool ok = false;
-   if (gl < ngroups) {
+   if (lane_id() < tile && gl < ngroups) {
      nm_l = nmain[gl];
      na_l = nap[gl];
      s0_l = slot_off[gl];

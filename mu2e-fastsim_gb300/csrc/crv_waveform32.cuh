@@ -14,10 +14,12 @@
 //                FP32 sums widened exactly; ADC as the FP32 stage rule (adc_of_f).
 //
 // Two kernels, one warp per SiPM group each:
-//   k_wf_prep32   lanes over the group's charges: cluster split by the gap test on consecutive fixed-point times
-//                 (ballots), then lanes over the clusters: keep rule, start tick, length, window sample range, digi
+//   k_wf_prep32   a tile of groups per warp: lanes over the groups (TDC0), over each group's charges (cluster split by
+//                 the gap test on consecutive fixed-point times, ballots), then over the clusters of all the tile's
+//                 groups, which wait in a shared queue: keep rule, start tick, length, window sample range, digi
 //                 bound; kept clusters are written to cl[group start + k] (the record layout of WfCluster, with the
-//                 fixed-point start in place of the double).
+//                 fixed-point start in place of the double).  A group has 1.2 clusters, so group by group the
+//                 cluster work ran on one or two lanes (65,536 events: 6.1 -> 3.0 ms).
 //   k_wf_synth32  per kept cluster: the charges' FP32 offsets from the cluster start and normalised charges are
 //                 staged in shared memory (coalesced loads), then lanes own samples (32 per tile) and sum the
 //                 template contributions of the staged charges in charge order (deterministic), keyed noise is
@@ -149,13 +151,21 @@ struct WfCluster32 {
 };
 static_assert(sizeof(WfCluster32) == sizeof(WfCluster), "FP32 cluster record layout");
 
+// Cluster starts waiting for a warp's lanes, and the totals of the tile's groups.
+constexpr int PREP_QUEUE = 96;
+struct PrepQueue {
+  int first[PREP_QUEUE];         // first charge of the cluster in its group
+  uint8_t group[PREP_QUEUE];     // its group in the tile
+  int nk[32], bound[32], maxlen[32];
+};
+
 __global__ void __launch_bounds__(256) k_wf_prep32(CrvParams p, CrvChannels ch, WfGroups G,
                                                    const double* __restrict__ time, const double* __restrict__ tmpl,
                                                    int tlen, const double* __restrict__ tdc0_rows,
                                                    double* __restrict__ g_tdc0, int32_t* __restrict__ g_bound,
                                                    int32_t* __restrict__ g_maxlen, int32_t* __restrict__ g_nkept,
-                                                   int32_t* __restrict__ cstart, WfCluster32* __restrict__ cl,
-                                                   Status* status) {
+                                                   WfCluster32* __restrict__ cl, Status* status) {
+  __shared__ PrepQueue queue[8];
   __shared__ WfFx fx_s;
   __shared__ unsigned long long vmax_s;
   __shared__ float ip_s, pf_s;
@@ -177,99 +187,139 @@ __global__ void __launch_bounds__(256) k_wf_prep32(CrvParams p, CrvChannels ch, 
   const int zs = p.samples_zs;
   const float Pf = pf_s, ip = ip_s;
   const int lane = lane_id();
+  const unsigned lt = (1u << lane) - 1u;
+  PrepQueue& Q = queue[warp_in_block()];
   const long long ng = *G.n;
   const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
-  for (long long g = blockIdx.x * (long long)(blockDim.x >> 5) + warp_in_block(); g < ng; g += warps) {
-    const int n = G.count[g];
-    const long long q0 = G.start[g];
-    const double* t = time + q0;
-    // keyed TDC0 of the group (unless the caller gives one per cluster)
-    long long tdc0g = 0;
-    if (!tdc0_rows) tdc0g = tdc0_fx_of(p, ch, G.label[g], G.run ? G.run[g] : 0u, F.width);
-    // 1) cluster starts: a new cluster where consecutive fixed-point times differ by more than the gap
-    int ncl = 0;
-    long long prev = 0;
-    bool bad = false;
-    for (int base = 0; base < n; base += 32) {
+  const int tile = tile_size(ng, warps);
+  for (long long g0 = (blockIdx.x * (long long)(blockDim.x >> 5) + warp_in_block()) * tile; g0 < ng; g0 += warps * tile) {
+    // lane = group of the tile: its rows and its keyed TDC0 (unless the caller gives one per cluster)
+    const int ntile = int(min((long long)tile, ng - g0));
+    const long long gl = g0 + lane;
+    int n_l = 0;
+    long long q0_l = 0, tdc0_l = 0;
+    if (lane < ntile) {
+      n_l = G.count[gl];
+      q0_l = G.start[gl];
+      if (!tdc0_rows) tdc0_l = tdc0_fx_of(p, ch, G.label[gl], G.run ? G.run[gl] : 0u, F.width);
+    }
+    Q.nk[lane] = 0;
+    Q.bound[lane] = 0;
+    Q.maxlen[lane] = 0;
+    __syncwarp();
+    // The clusters queued in Q (start rows, in order), the first `full` of them with known ends: keep rule, start tick,
+    // length, window range, digi bound, one cluster per lane.
+    auto clusters = [&](int cnt, int full) {
+#pragma unroll 1
+      for (int base = 0; base < full; base += 32) {
+        const int e = base + lane;
+        const bool on = e < full;
+        const int gi = on ? Q.group[e] : 0, a = on ? Q.first[e] : 0;
+        const int gn = e + 1 < cnt ? int(Q.group[e + 1]) : -1;
+        const int n = __shfl_sync(0xffffffffu, n_l, gi);
+        const long long q0 = __shfl_sync(0xffffffffu, q0_l, gi), tdc0g = __shfl_sync(0xffffffffu, tdc0_l, gi);
+        const int b = on && gn == gi ? Q.first[e + 1] : n;
+        const bool keep = on && (b - a) >= F.nmin;
+        WfCluster32 rec{};
+        int L = 0;
+        if (keep) {
+          long long tdc0 = tdc0g;
+          if (tdc0_rows && !d2fx(tdc0_rows[q0 + a], &tdc0)) {
+            set_flag(status, CRV_ST_LIMIT);
+            tdc0 = 0;
+          }
+          long long tf, tl;
+          d2fx(time[q0 + a], &tf);
+          d2fx(time[q0 + b - 1], &tl);
+          const long long k0 = fx_ceil_div(tf - F.P - tdc0, F.P, F.invP);
+          const long long ts = k0 * F.P + tdc0;
+          const long long est = fx_floor_div(tl - tf + F.maxt, F.P, F.invP);
+          // the last charge reaches the last sample (the reach only grows with the charge time)
+          const float dt = fx2f(tl - ts);
+          long long used = 0;
+          const int j0 = first_sample_f(dt, Pf);
+          for (int k = nr - 1; k >= 0; --k)
+            if (tmpl_index_f(j0 + k, dt, Pf, ip, tlen) >= 0) {
+              used = j0 + k + 1;
+              break;
+            }
+          L = int(est > used ? est : used);
+          int ilo = 0, ihi = -1;
+          if (L <= 16384) {
+            const long long last = ts + (long long)(L - 1) * F.P;
+            ilo = ts >= F.wlo ? 0 : int(min((long long)L, fx_ceil_div(F.wlo - ts, F.P, F.invP)));
+            ihi = last <= F.whi ? L - 1 : int(max(-1ll, fx_floor_div(F.whi - ts, F.P, F.invP)));
+          }
+          rec = WfCluster32{ts, k0, a, b, L, int16_t(ilo), int16_t(ihi)};
+        }
+        const unsigned mine = __match_any_sync(0xffffffffu, on ? gi : 32 + lane);
+        const unsigned km = __ballot_sync(0xffffffffu, keep);
+        if (keep) cl[q0 + Q.nk[gi] + __popc(km & mine & lt)] = rec;
+        __syncwarp();
+        if (keep) {
+          if ((km & mine & lt) == 0u) Q.nk[gi] += __popc(km & mine);
+          atomicAdd(&Q.bound[gi], (L + zs - 1) / zs);
+          atomicMax(&Q.maxlen[gi], L);
+        }
+        __syncwarp();
+      }
+    };
+    // cluster starts of every group: a new cluster where consecutive fixed-point times differ by more than the gap
+    int cnt = 0, gi = 0, base = 0, n = __shfl_sync(0xffffffffu, n_l, 0);
+    long long q0 = __shfl_sync(0xffffffffu, q0_l, 0), prev = 0;
+    unsigned bad = 0;
+    bool odd = false;
+#pragma unroll 1
+    while (true) {
+      if (gi < ntile && base >= n) {               // next group
+        if (__any_sync(0xffffffffu, odd)) {
+          bad |= 1u << gi;
+          if (lane == 0) set_flag(status, CRV_ST_LIMIT);
+        }
+        odd = false;
+        ++gi;
+        base = 0;
+        n = __shfl_sync(0xffffffffu, n_l, gi & 31);
+        q0 = __shfl_sync(0xffffffffu, q0_l, gi & 31);
+        if (gi < ntile && n <= 0) continue;
+      }
+      const bool end = gi >= ntile;
+      if (end || cnt > PREP_QUEUE - 32) {          // all clusters, or those with known ends to make room for 32 more
+        clusters(cnt, end ? cnt : cnt - 1);
+        if (end) break;
+        const int f = Q.first[cnt - 1];
+        const uint8_t q = Q.group[cnt - 1];
+        __syncwarp();
+        if (lane == 0) { Q.first[0] = f; Q.group[0] = q; }
+        cnt = 1;
+        __syncwarp();
+      }
       const int q = base + lane;
       long long tf = 0;
-      if (q < n) bad |= !d2fx(t[q], &tf);
+      if (q < n) odd |= !d2fx(time[q0 + q], &tf);
       long long tp = __shfl_up_sync(0xffffffffu, tf, 1);
       if (lane == 0) tp = prev;
       const bool isnew = q < n && (q == 0 || tf - tp > F.gap);
       const unsigned m = __ballot_sync(0xffffffffu, isnew);
-      if (isnew) cstart[q0 + ncl + __popc(m & ((1u << lane) - 1u))] = q;
-      ncl += __popc(m);
+      if (isnew) {
+        const int at = cnt + __popc(m & lt);
+        Q.first[at] = q;
+        Q.group[at] = uint8_t(gi);
+      }
+      cnt += __popc(m);
       prev = __shfl_sync(0xffffffffu, tf, 31);
-    }
-    if (__any_sync(0xffffffffu, bad)) {
-      if (lane == 0) set_flag(status, CRV_ST_LIMIT);
-      if (lane == 0) { g_bound[g] = 0; g_maxlen[g] = 0; g_nkept[g] = 0; g_tdc0[g] = 0.0; }
-      continue;
+      base += 32;
+      __syncwarp();
     }
     __syncwarp();
-    // 2) lanes over clusters: keep rule, start tick, length, window range, digi bound
-    long long bound = 0;
-    int maxlen = 0, nk = 0;
-    for (int cb = 0; cb < ncl; cb += 32) {
-      const int c = cb + lane;
-      int a = 0, b = 0;
-      if (c < ncl) {
-        a = cstart[q0 + c];
-        b = c + 1 < ncl ? cstart[q0 + c + 1] : n;
-      }
-      __syncwarp();                              // every lane has read its starts before records are written
-      bool keep = c < ncl && (b - a) >= F.nmin;
-      WfCluster32 rec{};
-      int L = 0;
-      if (keep) {
-        long long tdc0 = tdc0g;
-        if (tdc0_rows && !d2fx(tdc0_rows[q0 + a], &tdc0)) {
-          set_flag(status, CRV_ST_LIMIT);
-          tdc0 = 0;
-        }
-        long long tf, tl;
-        d2fx(t[a], &tf);
-        d2fx(t[b - 1], &tl);
-        const long long k0 = fx_ceil_div(tf - F.P - tdc0, F.P, F.invP);
-        const long long ts = k0 * F.P + tdc0;
-        const long long est = fx_floor_div(tl - tf + F.maxt, F.P, F.invP);
-        // the last charge reaches the last sample (the reach only grows with the charge time)
-        const float dt = fx2f(tl - ts);
-        long long used = 0;
-        const int j0 = first_sample_f(dt, Pf);
-        for (int k = nr - 1; k >= 0; --k)
-          if (tmpl_index_f(j0 + k, dt, Pf, ip, tlen) >= 0) {
-            used = j0 + k + 1;
-            break;
-          }
-        L = int(est > used ? est : used);
-        int ilo = 0, ihi = -1;
-        if (L <= 16384) {
-          const long long last = ts + (long long)(L - 1) * F.P;
-          ilo = ts >= F.wlo ? 0 : int(min((long long)L, fx_ceil_div(F.wlo - ts, F.P, F.invP)));
-          ihi = last <= F.whi ? L - 1 : int(max(-1ll, fx_floor_div(F.whi - ts, F.P, F.invP)));
-        }
-        rec = WfCluster32{ts, k0, a, b, L, int16_t(ilo), int16_t(ihi)};
-      }
-      const unsigned km = __ballot_sync(0xffffffffu, keep);
-      if (keep) cl[q0 + nk + __popc(km & ((1u << lane) - 1u))] = rec;
-      nk += __popc(km);
-      long long bnd = keep ? (L + zs - 1) / zs : 0;
-      int ml = keep ? L : 0;
-      for (int o = 16; o > 0; o >>= 1) {
-        bnd += __shfl_xor_sync(0xffffffffu, bnd, o);
-        ml = max(ml, __shfl_xor_sync(0xffffffffu, ml, o));
-      }
-      bound += bnd;
-      maxlen = max(maxlen, ml);
+    if (lane < ntile) {
+      const bool drop = (bad >> lane) & 1u;
+      g_bound[gl] = drop ? 0 : Q.bound[lane];
+      g_maxlen[gl] = drop ? 0 : Q.maxlen[lane];
+      g_nkept[gl] = drop ? 0 : Q.nk[lane];
+      g_tdc0[gl] = drop ? 0.0 : fx2d(tdc0_l);
     }
-    if (lane == 0) {
-      g_bound[g] = int32_t(bound);
-      g_maxlen[g] = maxlen;
-      g_nkept[g] = nk;
-      g_tdc0[g] = fx2d(tdc0g);
-    }
+    __syncwarp();
   }
 }
 
@@ -323,11 +373,13 @@ __global__ void __launch_bounds__(256, 4) k_wf_synth32(CrvParams p, WfGroups G, 
   const float conv_f = cf_s[5], off_f = cf_s[6];
   const long long ng = *G.n;
   const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
-  // groups in tiles of 32 per warp: one coalesced load of their longest clusters and a ballot pick this pass's groups
-  for (long long g0 = (blockIdx.x * (long long)(blockDim.x >> 5) + warp_in_block()) * 32; g0 < ng; g0 += warps * 32) {
+  // groups in tiles per warp: one coalesced load of their longest clusters and a ballot pick this pass's groups
+  const int tile = tile_size(ng, warps);
+  for (long long g0 = (blockIdx.x * (long long)(blockDim.x >> 5) + warp_in_block()) * tile; g0 < ng; g0 += warps * tile) {
    const long long gl = g0 + lane;
-   const int mll = gl < ng ? g_maxlen[gl] : 0;
-   unsigned todo = __ballot_sync(0xffffffffu, gl < ng && mll > lo);
+   const bool in = lane < tile && gl < ng;
+   const int mll = in ? g_maxlen[gl] : 0;
+   unsigned todo = __ballot_sync(0xffffffffu, in && mll > lo);
    while (todo) {
     const int bsel = __ffs(todo) - 1;
     todo &= todo - 1;
@@ -375,28 +427,31 @@ __global__ void __launch_bounds__(256, 4) k_wf_synth32(CrvParams p, WfGroups G, 
         const int jB = min(sj[nq - 1] + nr - 1, L - 1);
         for (int T = (jA >> 5) << 5; T <= jB; T += 32) {
           // charges of the chunk that can reach the tile: first sample in (T - nr, T + 31]
-          int q1 = 0, hi = nq;
-          while (q1 < hi) {
-            const int m = (q1 + hi) >> 1;
-            if (sj[m] > T - nr) hi = m; else q1 = m + 1;
-          }
-          int q2 = q1;
-          hi = nq;
-          while (q2 < hi) {
-            const int m = (q2 + hi) >> 1;
-            if (sj[m] > T + 31) hi = m; else q2 = m + 1;
+          int q1 = 0, q2 = nq;
+          if (L > 32) {                            // (one tile: all of them)
+            int hi = nq;
+            while (q1 < hi) {
+              const int m = (q1 + hi) >> 1;
+              if (sj[m] > T - nr) hi = m; else q1 = m + 1;
+            }
+            q2 = q1;
+            hi = nq;
+            while (q2 < hi) {
+              const int m = (q2 + hi) >> 1;
+              if (sj[m] > T + 31) hi = m; else q2 = m + 1;
+            }
           }
           // a cluster of at most 16 samples (most of them) takes two lanes per sample, each summing every other
           // charge; the two partial sums are added in a fixed order, so the result is the same on every run
           const int split = L <= 16 ? 1 : 0;
           const int J = T + (split ? (lane & 15) : lane);
           const int part = split ? (lane >> 4) : 0;
-          const float JP = float(J) * Pf;
+          const float JP = __fmul_rn(float(J), Pf);      // rounded before the subtraction, never fused with it
           float acc = 0.0f;
 #pragma unroll 4
           for (int q = q1 + part; q < q2; q += 1 + split) {
             const float2 v = sq[q];
-            const float st = JP - v.x;
+            const float st = __fsub_rn(JP, v.x);
             // nearest integer of st / precision (ties to even) by the 1.5 x 2^23 shift; |st / precision| < 2^22
             const int ti = __float_as_int(fmaf(st, ip, 12582912.0f)) - 0x4B400000;
             if (st >= 0.0f && ti < tlen) acc = fmaf(tmpl_f[ti], v.y, acc);
