@@ -368,7 +368,13 @@ extern __shared__ __align__(16) char sipm_smem[];
 template <typename R, int CAP, bool LOC>
 struct SipmShared {
   static constexpr int TCAP = sipm_tcap(CAP);                      // afterpulse queue length
-  static constexpr int O_T = NPS_ALLOC * int(sizeof(R)), O_TRT = O_T + CAP * int(sizeof(R)),
+  // Last-discharge times.  First pass: per pixel the number of its last charge record, and the records' times (FT of
+  // them; a SiPM of at most 256 photons has at most 272 charge slots, and one with more charges is reported, its
+  // results dropped).  Other passes, where a pixel fires over and over: the time per pixel.
+  static constexpr bool BY_RECORD = CAP <= 256;
+  static constexpr int FT = 288;
+  static constexpr int O_FT = NPS_ALLOC * 2;
+  static constexpr int O_T = BY_RECORD ? O_FT + FT * int(sizeof(R)) : NPS_ALLOC * int(sizeof(R)), O_TRT = O_T + CAP * int(sizeof(R)),
                        O_TRU = O_TRT + TCAP * int(sizeof(R)), O_TRI = O_TRU + TCAP * int(sizeof(R)),
                        O_KEY = O_TRI + TCAP * 8, O_LOC = O_KEY + CAP * 4, O_BM = O_LOC + (LOC ? CAP * 4 : 0),
                        O_MISC = O_BM + 64 * 4, O_CAND = O_MISC + 16, O_TRP = O_CAND + 256 * 2,
@@ -378,7 +384,20 @@ struct SipmShared {
   int base;
   template <typename T>
   __device__ __forceinline__ T* at(int off) const { return reinterpret_cast<T*>(sipm_smem + base + off); }
-  __device__ __forceinline__ R* last() const { return at<R>(0); }
+  __device__ __forceinline__ R last(int q) const {
+    if constexpr (BY_RECORD) return at<R>(O_FT)[at<uint16_t>(0)[q]];
+    else return at<R>(0)[q];
+  }
+  // pixel q fired at time t, charge record k; `top`: no later touch of q in this step
+  __device__ __forceinline__ void set_last(int q, int k, R t, bool top = true) const {
+    if constexpr (BY_RECORD) {
+      k = min(k, FT - 1);
+      at<R>(O_FT)[k] = t;
+      if (top) at<uint16_t>(0)[q] = uint16_t(k);
+    } else {
+      if (top) at<R>(0)[q] = t;
+    }
+  }
   __device__ __forceinline__ R* ph_t() const { return at<R>(O_T); }
   __device__ __forceinline__ uint32_t* ph_key() const { return at<uint32_t>(O_KEY); }
   __device__ __forceinline__ uint32_t* ph_loc() const { return at<uint32_t>(O_LOC); }
@@ -473,6 +492,8 @@ __device__ __forceinline__ int draw_pixel(const CrvParams& p, const CrvPixels& p
 template <typename R>
 struct SipmK {
   R vov, tau, p1, p2, life0, life1, t_end;
+  R inv_tau, inv_p2;             // reciprocals, rounded
+  int plain;                     // tau or p2 too large or small for div_const
   typename UniBits<R>::T t_ct, t_t0, t_t1;       // cross-talk and trap draws
   typename UniBits<R>::T t_fire;                 // a pixel at full overvoltage fires
   typename UniBits<R>::T t_cand;                 // a photon at or above it fires on no pixel, whatever its state
@@ -480,10 +501,29 @@ struct SipmK {
   int ct_on, t0_on, t1_on, npx, npy;
 };
 
+// Correctly rounded a / b for a constant b of ordinary size, from y = 1 / b rounded (Markstein, "Computation of elementary
+// functions on the IBM RISC System/6000 processor", 1990: two corrections by the exact remainder).  Five instructions;
+// the division's own sequence and slow path are 1.9 KB of code a copy in FP32, a dozen FP64 instructions in FP64.
+// Quotients below the normal range may differ in their last bits and a zero's sign is lost, neither of which an
+// exponential of the result sees.
+template <typename R>
+__device__ __noinline__ R div_plain(R a, R b) { return a / b; }
+__device__ __forceinline__ float fma_r(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double fma_r(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float mul_r(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_r(double a, double b) { return __dmul_rn(a, b); }
+template <typename R>
+__device__ __forceinline__ R div_const(R a, R b, R y, int plain) {
+  if (plain) return div_plain<R>(a, b);
+  R q = mul_r(a, y);
+  q = fma_r(fma_r(-q, b, a), y, q);
+  return fma_r(fma_r(-q, b, a), y, q);
+}
+
 template <typename R>
 __device__ __forceinline__ R pfire(const SipmK<R>& K, R v) {
   using M = Math<R>;
-  return K.p1 * (R(1) - M::exp(-v / K.p2));
+  return K.p1 * (R(1) - M::exp(div_const<R>(-v, K.p2, K.inv_p2, K.plain)));
 }
 
 // probability that a node hit m times fires: 1 - (1 - pfire)^m
@@ -497,14 +537,17 @@ __device__ __forceinline__ R pfire_m(const SipmK<R>& K, R v, int m) {
 }
 
 template <typename R>
-__device__ __forceinline__ SipmK<R> sipm_consts(const CrvParams& p) {
-  SipmK<R> K;
+__device__ __noinline__ void sipm_consts(const CrvParams& p, SipmK<R>& K) {
   K.vov = R(p.overvoltage); K.tau = R(p.time_constant); K.p1 = R(p.p1); K.p2 = R(p.p2);
   K.life0 = R(p.trap0_lifetime); K.life1 = R(p.trap1_lifetime); K.t_end = R(p.t_end);
   K.t_end_dn = __double2float_rd(p.t_end);
   K.ct_on = p.q_ct > 0.0; K.t0_on = p.q_t0 > 0.0; K.t1_on = p.q_t1 > 0.0;
   K.t_ct = UniBits<R>::below(R(p.q_ct)); K.t_t0 = UniBits<R>::below(R(p.q_t0)); K.t_t1 = UniBits<R>::below(R(p.q_t1));
   K.npx = p.n_pixels_x; K.npy = p.n_pixels_y;
+  K.inv_tau = R(1) / K.tau;
+  K.inv_p2 = R(1) / K.p2;
+  const auto odd = [](R x) { return !((x > R(1e-9) && x < R(1e9)) || (x < R(-1e-9) && x > R(-1e9))); };
+  K.plain = odd(K.tau) || odd(K.p2) || !(K.vov > R(-1e9) && K.vov < R(1e9));
   const R pm = pfire_m<R>(K, K.vov, 1);
   K.t_fire = UniBits<R>::below(pm);
   // A recovering pixel has 0 <= v <= overvoltage (photons come in time order), and pfire grows with v, so no state
@@ -512,20 +555,19 @@ __device__ __forceinline__ SipmK<R> sipm_consts(const CrvParams& p) {
   // constants of other signs every photon on a live pixel is kept.
   const bool grows = K.vov >= R(0) && K.tau > R(0) && K.p1 >= R(0) && K.p2 > R(0);
   K.t_cand = grows ? UniBits<R>::below(pm + R(1e-6)) : UniBits<R>::below(R(2));
-  return K;
 }
 
 // recovered overvoltage at time t of a pixel that fired last at t0
 template <typename R>
 __device__ __forceinline__ R recovered_from(const SipmK<R>& K, R t, R t0) {
   using M = Math<R>;
-  return K.vov * (R(1) - M::exp(-(t - t0) / K.tau));
+  return K.vov * (R(1) - M::exp(div_const<R>(-(t - t0), K.tau, K.inv_tau, K.plain)));
 }
 // recovered overvoltage of pixel q at time t (Vov if it never fired)
 template <typename R, int CAP, bool LOC>
 __device__ __forceinline__ R recovered(const SipmK<R>& K, const SipmShared<R, CAP, LOC>& S, int q, R t) {
   if (!bm_test(S.bm(), q)) return K.vov;
-  return recovered_from<R>(K, t, S.last()[q]);
+  return recovered_from<R>(K, t, S.last(q));
 }
 
 // Per SiPM context while simulating.
@@ -688,6 +730,19 @@ __device__ __forceinline__ int make_frontier(const SipmShared<R, CAP, LOC>& S, i
   return nf;
 }
 
+// Append the drawn neighbours ct of every lane's pixel q to the n candidates; returns how many there are then (at most
+// 256 are kept).
+template <typename R, int CAP, bool LOC>
+__device__ __forceinline__ int put_candidates(const SipmShared<R, CAP, LOC>& S, unsigned ct, int q, int n) {
+  const int c = __popc(ct);
+  const unsigned b0 = __ballot_sync(FULL, c & 1), b1 = __ballot_sync(FULL, c & 2), b2 = __ballot_sync(FULL, c & 4);
+  int at = n + __popc(b0 & lanemask_lt()) + 2 * __popc(b1 & lanemask_lt()) + 4 * __popc(b2 & lanemask_lt());
+#pragma unroll 1
+  for (unsigned m = ct; m; m &= m - 1u, ++at)
+    if (at < 256) S.cand()[at] = uint16_t(neighbour(q, __ffs(m) - 1));
+  return n + __popc(b0) + 2 * __popc(b1) + 4 * __popc(b2);
+}
+
 // Cross-talk cascade of one photon from generation 2 on; the frontier is spread over the lanes.  ct: the lane's drawn
 // neighbours of its pixel pix (0: none, or a node of another photon).  Generation 1 is part of the photon step (simulate_sipm), so this runs for the few photons whose
 // cascade goes further; called, not inlined, to keep the photon step's code and registers small.  C.nq, C.ntr and
@@ -699,9 +754,7 @@ __device__ __noinline__ void run_cascade(uint32_t seed, const SipmK<R>& K, SipmS
   t = __shfl_sync(FULL, t, src);
   key = __shfl_sync(FULL, key, src);
   id = __shfl_sync(FULL, id, src);
-  int nc, at = warp_excl(__popc(ct), &nc);
-#pragma unroll 1
-  for (unsigned m = ct; m; m &= m - 1u) S.cand()[at++] = uint16_t(neighbour(pix, __ffs(m) - 1));
+  int nc = put_candidates(S, ct, pix, 0);
   __syncwarp();
   uint32_t gen = 2;
   int lim = 0;
@@ -732,7 +785,7 @@ __device__ __noinline__ void run_cascade(uint32_t seed, const SipmK<R>& K, SipmS
       unsigned ct = 0;
       if (fire) {
         put_charge<R>(O, C, pos, t, v, id);
-        S.last()[q] = t;
+        S.set_last(q, C.nq + pos, t);
         bm_set(S.bm(), q);
         if (K.t0_on || K.t1_on) {
           const U4 a = keyed_call(seed, C.ek, w2_of(ST_SIPM, gen, uint32_t(i), 1, C.chan), key);
@@ -741,21 +794,11 @@ __device__ __noinline__ void run_cascade(uint32_t seed, const SipmK<R>& K, SipmS
         ct = node_crosstalk<R>(seed, K, C, gen, uint32_t(i), key, q);
       }
       C.nq += __popc(fm);
-      // traps in node order
-      int tot;
-      int tpos = warp_excl(ntr, &tot);
-      put_traps(S, C.ntr + tpos, ntr, tt, uf, q, id);
-      C.ntr += tot;
-      // candidates
-      int nct = __popc(ct);
-      int cpos = warp_excl(nct, &tot);
-      int a = 0;
-#pragma unroll 1
-      for (unsigned m = ct; m; m &= m - 1u) {
-        int k = ncand + cpos + a++;
-        if (k < 256) S.cand()[k] = uint16_t(neighbour(q, __ffs(m) - 1));
-      }
-      ncand += tot;
+      // traps and candidates in node order
+      const unsigned a1 = __ballot_sync(FULL, ntr > 0), a2 = __ballot_sync(FULL, ntr > 1);
+      put_traps(S, C.ntr + __popc(a1 & lanemask_lt()) + __popc(a2 & lanemask_lt()), ntr, tt, uf, q, id);
+      C.ntr += __popc(a1) + __popc(a2);
+      ncand = put_candidates(S, ct, q, ncand);
       __syncwarp();
     }
     if (ncand > 256) { lim = 1; break; }
@@ -861,7 +904,7 @@ __device__ __forceinline__ void simulate_sipm(const CrvParams& p, const SipmK<R>
       const typename B::T fb = B::of(w0, 1);
       if (node) fire = fb < K.t_fire;
       if (set) {
-        const Touch<R> o = touch_again<R>(K, t, S.last()[pix], fb);
+        const Touch<R> o = touch_again<R>(K, t, S.last(pix), fb);
         v = o.v;
         fire = o.fire;
       }
@@ -881,7 +924,7 @@ __device__ __forceinline__ void simulate_sipm(const CrvParams& p, const SipmK<R>
           v = K.vov;
           fire = fb < K.t_fire;
           if (m || set) {
-            const Touch<R> o = touch_again<R>(K, t, m ? tl : S.last()[pix], fb);
+            const Touch<R> o = touch_again<R>(K, t, m ? tl : S.last(pix), fb);
             v = o.v;
             fire = o.fire;
           }
@@ -925,7 +968,7 @@ __device__ __forceinline__ void simulate_sipm(const CrvParams& p, const SipmK<R>
     if (fire) {
       put_charge<R>(O, C, __popc(fm & lt), t, v, id);
       bm_set(S.bm(), pix);
-      if ((same & fm & ~lt) == (1u << lane)) S.last()[pix] = t;
+      S.set_last(pix, C.nq + __popc(fm & lt), t, (same & fm & ~lt) == (1u << lane));
       if (K.t0_on || K.t1_on) {
         const U4 a = draw<CAP>(p.seed, C.ek, w2_of(ST_SIPM, node, idx, 1, C.chan), key);
         ntr = node_traps<R>(p.seed, K, C, node, idx, key, t, a, tt, uf);
@@ -953,11 +996,12 @@ __device__ __forceinline__ void simulate_sipm(const CrvParams& p, const SipmK<R>
 }
 
 // Afterpulses after all photons, in (time, schedule order); stored after the main records.  Returns the count.
+// Lane 0, one after the other (rare, see run_afterpulses).
 template <typename R, int CAP, bool LOC>
-__device__ __noinline__ int run_afterpulses(const SipmK<R>& K, SipmShared<R, CAP, LOC> S, SipmCtx C, const SipmOut& O) {
-  int ntr = min(C.ntr, S.TCAP);
+__device__ __noinline__ int afterpulses_serial(const SipmK<R>& K, SipmShared<R, CAP, LOC> S, SipmCtx C, const SipmOut& O) {
+  const int ntr = min(C.ntr, S.TCAP);
   int nap = 0;
-  if (lane_id() == 0 && ntr > 0) {
+  if (lane_id() == 0) {
     // insertion sort by time (stable: equal times keep schedule order)
 #pragma unroll 1
     for (int a = 1; a < ntr; ++a) {
@@ -980,16 +1024,9 @@ __device__ __noinline__ int run_afterpulses(const SipmK<R>& K, SipmShared<R, CAP
       int q = S.tr_pix()[a];
       R v = recovered(K, S, q, t1);
       if (S.tr_uf()[a] < pfire<R>(K, v)) {
-        S.last()[q] = t1;
+        S.set_last(q, C.nq + nap, t1);
         S.bm()[q >> 5] |= 1u << (q & 31);
-        long long id = S.tr_id()[a];
-        int kk = C.nq + nap;
-        if (kk < C.cap) {
-          long long o = C.slot + kk;
-          O.t[o] = widen(t1);
-          O.v[o] = widen(v);
-          O.id[o] = id;
-        }
+        put_charge<R>(O, C, nap, t1, v, S.tr_id()[a]);
         ++nap;
       }
     }
@@ -997,6 +1034,34 @@ __device__ __noinline__ int run_afterpulses(const SipmK<R>& K, SipmShared<R, CAP
   nap = __shfl_sync(FULL, nap, 0);
   __syncwarp();
   return nap;
+}
+
+// One per lane when there are at most 32, on pixels that differ: then none decides another.
+template <typename R, int CAP, bool LOC>
+__device__ __noinline__ int run_afterpulses(const SipmK<R>& K, SipmShared<R, CAP, LOC> S, SipmCtx C,
+                                            const SipmOut& O) {
+  const int lane = lane_id();
+  const bool on = lane < C.ntr;
+  const R t = on ? S.tr_t()[lane & (S.TCAP - 1)] : R(0);
+  const int q = on ? int(S.tr_pix()[lane & (S.TCAP - 1)]) : 0;
+  const unsigned same = __match_any_sync(FULL, on ? q : -1 - lane);
+  if (C.ntr > 32 || __any_sync(FULL, on && (same & (same - 1u)) != 0u)) return afterpulses_serial(K, S, C, O);
+  R v = R(0);
+  bool fire = false;
+  if (on && !(t > K.t_end)) {
+    v = recovered_from<R>(K, t, S.last(q));        // its pixel has fired
+    fire = S.tr_uf()[lane] < pfire<R>(K, v);
+  }
+  const unsigned fm = __ballot_sync(FULL, fire);
+  int pos = 0;                                     // fired before it in (time, schedule) order
+#pragma unroll 1
+  for (unsigned m = fm; m; m &= m - 1u) {
+    const int j = __ffs(m) - 1;
+    const R tj = __shfl_sync(FULL, t, j);
+    pos += tj < t || (tj == t && j < lane);
+  }
+  if (fire) put_charge<R>(O, C, pos, t, v, S.tr_id()[lane]);
+  return __popc(fm);
 }
 
 // Order-preserving integer image of an FP64 time, -0 taken as +0 (as the numeric comparison does): FP64 sort
@@ -1056,25 +1121,43 @@ __device__ __noinline__ void sort_photons(SipmShared<R, CAP, LOC> S, int n) {
   }
 }
 
-// Warps per block.  20 warps of the first pass (11 KB of shared memory each, FP32) fit an SM, as two blocks of 102
-// registers a thread; the later passes have room for 11 warps or fewer, in one block.
-__host__ __device__ constexpr int sipm_block_warps(int cap) { return cap <= 256 ? 10 : 16; }
+// Errors of a SiPM: more charges than slots, a key limit (limit > 0), more photons than the last pass takes (limit < 0).
+static __device__ __noinline__ void sipm_report(Status* status, int charges, int cap, int photons, int limit) {
+  if (limit < 0) {
+    set_flag(status, CRV_ST_CAPACITY);
+    need_at_least(status, CRV_NEED_PHOTONS_PER_SIPM, photons);
+    return;
+  }
+  if (charges > cap) {
+    set_flag(status, CRV_ST_CAPACITY);
+    const long long per = photons > 0 ? (charges - 16 + photons - 1) / photons : 1;
+    need_at_least(status, CRV_NEED_CHARGE_FACTOR, per < 1 ? 1 : per);
+  }
+  if (limit) set_flag(status, CRV_ST_LIMIT);
+}
+
+// Warps per block.  First pass: 24 warps of 8.8 KB of shared memory fit an SM in FP32, as two blocks of 80 registers a
+// thread (20 warps of 96 registers: 29.2 instead of 27.3 ms for 65,536 events); 20 of 11.2 KB in FP64 (24 with their
+// spills: 2.28 instead of 2.12 ms for 1,500 events).  The later passes have room for 11 warps or fewer, in one block.
+template <typename R>
+__host__ __device__ constexpr int sipm_block_warps(int cap) { return cap > 256 ? 16 : sizeof(R) == 4 ? 12 : 10; }
 
 // draw key of photon i of a group that starts at row a
+template <bool LOC>
 __device__ __forceinline__ uint32_t draw_key(const SipmGroups& G, long long a, int i) {
-  return G.key32 ? G.key32[a + i] : G.key64 ? uint32_t(G.key64[a + i]) : uint32_t(i);
+  if constexpr (!LOC) return G.key32[a + i];       // the chain's own photons
+  else return G.key64 ? uint32_t(G.key64[a + i]) : uint32_t(i);
 }
 
 // SiPM stage over photon groups (PT: storage type of the photon times)
 template <typename R, typename PT, int CAP, bool LOC>
-__global__ void __launch_bounds__(sipm_block_warps(CAP) * 32, CAP <= 256 ? 2 : 1) k_sipm_sim(const __grid_constant__ CrvParams p, CrvPixels px, SipmGroups G,
+__global__ void __launch_bounds__(sipm_block_warps<R>(CAP) * 32, CAP <= 256 ? 2 : 1) k_sipm_sim(const __grid_constant__ CrvParams p, CrvPixels px, SipmGroups G,
                                                  const PT* __restrict__ ph_time, int lo, int last_pass,
                                                  const __grid_constant__ SipmOut O, Status* status) {
-  constexpr int cap = CAP;
   __shared__ uint32_t dead[64];
   __shared__ SipmK<R> K;
   for (int i = threadIdx.x; i < 64; i += blockDim.x) dead[i] = i < DEAD_WORDS ? px.dead_bits[i] : 0u;
-  if (threadIdx.x == 0) K = sipm_consts<R>(p);
+  if (threadIdx.x == 0) sipm_consts<R>(p, K);
   __syncthreads();
   const SipmShared<R, CAP, LOC> S{warp_in_block() * SipmShared<R, CAP, LOC>::BYTES};
   for (int q = 0; q < 2; ++q)
@@ -1106,10 +1189,9 @@ __global__ void __launch_bounds__(sipm_block_warps(CAP) * 32, CAP <= 256 ? 2 : 1
     C.nq = 0;
     C.ntr = 0;
     C.limit = 0;
-    if (cnt > cap) {
+    if (cnt > CAP) {
       if (lane_id() == 0 && last_pass) {
-        set_flag(status, CRV_ST_CAPACITY);
-        need_at_least(status, CRV_NEED_PHOTONS_PER_SIPM, cnt);
+        sipm_report(status, 0, 0, cnt, -1);
         O.nmain[g] = 0; O.nap[g] = 0; O.fired[g] = 0;
       }
       continue;
@@ -1122,7 +1204,7 @@ __global__ void __launch_bounds__(sipm_block_warps(CAP) * 32, CAP <= 256 ? 2 : 1
     uint32_t kn = 0;
     if (lane_id() < cnt) {
       tn = ph_time[a + lane_id()];
-      kn = draw_key(G, a, lane_id());
+      kn = draw_key<LOC>(G, a, lane_id());
     }
 #pragma unroll 1
     for (int base = 0; base < cnt; base += 32) {
@@ -1131,7 +1213,7 @@ __global__ void __launch_bounds__(sipm_block_warps(CAP) * 32, CAP <= 256 ? 2 : 1
       const uint32_t kv = kn;
       if (i + 32 < cnt) {
         tn = ph_time[a + i + 32];
-        kn = draw_key(G, a, i + 32);
+        kn = draw_key<LOC>(G, a, i + 32);
       }
       bool keep;
       if constexpr (sizeof(PT) == 4) keep = i < cnt && (float(tv) <= K.t_end_dn);
@@ -1171,12 +1253,7 @@ __global__ void __launch_bounds__(sipm_block_warps(CAP) * 32, CAP <= 256 ? 2 : 1
       O.nmain[g] = C.nq;
       O.nap[g] = nap;
       O.fired[g] = fired;
-      if (C.nq + nap > C.cap) {
-        set_flag(status, CRV_ST_CAPACITY);
-        long long per = cnt > 0 ? (C.nq + nap - 16 + cnt - 1) / cnt : 1;
-        need_at_least(status, CRV_NEED_CHARGE_FACTOR, per < 1 ? 1 : per);
-      }
-      if (C.limit) set_flag(status, CRV_ST_LIMIT);
+      if (C.nq + nap > C.cap || C.limit) sipm_report(status, C.nq + nap, C.cap, cnt, C.limit);
     }
     __syncwarp();
    }

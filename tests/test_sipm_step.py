@@ -66,3 +66,24 @@ def test_step_edges_bit_exact(pixel_id, where, cross_talk):
     for c in ("chan", "time", "charge", "pe", "photon"):
         assert np.array_equal(G[c], Qo[c]), c
     assert np.array_equal(G["_group_fired"], nfp) and np.array_equal(G["_group_charges"], nq)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_charge_factor_takes_the_time_per_pixel_pass(precision):
+    """More charge slots per photon (charge_factor) send every SiPM to the passes that keep a time per pixel: same charges
+    as the first pass's times per record."""
+    from crvgpu import response as R
+    from crvgpu.params import make_params
+    from tests.helpers import workload
+    geom, cond, cfg, steps = workload(40, seed=8)
+    cfg.precision = precision
+    ds, tabs = R.upload_steps(steps, nbars=geom.nbars), R.DeviceTables(geom, cond, cfg)
+    out = []
+    for factor in (1, 3):
+        P = make_params(cfg, 9, charge_factor=factor)
+        r = R.ResponseEngine().run(P, ds, tabs)
+        out.append([getattr(r, k).cpu().numpy() for k in ("label", "time", "charge", "pe", "photon")])
+    assert len(out[0][0]) > 1000
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
