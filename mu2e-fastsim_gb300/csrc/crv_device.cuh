@@ -187,6 +187,26 @@ __device__ __forceinline__ float d2f_trunc(double x) {
   return __uint_as_float(u);
 }
 
+// Correctly rounded a / b from y = 1 / b rounded to nearest (Markstein, "Computation of elementary functions on the IBM
+// RISC System/6000 processor", 1990): a quotient within an ulp, its exact remainder, one correction; the first
+// correction makes sure of the ulp.  Five FP64 instructions instead of a division's dozen; for operands far from the ends
+// of the exponent range.
+__device__ __forceinline__ double quotient(double a, double b, double y) {
+  double q = a * y;
+  q = __fma_rn(__fma_rn(-q, b, a), y, q);
+  return __fma_rn(__fma_rn(-q, b, a), y, q);
+}
+
+// x > y on integers (false with a NaN): an FP64 compare issues on the FP64 pipe
+__device__ __forceinline__ bool above(double x, double y) {
+  const unsigned long long ux = (unsigned long long)__double_as_longlong(x), uy = (unsigned long long)__double_as_longlong(y);
+  const unsigned long long ax = ux << 1, ay = uy << 1;
+  if (ax > 0xFFE0000000000000ull || ay > 0xFFE0000000000000ull) return false;
+  const long long kx = (ux >> 63) ? -(long long)(ax >> 1) : (long long)(ax >> 1);
+  const long long ky = (uy >> 63) ? -(long long)(ay >> 1) : (long long)(ay >> 1);
+  return kx > ky;
+}
+
 // finite and non-zero, tested on the bits
 __device__ __forceinline__ bool finite_nonzero(double x) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(x);

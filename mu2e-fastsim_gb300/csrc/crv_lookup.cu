@@ -224,14 +224,6 @@ struct SubRow {
   int bb, bth;
 };
 
-// correctly rounded a / b from y = 1 / b rounded, operands far from the ends of the exponent range (Markstein's corrections,
-// see div_by in crv_pulsefit.cuh)
-__device__ __forceinline__ double quotient(double a, double b, double y) {
-  double q = a * y;
-  q = __fma_rn(__fma_rn(-q, b, a), y, q);
-  return __fma_rn(__fma_rn(-q, b, a), y, q);
-}
-
 // Geometry and bins of substep k of a row (photons.py:139-196).  The scintillator's hole and the fibres are tested only
 // inside their bounding boxes: outside, ex or ey is at least 1 and so is ex^2 + ey^2, and a radius is at least the
 // larger of its two distances, in rounded arithmetic too (rounding is monotone).

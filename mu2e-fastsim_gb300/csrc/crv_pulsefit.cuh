@@ -50,16 +50,12 @@ __device__ __forceinline__ double round_half_away(double x) {
 __device__ __forceinline__ unsigned long long abs_bits(double x) {
   return (unsigned long long)__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFull;
 }
-// Correctly rounded a / b from y = 1 / b rounded to nearest (Markstein, "Computation of elementary functions on the IBM
-// RISC System/6000 processor", 1990): a quotient within an ulp, its exact remainder, one correction; the first
-// correction makes sure of the ulp.  Five FP64 instructions instead of a division's dozen.  Operands outside
-// 2^-500 .. 2^500 (quotient and remainder could leave the normal range; zero) take the division.
+// a / b from y = 1 / b rounded (quotient); operands outside 2^-500 .. 2^500 (quotient and remainder could leave the normal
+// range; zero) take the division
 __device__ __forceinline__ double div_by(double a, double b, double y) {
   const int ea = int((abs_bits(a) >> 52)), eb = int((abs_bits(b) >> 52));
   if (unsigned(eb - 523) > 1000u || unsigned(ea - 523) > 1000u) return a / b;
-  double q = a * y;
-  q = __fma_rn(__fma_rn(-q, b, a), y, q);
-  return __fma_rn(__fma_rn(-q, b, a), y, q);
+  return quotient(a, b, y);
 }
 
 // whether |x| > |y| (false with a NaN, as the floating-point compare)

@@ -56,14 +56,9 @@ __device__ __forceinline__ double tdc0_of(const CrvParams& p, const CrvChannels&
 __device__ __forceinline__ int reach_samples(const CrvParams& p) { return int(ceil(p.spe_max_time / p.period)) + 2; }
 
 // first sample a charge at time t reaches in a cluster starting at ts
-template <typename R>
 __device__ __forceinline__ long long first_sample(const CrvParams& p, double t, double ts) {
-  if (sizeof(R) == 8) {
-    double v = ceil((t - ts) / p.period);
-    return v > 0.0 ? (long long)v : 0;
-  }
-  float v = ceilf(float(t - ts) / float(p.period));
-  return v > 0.0f ? (long long)v : 0;
+  double v = ceil((t - ts) / p.period);
+  return v > 0.0 ? (long long)v : 0;
 }
 
 // x / d, exactly: a multiplication by 1/d when d is a power of two (the quotient rounds identically), else a division
@@ -74,18 +69,11 @@ __device__ __forceinline__ double exact_div(double x, double d) {
 }
 
 // template index of sample J for a charge at t (returns -1 when the pair does not contribute)
-template <typename R>
 __device__ __forceinline__ int tmpl_index(const CrvParams& p, long long J, double t, double ts, int tlen) {
-  if (sizeof(R) == 8) {
-    double st = double(J) * p.period + ts - t;
-    if (!(st >= 0.0)) return -1;
-    double ti = rint(exact_div(st, p.spe_precision));
-    return ti < double(tlen) ? int(ti) : -1;
-  }
-  float st = float(J) * float(p.period) - float(t - ts);
-  if (!(st >= 0.0f)) return -1;
-  float ti = rintf(st / float(p.spe_precision));
-  return ti < float(tlen) ? int(ti) : -1;
+  double st = double(J) * p.period + ts - t;
+  if (!(st >= 0.0)) return -1;
+  double ti = rint(exact_div(st, p.spe_precision));
+  return ti < double(tlen) ? int(ti) : -1;
 }
 
 // FP32-mixed forms on dt = t - t_start (one FP64 subtraction per charge, then FP32)
@@ -135,98 +123,264 @@ __device__ __forceinline__ void window_bounds(const CrvParams& p, double ts, int
   *hi_o = int(d);
 }
 
-// cluster_length for one thread (charges a..b-1 in turn); nr = reach_samples(p), ip = 1 / template precision
-template <typename R>
-__device__ __forceinline__ int cluster_length_serial(const CrvParams& p, const double* t, int a, int b, double ts,
-                                                     int tlen, int nr, float ip) {
-  long long est = (long long)floor((t[b - 1] - t[a] + p.spe_max_time) / p.period);
-  long long used = 0;
-  const float Pf = float(p.period);
-  for (int q = a; q < b; ++q) {
-    if (sizeof(R) == 8) {
-      long long j0 = first_sample<R>(p, t[q], ts);
-      for (int k = nr - 1; k >= 0; --k) {
-        if (tmpl_index<R>(p, j0 + k, t[q], ts, tlen) >= 0) {
-          if (j0 + k + 1 > used) used = j0 + k + 1;
-          break;
-        }
-      }
-    } else {
-      float dt = float(t[q] - ts);
-      int j0 = first_sample_f(dt, Pf);
-      for (int k = nr - 1; k >= 0; --k) {
-        if (tmpl_index_f(j0 + k, dt, Pf, ip, tlen) >= 0) {
-          if (j0 + k + 1 > used) used = j0 + k + 1;
-          break;
-        }
-      }
-    }
+constexpr int WF_FX = 32;                      // fractional bits of fixed-point times
+
+// trunc(x * 2^32) for |x| < 2^30; false for non-finite or larger values
+__device__ __forceinline__ bool d2fx(double x, long long* out) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+  const int e = int((b >> 52) & 0x7FF);
+  if (e == 0x7FF || e >= 1023 + 30) return false;
+  if (e < 1023 - WF_FX - 1) {                  // |x| < 2^-33: below the resolution
+    *out = 0;
+    return true;
   }
-  return int(est > used ? est : used);
+  const unsigned long long m = (b & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull;
+  const int sh = e - 1075 + WF_FX;             // in [-54, 10]
+  const unsigned long long v = sh >= 0 ? (m << sh) : (m >> (-sh));
+  *out = (b >> 63) ? -(long long)v : (long long)v;
+  return true;
 }
 
-// Per group, one thread each (the per-cluster FP64 scalars are then computed once per cluster, not by a whole
-// warp): TDC0, the kept clusters (into cl[group start + k]), the digi bound (sum over kept clusters of
-// ceil(length / samples_zs)) and the longest kept cluster.
-template <typename R>
-__global__ void __launch_bounds__(256) k_wf_prepass(CrvParams p, CrvChannels ch, WfGroups G,
-                                                    const double* __restrict__ time, const double* __restrict__ tmpl,
-                                                    int tlen, const double* __restrict__ tdc0_rows,
-                                                    double* __restrict__ g_tdc0, int32_t* __restrict__ g_bound,
-                                                    int32_t* __restrict__ g_maxlen, int32_t* __restrict__ g_nkept,
-                                                    WfCluster* __restrict__ cl) {
-  __shared__ double vmax_s;
-  if (threadIdx.x < 32) {
-    double v = -1e300;
-    for (int i = threadIdx.x; i < tlen; i += 32) v = fmax(v, tmpl[i]);
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-    if (threadIdx.x == 0) vmax_s = v;
-  }
+// order-preserving unsigned key of a double's bits (larger key = larger value), so a maximum over a table is
+// integer work: a warp-wide FP64 instruction costs ~60-70 FP32 issue slots on this GPU
+__device__ __forceinline__ unsigned long long dkey(double x) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+  return (b >> 63) ? ~b : (b | 0x8000000000000000ull);
+}
+__device__ __forceinline__ double dkey_value(unsigned long long k) {
+  return __longlong_as_double((long long)((k >> 63) ? (k & 0x7FFFFFFFFFFFFFFFull) : ~k));
+}
+
+// the template's maximum (NaN entries ignored, as fmax does) by every thread of the block; call from all threads
+__device__ __forceinline__ double block_tmpl_max(const double* tmpl, int tlen, unsigned long long* slot) {
+  if (threadIdx.x == 0) *slot = dkey(-1e300);
   __syncthreads();
-  const double vmax = vmax_s;
-  const double gap = p.spe_max_time + 4.0 * p.period;
-  const int nr = reach_samples(p);
-  const float ip = float(1.0 / p.spe_precision);
+  unsigned long long m = dkey(-1e300);
+  for (int i = threadIdx.x; i < tlen; i += blockDim.x) {
+    const double v = tmpl[i];
+    const unsigned long long k = dkey(v);
+    if (v == v && k > m) m = k;
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    const unsigned long long x = __shfl_xor_sync(0xffffffffu, m, o);
+    if (x > m) m = x;
+  }
+  if (lane_id() == 0) atomicMax(slot, m);
+  __syncthreads();
+  return dkey_value(*slot);
+}
+
+// Cluster starts waiting for a warp's lanes, and the totals of the tile's groups.
+constexpr int PREP_QUEUE = 96;
+struct PrepQueue {
+  int first[PREP_QUEUE];         // first charge of the cluster in its group
+  uint8_t group[PREP_QUEUE];     // its group in the tile
+  int nk[32], bound[32], maxlen[32];
+};
+
+// The prepass of both precisions (Prep: Prep32, Prep64): the groups' kept clusters, TDC0, digi bounds and longest
+// clusters.  Warps take tiles of groups: lanes over the groups (TDC0), over each group's charges (cluster starts), then
+// over the clusters of all the tile's groups, which wait in a shared queue.
+template <typename Prep>
+__global__ void __launch_bounds__(256, 3) k_wf_prep(CrvParams p, CrvChannels ch, WfGroups G,
+                                                 const double* __restrict__ time, const double* __restrict__ tmpl,
+                                                 int tlen, const double* __restrict__ tdc0_rows,
+                                                 double* __restrict__ g_tdc0, int32_t* __restrict__ g_bound,
+                                                 int32_t* __restrict__ g_maxlen, int32_t* __restrict__ g_nkept,
+                                                 typename Prep::Record* __restrict__ cl, Status* status) {
+  __shared__ PrepQueue queue[8];
+  __shared__ typename Prep::Consts K_s;
+  __shared__ unsigned long long vmax_s;
+  const double vmax = block_tmpl_max(tmpl, tlen, &vmax_s);
+  if (threadIdx.x == 0) K_s = Prep::consts(p, vmax);           // FP64 scalars once per block, in one thread
+  __syncthreads();
+  const typename Prep::Consts& K = K_s;
+  if (Prep::LIMIT && (!Prep::ok(K) || tlen > 1024)) {
+    if (threadIdx.x == 0 && blockIdx.x == 0) set_flag(status, CRV_ST_LIMIT);
+    return;
+  }
   const int zs = p.samples_zs;
+  const int lane = lane_id();
+  const unsigned lt = (1u << lane) - 1u;
+  PrepQueue& Q = queue[warp_in_block()];
   const long long ng = *G.n;
-  for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < ng; g += (long long)gridDim.x * blockDim.x) {
-    const int n = G.count[g];
-    const long long q0 = G.start[g];
-    const double* t = time + q0;
-    // keyed TDC0 of the group, unless the caller gives one per cluster (then the channel tables are not read)
-    const double tdc0 = tdc0_rows ? 0.0 : tdc0_of(p, ch, G.label[g], G.run ? G.run[g] : 0u);
-    long long bound = 0;
-    int maxlen = 0, nk = 0;
-    for (int a = 0; a < n;) {
-      int b = a + 1;
-      while (b < n && !(t[b] - t[b - 1] > gap)) ++b;
-      if (double(b - a) * vmax >= p.min_voltage) {
-        const double tdc0c = tdc0_rows ? tdc0_rows[q0 + a] : tdc0;
-        const long long k0 = (long long)ceil((t[a] - p.period - tdc0c) / p.period);
-        const double ts = cluster_ts(k0, p.period, tdc0c);
-        const int L = cluster_length_serial<R>(p, t, a, b, ts, tlen, nr, ip);
-        bound += (L + zs - 1) / zs;
-        maxlen = L > maxlen ? L : maxlen;
-        int ilo = 0, ihi = -1;
-        if (L <= 16384) window_bounds(p, ts, L, &ilo, &ihi);
-        cl[q0 + nk] = WfCluster{ts, k0, a, b, L, int16_t(ilo), int16_t(ihi)};
-        ++nk;
-      }
-      a = b;
+  const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
+  const int tile = tile_size(ng, warps);
+  for (long long g0 = (blockIdx.x * (long long)(blockDim.x >> 5) + warp_in_block()) * tile; g0 < ng; g0 += warps * tile) {
+    // lane = group of the tile: its rows and its keyed TDC0 (unless the caller gives one per cluster)
+    const int ntile = int(min((long long)tile, ng - g0));
+    const long long gl = g0 + lane;
+    int n_l = 0;
+    long long q0_l = 0;
+    typename Prep::Tdc0 tdc0_l = 0;
+    if (lane < ntile) {
+      n_l = G.count[gl];
+      q0_l = G.start[gl];
+      if (!tdc0_rows) tdc0_l = Prep::tdc0(p, ch, K, G.label[gl], G.run ? G.run[gl] : 0u);
     }
-    g_tdc0[g] = tdc0;
-    g_bound[g] = int32_t(bound);
-    g_maxlen[g] = maxlen;
-    g_nkept[g] = nk;
+    Q.nk[lane] = 0;
+    Q.bound[lane] = 0;
+    Q.maxlen[lane] = 0;
+    __syncwarp();
+    // The clusters queued in Q (start rows, in order), the first `full` of them with known ends: keep rule, start tick,
+    // length, window range, digi bound, one cluster per lane.
+    auto clusters = [&](int cnt, int full) {
+#pragma unroll 1
+      for (int base = 0; base < full; base += 32) {
+        const int e = base + lane;
+        const bool on = e < full;
+        const int gi = on ? Q.group[e] : 0, a = on ? Q.first[e] : 0;
+        const int gn = e + 1 < cnt ? int(Q.group[e + 1]) : -1;
+        const int n = __shfl_sync(0xffffffffu, n_l, gi);
+        const long long q0 = __shfl_sync(0xffffffffu, q0_l, gi);
+        const typename Prep::Tdc0 tdc0g = __shfl_sync(0xffffffffu, tdc0_l, gi);
+        const int b = on && gn == gi ? Q.first[e + 1] : n;
+        const bool keep = on && Prep::keep(p, K, b - a);
+        typename Prep::Record rec{};
+        int L = 0;
+        if (keep) {
+          const typename Prep::Tdc0 tdc0 = tdc0_rows ? Prep::caller_tdc0(tdc0_rows[q0 + a], status) : tdc0g;
+          rec = Prep::record(p, K, time + q0, a, b, tdc0, tlen);
+          L = rec.L;
+        }
+        const unsigned mine = __match_any_sync(0xffffffffu, on ? gi : 32 + lane);
+        const unsigned km = __ballot_sync(0xffffffffu, keep);
+        if (keep) cl[q0 + Q.nk[gi] + __popc(km & mine & lt)] = rec;
+        __syncwarp();
+        if (keep) {
+          if ((km & mine & lt) == 0u) Q.nk[gi] += __popc(km & mine);
+          atomicAdd(&Q.bound[gi], (L + zs - 1) / zs);
+          atomicMax(&Q.maxlen[gi], L);
+        }
+        __syncwarp();
+      }
+    };
+    // cluster starts of every group: a new cluster where consecutive fixed-point times differ by more than the gap
+    int cnt = 0, gi = 0, base = 0, n = __shfl_sync(0xffffffffu, n_l, 0);
+    long long q0 = __shfl_sync(0xffffffffu, q0_l, 0), prev = 0;
+    unsigned bad = 0;
+    bool odd = false, prev_ok = false;
+#pragma unroll 1
+    while (true) {
+      if (gi < ntile && base >= n) {               // next group
+        if (Prep::LIMIT && __any_sync(0xffffffffu, odd)) {
+          bad |= 1u << gi;
+          if (lane == 0) set_flag(status, CRV_ST_LIMIT);
+        }
+        odd = false;
+        ++gi;
+        base = 0;
+        n = __shfl_sync(0xffffffffu, n_l, gi & 31);
+        q0 = __shfl_sync(0xffffffffu, q0_l, gi & 31);
+        if (gi < ntile && n <= 0) continue;
+      }
+      const bool end = gi >= ntile;
+      if (end || cnt > PREP_QUEUE - 32) {          // all clusters, or those with known ends to make room for 32 more
+        clusters(cnt, end ? cnt : cnt - 1);
+        if (end) break;
+        const int f = Q.first[cnt - 1];
+        const uint8_t q = Q.group[cnt - 1];
+        __syncwarp();
+        if (lane == 0) { Q.first[0] = f; Q.group[0] = q; }
+        cnt = 1;
+        __syncwarp();
+      }
+      const int q = base + lane;
+      long long tf = 0;
+      const bool known = q < n && d2fx(time[q0 + q], &tf);
+      odd |= q < n && !known;
+      long long tp = __shfl_up_sync(0xffffffffu, tf, 1);
+      const unsigned okm = __ballot_sync(0xffffffffu, known);
+      bool pk = (okm >> ((lane + 31) & 31)) & 1u;
+      if (lane == 0) { tp = prev; pk = prev_ok; }
+      const bool isnew = q < n && (q == 0 || Prep::is_new(K, tf, tp, known && pk, time + q0 + q));
+      const unsigned m = __ballot_sync(0xffffffffu, isnew);
+      if (isnew) {
+        const int at = cnt + __popc(m & lt);
+        Q.first[at] = q;
+        Q.group[at] = uint8_t(gi);
+      }
+      cnt += __popc(m);
+      prev = __shfl_sync(0xffffffffu, tf, 31);
+      prev_ok = okm >> 31;
+      base += 32;
+      __syncwarp();
+    }
+    __syncwarp();
+    if (lane < ntile) {
+      const bool drop = (bad >> lane) & 1u;
+      g_bound[gl] = drop ? 0 : Q.bound[lane];
+      g_maxlen[gl] = drop ? 0 : Q.maxlen[lane];
+      g_nkept[gl] = drop ? 0 : Q.nk[lane];
+      g_tdc0[gl] = drop ? 0.0 : Prep::tdc0_value(tdc0_l);
+    }
+    __syncwarp();
   }
 }
 
+// FP64 form of the prepass.  The gap test on consecutive times is decided on fixed-point copies (2^-32 ns, truncated)
+// unless they lie within a few units of the gap; everything else runs once per cluster, 32 clusters at a time.
+struct Prep64 {
+  using Record = WfCluster;
+  static constexpr bool LIMIT = false;
+  struct Consts {
+    double vmax, gap;
+    long long gap_fx;
+    int nr, gap_ok;
+  };
+  static __device__ __forceinline__ Consts consts(const CrvParams& p, double vmax) {
+    Consts K;
+    K.vmax = vmax;
+    K.gap = p.spe_max_time + 4.0 * p.period;
+    K.nr = reach_samples(p);
+    K.gap_ok = d2fx(K.gap, &K.gap_fx);
+    return K;
+  }
+  static __device__ __forceinline__ bool ok(const Consts&) { return true; }
+  static __device__ __forceinline__ bool is_new(const Consts& K, long long tf, long long tp, bool known,
+                                                const double* t) {
+    if (known && K.gap_ok) {
+      const long long d = tf - tp - K.gap_fx;      // within 2 units of the difference
+      if (d > 4 || d < -4) return d > 0;
+    }
+    return t[0] - t[-1] > K.gap;
+  }
+  static __device__ __forceinline__ bool keep(const CrvParams& p, const Consts& K, int n) {
+    return double(n) * K.vmax >= p.min_voltage;
+  }
+  using Tdc0 = double;
+  static __device__ __forceinline__ double tdc0(const CrvParams& p, const CrvChannels& ch, const Consts&,
+                                                long long label, uint32_t run) {
+    return tdc0_of(p, ch, label, run);
+  }
+  static __device__ __forceinline__ double caller_tdc0(double x, Status*) { return x; }
+  static __device__ __forceinline__ double tdc0_value(double v) { return v; }
+  static __device__ __forceinline__ WfCluster record(const CrvParams& p, const Consts& K, const double* t, int a, int b,
+                                                     double tdc0, int tlen) {
+    const long long k0 = (long long)ceil((t[a] - p.period - tdc0) / p.period);
+    const double ts = cluster_ts(k0, p.period, tdc0);
+    const long long est = (long long)floor((t[b - 1] - t[a] + p.spe_max_time) / p.period);
+    // the last charge reaches the last sample: a later charge's sample times are no larger, so its reach is no shorter
+    long long used = 0;
+    const long long j0 = first_sample(p, t[b - 1], ts);
+#pragma unroll 1
+    for (int k = K.nr - 1; k >= 0; --k)
+      if (tmpl_index(p, j0 + k, t[b - 1], ts, tlen) >= 0) {
+        used = j0 + k + 1;
+        break;
+      }
+    const int L = int(est > used ? est : used);
+    int ilo = 0, ihi = -1;
+    if (L <= 16384) window_bounds(p, ts, L, &ilo, &ihi);
+    return WfCluster{ts, k0, a, b, L, int16_t(ilo), int16_t(ihi)};
+  }
+};
 
 constexpr int WF_QSTAGE = 512;    // charges of a cluster staged in shared memory (larger clusters: on the fly)
+constexpr int WF_TMPL = 1024;     // template entries kept in shared memory (longer templates: from global memory)
 
-template <typename R>
 __host__ __device__ inline size_t wf_smem_per_warp(int cap) {
-  return (size_t(cap) * sizeof(R) + size_t(WF_QSTAGE) * (sizeof(R) + 8) + 15) & ~size_t(15);
+  return (size_t(cap) * 8 + size_t(WF_QSTAGE) * 16 + 15) & ~size_t(15);
 }
 
 __device__ __forceinline__ int16_t adc_of(const CrvParams& p, double v) {
@@ -255,8 +409,79 @@ __device__ __forceinline__ int16_t adc_of_f(const CrvParams& p, float v, float c
   return int16_t(r);
 }
 
+#if defined(CRV_REAL_IS_FLOAT) && !CRV_REAL_IS_FLOAT    // the FP64 kernels' unit
+// Synthesis in FP64 without FP64 decisions.  A warp-wide FP64 instruction takes 19 cycles of the whole SM, so only the
+// arithmetic whose rounding is the result (sample sums, noise, volts, start times) is FP64; what a comparison or a
+// rounding to an integer decides is decided on fixed-point copies where that is certain, and by the FP64 form elsewhere:
+//   first sample  ceil((t - ts) / P) from t - ts in units of 2^-32 ns, unless it lies within j + 8 units of a sample;
+//   template index rint((J P + ts - t) / precision) and the sign of the time, from 32-bit differences in 2^-20 ns (a
+//                 charge of the sample's range lies within the template's length, so the differences fit; both
+//                 terms truncated, J P within J 2^-32: 7 units at most; the FP32 quotient within 2^-22), unless within
+//                 four times those errors of a half (4e-4 here) or 16 units of 0;
+//   ADC           truncation of v conversion + pedestal + 1/2, from FP32 unless within 0.01 of an integer.
+// 1,500 events: synthesis 5.9 -> 2.9 ms, of which the noise normals are a third, prepass (Prep64) 2.9 -> 0.5 ms.
+struct WfFixed {
+  long long P;                   // period, 2^-32 ns
+  float P_ns, inv_P;
+  double inv_ref;                // 1 / reference charge, rounded
+  float unit, half;              // 2^-20 ns in template steps; 1/2 less the index quotient's error
+  float conv, off;
+  int plain;                     // settings outside the fixed-point forms' range: FP64 forms only
+};
+
+__device__ __forceinline__ WfFixed wf_fixed(const CrvParams& p) {
+  WfFixed F;
+  const double reach = p.spe_max_time + 3.0 * p.period;
+  F.plain = !d2fx(p.period, &F.P) || !(p.period > 0.5) || !(p.spe_max_time >= 0.0 && reach < 1000.0) ||
+            !(p.spe_precision > 0.0 && reach / p.spe_precision < 4000.0) || !(fabs(p.adc_conversion) < 1e6) ||
+            !(fabs(double(p.adc_pedestal)) < 8000.0);
+  F.P_ns = float(p.period);
+  F.inv_P = float(1.0 / p.period);
+  F.inv_ref = 1.0 / p.spe_ref_charge;
+  F.unit = float(0x1p-20 / p.spe_precision);
+  F.half = 0.5f - 4.0f * (float(reach / p.spe_precision) * 0x1p-22f + 16.0f * F.unit);
+  F.conv = float(p.adc_conversion);
+  F.off = float(double(p.adc_pedestal) + 0.5);
+  return F;
+}
+
+// first sample of a charge whose time from the cluster start is x (2^-32 ns), given where that is certain
+__device__ __forceinline__ bool first_sample_fx(const WfFixed& F, long long x, int* j) {
+  if (x <= -16) { *j = 0; return true; }
+  if (x < 16 || x > (1ll << 50)) return false;
+  long long k = (long long)(__int2float_rn(int(x >> 32)) * F.inv_P);    // floor estimate, within a sample or two
+  while (k * F.P > x) --k;
+  while ((k + 1) * F.P <= x) ++k;
+  const long long r = x - k * F.P, tol = k + 8;                          // in [0, P)
+  if (r < tol || F.P - r < tol) return false;
+  *j = int(k) + 1;
+  return true;
+}
+
+__device__ __forceinline__ int16_t adc_near(const CrvParams& p, const WfFixed& F, double v) {
+  if (!F.plain) {
+    const float x = fmaf(d2f_trunc(v), F.conv, F.off), t = truncf(x), d = fabsf(x - t);
+    // value, conversion and offset in FP32: within 2^-22 of |v conversion| + |off|, 4e-3 below 16,000
+    if (fabsf(x) < 8000.0f && d > 0.01f && d < 0.99f) {
+      int r = int(t);
+      if (r < p.min_adc) r = p.min_adc;
+      if (r > p.max_adc) r = p.max_adc;
+      return int16_t(r);
+    }
+  }
+  return adc_of(p, v);
+}
+
+// normal of one sample: the pair of the block, only the half that is used
+__device__ __noinline__ double noise_normal(U4 w, int odd) {
+  const double u1 = u01_open(w.x, w.y), u2 = u01(w.z, w.w);
+  const double r = sqrt(-2.0 * dlog(u1));
+  double s, c;
+  dsincospi(2.0 * u2, &s, &c);
+  return r * (odd ? s : c);
+}
+
 // Synthesis + zero suppression of the groups whose longest kept cluster is in (lo, cap].
-template <typename R>
 __global__ void __launch_bounds__(256, 3) k_wf_synth(CrvParams p, WfGroups G, const double* __restrict__ time,
                                                   const double* __restrict__ charge, const double* __restrict__ tmpl,
                                                   int tlen, const double* __restrict__ tdc0_rows,
@@ -266,29 +491,30 @@ __global__ void __launch_bounds__(256, 3) k_wf_synth(CrvParams p, WfGroups G, co
                                                   const WfCluster* __restrict__ cl, int lo, int cap, int last_pass,
                                                   DigiSlots D, Status* status) {
   extern __shared__ __align__(16) char smem[];
-  char* wbase = smem + size_t(warp_in_block()) * wf_smem_per_warp<R>(cap);
-  R* wave = reinterpret_cast<R*>(wbase);
-  R* qn_s = reinterpret_cast<R*>(wbase + size_t(cap) * sizeof(R));
-  int32_t* j0_s = reinterpret_cast<int32_t*>(wbase + size_t(cap) * sizeof(R) + size_t(WF_QSTAGE) * sizeof(R));
-  float* dt_s = reinterpret_cast<float*>(wbase + size_t(cap) * sizeof(R) + size_t(WF_QSTAGE) * (sizeof(R) + 4));
-  __shared__ float tmpl_f[1024];
-  if (sizeof(R) == 4)
-    for (int i = threadIdx.x; i < tlen && i < 1024; i += blockDim.x) tmpl_f[i] = float(tmpl[i]);
+  char* wbase = smem + size_t(warp_in_block()) * wf_smem_per_warp(cap);
+  double* wave = reinterpret_cast<double*>(wbase);
+  double* qn_s = reinterpret_cast<double*>(wbase + size_t(cap) * 8);
+  int32_t* j0_s = reinterpret_cast<int32_t*>(wbase + size_t(cap) * 8 + size_t(WF_QSTAGE) * 8);
+  int32_t* dt_s = j0_s + WF_QSTAGE;                // t - ts in 2^-20 ns, modulo 2^32
+  __shared__ double tmpl_s[WF_TMPL];
+  __shared__ WfFixed F_s;
+  for (int i = threadIdx.x; i < tlen && i < WF_TMPL; i += blockDim.x) tmpl_s[i] = tmpl[i];
+  if (threadIdx.x == 0) F_s = wf_fixed(p);
   __syncthreads();
+  const WfFixed& F = F_s;
+  const double* tm = tlen <= WF_TMPL ? tmpl_s : tmpl;
   const int nr = reach_samples(p);
   const int zs = p.samples_zs;
-  const float Pf = float(p.period), ip = float(1.0 / p.spe_precision);
-  const R inv_q = R(1.0 / p.spe_ref_charge);
-  const R vthr = R(p.min_voltage);
-  const R sigma = R(p.noise_sigma);
-  const float conv_f = float(p.adc_conversion), off_f = float(double(p.adc_pedestal) + 0.5);
+  const double vthr = p.min_voltage;
+  const double sigma = p.noise_sigma;
+  const int lane = lane_id();
   long long ng = *G.n;
   long long warps = (long long)gridDim.x * (blockDim.x >> 5);
   for (long long g = blockIdx.x * (long long)(blockDim.x >> 5) + warp_in_block(); g < ng; g += warps) {
     int ml = g_maxlen[g];
     if (ml <= lo) continue;
     if (ml > cap) {
-      if (last_pass && lane_id() == 0) {
+      if (last_pass && lane == 0) {
         set_flag(status, CRV_ST_CAPACITY);
         need_at_least(status, CRV_NEED_SAMPLES, ml);
       }
@@ -313,24 +539,29 @@ __global__ void __launch_bounds__(256, 3) k_wf_synth(CrvParams p, WfGroups G, co
       const long long k0 = C.k0;
       const double ts = C.ts;
       const double tdc0c = tdc0_rows ? tdc0_rows[q0 + a] : tdc0;
-      // stage each charge's first reached sample and normalised charge (once per charge, not per sample)
+      // stage each charge's first reached sample, time from the cluster start and normalised charge
       const bool staged = (b - a) <= WF_QSTAGE;
+      bool fixed = staged && !F.plain;
       if (staged) {
-        for (int q = a + lane_id(); q < b; q += 32) {
-          if (sizeof(R) == 8) {
-            j0_s[q - a] = int32_t(first_sample<R>(p, t[q], ts));
-            qn_s[q - a] = R(qc[q] / p.spe_ref_charge);
-          } else {
-            float dt = float(t[q] - ts);
-            dt_s[q - a] = dt;
-            j0_s[q - a] = first_sample_f(dt, Pf);
-            qn_s[q - a] = R(d2f_trunc(qc[q])) * inv_q;        // FP32-stage charges: exact FP32 values
-          }
+        for (int q = a + lane; q < b; q += 32) {
+          const double tq = t[q];
+          long long x = 0;
+          const bool fx = d2fx(tq - ts, &x);
+          int j = 0;
+          if (!fx || F.plain || !first_sample_fx(F, x, &j)) j = int32_t(first_sample(p, tq, ts));
+          j0_s[q - a] = j;
+          dt_s[q - a] = int32_t(x >> 12);
+          fixed = fixed && fx;
+          const double qq = qc[q];
+          const int e = int((__double_as_longlong(qq) >> 52) & 0x7FF);
+          qn_s[q - a] = unsigned(e - 723) < 600u && F.inv_ref > 1e-90 && F.inv_ref < 1e90
+                            ? quotient(qq, p.spe_ref_charge, F.inv_ref) : qq / p.spe_ref_charge;
         }
+        fixed = __all_sync(0xffffffffu, fixed);
         __syncwarp();
       }
       // samples: sum of the charges reaching each sample, in charge order
-      for (int j = lane_id(); j < L; j += 32) {
+      for (int j = lane; j < L; j += 32) {
         // charges with first_sample in (j - nr, j]: first_sample is non-decreasing along the cluster.  The staged
         // and the on-the-fly searches are separate loops, so the staged one carries no FP64 work.
         int q1, lo2;
@@ -351,34 +582,38 @@ __global__ void __launch_bounds__(256, 3) k_wf_synth(CrvParams p, WfGroups G, co
           int lo_q = a, hi_q = b;
           while (lo_q < hi_q) {
             int m = (lo_q + hi_q) >> 1;
-            if (first_sample<R>(p, t[m], ts) > (long long)j - nr) hi_q = m; else lo_q = m + 1;
+            if (first_sample(p, t[m], ts) > (long long)j - nr) hi_q = m; else lo_q = m + 1;
           }
           q1 = lo_q;
           int hi2 = b;
           lo2 = q1;
           while (lo2 < hi2) {
             int m = (lo2 + hi2) >> 1;
-            if (first_sample<R>(p, t[m], ts) > (long long)j) hi2 = m; else lo2 = m + 1;
+            if (first_sample(p, t[m], ts) > (long long)j) hi2 = m; else lo2 = m + 1;
           }
         }
-        R acc = R(0);
-        if (sizeof(R) == 4 && staged) {
+        double acc = 0.0;
+        if (fixed) {
+          const int32_t JP = int32_t(((long long)j * F.P) >> 12);
+#pragma unroll 1
           for (int q = q1; q < lo2; ++q) {
-            int ti = tmpl_index_f(j, dt_s[q - a], Pf, ip, tlen);
-            if (ti >= 0) acc += R(tmpl_f[ti]) * qn_s[q - a];
+            const int32_t st = int32_t(uint32_t(JP) - uint32_t(dt_s[q - a]));
+            const float x = float(st) * F.unit;
+            const float r = rintf(x);
+            int ti = int(r);
+            if (st < 16 || fabsf(x - r) > F.half) ti = st < -16 ? -1 : tmpl_index(p, j, t[q], ts, tlen);
+            if (ti >= 0 && ti < tlen) acc += tm[ti] * qn_s[q - a];
           }
         } else {
           for (int q = q1; q < lo2; ++q) {
-            int ti = tmpl_index<R>(p, j, t[q], ts, tlen);
-            if (ti >= 0) acc += R(tmpl[ti]) * (staged ? qn_s[q - a] : R(qc[q] / p.spe_ref_charge));
+            int ti = tmpl_index(p, j, t[q], ts, tlen);
+            if (ti >= 0) acc += tm[ti] * (staged ? qn_s[q - a] : qc[q] / p.spe_ref_charge);
           }
         }
         if (p.noise_on) {
           long long tk = k0 + j;
           U4 w = keyed(p.seed, ek, (ST_NOISE << 28) | (chan & 0x7FFFu), uint32_t(tk >> 1));
-          R z0, z1;
-          Math<R>::normal_pair(w, &z0, &z1);
-          acc = acc + sigma * ((tk & 1) ? z1 : z0);
+          acc = acc + sigma * noise_normal(w, int(tk & 1));
         }
         wave[j] = acc;
       }
@@ -387,12 +622,12 @@ __global__ void __launch_bounds__(256, 3) k_wf_synth(CrvParams p, WfGroups G, co
       // zero suppression over chunks of 32 samples
       int next_i = 0;
       for (int base = 0; base < L; base += 32) {
-        int i = base + lane_id();
+        int i = base + lane;
         bool w = false;
         if (i < L) {
           for (int d = -2; d <= 2 && !w; ++d) {
             int k = i + d;
-            if (k >= 0 && k < L && wave[k] > vthr) w = true;
+            if (k >= 0 && k < L && above(wave[k], vthr)) w = true;
           }
         }
         bool inwin = i >= i_lo && i <= i_hi;
@@ -405,19 +640,13 @@ __global__ void __launch_bounds__(256, 3) k_wf_synth(CrvParams p, WfGroups G, co
           // emit digi at i0; its start TDC (start - TDC0) / P is the integer tick k0 + i0
           if (nd < scap) {
             long long o = slot + nd;
-            if (lane_id() < zs) {
-              int c = i0 + lane_id();
-              if constexpr (sizeof(R) == 4) {
-                const float v = c < L ? float(wave[c]) : 0.0f;
-                if (D.volt) D.volt[o * zs + lane_id()] = f2d(v);
-                D.adc[o * zs + lane_id()] = adc_of_f(p, v, conv_f, off_f);
-              } else {
-                double v = c < L ? double(wave[c]) : 0.0;
-                if (D.volt) D.volt[o * zs + lane_id()] = v;
-                D.adc[o * zs + lane_id()] = adc_of(p, v);
-              }
+            if (lane < zs) {
+              int c = i0 + lane;
+              double v = c < L ? wave[c] : 0.0;
+              if (D.volt) D.volt[o * zs + lane] = v;
+              D.adc[o * zs + lane] = adc_near(p, F, v);
             }
-            if (lane_id() == 0) {
+            if (lane == 0) {
               D.chan[o] = lab;
               D.start[o] = __dadd_rn(ts, __dmul_rn(double(i0), p.period));
               D.tdc0[o] = tdc0c;
@@ -430,12 +659,14 @@ __global__ void __launch_bounds__(256, 3) k_wf_synth(CrvParams p, WfGroups G, co
       }
       __syncwarp();
     }
-    if (lane_id() == 0) {
+    if (lane == 0) {
       D.n[g] = nd;
       if (nd > scap) set_flag(status, CRV_ST_CAPACITY);
     }
   }
 }
+
+#endif
 
 }  // namespace crv
 

@@ -14,7 +14,7 @@
 //                FP32 sums widened exactly; ADC as the FP32 stage rule (adc_of_f).
 //
 // Two kernels, one warp per SiPM group each:
-//   k_wf_prep32   a tile of groups per warp: lanes over the groups (TDC0), over each group's charges (cluster split by
+//   k_wf_prep     (crv_waveform.cuh) a tile of groups per warp: lanes over the groups (TDC0), over each group's charges (cluster split by
 //                 the gap test on consecutive fixed-point times, ballots), then over the clusters of all the tile's
 //                 groups, which wait in a shared queue: keep rule, start tick, length, window sample range, digi
 //                 bound; kept clusters are written to cl[group start + k] (the record layout of WfCluster, with the
@@ -28,24 +28,6 @@
 #include "crv_waveform.cuh"
 
 namespace crv {
-
-constexpr int WF_FX = 32;                      // fractional bits of fixed-point times
-
-// trunc(x * 2^32) for |x| < 2^30; false for non-finite or larger values
-__device__ __forceinline__ bool d2fx(double x, long long* out) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
-  const int e = int((b >> 52) & 0x7FF);
-  if (e == 0x7FF || e >= 1023 + 30) return false;
-  if (e < 1023 - WF_FX - 1) {                  // |x| < 2^-33: below the resolution
-    *out = 0;
-    return true;
-  }
-  const unsigned long long m = (b & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull;
-  const int sh = e - 1075 + WF_FX;             // in [-54, 10]
-  const unsigned long long v = sh >= 0 ? (m << sh) : (m >> (-sh));
-  *out = (b >> 63) ? -(long long)v : (long long)v;
-  return true;
-}
 
 // v * 2^-32 as FP32: integer part and fraction converted separately, one final rounding
 __device__ __forceinline__ float fx2f(long long v) {
@@ -98,35 +80,6 @@ struct WfFx {                   // per-launch constants of the fixed-point forms
   bool ok;
 };
 
-// order-preserving unsigned key of a double's bits (larger key = larger value), so a maximum over a table is
-// integer work: a warp-wide FP64 instruction costs ~60-70 FP32 issue slots on this GPU
-__device__ __forceinline__ unsigned long long dkey(double x) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
-  return (b >> 63) ? ~b : (b | 0x8000000000000000ull);
-}
-__device__ __forceinline__ double dkey_value(unsigned long long k) {
-  return __longlong_as_double((long long)((k >> 63) ? (k & 0x7FFFFFFFFFFFFFFFull) : ~k));
-}
-
-// the template's maximum (NaN entries ignored, as fmax does) by every thread of the block; call from all threads
-__device__ __forceinline__ double block_tmpl_max(const double* tmpl, int tlen, unsigned long long* slot) {
-  if (threadIdx.x == 0) *slot = dkey(-1e300);
-  __syncthreads();
-  unsigned long long m = dkey(-1e300);
-  for (int i = threadIdx.x; i < tlen; i += blockDim.x) {
-    const double v = tmpl[i];
-    const unsigned long long k = dkey(v);
-    if (v == v && k > m) m = k;
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    const unsigned long long x = __shfl_xor_sync(0xffffffffu, m, o);
-    if (x > m) m = x;
-  }
-  if (lane_id() == 0) atomicMax(slot, m);
-  __syncthreads();
-  return dkey_value(*slot);
-}
-
 __device__ __forceinline__ WfFx wf_fx_consts(const CrvParams& p, double vmax) {
   WfFx f;
   f.ok = d2fx(p.period, &f.P) && d2fx(p.spe_max_time + 4.0 * p.period, &f.gap) && d2fx(p.spe_max_time, &f.maxt) &&
@@ -151,177 +104,65 @@ struct WfCluster32 {
 };
 static_assert(sizeof(WfCluster32) == sizeof(WfCluster), "FP32 cluster record layout");
 
-// Cluster starts waiting for a warp's lanes, and the totals of the tile's groups.
-constexpr int PREP_QUEUE = 96;
-struct PrepQueue {
-  int first[PREP_QUEUE];         // first charge of the cluster in its group
-  uint8_t group[PREP_QUEUE];     // its group in the tile
-  int nk[32], bound[32], maxlen[32];
+// FP32 form of the prepass (k_wf_prep): fixed-point times, cluster records with the fixed-point start
+struct Prep32 {
+  using Record = WfCluster32;
+  static constexpr bool LIMIT = true;          // times beyond the fixed-point range are refused
+  struct Consts {
+    WfFx F;
+    float ip, Pf;
+    int nr;
+  };
+  static __device__ __forceinline__ Consts consts(const CrvParams& p, double vmax) {
+    return Consts{wf_fx_consts(p, vmax), float(1.0 / p.spe_precision), float(p.period), reach_samples(p)};
+  }
+  static __device__ __forceinline__ bool ok(const Consts& K) { return K.F.ok; }
+  static __device__ __forceinline__ bool is_new(const Consts& K, long long tf, long long tp, bool, const double*) {
+    return tf - tp > K.F.gap;
+  }
+  static __device__ __forceinline__ bool keep(const CrvParams&, const Consts& K, int n) { return n >= K.F.nmin; }
+  using Tdc0 = long long;
+  static __device__ __forceinline__ long long tdc0(const CrvParams& p, const CrvChannels& ch, const Consts& K,
+                                                   long long label, uint32_t run) {
+    return tdc0_fx_of(p, ch, label, run, K.F.width);
+  }
+  static __device__ __forceinline__ long long caller_tdc0(double x, Status* status) {
+    long long v = 0;
+    if (!d2fx(x, &v)) {
+      set_flag(status, CRV_ST_LIMIT);
+      v = 0;
+    }
+    return v;
+  }
+  static __device__ __forceinline__ double tdc0_value(long long v) { return fx2d(v); }
+  static __device__ __forceinline__ WfCluster32 record(const CrvParams&, const Consts& K, const double* t, int a, int b,
+                                                       long long tdc0, int tlen) {
+    const WfFx& F = K.F;
+    long long tf, tl;
+    d2fx(t[a], &tf);
+    d2fx(t[b - 1], &tl);
+    const long long k0 = fx_ceil_div(tf - F.P - tdc0, F.P, F.invP);
+    const long long ts = k0 * F.P + tdc0;
+    const long long est = fx_floor_div(tl - tf + F.maxt, F.P, F.invP);
+    // the last charge reaches the last sample (the reach only grows with the charge time)
+    const float dt = fx2f(tl - ts);
+    long long used = 0;
+    const int j0 = first_sample_f(dt, K.Pf);
+    for (int k = K.nr - 1; k >= 0; --k)
+      if (tmpl_index_f(j0 + k, dt, K.Pf, K.ip, tlen) >= 0) {
+        used = j0 + k + 1;
+        break;
+      }
+    const int L = int(est > used ? est : used);
+    int ilo = 0, ihi = -1;
+    if (L <= 16384) {
+      const long long last = ts + (long long)(L - 1) * F.P;
+      ilo = ts >= F.wlo ? 0 : int(min((long long)L, fx_ceil_div(F.wlo - ts, F.P, F.invP)));
+      ihi = last <= F.whi ? L - 1 : int(max(-1ll, fx_floor_div(F.whi - ts, F.P, F.invP)));
+    }
+    return WfCluster32{ts, k0, a, b, L, int16_t(ilo), int16_t(ihi)};
+  }
 };
-
-__global__ void __launch_bounds__(256) k_wf_prep32(CrvParams p, CrvChannels ch, WfGroups G,
-                                                   const double* __restrict__ time, const double* __restrict__ tmpl,
-                                                   int tlen, const double* __restrict__ tdc0_rows,
-                                                   double* __restrict__ g_tdc0, int32_t* __restrict__ g_bound,
-                                                   int32_t* __restrict__ g_maxlen, int32_t* __restrict__ g_nkept,
-                                                   WfCluster32* __restrict__ cl, Status* status) {
-  __shared__ PrepQueue queue[8];
-  __shared__ WfFx fx_s;
-  __shared__ unsigned long long vmax_s;
-  __shared__ float ip_s, pf_s;
-  __shared__ int nr_s;
-  const double vmax = block_tmpl_max(tmpl, tlen, &vmax_s);
-  if (threadIdx.x == 0) {                      // FP64 scalars once per block, in one thread
-    fx_s = wf_fx_consts(p, vmax);
-    ip_s = float(1.0 / p.spe_precision);
-    pf_s = float(p.period);
-    nr_s = reach_samples(p);
-  }
-  __syncthreads();
-  const WfFx F = fx_s;
-  if (!F.ok || tlen > 1024) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) set_flag(status, CRV_ST_LIMIT);
-    return;
-  }
-  const int nr = nr_s;
-  const int zs = p.samples_zs;
-  const float Pf = pf_s, ip = ip_s;
-  const int lane = lane_id();
-  const unsigned lt = (1u << lane) - 1u;
-  PrepQueue& Q = queue[warp_in_block()];
-  const long long ng = *G.n;
-  const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
-  const int tile = tile_size(ng, warps);
-  for (long long g0 = (blockIdx.x * (long long)(blockDim.x >> 5) + warp_in_block()) * tile; g0 < ng; g0 += warps * tile) {
-    // lane = group of the tile: its rows and its keyed TDC0 (unless the caller gives one per cluster)
-    const int ntile = int(min((long long)tile, ng - g0));
-    const long long gl = g0 + lane;
-    int n_l = 0;
-    long long q0_l = 0, tdc0_l = 0;
-    if (lane < ntile) {
-      n_l = G.count[gl];
-      q0_l = G.start[gl];
-      if (!tdc0_rows) tdc0_l = tdc0_fx_of(p, ch, G.label[gl], G.run ? G.run[gl] : 0u, F.width);
-    }
-    Q.nk[lane] = 0;
-    Q.bound[lane] = 0;
-    Q.maxlen[lane] = 0;
-    __syncwarp();
-    // The clusters queued in Q (start rows, in order), the first `full` of them with known ends: keep rule, start tick,
-    // length, window range, digi bound, one cluster per lane.
-    auto clusters = [&](int cnt, int full) {
-#pragma unroll 1
-      for (int base = 0; base < full; base += 32) {
-        const int e = base + lane;
-        const bool on = e < full;
-        const int gi = on ? Q.group[e] : 0, a = on ? Q.first[e] : 0;
-        const int gn = e + 1 < cnt ? int(Q.group[e + 1]) : -1;
-        const int n = __shfl_sync(0xffffffffu, n_l, gi);
-        const long long q0 = __shfl_sync(0xffffffffu, q0_l, gi), tdc0g = __shfl_sync(0xffffffffu, tdc0_l, gi);
-        const int b = on && gn == gi ? Q.first[e + 1] : n;
-        const bool keep = on && (b - a) >= F.nmin;
-        WfCluster32 rec{};
-        int L = 0;
-        if (keep) {
-          long long tdc0 = tdc0g;
-          if (tdc0_rows && !d2fx(tdc0_rows[q0 + a], &tdc0)) {
-            set_flag(status, CRV_ST_LIMIT);
-            tdc0 = 0;
-          }
-          long long tf, tl;
-          d2fx(time[q0 + a], &tf);
-          d2fx(time[q0 + b - 1], &tl);
-          const long long k0 = fx_ceil_div(tf - F.P - tdc0, F.P, F.invP);
-          const long long ts = k0 * F.P + tdc0;
-          const long long est = fx_floor_div(tl - tf + F.maxt, F.P, F.invP);
-          // the last charge reaches the last sample (the reach only grows with the charge time)
-          const float dt = fx2f(tl - ts);
-          long long used = 0;
-          const int j0 = first_sample_f(dt, Pf);
-          for (int k = nr - 1; k >= 0; --k)
-            if (tmpl_index_f(j0 + k, dt, Pf, ip, tlen) >= 0) {
-              used = j0 + k + 1;
-              break;
-            }
-          L = int(est > used ? est : used);
-          int ilo = 0, ihi = -1;
-          if (L <= 16384) {
-            const long long last = ts + (long long)(L - 1) * F.P;
-            ilo = ts >= F.wlo ? 0 : int(min((long long)L, fx_ceil_div(F.wlo - ts, F.P, F.invP)));
-            ihi = last <= F.whi ? L - 1 : int(max(-1ll, fx_floor_div(F.whi - ts, F.P, F.invP)));
-          }
-          rec = WfCluster32{ts, k0, a, b, L, int16_t(ilo), int16_t(ihi)};
-        }
-        const unsigned mine = __match_any_sync(0xffffffffu, on ? gi : 32 + lane);
-        const unsigned km = __ballot_sync(0xffffffffu, keep);
-        if (keep) cl[q0 + Q.nk[gi] + __popc(km & mine & lt)] = rec;
-        __syncwarp();
-        if (keep) {
-          if ((km & mine & lt) == 0u) Q.nk[gi] += __popc(km & mine);
-          atomicAdd(&Q.bound[gi], (L + zs - 1) / zs);
-          atomicMax(&Q.maxlen[gi], L);
-        }
-        __syncwarp();
-      }
-    };
-    // cluster starts of every group: a new cluster where consecutive fixed-point times differ by more than the gap
-    int cnt = 0, gi = 0, base = 0, n = __shfl_sync(0xffffffffu, n_l, 0);
-    long long q0 = __shfl_sync(0xffffffffu, q0_l, 0), prev = 0;
-    unsigned bad = 0;
-    bool odd = false;
-#pragma unroll 1
-    while (true) {
-      if (gi < ntile && base >= n) {               // next group
-        if (__any_sync(0xffffffffu, odd)) {
-          bad |= 1u << gi;
-          if (lane == 0) set_flag(status, CRV_ST_LIMIT);
-        }
-        odd = false;
-        ++gi;
-        base = 0;
-        n = __shfl_sync(0xffffffffu, n_l, gi & 31);
-        q0 = __shfl_sync(0xffffffffu, q0_l, gi & 31);
-        if (gi < ntile && n <= 0) continue;
-      }
-      const bool end = gi >= ntile;
-      if (end || cnt > PREP_QUEUE - 32) {          // all clusters, or those with known ends to make room for 32 more
-        clusters(cnt, end ? cnt : cnt - 1);
-        if (end) break;
-        const int f = Q.first[cnt - 1];
-        const uint8_t q = Q.group[cnt - 1];
-        __syncwarp();
-        if (lane == 0) { Q.first[0] = f; Q.group[0] = q; }
-        cnt = 1;
-        __syncwarp();
-      }
-      const int q = base + lane;
-      long long tf = 0;
-      if (q < n) odd |= !d2fx(time[q0 + q], &tf);
-      long long tp = __shfl_up_sync(0xffffffffu, tf, 1);
-      if (lane == 0) tp = prev;
-      const bool isnew = q < n && (q == 0 || tf - tp > F.gap);
-      const unsigned m = __ballot_sync(0xffffffffu, isnew);
-      if (isnew) {
-        const int at = cnt + __popc(m & lt);
-        Q.first[at] = q;
-        Q.group[at] = uint8_t(gi);
-      }
-      cnt += __popc(m);
-      prev = __shfl_sync(0xffffffffu, tf, 31);
-      base += 32;
-      __syncwarp();
-    }
-    __syncwarp();
-    if (lane < ntile) {
-      const bool drop = (bad >> lane) & 1u;
-      g_bound[gl] = drop ? 0 : Q.bound[lane];
-      g_maxlen[gl] = drop ? 0 : Q.maxlen[lane];
-      g_nkept[gl] = drop ? 0 : Q.nk[lane];
-      g_tdc0[gl] = drop ? 0.0 : fx2d(tdc0_l);
-    }
-    __syncwarp();
-  }
-}
 
 constexpr int WF32_QS = 256;      // charges staged per chunk (per warp)
 
