@@ -953,7 +953,11 @@ __global__ void __launch_bounds__(32, 16) k_coinc(const __grid_constant__ CrvPar
       if (H > hcap) break;
     }
     if (H > hcap) {
-      if (lane_id() == 0) deferred[e] = 1;
+      if (lane_id() == 0) {
+        deferred[e] = 1;
+        O.ncl[e] = 0;
+        O.nmem[e] = 0;
+      }
       continue;
     }
     __syncwarp();
@@ -961,6 +965,7 @@ __global__ void __launch_bounds__(32, 16) k_coinc(const __grid_constant__ CrvPar
     for (int ti = 0; ti < G.ntypes; ++ti)
       finder_type<false>(p, G, S, W, H, ti, r0, np_, O, ncl_ev, nmem_ev);
     if (lane_id() == 0) {
+      deferred[e] = 0;
       O.ncl[e] = ncl_ev;
       O.nmem[e] = nmem_ev;
     }
@@ -1055,7 +1060,6 @@ __global__ void __launch_bounds__(CO_GWARPS * 32) k_coinc_global(const __grid_co
       if (lane_id() == 0) {
         O.ncl[e] = ncl;
         O.nmem[e] = nmem;
-        deferred[e] = 0;
         if (ncl > np_ || nmem > np_) set_flag(status, CRV_ST_LIMIT);
       }
     }

@@ -73,51 +73,6 @@ Mark::~Mark() {
   cudaEventRecord(g_prof[slot].b, stream);
 }
 
-__global__ void k_scan_parts(long long* __restrict__ part, long long nb, long long* __restrict__ total) {
-  // single block: running exclusive scan over chunks of blockDim.x
-  __shared__ long long carry;
-  __shared__ long long wsum[32];
-  if (threadIdx.x == 0) carry = 0;
-  __syncthreads();
-  for (long long base = 0; base < nb; base += blockDim.x) {
-    long long i = base + threadIdx.x;
-    long long v = i < nb ? part[i] : 0;
-    int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    long long x = v;
-    for (int o = 1; o < 32; o <<= 1) {
-      long long y = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= o) x += y;
-    }
-    if (lane == 31) wsum[w] = x;
-    __syncthreads();
-    if (w == 0) {
-      long long q = lane < (int)(blockDim.x >> 5) ? wsum[lane] : 0;
-      long long qq = q;
-      for (int o = 1; o < 32; o <<= 1) {
-        long long y = __shfl_up_sync(0xffffffffu, qq, o);
-        if (lane >= o) qq += y;
-      }
-      if (lane < (int)(blockDim.x >> 5)) wsum[lane] = qq - q;
-    }
-    __syncthreads();
-    long long ex = carry + wsum[w] + x - v;
-    if (i < nb) part[i] = ex;
-    __syncthreads();
-    if (threadIdx.x == blockDim.x - 1) carry = ex + v;
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) *total = carry;
-}
-
-__global__ void k_check_caps(const long long* __restrict__ total, long long cap, int need_slot, Status* status) {
-  if (threadIdx.x == 0 && blockIdx.x == 0 && *total > cap) {
-    set_flag(status, CRV_ST_CAPACITY);
-    need_at_least(status, need_slot, *total);
-  }
-}
-
-__global__ void k_copy_i64(const long long* __restrict__ src, long long* __restrict__ dst) { *dst = *src; }
-
 __global__ void k_sipm_diag(const long long* __restrict__ nsipm_dev, long long cap, const long long* __restrict__ label,
                             const int32_t* __restrict__ nphot, const int32_t* __restrict__ fired,
                             int64_t* __restrict__ o_label, int32_t* __restrict__ o_phot, int32_t* __restrict__ o_fired,
@@ -134,10 +89,32 @@ __global__ void k_sipm_diag(const long long* __restrict__ nsipm_dev, long long c
   }
 }
 
-__global__ void k_slot_caps(long long ng, const int32_t* __restrict__ gcount, int factor, int32_t* __restrict__ cap) {
-  for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < ng; g += (long long)gridDim.x * blockDim.x)
+// charge slots per group of photons; *n = ng for the kernels after it; counts cleared (groups without photons keep them)
+__global__ void k_slot_caps(long long ng, const int32_t* __restrict__ gcount, int factor, int32_t* __restrict__ cap,
+                            int32_t* __restrict__ nmain, int32_t* __restrict__ nap, int32_t* __restrict__ fired,
+                            long long* __restrict__ n) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) *n = ng;
+  for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < ng; g += (long long)gridDim.x * blockDim.x) {
     cap[g] = gcount[g] > 0 ? factor * gcount[g] + 16 : 0;
+    nmain[g] = 0;
+    nap[g] = 0;
+    fired[g] = 0;
+  }
 }
+
+// charges per group: main and afterpulse records
+struct ChargeCounts {
+  using V = long long;
+  static constexpr bool FLAG = false;
+  const int32_t *nmain, *nap;
+  long long* off;
+  int32_t* sum;                  // may be null
+  __device__ __forceinline__ long long item(long long i) const { return nmain[i] + nap[i]; }
+  __device__ __forceinline__ void put(long long i, long long v, long long before) const {
+    off[i] = before;
+    if (sum) sum[i] = int32_t(v);
+  }
+};
 
 __global__ void k_fill_step_event(CrvEvents ev, long long nevents, int32_t* __restrict__ step_event) {
   long long warps = (long long)gridDim.x * (blockDim.x >> 5);
@@ -145,14 +122,6 @@ __global__ void k_fill_step_event(CrvEvents ev, long long nevents, int32_t* __re
     long long f = ev.first_step[e];
     for (int i = threadIdx.x & 31; i < ev.nsteps[e]; i += 32) step_event[f + i] = int32_t(e);
   }
-}
-
-__global__ void k_set_i64(long long* __restrict__ dst, long long v) { *dst = v; }
-
-// *out = (*total <= cap) ? *n : 0  (downstream kernels then see no groups)
-__global__ void k_guard_groups(const long long* __restrict__ total, long long cap, const long long* __restrict__ n,
-                               long long* __restrict__ out) {
-  *out = (*total <= cap) ? *n : 0;
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
@@ -173,7 +142,7 @@ struct Carve {
 struct RespWs {
   int32_t *step_event, *step_order, *count, *sipm_count;
   long long* sipm_off;
-  int32_t *s_event, *s_chan, *s_nseg, *nphot, *slot_cap, *nmain, *nap, *fired, *ntot;
+  int32_t *s_event, *s_chan, *s_nseg, *nphot, *slot_cap, *nmain, *nap, *fired;
   long long *s_seg, *id_base, *label, *ph_off, *slot_off, *out_off, *parts, *totals;
   uint32_t* run;
   void* ph_t;
@@ -206,7 +175,6 @@ static RespWs resp_layout(char* base, const CrvParams& p, long long ne, long lon
   w.nmain = c.take<int32_t>(w.nb);
   w.nap = c.take<int32_t>(w.nb);
   w.fired = c.take<int32_t>(w.nb);
-  w.ntot = c.take<int32_t>(w.nb);
   w.s_seg = c.take<long long>(w.nb);
   w.id_base = c.take<long long>(w.nb);
   w.label = c.take<long long>(w.nb);
@@ -374,7 +342,8 @@ static int response_run(const CrvParams* p, const CrvEvents* ev, int64_t nevents
                         int64_t out_cap, int64_t* n_out_dev, int64_t* sipm_label, int32_t* sipm_photons,
                         int32_t* sipm_fired, int64_t sipm_cap, int64_t* n_sipm_dev, void* workspace,
                         int64_t workspace_bytes, void* stream, CrvStatus* status_dev,
-                        const CrvLookupChain* lk = nullptr) {
+                        const CrvLookupChain* lk = nullptr,
+                        long long* photons_dev = nullptr, long long* pass_dev = nullptr) {
   if (!p || !ev || !st || !bars || !ch || !px || !out || !n_out_dev || !status_dev) return CRV_ERR_ARG;
   if (st->real_bytes != 4 && st->real_bytes != 8) return CRV_ERR_ARG;
   if (nevents < 0 || nsteps < 0 || photon_cap < 0 || out_cap < 0 || max_steps_per_event < 0) return CRV_ERR_ARG;
@@ -387,18 +356,11 @@ static int response_run(const CrvParams* p, const CrvEvents* ev, int64_t nevents
   char* base = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(workspace) + 255) & ~uintptr_t(255));
   size_t dummy;
   RespWs w = resp_layout(base, *p, nevents, nsteps, photon_cap, &dummy, lk != nullptr);
-  CK(cudaMemsetAsync(w.totals, 0, 8 * sizeof(long long), s));
   if (nevents == 0 || nsteps == 0) {
     CK(cudaMemsetAsync(n_out_dev, 0, sizeof(long long), s));
     if (n_sipm_dev) CK(cudaMemsetAsync(n_sipm_dev, 0, sizeof(long long), s));
     return CRV_OK;
   }
-  CK(cudaMemsetAsync(w.nphot, 0, sizeof(int32_t) * w.nb, s));
-  CK(cudaMemsetAsync(w.slot_cap, 0, sizeof(int32_t) * w.nb, s));
-  CK(cudaMemsetAsync(w.nmain, 0, sizeof(int32_t) * w.nb, s));
-  CK(cudaMemsetAsync(w.nap, 0, sizeof(int32_t) * w.nb, s));
-  CK(cudaMemsetAsync(w.fired, 0, sizeof(int32_t) * w.nb, s));
-  CK(cudaMemsetAsync(w.ntot, 0, sizeof(int32_t) * w.nb, s));
   // 1. events: steps grouped by bar, SiPM counts; 2. scan; 3. SiPM table
   int stepcap = 1;
   while (stepcap < max_steps_per_event) stepcap <<= 1;
@@ -413,7 +375,7 @@ static int response_run(const CrvParams* p, const CrvEvents* ev, int64_t nevents
                                                   w.sipm_count, nullptr, nullptr, nullptr, nullptr, nullptr, S, 0);
   }
   CK(cudaGetLastError());
-  CK(exclusive_scan(w.sipm_count, nevents, Identity(), w.sipm_off, &w.totals[0], w.parts, s));
+  CK(exclusive_scan(column(w.sipm_count, w.sipm_off), nevents, nullptr, scan_end(&w.totals[0], n_sipm_dev), w.parts, s));
   {
     crv::Mark mark_("k_event_prep", s);
     k_event_prep<<<gp, PREP_THREADS, psmem, s>>>(*ev, nevents, *st, *ch, 1, stepcap, nullptr, nullptr, nullptr,
@@ -434,20 +396,12 @@ static int response_run(const CrvParams* p, const CrvEvents* ev, int64_t nevents
     crv::Mark mark_("k_sipm_sizes", s);
     k_sipm_sizes<<<grid_for(w.nb, 256, 8), 256, 0, s>>>(&w.totals[0], w.s_event, w.s_chan, w.s_seg, w.s_nseg,
                                                         w.step_order, w.count, *ev, factor, w.nphot, w.slot_cap,
-                                                        w.id_base, w.label, w.run);
+                                                        w.id_base, w.label, w.run, w.nmain, w.nap, w.fired);
   }
   CK(cudaGetLastError());
-  CK(exclusive_scan(w.nphot, w.nb, Identity(), w.ph_off, &w.totals[1], w.parts, s, &w.totals[0]));
-  CK(exclusive_scan(w.slot_cap, w.nb, Identity(), w.slot_off, &w.totals[2], w.parts, s, &w.totals[0]));
-  {
-    crv::Mark mark_("k_check_caps", s);
-    k_check_caps<<<1, 32, 0, s>>>(&w.totals[1], w.pc, CRV_NEED_PHOTONS_TOTAL, S);
-  }
-  {
-    crv::Mark mark_("k_check_caps", s);
-    k_check_caps<<<1, 32, 0, s>>>(&w.totals[2], w.sc, CRV_NEED_SLOTS_TOTAL, S);
-  }
-  CK(cudaGetLastError());
+  CK(exclusive_scan(Columns{w.nphot, w.slot_cap, w.ph_off, w.slot_off}, w.nb, &w.totals[0],
+                    ScanEnds{{scan_end(&w.totals[1], photons_dev).check(S, CRV_NEED_PHOTONS_TOTAL, w.pc),
+                              scan_end(&w.totals[2]).check(S, CRV_NEED_SLOTS_TOTAL, w.sc)}}, w.parts, s));
   // 6. photons of every SiPM (lookup model: each row's photons at the offset of its step in its SiPM)
   if (lk) {
     CK(cudaMemsetAsync(w.lk.row_off, 0xFF, sizeof(long long) * size_t(w.nb), s));
@@ -489,16 +443,9 @@ static int response_run(const CrvParams* p, const CrvEvents* ev, int64_t nevents
   else
     CK((launch_sipm<double, double>(*p, *px, G, &w.totals[0], (const double*)w.ph_t, O, S, s)));
   // 8. compaction into label/time order
-  {
-    crv::Mark mark_("k_counts_total", s);
-    k_counts_total<<<grid_for(w.nb, 256, 8), 256, 0, s>>>(&w.totals[0], w.nmain, w.nap, w.ntot);
-  }
-  CK(cudaGetLastError());
-  CK(exclusive_scan(w.ntot, w.nb, Identity(), w.out_off, &w.totals[3], w.parts, s, &w.totals[0]));
-  {
-    crv::Mark mark_("k_check_caps", s);
-    k_check_caps<<<1, 32, 0, s>>>(&w.totals[3], out_cap, CRV_NEED_CHARGES_OUT, S);
-  }
+  CK(exclusive_scan(ChargeCounts{w.nmain, w.nap, w.out_off, nullptr}, w.nb, &w.totals[0],
+                    scan_end(&w.totals[3], n_out_dev).check(S, CRV_NEED_CHARGES_OUT, out_cap).guard(pass_dev, out_cap),
+                    w.parts, s));
   {
     crv::Mark mark_("k_charge_compact", s);
     k_charge_compact<<<grid_for(w.nb, 8, 16), 256, 0, s>>>(&w.totals[0], w.label, w.slot_off, w.slot_cap, w.nmain,
@@ -507,14 +454,6 @@ static int response_run(const CrvParams* p, const CrvEvents* ev, int64_t nevents
                                                             *out, out_cap);
   }
   CK(cudaGetLastError());
-  {
-    crv::Mark mark_("k_copy_i64", s);
-    k_copy_i64<<<1, 1, 0, s>>>(&w.totals[3], reinterpret_cast<long long*>(n_out_dev));
-  }
-  if (n_sipm_dev) {
-    crv::Mark mark_("k_copy_i64", s);
-    k_copy_i64<<<1, 1, 0, s>>>(&w.totals[0], reinterpret_cast<long long*>(n_sipm_dev));
-  }
   if (sipm_label || sipm_photons || sipm_fired)
     {
       crv::Mark mark_("k_sipm_diag", s);
@@ -539,7 +478,7 @@ int crv_response(const CrvParams* p, const CrvEvents* ev, int64_t nevents, const
 
 struct SipmWs {
   long long *slot_off, *out_off, *parts, *totals, *label_dummy;
-  int32_t *slot_cap, *nmain, *nap, *ntot;
+  int32_t *slot_cap, *nmain, *nap;
   double *slot_t, *slot_v;
   long long* slot_id;
   long long sc;
@@ -557,7 +496,6 @@ static SipmWs sipm_layout(char* base, const CrvParams& p, long long ng, long lon
   w.slot_cap = c.take<int32_t>(ng);
   w.nmain = c.take<int32_t>(ng);
   w.nap = c.take<int32_t>(ng);
-  w.ntot = c.take<int32_t>(ng);
   w.slot_t = c.take<double>(w.sc);
   w.slot_v = c.take<double>(w.sc);
   w.slot_id = c.take<long long>(w.sc);
@@ -595,24 +533,14 @@ extern "C" int crv_sipm(const CrvParams* p, const CrvPixels* px, int64_t ngroups
   size_t dummy;
   SipmWs w = sipm_layout(base, *p, ngroups, nph_bound, &dummy);
   int factor = p->charge_factor > 0 ? p->charge_factor : 1;
-  CK(cudaMemsetAsync(w.totals, 0, 8 * sizeof(long long), s));
-  CK(cudaMemsetAsync(w.nmain, 0, sizeof(int32_t) * ngroups, s));
-  CK(cudaMemsetAsync(w.nap, 0, sizeof(int32_t) * ngroups, s));
-  CK(cudaMemsetAsync(g_fired, 0, sizeof(int32_t) * ngroups, s));
-  {
-    crv::Mark mark_("k_set_i64", s);
-    k_set_i64<<<1, 1, 0, s>>>(&w.totals[0], ngroups);
-  }
   {
     crv::Mark mark_("k_slot_caps", s);
-    k_slot_caps<<<grid_for(ngroups, 256, 8), 256, 0, s>>>(ngroups, gcount, factor, w.slot_cap);
+    k_slot_caps<<<grid_for(ngroups, 256, 8), 256, 0, s>>>(ngroups, gcount, factor, w.slot_cap, w.nmain, w.nap, g_fired,
+                                                          &w.totals[0]);
   }
   CK(cudaGetLastError());
-  CK(exclusive_scan(w.slot_cap, ngroups, Identity(), w.slot_off, &w.totals[2], w.parts, s));
-  {
-    crv::Mark mark_("k_check_caps", s);
-    k_check_caps<<<1, 32, 0, s>>>(&w.totals[2], w.sc, CRV_NEED_SLOTS_TOTAL, S);
-  }
+  CK(exclusive_scan(column(w.slot_cap, w.slot_off), ngroups, nullptr,
+                    scan_end(&w.totals[2]).check(S, CRV_NEED_SLOTS_TOTAL, w.sc), w.parts, s));
   SipmGroups G{};
   G.n = &w.totals[0];
   G.guard[0] = &w.totals[2];
@@ -633,16 +561,8 @@ extern "C" int crv_sipm(const CrvParams* p, const CrvPixels* px, int64_t ngroups
     CK((launch_sipm<float, double>(*p, *px, G, &w.totals[0], time, O, S, s)));
   else
     CK((launch_sipm<double, double>(*p, *px, G, &w.totals[0], time, O, S, s)));
-  {
-    crv::Mark mark_("k_counts_total", s);
-    k_counts_total<<<grid_for(ngroups, 256, 8), 256, 0, s>>>(&w.totals[0], w.nmain, w.nap, w.ntot);
-  }
-  CK(cudaGetLastError());
-  CK(exclusive_scan(w.ntot, ngroups, Identity(), w.out_off, &w.totals[3], w.parts, s));
-  {
-    crv::Mark mark_("k_check_caps", s);
-    k_check_caps<<<1, 32, 0, s>>>(&w.totals[3], out_cap, CRV_NEED_CHARGES_OUT, S);
-  }
+  CK(exclusive_scan(ChargeCounts{w.nmain, w.nap, w.out_off, g_charges}, ngroups, nullptr,
+                    scan_end(&w.totals[3], n_out_dev).check(S, CRV_NEED_CHARGES_OUT, out_cap), w.parts, s));
   {
     crv::Mark mark_("k_charge_compact", s);
     k_charge_compact<<<grid_for(ngroups, 8, 16), 256, 0, s>>>(&w.totals[0], G.label, w.slot_off, w.slot_cap, w.nmain,
@@ -651,12 +571,6 @@ extern "C" int crv_sipm(const CrvParams* p, const CrvPixels* px, int64_t ngroups
                                                             *out, out_cap);
   }
   CK(cudaGetLastError());
-  if (g_charges)
-    CK(cudaMemcpyAsync(g_charges, w.ntot, sizeof(int32_t) * ngroups, cudaMemcpyDeviceToDevice, s));
-  {
-    crv::Mark mark_("k_copy_i64", s);
-    k_copy_i64<<<1, 1, 0, s>>>(&w.totals[3], reinterpret_cast<long long*>(n_out_dev));
-  }
   CK(cudaGetLastError());
   return CRV_OK;
 }
@@ -665,9 +579,9 @@ extern "C" int crv_sipm(const CrvParams* p, const CrvPixels* px, int64_t ngroups
 
 namespace crv {
 struct DigiWs {
-  int32_t *head, *gcount, *g_bound, *g_maxlen, *g_nkept, *dn;
-  WfCluster* cl;                 // kept clusters by charge row (shares the group index memory, free after grouping)
-  long long *gidx, *gstart, *glabel, *slot_off, *out_off, *parts, *totals;
+  int32_t *gcount, *g_bound, *g_maxlen, *g_nkept, *dn;
+  WfCluster* cl;                 // kept clusters by charge row
+  long long *gstart, *glabel, *slot_off, *out_off, *parts, *totals;
   uint32_t* grun;
   double* g_tdc0;
   DigiSlots D;
@@ -678,10 +592,7 @@ static DigiWs digi_layout(char* base, long long nq, long long slot_cap, int zs, 
   Carve c{base};
   DigiWs w;
   w.sc = slot_cap;
-  w.head = c.take<int32_t>(nq);
-  static_assert(sizeof(WfCluster) == 4 * sizeof(long long), "cluster record size");
-  w.gidx = c.take<long long>(4 * nq);
-  w.cl = reinterpret_cast<WfCluster*>(w.gidx);
+  w.cl = c.take<WfCluster>(nq);
   w.gstart = c.take<long long>(nq);
   w.glabel = c.take<long long>(nq);
   w.gcount = c.take<int32_t>(nq);
@@ -721,7 +632,8 @@ static int digis_run(const CrvParams* p, const CrvChannels* ch, int64_t ncharges
                      const double* tmpl, int32_t tlen,
                      const int64_t* ev_keys, const uint32_t* ev_runs, int64_t n_events, int64_t slot_cap,
                      CrvDigis* out, int64_t out_cap, int64_t* n_out_dev, void* workspace, int64_t workspace_bytes,
-                     void* stream, CrvStatus* status_dev) {
+                     void* stream, CrvStatus* status_dev,
+                     long long* slots_dev = nullptr, long long* pass_dev = nullptr) {
   if (!p || !ch || !out || !n_out_dev || !status_dev || ncharges < 0 || slot_cap < 0 || out_cap < 0) return CRV_ERR_ARG;
   if (p->samples_zs <= 0 || p->samples_zs > 32 || tlen <= 0 || !tmpl) return CRV_ERR_ARG;
   if (p->precision == 1 && tlen > 1024) return CRV_ERR_ARG;      // FP32-mixed: template copy in shared memory
@@ -740,20 +652,8 @@ static int digis_run(const CrvParams* p, const CrvChannels* ch, int64_t ncharges
   DigiWs w = digi_layout(base, ncharges, slot_cap, p->samples_zs, &dummy);
   if (!out->volt) w.D.volt = nullptr;       // volts not asked for: the slots keep none either
   const long long* lab = reinterpret_cast<const long long*>(label);
-  CK(cudaMemsetAsync(w.totals, 0, 8 * sizeof(long long), s));
-  CK(cudaMemsetAsync(w.g_maxlen, 0, sizeof(int32_t) * ncharges, s));
-  CK(cudaMemsetAsync(w.g_bound, 0, sizeof(int32_t) * ncharges, s));
-  CK(cudaMemsetAsync(w.dn, 0, sizeof(int32_t) * ncharges, s));
   unsigned gq = grid_for(ncharges, 256, 8);
-  {
-    crv::Mark mark_("k_label_heads", s);
-    k_label_heads<<<gq, 256, 0, s>>>(ncharges, nq_dev, lab, w.head);
-  }
-  CK(exclusive_scan(w.head, ncharges, Identity(), w.gidx, &w.totals[0], w.parts, s, nq_dev));
-  {
-    crv::Mark mark_("k_label_groups", s);
-    k_label_groups<<<gq, 256, 0, s>>>(ncharges, nq_dev, lab, w.head, w.gidx, w.gstart, w.glabel);
-  }
+  CK(exclusive_scan(LabelRuns{lab, w.gstart, w.glabel}, ncharges, nq_dev, scan_end(&w.totals[0]), w.parts, s));
   {
     crv::Mark mark_("k_group_counts", s);
     k_group_counts<<<gq, 256, 0, s>>>(&w.totals[0], ncharges, nq_dev, w.gstart, w.glabel, w.gcount,
@@ -763,21 +663,14 @@ static int digis_run(const CrvParams* p, const CrvChannels* ch, int64_t ncharges
   WfGroups G{&w.totals[0], w.gstart, w.gcount, w.glabel, w.grun};
   if (p->precision == 1)
     CK(launch_wf_prepass<float>(*p, *ch, G, ncharges, time, tmpl, tlen, tdc0_rows, w.g_tdc0, w.g_bound,
-                                w.g_maxlen, w.g_nkept, w.cl, S, s));
+                                w.g_maxlen, w.g_nkept, w.dn, w.cl, S, s));
   else
     CK(launch_wf_prepass<double>(*p, *ch, G, ncharges, time, tmpl, tlen, tdc0_rows, w.g_tdc0, w.g_bound,
-                                 w.g_maxlen, w.g_nkept, w.cl, S, s));
-  CK(exclusive_scan(w.g_bound, ncharges, Identity(), w.slot_off, &w.totals[1], w.parts, s, &w.totals[0]));
-  {
-    crv::Mark mark_("k_check_caps", s);
-    k_check_caps<<<1, 32, 0, s>>>(&w.totals[1], slot_cap, CRV_NEED_DIGIS, S);
-  }
-  // synthesis only when the slots fit: guard by zeroing the group count otherwise
-  {
-    crv::Mark mark_("k_guard_groups", s);
-    k_guard_groups<<<1, 32, 0, s>>>(&w.totals[1], slot_cap, &w.totals[0], &w.totals[2]);
-  }
-  CK(cudaGetLastError());
+                                 w.g_maxlen, w.g_nkept, w.dn, w.cl, S, s));
+  // synthesis only when the slots fit: it sees no groups otherwise
+  CK(exclusive_scan(column(w.g_bound, w.slot_off), ncharges, &w.totals[0],
+                    scan_end(&w.totals[1], slots_dev).check(S, CRV_NEED_DIGIS, slot_cap)
+                        .guard(&w.totals[2], slot_cap, &w.totals[0]), w.parts, s));
   G.n = &w.totals[2];
   if (p->precision == 1)
     CK(launch_wf_synth<float>(*p, G, ncharges, time, charge, tmpl, tlen, tdc0_rows, w.g_tdc0, w.g_maxlen,
@@ -785,20 +678,14 @@ static int digis_run(const CrvParams* p, const CrvChannels* ch, int64_t ncharges
   else
     CK(launch_wf_synth<double>(*p, G, ncharges, time, charge, tmpl, tlen, tdc0_rows, w.g_tdc0, w.g_maxlen,
                                w.g_nkept, w.cl, w.D, S, s));
-  CK(exclusive_scan(w.dn, ncharges, Identity(), w.out_off, &w.totals[3], w.parts, s, &w.totals[2]));
-  {
-    crv::Mark mark_("k_check_caps", s);
-    k_check_caps<<<1, 32, 0, s>>>(&w.totals[3], out_cap, CRV_NEED_DIGIS_OUT, S);
-  }
+  CK(exclusive_scan(column(w.dn, w.out_off), ncharges, &w.totals[2],
+                    scan_end(&w.totals[3], n_out_dev).check(S, CRV_NEED_DIGIS_OUT, out_cap).guard(pass_dev, out_cap),
+                    w.parts, s));
   Digis O{reinterpret_cast<long long*>(out->chan), out->start, out->tdc0, reinterpret_cast<long long*>(out->starttdc),
           out->volt, out->adc};
   {
     crv::Mark mark_("k_digi_compact", s);
     k_digi_compact<<<grid_for(ncharges, 8, 16), 256, 0, s>>>(&w.totals[2], w.D, w.out_off, p->samples_zs, O, out_cap);
-  }
-  {
-    crv::Mark mark_("k_copy_i64", s);
-    k_copy_i64<<<1, 1, 0, s>>>(&w.totals[3], reinterpret_cast<long long*>(n_out_dev));
   }
   CK(cudaGetLastError());
   return CRV_OK;
@@ -915,19 +802,27 @@ static PulseWs pulse_layout(char* base, long long nw, long long nsamples, size_t
   return w;
 }
 
-__global__ void k_pulse_caps(long long nw, const long long* __restrict__ nw_dev, const long long* __restrict__ off,
-                             const int32_t* __restrict__ n, long long nsamples, int max_pulses,
-                             int32_t* __restrict__ cap) {
-  nw = bounded_count(nw, nw_dev);
-  for (long long w = blockIdx.x * (long long)blockDim.x + threadIdx.x; w < nw; w += (long long)gridDim.x * blockDim.x) {
-    if (!wave_in_bounds(off[w], n[w], nsamples)) {     // no slots: the fit skips it and reports CRV_ST_BOUNDS
-      cap[w] = 0;
-      continue;
-    }
-    int b = n[w] / 2 + 1;
-    cap[w] = b < max_pulses ? b : max_pulses;
+// record slots of each waveform: at most max_pulses, none for one out of bounds (the fit skips it and reports
+// CRV_ST_BOUNDS)
+struct PulseCaps {
+  using V = long long;
+  static constexpr bool FLAG = false;
+  const long long* off;
+  const int32_t* n;
+  long long nsamples;
+  int max_pulses;
+  int32_t* cap;
+  long long* slot_off;
+  __device__ __forceinline__ long long item(long long w) const {
+    if (!wave_in_bounds(off[w], n[w], nsamples)) return 0;
+    const int b = n[w] / 2 + 1;
+    return b < max_pulses ? b : max_pulses;
   }
-}
+  __device__ __forceinline__ void put(long long w, long long v, long long before) const {
+    cap[w] = int32_t(v);
+    slot_off[w] = before;
+  }
+};
 
 __global__ void k_pulse_compact(long long nw, const long long* __restrict__ nw_dev,
                                 const long long* __restrict__ slot_off, const int32_t* __restrict__ count,
@@ -972,7 +867,8 @@ static int pulses_run(const CrvParams* p, int64_t nw, const long long* nw_dev, i
                       const int32_t* n, const int64_t* start_tdc, const double* ped_db, const double* area,
                       const double* height, const int16_t* adc16, const int64_t* adc64, int32_t max_pulses,
                       CrvPulses* out, int64_t out_cap, int64_t* n_out_dev, uint8_t* wf_near, void* workspace,
-                      int64_t workspace_bytes, void* stream, CrvStatus* status_dev) {
+                      int64_t workspace_bytes, void* stream, CrvStatus* status_dev,
+                      long long* pass_dev = nullptr) {
   if (!p || !out || !n_out_dev || !status_dev || nw < 0 || nsamples < 0 || out_cap < 0 || max_pulses < 0)
     return CRV_ERR_ARG;
   if (nw > 0 && (!off || !n || !start_tdc || !ped_db || !area || !height || !wf_near || (!adc16 == !adc64)))
@@ -989,15 +885,10 @@ static int pulses_run(const CrvParams* p, int64_t nw, const long long* nw_dev, i
   char* base = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(workspace) + 255) & ~uintptr_t(255));
   size_t dummy;
   PulseWs w = pulse_layout(base, nw, nsamples, &dummy);
-  CK(cudaMemsetAsync(w.totals, 0, 8 * sizeof(long long), s));
   CK(cudaMemsetAsync(w.q.counts, 0, (kPulseRoundsMax + 2) * sizeof(long long), s));
   unsigned g = grid_for(nw, 256, 8);
-  {
-    crv::Mark mark_("k_pulse_caps", s);
-    k_pulse_caps<<<g, 256, 0, s>>>(nw, nw_dev, reinterpret_cast<const long long*>(off), n, nsamples, max_pulses,
-                                   w.cap);
-  }
-  CK(exclusive_scan(w.cap, nw, Identity(), w.slot_off, &w.totals[0], w.parts, s, nw_dev));
+  CK(exclusive_scan(PulseCaps{reinterpret_cast<const long long*>(off), n, nsamples, max_pulses, w.cap, w.slot_off}, nw,
+                    nw_dev, scan_end(&w.totals[0]), w.parts, s));
   WaveIn W{nw, nw_dev, reinterpret_cast<const long long*>(off), n, reinterpret_cast<const long long*>(start_tdc), ped_db,
            area, height, adc16, reinterpret_cast<const long long*>(adc64), nsamples};
   PulseSlots PS{w.slot_off, w.cap, w.count, wf_near, w.rec, w.rc};
@@ -1005,18 +896,12 @@ static int pulses_run(const CrvParams* p, int64_t nw, const long long* nw_dev, i
     CK(launch_pulsefit<float>(*p, W, w.yscr, max_pulses, PS, w.q, S, s));
   else
     CK(launch_pulsefit<double>(*p, W, w.yscr, max_pulses, PS, w.q, S, s));
-  CK(exclusive_scan(w.count, nw, Identity(), w.out_off, &w.totals[1], w.parts, s, nw_dev));
-  {
-    crv::Mark mark_("k_check_caps", s);
-    k_check_caps<<<1, 32, 0, s>>>(&w.totals[1], out_cap, CRV_NEED_PULSES_OUT, S);
-  }
+  CK(exclusive_scan(column(w.count, w.out_off), nw, nw_dev,
+                    scan_end(&w.totals[1], n_out_dev).check(S, CRV_NEED_PULSES_OUT, out_cap).guard(pass_dev, out_cap),
+                    w.parts, s));
   {
     crv::Mark mark_("k_pulse_compact", s);
     k_pulse_compact<<<g, 256, 0, s>>>(nw, nw_dev, w.slot_off, w.count, w.out_off, w.rec, *out, out_cap);
-  }
-  {
-    crv::Mark mark_("k_copy_i64", s);
-    k_copy_i64<<<1, 1, 0, s>>>(&w.totals[1], reinterpret_cast<long long*>(n_out_dev));
   }
   CK(cudaGetLastError());
   return CRV_OK;
@@ -1128,10 +1013,6 @@ static int coinc_run(const CrvParams* p, const CrvFinderGeom* g, int64_t nevents
   char* base = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(workspace) + 255) & ~uintptr_t(255));
   size_t dummy;
   CoincWs w = coinc_layout(base, nevents, npulses, &dummy);
-  CK(cudaMemsetAsync(w.totals, 0, 8 * sizeof(long long), s));
-  CK(cudaMemsetAsync(w.ncl, 0, sizeof(int32_t) * nevents, s));
-  CK(cudaMemsetAsync(w.nmem, 0, sizeof(int32_t) * nevents, s));
-  CK(cudaMemsetAsync(w.deferred, 0, sizeof(int32_t) * nevents, s));
   CoincGeom G;
   memcpy(&G, g, sizeof(G));
   CoincIn I{nevents, nev_dev, reinterpret_cast<const long long*>(ev_start), ev_count, bar, sipm, seq, time, pe, status};
@@ -1156,30 +1037,15 @@ static int coinc_run(const CrvParams* p, const CrvFinderGeom* g, int64_t nevents
                                                                                          w.gscratch, S);
   }
   CK(cudaGetLastError());
-  CK(exclusive_scan(w.ncl, nevents, Identity(), w.cl_off, &w.totals[0], w.parts, s, nev_dev));
-  CK(exclusive_scan(w.nmem, nevents, Identity(), w.mem_off, &w.totals[1], w.parts, s, nev_dev));
-  {
-    crv::Mark mark_("k_check_caps", s);
-    k_check_caps<<<1, 32, 0, s>>>(&w.totals[0], cl_cap, CRV_NEED_CLUSTERS, S);
-  }
-  {
-    crv::Mark mark_("k_check_caps", s);
-    k_check_caps<<<1, 32, 0, s>>>(&w.totals[1], mem_cap, CRV_NEED_MEMBERS, S);
-  }
+  CK(exclusive_scan(Columns{w.ncl, w.nmem, w.cl_off, w.mem_off}, nevents, nev_dev,
+                    ScanEnds{{scan_end(&w.totals[0], n_cl_dev).check(S, CRV_NEED_CLUSTERS, cl_cap),
+                              scan_end(&w.totals[1], n_mem_dev).check(S, CRV_NEED_MEMBERS, mem_cap)}}, w.parts, s));
   {
     crv::Mark mark_("k_coinc_compact", s);
     k_coinc_compact<<<grid_for(nevents, 256, 8), 256, 0, s>>>(nevents, nev_dev,
                                                             reinterpret_cast<const long long*>(ev_start),
                                                             reinterpret_cast<const long long*>(ev_key), w.ncl, w.cl_off,
                                                             w.mem_off, w.rec, w.mem_idx, *out, cl_cap, *mem, mem_cap);
-  }
-  {
-    crv::Mark mark_("k_copy_i64", s);
-    k_copy_i64<<<1, 1, 0, s>>>(&w.totals[0], reinterpret_cast<long long*>(n_cl_dev));
-  }
-  {
-    crv::Mark mark_("k_copy_i64", s);
-    k_copy_i64<<<1, 1, 0, s>>>(&w.totals[1], reinterpret_cast<long long*>(n_mem_dev));
   }
   CK(cudaGetLastError());
   return CRV_OK;
@@ -1198,26 +1064,27 @@ extern "C" int crv_coincidences(const CrvParams* p, const CrvFinderGeom* g, int6
 // ---- reco waveforms and pulse glue ---------------------------------------------------------------------------------
 
 namespace crv {
-__global__ void k_wf_heads(long long nd, const long long* __restrict__ nd_dev, const long long* __restrict__ label,
-                           const long long* __restrict__ tdc, int zs, int32_t* __restrict__ head) {
-  nd = bounded_count(nd, nd_dev);
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nd; i += (long long)gridDim.x * blockDim.x)
-    head[i] = (i == 0 || label[i] != label[i - 1] || tdc[i] != tdc[i - 1] + zs) ? 1 : 0;
-}
-
-__global__ void k_wf_fill(long long nd, const long long* __restrict__ nd_dev, const long long* __restrict__ label,
-                          const long long* __restrict__ tdc, int zs, const int32_t* __restrict__ head,
-                          const long long* __restrict__ gidx, CrvChannels ch, long long* __restrict__ w_label,
-                          long long* __restrict__ w_off, int32_t* __restrict__ w_n, long long* __restrict__ w_start,
-                          double* __restrict__ w_ped, double* __restrict__ w_area, double* __restrict__ w_height,
-                          double* __restrict__ w_toff) {
-  nd = bounded_count(nd, nd_dev);
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nd; i += (long long)gridDim.x * blockDim.x) {
-    if (!head[i]) continue;
-    long long g = gidx[i];
+// Waveforms: runs of digis of one channel whose windows follow one another
+struct WaveRuns {
+  using V = long long;
+  static constexpr bool FLAG = true;
+  const long long *label, *tdc;
+  long long nd;                  // bound and device count of the digis (a run ends with the last one)
+  const long long* nd_dev;
+  int zs;
+  CrvChannels ch;
+  long long *w_label, *w_off;
+  int32_t* w_n;
+  long long* w_start;
+  double *w_ped, *w_area, *w_height, *w_toff;
+  __device__ __forceinline__ long long item(long long i) const {
+    return i == 0 || label[i] != label[i - 1] || tdc[i] != tdc[i - 1] + zs;
+  }
+  __device__ __forceinline__ void put(long long i, long long, long long g) const {
+    const long long n = bounded_count(nd, nd_dev);
     long long j = i + 1;
-    while (j < nd && !head[j]) ++j;
-    int c = int(label[i] % 32768);
+    while (j < n && !item(j)) ++j;
+    const int c = int(label[i] % 32768);
     w_label[g] = label[i];
     w_off[g] = i * zs;
     w_n[g] = int32_t((j - i) * zs);
@@ -1227,34 +1094,31 @@ __global__ void k_wf_fill(long long nd, const long long* __restrict__ nd_dev, co
     w_height[g] = ch.pulseheight[c];
     w_toff[g] = ch.timeoffset[c];
   }
-}
+};
 
-__global__ void k_hit_keep(const CrvParams p, const int32_t* __restrict__ status, const long long* __restrict__ w_label,
-                           long long np, const long long* __restrict__ np_dev, const long long* __restrict__ p_wf,
-                           int32_t* __restrict__ keep) {
-  np = bounded_count(np, np_dev);
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < np; i += (long long)gridDim.x * blockDim.x) {
-    int c = int(w_label[p_wf[i]] % 32768);
-    keep[i] = (p.ignore_channels && (status[c] & 0b010)) ? 0 : 1;
+// Hits: the pulses of channels that are not ignored, in order
+struct KeptHits {
+  using V = long long;
+  static constexpr bool FLAG = true;
+  int ignore_channels, use_time_offset_db;
+  double time_offset_scale;
+  const int32_t* status;
+  const long long* w_label;
+  const double *w_toff, *event_t0;
+  const long long *p_wf, *p_seq;
+  const double *p_time, *p_pe;
+  int32_t *bar, *sipm, *seq;
+  double *time, *pe;
+  long long* hev;
+  __device__ __forceinline__ long long item(long long i) const {
+    if (!ignore_channels) return 1;
+    return !(status[int(w_label[p_wf[i]] % 32768)] & 0b010);
   }
-}
-
-__global__ void k_hit_fill(const CrvParams p, const long long* __restrict__ w_label, const double* __restrict__ w_toff,
-                           const double* __restrict__ event_t0, long long np, const long long* __restrict__ np_dev,
-                           const long long* __restrict__ p_wf, const long long* __restrict__ p_seq,
-                           const double* __restrict__ p_time, const double* __restrict__ p_pe,
-                           const int32_t* __restrict__ keep, const long long* __restrict__ kidx,
-                           int32_t* __restrict__ bar, int32_t* __restrict__ sipm, int32_t* __restrict__ seq,
-                           double* __restrict__ time, double* __restrict__ pe, long long* __restrict__ hev) {
-  np = bounded_count(np, np_dev);
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < np; i += (long long)gridDim.x * blockDim.x) {
-    if (!keep[i]) continue;
-    long long k = kidx[i];
-    long long w = p_wf[i];
-    long long lab = w_label[w];
-    int c = int(lab % 32768);
+  __device__ __forceinline__ void put(long long i, long long, long long k) const {
+    const long long w = p_wf[i], lab = w_label[w];
+    const int c = int(lab % 32768);
     double t = p_time[i];
-    if (p.use_time_offset_db) t = t + w_toff[w] * p.time_offset_scale;
+    if (use_time_offset_db) t = t + w_toff[w] * time_offset_scale;
     if (event_t0) t = t + event_t0[w];
     bar[k] = c / 4;
     sipm[k] = c % 4;
@@ -1263,37 +1127,34 @@ __global__ void k_hit_fill(const CrvParams p, const long long* __restrict__ w_la
     pe[k] = p_pe[i];
     hev[k] = lab / 32768;
   }
-}
+};
 
-__global__ void k_ev_heads(const long long* __restrict__ n_dev, const long long* __restrict__ hev,
-                           int32_t* __restrict__ head) {
-  long long n = *n_dev;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    head[i] = (i == 0 || hev[i] != hev[i - 1]) ? 1 : 0;
-}
-
-__global__ void k_ev_fill(const long long* __restrict__ n_dev, const long long* __restrict__ hev,
-                          const int32_t* __restrict__ head, const long long* __restrict__ eidx,
-                          long long* __restrict__ ev_start, int32_t* __restrict__ ev_count,
-                          long long* __restrict__ ev_key) {
-  long long n = *n_dev;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    if (!head[i]) continue;
-    long long e = eidx[i];
-    long long j = i + 1;
-    while (j < n && !head[j]) ++j;
-    ev_start[e] = i;
-    ev_count[e] = int32_t(j - i);
-    ev_key[e] = hev[i];
+// Events: runs of hits of one event
+struct EventRuns {
+  using V = long long;
+  static constexpr bool FLAG = true;
+  const long long* hev;
+  long long *start, *key;
+  __device__ __forceinline__ long long item(long long i) const { return i == 0 || hev[i] != hev[i - 1]; }
+  __device__ __forceinline__ void put(long long i, long long, long long e) const {
+    start[e] = i;
+    key[e] = hev[i];
   }
+};
+
+// hits of each event, from consecutive starts (a walk over the hits of each event, by one thread, took 215 us at 65,536
+// events and 12 us at 16)
+__global__ void k_run_lengths(const long long* __restrict__ runs_dev, const long long* __restrict__ n_dev,
+                              const long long* __restrict__ start, int32_t* __restrict__ count) {
+  const long long runs = *runs_dev, n = *n_dev;
+  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < runs; e += (long long)gridDim.x * blockDim.x)
+    count[e] = int32_t((e + 1 < runs ? start[e + 1] : n) - start[e]);
 }
 }  // namespace crv
 
 extern "C" int64_t crv_reco_waveforms_workspace(int64_t nd) {
   if (nd < 0) return -1;
   Carve c{nullptr};
-  c.take<int32_t>(nd);
-  c.take<long long>(nd);
   c.take<long long>(scan_parts_len(nd) + 1);
   c.take<long long>(8);
   return (int64_t)(c.off + 256);
@@ -1303,7 +1164,8 @@ static int reco_waveforms_run(const CrvParams* p, const CrvChannels* ch, int64_t
                               const int64_t* label, const int64_t* starttdc, int64_t* w_label, int64_t* w_off,
                               int32_t* w_n, int64_t* w_start, double* w_ped, double* w_area, double* w_height,
                               double* w_toff, int64_t* n_w_dev, void* workspace, int64_t workspace_bytes, void* stream,
-                              CrvStatus* status_dev) {
+                              CrvStatus* status_dev,
+                              long long* pass_dev = nullptr) {
   if (!p || !ch || !n_w_dev || !status_dev || nd < 0) return CRV_ERR_ARG;
   cudaStream_t s = (cudaStream_t)stream;
   if (nd == 0) {
@@ -1313,29 +1175,14 @@ static int reco_waveforms_run(const CrvParams* p, const CrvChannels* ch, int64_t
   if (crv_reco_waveforms_workspace(nd) > workspace_bytes || !workspace) return CRV_ERR_ARG;
   char* base = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(workspace) + 255) & ~uintptr_t(255));
   Carve c{base};
-  int32_t* head = c.take<int32_t>(nd);
-  long long* gidx = c.take<long long>(nd);
   long long* parts = c.take<long long>(scan_parts_len(nd) + 1);
   long long* totals = c.take<long long>(8);
   const long long* lab = reinterpret_cast<const long long*>(label);
   const long long* tdc = reinterpret_cast<const long long*>(starttdc);
-  unsigned g = grid_for(nd, 256, 8);
-  {
-    crv::Mark mark_("k_wf_heads", s);
-    k_wf_heads<<<g, 256, 0, s>>>(nd, nd_dev, lab, tdc, p->samples_zs, head);
-  }
-  CK(exclusive_scan(head, nd, Identity(), gidx, &totals[0], parts, s, nd_dev));
-  {
-    crv::Mark mark_("k_wf_fill", s);
-    k_wf_fill<<<g, 256, 0, s>>>(nd, nd_dev, lab, tdc, p->samples_zs, head, gidx, *ch,
-                                reinterpret_cast<long long*>(w_label), reinterpret_cast<long long*>(w_off), w_n,
-                                reinterpret_cast<long long*>(w_start), w_ped, w_area, w_height, w_toff);
-  }
-  {
-    crv::Mark mark_("k_copy_i64", s);
-    k_copy_i64<<<1, 1, 0, s>>>(&totals[0], reinterpret_cast<long long*>(n_w_dev));
-  }
-  CK(cudaGetLastError());
+  const WaveRuns R{lab, tdc, nd, nd_dev, p->samples_zs, *ch, reinterpret_cast<long long*>(w_label),
+                   reinterpret_cast<long long*>(w_off), w_n, reinterpret_cast<long long*>(w_start), w_ped, w_area,
+                   w_height, w_toff};
+  CK(exclusive_scan(R, nd, nd_dev, scan_end(&totals[0], n_w_dev).guard(pass_dev, nd), parts, s));
   return CRV_OK;
 }
 
@@ -1351,10 +1198,6 @@ extern "C" int crv_reco_waveforms(const CrvParams* p, const CrvChannels* ch, int
 extern "C" int64_t crv_pulse_hits_workspace(int64_t np) {
   if (np < 0) return -1;
   Carve c{nullptr};
-  c.take<int32_t>(np);
-  c.take<long long>(np);
-  c.take<long long>(np);
-  c.take<int32_t>(np);
   c.take<long long>(np);
   c.take<long long>(scan_parts_len(np) + 1);
   c.take<long long>(8);
@@ -1366,7 +1209,8 @@ static int pulse_hits_run(const CrvParams* p, const int32_t* status, int64_t nw,
                           const int64_t* p_wf, const int64_t* p_seq, const double* p_time, const double* p_pe,
                           int64_t* ev_start, int32_t* ev_count, int64_t* ev_key, int32_t* bar, int32_t* sipm,
                           int32_t* seq, double* time, double* pe, int64_t* n_ev_dev, int64_t* n_hit_dev,
-                          void* workspace, int64_t workspace_bytes, void* stream, CrvStatus* status_dev) {
+                          void* workspace, int64_t workspace_bytes, void* stream, CrvStatus* status_dev,
+                          long long* pass_dev = nullptr, long long pass_cap = 0) {
   if (!p || !status || !n_ev_dev || !n_hit_dev || !status_dev || np < 0 || nw < 0) return CRV_ERR_ARG;
   cudaStream_t s = (cudaStream_t)stream;
   if (np == 0) {
@@ -1377,45 +1221,20 @@ static int pulse_hits_run(const CrvParams* p, const int32_t* status, int64_t nw,
   if (crv_pulse_hits_workspace(np) > workspace_bytes || !workspace) return CRV_ERR_ARG;
   char* base = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(workspace) + 255) & ~uintptr_t(255));
   Carve c{base};
-  int32_t* keep = c.take<int32_t>(np);
-  long long* kidx = c.take<long long>(np);
   long long* hev = c.take<long long>(np);
-  int32_t* head = c.take<int32_t>(np);
-  long long* eidx = c.take<long long>(np);
   long long* parts = c.take<long long>(scan_parts_len(np) + 1);
   long long* totals = c.take<long long>(8);
-  unsigned g = grid_for(np, 256, 8);
-  const long long* wl = reinterpret_cast<const long long*>(w_label);
+  const KeptHits K{p->ignore_channels, p->use_time_offset_db, p->time_offset_scale, status,
+                   reinterpret_cast<const long long*>(w_label), w_toff, event_t0,
+                   reinterpret_cast<const long long*>(p_wf), reinterpret_cast<const long long*>(p_seq), p_time, p_pe,
+                   bar, sipm, seq, time, pe, hev};
+  CK(exclusive_scan(K, np, np_dev, scan_end(&totals[0], n_hit_dev), parts, s));
+  CK(exclusive_scan(EventRuns{hev, reinterpret_cast<long long*>(ev_start), reinterpret_cast<long long*>(ev_key)}, np,
+                    &totals[0], scan_end(&totals[1], n_ev_dev).guard(pass_dev, pass_cap), parts, s));
   {
-    crv::Mark mark_("k_hit_keep", s);
-    k_hit_keep<<<g, 256, 0, s>>>(*p, status, wl, np, np_dev, reinterpret_cast<const long long*>(p_wf), keep);
-  }
-  CK(exclusive_scan(keep, np, Identity(), kidx, &totals[0], parts, s, np_dev));
-  {
-    crv::Mark mark_("k_hit_fill", s);
-    k_hit_fill<<<g, 256, 0, s>>>(*p, wl, w_toff, event_t0, np, np_dev, reinterpret_cast<const long long*>(p_wf),
-                                 reinterpret_cast<const long long*>(p_seq), p_time, p_pe, keep, kidx, bar, sipm, seq,
-                                 time, pe, hev);
-  }
-  // rows beyond the kept count stay 0 so the event scan counts kept pulses only
-  CK(cudaMemsetAsync(head, 0, sizeof(int32_t) * np, s));
-  {
-    crv::Mark mark_("k_ev_heads", s);
-    k_ev_heads<<<g, 256, 0, s>>>(&totals[0], hev, head);
-  }
-  CK(exclusive_scan(head, np, Identity(), eidx, &totals[1], parts, s));
-  {
-    crv::Mark mark_("k_ev_fill", s);
-    k_ev_fill<<<g, 256, 0, s>>>(&totals[0], hev, head, eidx, reinterpret_cast<long long*>(ev_start), ev_count,
-                                reinterpret_cast<long long*>(ev_key));
-  }
-  {
-    crv::Mark mark_("k_copy_i64", s);
-    k_copy_i64<<<1, 1, 0, s>>>(&totals[1], reinterpret_cast<long long*>(n_ev_dev));
-  }
-  {
-    crv::Mark mark_("k_copy_i64", s);
-    k_copy_i64<<<1, 1, 0, s>>>(&totals[0], reinterpret_cast<long long*>(n_hit_dev));
+    crv::Mark mark_("k_run_lengths", s);
+    k_run_lengths<<<grid_for(np, 256, 8), 256, 0, s>>>(&totals[1], &totals[0], reinterpret_cast<long long*>(ev_start),
+                                                     ev_count);
   }
   CK(cudaGetLastError());
   return CRV_OK;
@@ -1557,53 +1376,29 @@ static int chain_run(const CrvParams* p, const CrvChainCaps* caps, const CrvEven
   long long* m = w.counts + 16;            // counts passed on: 0 when the stage overflowed its capacity
   const long long zs = p->samples_zs;
   CK(cudaMemsetAsync(w.counts, 0, 32 * sizeof(long long), s));
-  // the stage totals that size the photon and slot capacities, from the stage workspaces (scratch is 256-aligned)
-  auto keep_total = [&](const long long* total, int k) -> cudaError_t {
-    crv::Mark mark_("k_copy_i64", s);
-    k_copy_i64<<<1, 1, 0, s>>>(total, &n[k]);
-    return cudaGetLastError();
-  };
   auto N = [&](int k) { return reinterpret_cast<int64_t*>(&n[k]); };
-  auto guard = [&](int k, long long cap) -> cudaError_t {
-    crv::Mark mark_("k_guard_groups", s);
-    k_guard_groups<<<1, 32, 0, s>>>(&n[k], cap, &n[k], &m[k]);
-    return cudaGetLastError();
-  };
   int rc = response_run(p, ev, c.events, st, c.steps, reinterpret_cast<const long long*>(nsteps_dev),
                         c.max_steps_per_event, bars, ch, px, c.photons, &w.Q, c.charges, N(CRV_CHAIN_CHARGES),
-                        nullptr, nullptr, nullptr, 0, nullptr, w.scratch, w.scratch_bytes, stream, status_dev, lk);
+                        nullptr, nullptr, nullptr, 0, nullptr, w.scratch, w.scratch_bytes, stream, status_dev, lk,
+                        &n[CRV_CHAIN_PHOTONS], &m[CRV_CHAIN_CHARGES]);
   if (rc != CRV_OK) return rc;
-  {
-    size_t b;
-    CK(keep_total(&resp_layout(w.scratch, *p, c.events, c.steps, c.photons, &b, lk != nullptr).totals[1],
-                  CRV_CHAIN_PHOTONS));
-  }
-  CK(guard(CRV_CHAIN_CHARGES, c.charges));
   rc = digis_run(p, ch, c.charges, &m[CRV_CHAIN_CHARGES], w.Q.label, w.Q.time, w.Q.charge, nullptr, tmpl, tlen, ev_keys,
                  ev_runs, c.events, c.slots, &w.D, c.digis, N(CRV_CHAIN_DIGIS), w.scratch, w.scratch_bytes, stream,
-                 status_dev);
+                 status_dev, &n[CRV_CHAIN_SLOTS], &m[CRV_CHAIN_DIGIS]);
   if (rc != CRV_OK) return rc;
-  {
-    size_t b;
-    CK(keep_total(&digi_layout(w.scratch, c.charges, c.slots, p->samples_zs, &b).totals[1], CRV_CHAIN_SLOTS));
-  }
-  CK(guard(CRV_CHAIN_DIGIS, c.digis));
   rc = reco_waveforms_run(p, ch, c.digis, &m[CRV_CHAIN_DIGIS], w.D.chan, w.D.starttdc, w.w_label, w.w_off, w.w_n,
                           w.w_start, w.w_ped, w.w_area, w.w_height, w.w_toff, N(CRV_CHAIN_WAVEFORMS), w.scratch,
-                          w.scratch_bytes, stream, status_dev);
+                          w.scratch_bytes, stream, status_dev, &m[CRV_CHAIN_WAVEFORMS]);
   if (rc != CRV_OK) return rc;
-  CK(guard(CRV_CHAIN_WAVEFORMS, c.digis));
   rc = pulses_run(p, c.digis, &m[CRV_CHAIN_WAVEFORMS], c.digis * zs, w.w_off, w.w_n, w.w_start, w.w_ped, w.w_area,
                   w.w_height, w.D.adc, nullptr, 0x7FFFFFFF, &w.P, c.pulses, N(CRV_CHAIN_PULSES), w.near, w.scratch,
-                  w.scratch_bytes, stream, status_dev);
+                  w.scratch_bytes, stream, status_dev, &m[CRV_CHAIN_PULSES]);
   if (rc != CRV_OK) return rc;
-  CK(guard(CRV_CHAIN_PULSES, c.pulses));
   rc = pulse_hits_run(p, ch->status, c.digis, w.w_label, w.w_toff, nullptr, c.pulses, &m[CRV_CHAIN_PULSES], w.P.wf,
                       w.P.seq, w.P.time, w.P.pe, w.h_ev_start, w.h_ev_count, w.h_ev_key, w.h_bar, w.h_sipm, w.h_seq,
                       w.h_time, w.h_pe, N(CRV_CHAIN_EVENTS), N(CRV_CHAIN_HITS), w.scratch, w.scratch_bytes, stream,
-                      status_dev);
+                      status_dev, &m[CRV_CHAIN_EVENTS], c.events);
   if (rc != CRV_OK) return rc;
-  CK(guard(CRV_CHAIN_EVENTS, c.events));
   rc = coinc_run(p, g, c.events, &m[CRV_CHAIN_EVENTS], w.h_ev_start, w.h_ev_count, w.h_ev_key, c.pulses, w.h_bar,
                  w.h_sipm, w.h_seq, w.h_time, w.h_pe, ch->status, out, c.pulses, N(CRV_CHAIN_CLUSTERS), mem, c.pulses,
                  N(CRV_CHAIN_MEMBERS), w.scratch, w.scratch_bytes, stream, status_dev);

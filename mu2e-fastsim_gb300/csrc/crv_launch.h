@@ -68,8 +68,8 @@ cudaError_t launch_sipm(const CrvParams& p, const CrvPixels& px, const SipmGroup
 template <typename R>
 cudaError_t launch_wf_prepass(const CrvParams& p, const CrvChannels& ch, const WfGroups& G, long long ng_bound,
                               const double* time, const double* tmpl, int tlen, const double* tdc0_rows,
-                              double* g_tdc0, int32_t* g_bound, int32_t* g_maxlen, int32_t* g_nkept, WfCluster* cl,
-                              Status* status, cudaStream_t s);
+                              double* g_tdc0, int32_t* g_bound, int32_t* g_maxlen, int32_t* g_nkept,
+                              int32_t* g_digis, WfCluster* cl, Status* status, cudaStream_t s);
 
 template <typename R>
 cudaError_t launch_wf_synth(const CrvParams& p, const WfGroups& G, long long ng_bound, const double* time,

@@ -832,15 +832,6 @@ __global__ void __launch_bounds__(SUB_ROWS_PER_BLOCK * 32) k_substep_emit_f32(Cr
   }
 }
 
-__global__ void k_substep_check(const long long* __restrict__ total, long long cap, long long* __restrict__ n_out,
-                                Status* status) {
-  if (*total > cap) {
-    set_flag(status, CRV_ST_CAPACITY);
-    need_at_least(status, CRV_NEED_PHOTONS_OUT, *total);
-  }
-  *n_out = *total;
-}
-
 struct SubWs {
   long long *count, *offset, *parts, *total;
 };
@@ -921,11 +912,9 @@ extern "C" int crv_substep_photons(const CrvLookup* L, uint32_t seed, const CrvS
     k_substep_count<<<grid, SUB_ROWS_PER_BLOCK * 32, 0, s>>>(*L, *rows, seed, nrows, RowSel{}, w.count, S);
   }
   if (cudaGetLastError() != cudaSuccess) return CRV_ERR_CUDA;
-  if (exclusive_scan(w.count, nrows, Identity(), w.offset, w.total, w.parts, s) != cudaSuccess) return CRV_ERR_CUDA;
-  {
-    crv::Mark mark_("k_substep_check", s);
-    k_substep_check<<<1, 1, 0, s>>>(w.total, cap, reinterpret_cast<long long*>(n_out_dev), S);
-  }
+  if (exclusive_scan(column(w.count, w.offset), nrows, nullptr,
+                     scan_end(w.total, n_out_dev).check(S, CRV_NEED_PHOTONS_OUT, cap), w.parts, s) != cudaSuccess)
+    return CRV_ERR_CUDA;
   if (f32) {
     crv::Mark mark_("k_substep_emit", s);
     k_substep_emit_f32<<<grid, SUB_ROWS_PER_BLOCK * 32, esm, s>>>(*L, *rows, seed, nrows, RowSel{}, w.offset,
@@ -1150,7 +1139,7 @@ extern "C" int crv_lookup_rows(const CrvLookupGroup* G, uint32_t seed, const Crv
     crv::Mark mark_("k_lrows_flag", s);
     k_lrows_flag<<<grid, 256, 0, s>>>(*G, *st, nsteps, flag);
   }
-  if (exclusive_scan(flag, nsteps, Identity(), rank, total, parts, s) != cudaSuccess) return CRV_ERR_CUDA;
+  if (exclusive_scan(column(flag, rank), nsteps, nullptr, scan_end(total), parts, s) != cudaSuccess) return CRV_ERR_CUDA;
   {
     crv::Mark mark_("k_lrows_fill", s);
     k_lrows_fill<<<grid, 256, 0, s>>>(*G, *st, seed, nsteps, rank, total, *out);

@@ -239,7 +239,8 @@ __global__ void k_sipm_sizes(const long long* __restrict__ nsipm_dev, const int3
                              const int32_t* __restrict__ step_order, const int32_t* __restrict__ count,
                              CrvEvents ev, int charge_factor, int32_t* __restrict__ nphot,
                              int32_t* __restrict__ slot_cap, long long* __restrict__ id_base,
-                             long long* __restrict__ label, uint32_t* __restrict__ run) {
+                             long long* __restrict__ label, uint32_t* __restrict__ run,
+                             int32_t* __restrict__ nmain, int32_t* __restrict__ nap, int32_t* __restrict__ fired) {
   long long nsipm = *nsipm_dev;
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < nsipm;
        g += (long long)gridDim.x * blockDim.x) {
@@ -254,6 +255,9 @@ __global__ void k_sipm_sizes(const long long* __restrict__ nsipm_dev, const int3
     long long evkey = ((long long)ev.subrun[e] << 20) | (long long)ev.event[e];
     label[g] = evkey * 32768 + s_chan[g];
     run[g] = ev.run[e];
+    nmain[g] = 0;                // the SiPM stage writes the SiPMs with photons only, and none at an overflow
+    nap[g] = 0;
+    fired[g] = 0;
   }
 }
 
@@ -1331,13 +1335,6 @@ __global__ void k_charge_compact(const long long* __restrict__ ngroups_dev, cons
     }
    }
   }
-}
-
-__global__ void k_counts_total(const long long* __restrict__ n_dev, const int32_t* __restrict__ a,
-                               const int32_t* __restrict__ b, int32_t* __restrict__ out) {
-  long long n = *n_dev;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    out[i] = a[i] + b[i];
 }
 
 #endif  // CRV_ENGINE_TU

@@ -187,6 +187,7 @@ __global__ void __launch_bounds__(256, 3) k_wf_prep(CrvParams p, CrvChannels ch,
                                                  int tlen, const double* __restrict__ tdc0_rows,
                                                  double* __restrict__ g_tdc0, int32_t* __restrict__ g_bound,
                                                  int32_t* __restrict__ g_maxlen, int32_t* __restrict__ g_nkept,
+                                                 int32_t* __restrict__ g_digis,
                                                  typename Prep::Record* __restrict__ cl, Status* status) {
   __shared__ PrepQueue queue[8];
   __shared__ typename Prep::Consts K_s;
@@ -312,6 +313,7 @@ __global__ void __launch_bounds__(256, 3) k_wf_prep(CrvParams p, CrvChannels ch,
       g_bound[gl] = drop ? 0 : Q.bound[lane];
       g_maxlen[gl] = drop ? 0 : Q.maxlen[lane];
       g_nkept[gl] = drop ? 0 : Q.nk[lane];
+      g_digis[gl] = 0;         // the synthesis writes the groups with kept clusters only
       g_tdc0[gl] = drop ? 0.0 : Prep::tdc0_value(tdc0_l);
     }
     __syncwarp();
@@ -734,25 +736,18 @@ __global__ void k_digi_compact(const long long* __restrict__ ng_dev, DigiSlots D
   }
 }
 
-// Segments of equal labels in a label-sorted array: heads, then group start/label/count.
-__global__ void k_label_heads(long long n, const long long* __restrict__ n_dev, const long long* __restrict__ label,
-                              int32_t* __restrict__ head) {
-  n = bounded_count(n, n_dev);
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    head[i] = (i == 0 || label[i] != label[i - 1]) ? 1 : 0;
-}
-
-__global__ void k_label_groups(long long n, const long long* __restrict__ n_dev, const long long* __restrict__ label,
-                               const int32_t* __restrict__ head, const long long* __restrict__ gidx,
-                               long long* __restrict__ gstart, long long* __restrict__ glabel) {
-  n = bounded_count(n, n_dev);
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    if (head[i]) {
-      long long g = gidx[i];
-      gstart[g] = i;
-      glabel[g] = label[i];
-    }
-}
+// Groups: runs of equal labels in a label-sorted array
+struct LabelRuns {
+  using V = long long;
+  static constexpr bool FLAG = true;
+  const long long* label;
+  long long *start, *group_label;
+  __device__ __forceinline__ long long item(long long i) const { return i == 0 || label[i] != label[i - 1]; }
+  __device__ __forceinline__ void put(long long i, long long, long long g) const {
+    start[g] = i;
+    group_label[g] = label[i];
+  }
+};
 
 // counts from consecutive starts; run per group from a sorted (event key -> run) table (run 0 if absent)
 __global__ void k_group_counts(const long long* __restrict__ ng_dev, long long n, const long long* __restrict__ n_dev,
