@@ -426,6 +426,17 @@ int crv_chain(const CrvParams *p, const CrvChainCaps *caps, const CrvEvents *ev,
               void *stream, CrvStatus *status_dev);
 
 /*
+ * Columns of a batch in one launch (at most CRV_COPY_COLUMNS): bytes[c] bytes from src[c] to dst[c], device memory, any
+ * alignment.  crv_chain_load also completes the event table of crv_chain in its static buffers: keys of the first
+ * nevents rows from (event, subrun), rows from there to events_cap cleared (no steps, key INT64_MAX), *nsteps_dev = n.
+ */
+#define CRV_COPY_COLUMNS 32
+int crv_copy_columns(int32_t ncols, const void *const *src, void *const *dst, const int64_t *bytes, void *stream);
+int crv_chain_load(int32_t ncols, const void *const *src, void *const *dst, const int64_t *bytes, const int32_t *event,
+                   const int32_t *subrun, int64_t nevents, int64_t events_cap, int64_t *first_step, int32_t *nsteps,
+                   int64_t *key, int64_t n, int64_t *nsteps_dev, void *stream);
+
+/*
  * The resident chain as one CUDA graph (no counterpart in the reference; the reference's resident JAX chain compiles
  * one program per shape): crv_chain_graph_create captures one crv_chain call with these arguments (plus the zeroing
  * of the status block) on `stream`, which must be a created stream, in thread-local capture mode, and instantiates

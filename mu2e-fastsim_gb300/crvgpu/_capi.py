@@ -231,6 +231,8 @@ _SIGS = {
     "crv_chain": (c_i32, [P(CrvParams), P(CrvChainCaps), P(CrvEvents), c_p, c_p, P(CrvSteps), c_p, P(CrvBars),
                           P(CrvChannels), P(CrvPixels), c_p, c_i32, P(CrvFinderGeom), P(CrvClusters), P(CrvMembers),
                           c_p, c_p, c_i64, c_p, c_p]),
+    "crv_copy_columns": (c_i32, [c_i32, c_p, c_p, c_p, c_p]),
+    "crv_chain_load": (c_i32, [c_i32, c_p, c_p, c_p, c_p, c_p, c_i64, c_i64, c_p, c_p, c_p, c_i64, c_p, c_p]),
     "crv_chain_graph_create": (c_i32, [P(CrvParams), P(CrvChainCaps), P(CrvEvents), c_p, c_p, P(CrvSteps), c_p,
                                        P(CrvBars), P(CrvChannels), P(CrvPixels), c_p, c_i32, P(CrvFinderGeom),
                                        P(CrvClusters), P(CrvMembers), c_p, c_p, c_i64, c_p, c_p, P(c_p)]),

@@ -27,6 +27,8 @@ from . import _capi
 from .response import DeviceSteps, EngineError, _stream, _torch
 
 INT64_MAX = (1 << 63) - 1
+_STEP_COLS = ("x", "y", "z", "t", "edep", "bar")
+_EVENT_COLS = ("event", "subrun", "run", "first", "nsteps")
 
 # one stream capture at a time in the process: entering a capture synchronises the device, which another thread's
 # capture in progress does not permit
@@ -145,7 +147,8 @@ class ResidentChain:
         self.graph_mode, self.grow, self.max_grow = bool(graph), bool(grow), int(max_grow)
         self.real_dtype = real_dtype if real_dtype is not None else torch.float32
         self.status = _capi.DeviceStatus(self.device)
-        self.counts = torch.zeros(10, dtype=torch.int64, device=self.device)
+        self._hdr = torch.zeros(10 + self.status.t.numel(), dtype=torch.int64, device=self.device)
+        self.counts, self.status.t = self._hdr[:10], self._hdr[10:]          # read in one copy
         self.last_counts = None
         self.launches_per_run = 0
         self.replays = 0                # graph replays (kernel launches of a replay: launches_per_run)
@@ -202,6 +205,15 @@ class ResidentChain:
         self._S = _capi.CrvSteps(*[_capi.ptr(self.st[k]) for k in ("x", "y", "z", "t", "edep", "bar")], rb, 0)
         self._E = _capi.CrvEvents(*[_capi.ptr(self.ev[k]) for k in ("event", "subrun", "run", "first", "nsteps")])
         self._LK = self._lookup_c() if self.lookup is not None else None
+        # what a batch is copied into and taken from in one launch each: key, type, bytes per row, address
+        col = lambda d, ks: [(k, d[k].dtype, int(d[k].element_size()) * int(d[k].numel() // max(len(d[k]), 1)),  # noqa: E731
+                              d[k].data_ptr()) for k in ks]
+        self._in_steps, self._in_events = col(self.st, _STEP_COLS), col(self.ev, _EVENT_COLS)
+        self._in_lookup = col(self.lst, self.lst) if self.lst is not None else []
+        ins = self._in_steps + self._in_events + self._in_lookup
+        self._in_dst = (ctypes.c_void_p * len(ins))(*[c[3] for c in ins])
+        self._out = [(*col(d, [k])[0], tuple(t.shape[1:]), t.device) for d in (self.cl, self.mem) for k, t in d.items()]
+        self._out_src = (ctypes.c_void_p * len(self._out))(*[c[3] for c in self._out])
         self.nbytes = int(self.ws.numel()) + sum(int(t.numel() * t.element_size()) for d in
                                                  (self.ev, self.st, self.cl, self.mem, self.lst or {})
                                                  for t in d.values())
@@ -248,22 +260,46 @@ class ResidentChain:
                              f"exceeds the chain capacities {c.events} / {c.steps} / {c.max_steps_per_event}")
         if ds.x.dtype != self.real_dtype:
             raise ValueError(f"step table dtype {ds.x.dtype} differs from the chain's {self.real_dtype}")
-        n, e = ds.nsteps, ds.nevents
         if self.lookup is not None:
             if ds.order is not None:
                 raise ValueError("the lookup-table chain needs steps grouped by event in increasing event key")
             for k in _capi.LOOKUP_STEP_COLS + ("pdg",):
-                if int(lookup_steps[k].numel()) != n:
-                    raise ValueError(f"lookup step column {k}: {int(lookup_steps[k].numel())} rows, the batch {n}")
+                if int(lookup_steps[k].numel()) != ds.nsteps:
+                    raise ValueError(f"lookup step column {k}: {int(lookup_steps[k].numel())} rows, the batch {ds.nsteps}")
+        if not self._load_columns(ds, lookup_steps):
+            self._load_each(ds, lookup_steps)
+        self._n_events = ds.nevents
+
+    def _load_columns(self, ds, lookup_steps):
+        """The batch in one launch; False when a column is not a dense one of the buffer's type and device."""
+        n, e, dev = ds.nsteps, ds.nevents, self.nsteps_dev.get_device()
+        cols = ([(getattr(ds, c[0]), c, n) for c in self._in_steps]
+                + [(getattr(ds, "ev_" + c[0]), c, e) for c in self._in_events]
+                + [(lookup_steps[c[0]], c, n) for c in self._in_lookup])
+        for t, c, rows in cols:
+            if (t.dtype is not c[1] or t.dim() != 1 or t.numel() != rows or t.get_device() != dev
+                    or not t.is_contiguous() or t.is_neg()):
+                return False
+        k, E = len(cols), self.ev
+        p = _capi.ptr
+        _capi.check(_capi.load().crv_chain_load(
+            k, (ctypes.c_void_p * k)(*[t.data_ptr() for t, _, _ in cols]), self._in_dst,
+            (ctypes.c_int64 * k)(*[rows * c[2] for _, c, rows in cols]), p(ds.ev_event), p(ds.ev_subrun), e,
+            self.caps.events, p(E["first"]), p(E["nsteps"]), p(E["key"]), n, p(self.nsteps_dev), _stream()),
+            "crv_chain_load")
+        return True
+
+    def _load_each(self, ds, lookup_steps):
+        """The batch column by column: other types, strides or devices than the buffers'."""
+        c, n, e = self.caps, ds.nsteps, ds.nevents
+        if self.lookup is not None:
+            for k in _capi.LOOKUP_STEP_COLS + ("pdg",):
                 self.lst[k][:n].copy_(lookup_steps[k])
-        for k in ("x", "y", "z", "t", "edep", "bar"):
+        for k in _STEP_COLS:
             self.st[k][:n].copy_(getattr(ds, k))
         E = self.ev
-        E["event"][:e].copy_(ds.ev_event)
-        E["subrun"][:e].copy_(ds.ev_subrun)
-        E["run"][:e].copy_(ds.ev_run)
-        E["first"][:e].copy_(ds.ev_first)
-        E["nsteps"][:e].copy_(ds.ev_nsteps)
+        for k in _EVENT_COLS:
+            E[k][:e].copy_(getattr(ds, "ev_" + k))
         E["key"][:e].copy_(((ds.ev_subrun.to(E["key"].dtype) & 0xFFFFFFFF) << 20)
                            | (ds.ev_event.to(E["key"].dtype) & 0xFFFFFFFF))
         if e < c.events:
@@ -271,7 +307,6 @@ class ResidentChain:
             E["first"][e:].zero_()
             E["key"][e:].fill_(INT64_MAX)
         self.nsteps_dev.fill_(n)
-        self._n_events = e
 
     # -- the call ---------------------------------------------------------------------------------------------------
     def _args(self, P):
@@ -345,16 +380,32 @@ class ResidentChain:
     def finish(self, copy=True):
         """Read counts and status (one host read); raise BatchRejected on any flag; the batch's clusters."""
         torch = _torch()
-        hdr = torch.cat([self.counts, self.status.t]).cpu().numpy()
+        hdr = (torch.cat([self.counts, self.status.t]) if getattr(self, "_hdr", None) is None else self._hdr).cpu().numpy()
         counts = {k: int(hdr[i]) for i, k in enumerate(_capi.CHAIN_COUNTS)}
         self.last_counts = counts
         flags = int(np.int64(hdr[10]) & 0xFFFFFFFF)
         if flags:
             raise BatchRejected(flags, hdr[11:27].copy(), counts)
         ncl, nm = counts["clusters"], counts["members"]
-        take = (lambda v, n: v[:n].clone()) if copy else (lambda v, n: v[:n])  # noqa: E731
-        return ResidentResult(self._n_events, counts, {k: take(v, ncl) for k, v in self.cl.items()},
-                              {k: take(v, nm) for k, v in self.mem.items()})
+        if copy and getattr(self, "_out", None):
+            cl, mem = self._take(ncl, nm)
+        else:
+            take = (lambda v, n: v[:n].clone()) if copy else (lambda v, n: v[:n])  # noqa: E731
+            cl, mem = {k: take(v, ncl) for k, v in self.cl.items()}, {k: take(v, nm) for k, v in self.mem.items()}
+        return ResidentResult(self._n_events, counts, cl, mem)
+
+    def _take(self, ncl, nm):
+        """Clusters and members in tensors of their own, copied in one launch."""
+        torch = _torch()
+        k, ncols = len(self._out), len(self.cl)
+        rows = [ncl] * ncols + [nm] * (k - ncols)
+        new = [torch.empty((n, *tail), dtype=dt, device=dev) for (_, dt, _, _, tail, dev), n in zip(self._out, rows)]
+        if ncl or nm:
+            _capi.check(_capi.load().crv_copy_columns(
+                k, self._out_src, (ctypes.c_void_p * k)(*[t.data_ptr() for t in new]),
+                (ctypes.c_int64 * k)(*[n * c[2] for c, n in zip(self._out, rows)]), _stream()), "crv_copy_columns")
+        named = [(c[0], t) for c, t in zip(self._out, new)]
+        return dict(named[:ncols]), dict(named[ncols:])
 
     def run(self, ds: DeviceSteps, seed, copy=True, lookup_steps=None):
         """One batch: load, launch, read.  With grow, a rejected batch for capacity alone is re-run with larger
