@@ -630,6 +630,11 @@ int crv_lookup_file_read(const uint8_t *image, int64_t size, const CrvLookupFile
 int64_t crv_lz4_block_decompress(const uint8_t *src, int64_t n, uint8_t *dst, int64_t cap);
 uint64_t crv_xxh64(const uint8_t *data, int64_t n, uint64_t seed);
 
+/* Waveform matrix of runs of digis (host code): row g of mat (width digis of L samples) takes the ndig[g] digis of the
+ * nd x L samples adc from row first[g] on, then zeros.  CRV_ERR_ARG when a run leaves the samples or its row. */
+int crv_waveform_matrix(int64_t rows, int64_t width, int64_t L, const int64_t *first, const int64_t *ndig,
+                        const int16_t *adc, int64_t nd, int64_t *mat);
+
 #ifdef __cplusplus
 }
 #endif

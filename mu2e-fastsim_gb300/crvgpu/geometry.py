@@ -56,26 +56,24 @@ def module_geometry(n_modules=1, lengths=None, seed=0, n_layers=4, n_counters=16
                    list(np.random.default_rng(seed).choice(LENGTHS, n_modules)))
     lengths = [float(v) for v in lengths]
     names = ["EX"] if n_modules == 1 else [f"L{int(round(v / 10))}" for v in sorted(set(lengths))]
-    sec_of = {v: (0 if n_modules == 1 else sorted(set(lengths)).index(v)) for v in lengths}
-    rows = {k: [] for k in ("sector", "module", "layer", "counter", "center", "halflen")}
-    mod_in_sec = {}
-    width_mod = n_counters * PITCH + MODULE_GAP
-    for m, L in enumerate(lengths):
+    order = sorted(set(lengths))
+    sec_of = {v: (0 if n_modules == 1 else order.index(v)) for v in order}
+    mod_in_sec, mods = {}, []
+    for L in lengths:
         s = sec_of[L]
-        mi = mod_in_sec.get(s, 0)
-        mod_in_sec[s] = mi + 1
-        for layer in range(n_layers):
-            for c in range(n_counters):
-                x = m * width_mod + (c - (n_counters - 1) / 2) * PITCH + STAGGER * (layer % 2)
-                y = (layer - (n_layers - 1) / 2) * LAYER_PITCH
-                rows["sector"].append(s); rows["module"].append(mi); rows["layer"].append(layer)
-                rows["counter"].append(c); rows["center"].append((x, y, 0.0))
-                rows["halflen"].append((WIDTH / 2, THICK / 2, L / 2))
-    nb = len(rows["sector"])
-    return CRVGeometry(sector_names=names, sector=np.array(rows["sector"]), module=np.array(rows["module"]),
-                       layer=np.array(rows["layer"]), counter=np.array(rows["counter"]),
-                       center=np.array(rows["center"], float), halflen=np.array(rows["halflen"], float),
-                       local_to_world=np.tile([1, 0, 2], (nb, 1)))
+        mods.append((s, mod_in_sec.get(s, 0)))
+        mod_in_sec[s] = mods[-1][1] + 1
+    width_mod = n_counters * PITCH + MODULE_GAP
+    per = n_layers * n_counters
+    nb = len(lengths) * per
+    m, layer, c = np.divmod(np.arange(nb), per)[0], np.arange(nb) // n_counters % n_layers, np.arange(nb) % n_counters
+    center, halflen = np.zeros((nb, 3)), np.empty((nb, 3))
+    center[:, 0] = m * width_mod + (c - (n_counters - 1) / 2) * PITCH + STAGGER * (layer % 2)
+    center[:, 1] = (layer - (n_layers - 1) / 2) * LAYER_PITCH
+    halflen[:, 0], halflen[:, 1], halflen[:, 2] = WIDTH / 2, THICK / 2, np.asarray(lengths)[m] / 2
+    mods = np.asarray(mods, np.int64).reshape(-1, 2)
+    return CRVGeometry(sector_names=names, sector=mods[m, 0], module=mods[m, 1], layer=layer, counter=c, center=center,
+                       halflen=halflen, local_to_world=np.tile([1, 0, 2], (nb, 1)))
 
 
 def sector_geom(geom, n_counters=16):

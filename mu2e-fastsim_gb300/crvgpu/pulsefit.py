@@ -255,8 +255,15 @@ def concat_waveforms(key, bar, sipm, start_tdc, adc_flat, lens):
         if int(ndig.max()) == 1:
             mat = rows.astype(np.int64)
         else:
+            W = int(ndig.max())
+            if rows.dtype == np.int16 and rows.flags.c_contiguous:
+                mat = np.empty((G, W * L), np.int64)
+                p = lambda a: a.ctypes.data  # noqa: E731
+                _capi.check(_capi.load().crv_waveform_matrix(G, W, L, p(first), p(ndig), p(rows), nd, p(mat)),
+                            "crv_waveform_matrix")
+                return gid, mat, glen, start_tdc[first], first
             pos = np.arange(nd) - np.repeat(first, ndig)
-            mat = np.zeros((G, int(ndig.max()), L), np.int64)
+            mat = np.zeros((G, W, L), np.int64)
             mat[gid, pos] = rows
             mat = mat.reshape(G, -1)
         return gid, mat, glen, start_tdc[first], first

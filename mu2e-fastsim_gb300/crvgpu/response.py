@@ -19,6 +19,7 @@ import numpy as np
 
 from . import _capi, readout
 from .config import CHAN_MULT, ChainConfig
+from .hostmem import to_host
 from .params import make_params, validate_sipm, validate_window
 
 
@@ -392,11 +393,11 @@ def charges(steps, parts, geom, cond, cfg: ChainConfig, rng, key=None, tabs=None
     T = tabs if isinstance(tabs, DeviceTables) else DeviceTables(geom, cond, cfg, pmap=pmap)
     P = make_params(cfg, seed, uniform_map=T.uniform_map)
     R = engine().run(P, ds, T)
-    photon = R.photon.cpu().numpy()
+    photon = to_host(R.photon)
     if ds.order is not None:
         photon = ds.order[photon]
-    Q = {"chan": R.label.cpu().numpy(), "time": R.time.cpu().numpy(), "charge": R.charge.cpu().numpy(),
-         "pe": R.pe.cpu().numpy(), "photon": photon}
+    Q = {"chan": to_host(R.label), "time": to_host(R.time), "charge": to_host(R.charge), "pe": to_host(R.pe),
+         "photon": photon}
     timers["response_s"] = timers.get("response_s", 0.0) + _time.perf_counter() - t0
     timers["photons"] = timers.get("photons", 0) + int(R.sipm_photons.sum().item()) if R.nsipm else 0
     timers["charges"] = timers.get("charges", 0) + R.n

@@ -17,6 +17,7 @@ import numpy as np
 
 from . import _capi
 from .config import CHAN_MULT, ChainConfig, WaveformConfig
+from .hostmem import to_host
 from .params import make_params, validate_window
 from .response import DeviceTables, _stream, _torch, raise_status, seed_of
 
@@ -126,8 +127,7 @@ def engine(device="cuda"):
 
 
 def _host(D):
-    out = {k: v.cpu().numpy() for k, v in D.items()}
-    return out
+    return {k: to_host(v) for k, v in D.items()}
 
 
 def charge_clusters(chan, time, wcfg: WaveformConfig):
@@ -148,8 +148,13 @@ def cluster_table(chan, time, tdc0_cluster, wcfg: WaveformConfig, tmpl, clusters
     template maximum >= min_voltage), for every cluster, kept or not.  The device forms the same start with the same
     operations for the clusters it synthesises.  clusters: charge_clusters' result when the caller has it."""
     cid, first = clusters if clusters is not None else charge_clusters(chan, time, wcfg)
-    P = wcfg.period
     nq = np.bincount(cid, minlength=len(first)) if len(first) else np.zeros(0, np.int64)
+    return _cluster_rows(chan, time, first, nq, tdc0_cluster, wcfg, tmpl)
+
+
+def _cluster_rows(chan, time, first, nq, tdc0_cluster, wcfg: WaveformConfig, tmpl):
+    """cluster_table from the first charge row and the charges of every cluster."""
+    P = wcfg.period
     t_first = np.asarray(time, np.float64)[first] - P
     tdc0_cluster = np.asarray(tdc0_cluster, np.float64)
     return {"cluster_chan": np.asarray(chan)[first], "cluster_tstart": np.ceil((t_first - tdc0_cluster) / P) * P
@@ -245,15 +250,32 @@ def _tdc0_device(P, tabs, labels_d, ek=None, er=None, host=True):
     return out[:n].cpu().numpy() if host else out[:n]
 
 
-def _part_starts(cid, first, max_charges):
-    """Charge rows where synthesize's batches start: whole clusters, a new batch at the first cluster start at or
-    after every multiple of max_charges (waveform.py:88-98)."""
+# label types that _charge_columns may take as int64 (others: charge_clusters compares them as they are)
+_LABEL_TYPES = tuple(np.dtype(t) for t in (np.int8, np.int16, np.int32, np.int64, np.uint8, np.uint16, np.uint32))
+
+
+def _part_starts(n, first, max_charges):
+    """Clusters where synthesize's batches of n charges start: whole clusters, a new batch at the first cluster start at
+    or after every multiple of max_charges (waveform.py:88-98)."""
     cuts = [0]
-    for v in range(max_charges, len(cid), max_charges):
-        j = np.searchsorted(first, v)
-        if j < len(first) and first[j] > cuts[-1]:
-            cuts.append(int(first[j]))
-    return cuts + [len(cid)]
+    for v in range(max_charges, n, max_charges):
+        j = int(np.searchsorted(first, v))
+        if j < len(first) and j > cuts[-1]:
+            cuts.append(j)
+    return cuts + [len(first)]
+
+
+def _charge_columns(lab_d, time_d, wcfg: WaveformConfig):
+    """charge_clusters' comparisons on device columns: (cluster mark of every charge, first row of every cluster on the
+    host, smallest label, largest channel, labels ascend)."""
+    torch = _torch()
+    n = int(lab_d.numel())
+    gap = wcfg.single_pe_max_time + N_DIGI_PERIODS_GAP * wcfg.period
+    new = torch.ones(n, dtype=torch.bool, device=lab_d.device)
+    new[1:] = (lab_d[1:] != lab_d[:-1]) | (time_d[1:] - time_d[:-1] > gap)
+    falls = (lab_d[1:] < lab_d[:-1]).any().to(torch.int64)
+    lo, ch, falls = torch.stack([lab_d.min(), (lab_d % CHAN_MULT).max(), falls]).cpu().tolist()
+    return new, torch.nonzero(new).squeeze(1).cpu().numpy(), lo, ch, not falls
 
 
 def synthesize(chan, time, charge, tdc0_of_chan, cfg=WaveformConfig(), window=(0.0, 1e5), rng=None,
@@ -267,45 +289,56 @@ def synthesize(chan, time, charge, tdc0_of_chan, cfg=WaveformConfig(), window=(0
     rng (the reference draws sequential normals from rng).  Returns per digi chan, start, tdc0, starttdc,
     volt [D, 12], adc [D, 12] sorted by (label, start), and per cluster cluster_chan, cluster_tstart, cluster_keep in
     input order."""
+    torch = _torch()
     chan = np.asarray(chan)
     time = np.asarray(time, np.float64)
     charge = np.asarray(charge, np.float64)
     if not (len(chan) == len(time) == len(charge)):
         raise ValueError("chan, time and charge must have the same length")
-    if len(chan) and int(np.min(chan)) < 0:
+    n, lab_d = len(chan), None
+    if n and torch.cuda.is_available() and chan.dtype in _LABEL_TYPES:
+        lab_d, time_d = _dev(chan, np.int64), _dev(time, np.float64)
+        new_d, first, lo, ch, ascend = _charge_columns(lab_d, time_d, cfg)
+    else:
+        cid, first = charge_clusters(chan, time, cfg)
+        lab = chan.astype(np.int64)
+        lo, ch = (int(np.min(chan)), int(np.max(lab % CHAN_MULT))) if n else (0, 255)
+        ascend = not np.any(np.diff(lab) < 0)
+    if lo < 0:
         raise ValueError("channel labels must be non-negative")
     tmpl = single_pe_template(cfg)
-    cid, first = charge_clusters(chan, time, cfg)
     # the caller's TDC0 per cluster, evaluated batch by batch as the reference does
     tdc0_cl = np.zeros(len(first))
-    cuts = _part_starts(cid, first, int(max_charges)) if len(cid) else [0, 0]
-    for a, b in zip(cuts[:-1], cuts[1:]):
-        ca, cb = cid[a], cid[b - 1] + 1
+    cuts = _part_starts(n, first, int(max_charges)) if n else [0, 0]
+    for ca, cb in zip(cuts[:-1], cuts[1:]):
         cch = chan[first[ca:cb]]
         tdc0_cl[ca:cb] = tdc0_of_chan(cch) if callable(tdc0_of_chan) else np.asarray(tdc0_of_chan)[cch]
-    table = cluster_table(chan, time, tdc0_cl, cfg, tmpl, clusters=(cid, first))
+    nq = np.diff(np.append(first, n))
+    table = _cluster_rows(chan, time, first, nq, tdc0_cl, cfg, tmpl)
     # the device wants labels ascending: a stable sort keeps every label's time order and its clusters
-    lab = chan.astype(np.int64)
     order = None
-    if len(lab) > 1 and np.any(np.diff(lab) < 0):
+    if not ascend:
+        lab = chan.astype(np.int64)
         runs = 1 + int(np.count_nonzero(lab[1:] != lab[:-1]))
         if runs != len(np.unique(lab)):
             raise ValueError("charges must be grouped by channel label (each label's charges contiguous)")
         order = np.argsort(lab, kind="stable")
-    rows = tdc0_cl[cid] if len(cid) else np.zeros(0)
-    if order is not None:
-        lab, time, charge, rows = lab[order], time[order], charge[order], rows[order]
     from .geometry import default_conditions, module_geometry
-    nb = int(np.max(lab % CHAN_MULT)) // 4 + 1 if len(lab) else 64
-    geom = module_geometry(n_modules=max(1, (nb + 63) // 64))
+    geom = module_geometry(n_modules=max(1, (ch // 4 + 1 + 63) // 64))
     cond = cond if cond is not None else default_conditions(geom)
     cc = ChainConfig(waveform=cfg, window=window, noise=rng is not None or key is not None)
     validate_window(cc.window)
     seed = seed_of(rng, key)
     tabs = DeviceTables(geom, cond, cc)
     P = make_params(cc, seed, template_len=len(tmpl))
-    D = engine().run(P, tabs, _dev(lab, np.int64), _dev(time, np.float64), _dev(charge, np.float64),
-                     _dev(tmpl, np.float64), tdc0_rows=_dev(rows, np.float64))
+    if lab_d is None:
+        lab_d, time_d, rows_d = _dev(lab, np.int64), _dev(time, np.float64), _dev(tdc0_cl[cid], np.float64)
+    else:
+        rows_d = _dev(tdc0_cl, np.float64)[torch.cumsum(new_d, 0) - 1]
+    columns = [lab_d, time_d, _dev(charge, np.float64), rows_d]
+    if order is not None:
+        columns = [c[_dev(order, np.int64)] for c in columns]
+    D = engine().run(P, tabs, *columns[:3], _dev(tmpl, np.float64), tdc0_rows=columns[3])
     out = _host(D)
     out.update(table)
     return out

