@@ -653,7 +653,10 @@ static int digis_run(const CrvParams* p, const CrvChannels* ch, int64_t ncharges
   if (!out->volt) w.D.volt = nullptr;       // volts not asked for: the slots keep none either
   const long long* lab = reinterpret_cast<const long long*>(label);
   unsigned gq = grid_for(ncharges, 256, 8);
-  CK(exclusive_scan(LabelRuns{lab, w.gstart, w.glabel}, ncharges, nq_dev, scan_end(&w.totals[0]), w.parts, s));
+  int* const longest = reinterpret_cast<int*>(&w.totals[4]);
+  ScanEnd groups = scan_end(&w.totals[0]);
+  groups.clear = longest;
+  CK(exclusive_scan(LabelRuns{lab, w.gstart, w.glabel}, ncharges, nq_dev, groups, w.parts, s));
   {
     crv::Mark mark_("k_group_counts", s);
     k_group_counts<<<gq, 256, 0, s>>>(&w.totals[0], ncharges, nq_dev, w.gstart, w.glabel, w.gcount,
@@ -663,10 +666,10 @@ static int digis_run(const CrvParams* p, const CrvChannels* ch, int64_t ncharges
   WfGroups G{&w.totals[0], w.gstart, w.gcount, w.glabel, w.grun};
   if (p->precision == 1)
     CK(launch_wf_prepass<float>(*p, *ch, G, ncharges, time, tmpl, tlen, tdc0_rows, w.g_tdc0, w.g_bound,
-                                w.g_maxlen, w.g_nkept, w.dn, w.cl, S, s));
+                                w.g_maxlen, w.g_nkept, w.dn, longest, w.cl, S, s));
   else
     CK(launch_wf_prepass<double>(*p, *ch, G, ncharges, time, tmpl, tlen, tdc0_rows, w.g_tdc0, w.g_bound,
-                                 w.g_maxlen, w.g_nkept, w.dn, w.cl, S, s));
+                                 w.g_maxlen, w.g_nkept, w.dn, longest, w.cl, S, s));
   // synthesis only when the slots fit: it sees no groups otherwise
   CK(exclusive_scan(column(w.g_bound, w.slot_off), ncharges, &w.totals[0],
                     scan_end(&w.totals[1], slots_dev).check(S, CRV_NEED_DIGIS, slot_cap)
@@ -674,10 +677,10 @@ static int digis_run(const CrvParams* p, const CrvChannels* ch, int64_t ncharges
   G.n = &w.totals[2];
   if (p->precision == 1)
     CK(launch_wf_synth<float>(*p, G, ncharges, time, charge, tmpl, tlen, tdc0_rows, w.g_tdc0, w.g_maxlen,
-                              w.g_nkept, w.cl, w.D, S, s));
+                              w.g_nkept, longest, w.cl, w.D, S, s));
   else
     CK(launch_wf_synth<double>(*p, G, ncharges, time, charge, tmpl, tlen, tdc0_rows, w.g_tdc0, w.g_maxlen,
-                               w.g_nkept, w.cl, w.D, S, s));
+                               w.g_nkept, longest, w.cl, w.D, S, s));
   CK(exclusive_scan(column(w.dn, w.out_off), ncharges, &w.totals[2],
                     scan_end(&w.totals[3], n_out_dev).check(S, CRV_NEED_DIGIS_OUT, out_cap).guard(pass_dev, out_cap),
                     w.parts, s));

@@ -69,13 +69,14 @@ template <typename R>
 cudaError_t launch_wf_prepass(const CrvParams& p, const CrvChannels& ch, const WfGroups& G, long long ng_bound,
                               const double* time, const double* tmpl, int tlen, const double* tdc0_rows,
                               double* g_tdc0, int32_t* g_bound, int32_t* g_maxlen, int32_t* g_nkept,
-                              int32_t* g_digis, WfCluster* cl, Status* status, cudaStream_t s);
+                              int32_t* g_digis, int* longest, WfCluster* cl, Status* status, cudaStream_t s);
 
 template <typename R>
 cudaError_t launch_wf_synth(const CrvParams& p, const WfGroups& G, long long ng_bound, const double* time,
                             const double* charge, const double* tmpl, int tlen, const double* tdc0_rows,
                             const double* g_tdc0, const int32_t* g_maxlen, const int32_t* g_nkept,
-                            const WfCluster* cl, const DigiSlots& D, Status* status, cudaStream_t s);
+                            const int* longest, const WfCluster* cl, const DigiSlots& D, Status* status,
+                            cudaStream_t s);
 
 // The lookup-table photon model inside the resident chain: dense rows (row 4 step + SiPM of the output channel; a
 // row of no group has group -1), their arrival counts in the chain's per-(step, SiPM) count array, and the photons

@@ -92,6 +92,7 @@ struct ScanEnd {
   long long* pass = nullptr;           // set: *pass = the sum (pass_n set: *pass_n), or 0 when the sum is above pass_cap
   const long long* pass_n = nullptr;
   long long pass_cap = 0;
+  int* clear = nullptr;                // set: *clear = 0
 
   ScanEnd& check(Status* s, int need_slot, long long most) {
     status = s;
@@ -112,6 +113,7 @@ struct ScanEnd {
       set_flag(status, CRV_ST_CAPACITY);
       need_at_least(status, slot, sum);
     }
+    if (clear) *clear = 0;
     if (pass) *pass = sum <= pass_cap ? (pass_n ? *pass_n : sum) : 0;
   }
 };

@@ -13,13 +13,14 @@
 //   outputs      start and TDC0 of a digi are the fixed-point values converted exactly to double; volts are the
 //                FP32 sums widened exactly; ADC as the FP32 stage rule (adc_of_f).
 //
-// Two kernels, one warp per SiPM group each:
+// Three kernels:
 //   k_wf_prep     (crv_waveform.cuh) a tile of groups per warp: lanes over the groups (TDC0), over each group's charges (cluster split by
 //                 the gap test on consecutive fixed-point times, ballots), then over the clusters of all the tile's
 //                 groups, which wait in a shared queue: keep rule, start tick, length, window sample range, digi
 //                 bound; kept clusters are written to cl[group start + k] (the record layout of WfCluster, with the
 //                 fixed-point start in place of the double).  A group has 1.2 clusters, so group by group the
 //                 cluster work ran on one or two lanes (65,536 events: 6.1 -> 3.0 ms).
+//   k_wf_synth16  the same as k_wf_synth32 for groups whose clusters have at most 16 samples, two groups per warp;
 //   k_wf_synth32  per kept cluster: the charges' FP32 offsets from the cluster start and normalised charges are
 //                 staged in shared memory (coalesced loads), then lanes own samples (32 per tile) and sum the
 //                 template contributions of the staged charges in charge order (deterministic), keyed noise is
@@ -170,6 +171,171 @@ __host__ __device__ inline size_t wf32_smem_per_warp(int cap) {
   return (size_t(cap) * 4 + size_t(WF32_QS) * 12 + 15) & ~size_t(15);
 }
 
+// Per-block scalars of the synthesis (FP64 work once per block, in one thread) and the template in FP32
+struct WfBlock32 {
+  float tmpl[1024];
+  long long P_fx;
+  float P, inv_prec, inv_q, vthr, sigma, conv, off;
+  int nr;
+};
+__device__ __forceinline__ void wf_block32(const CrvParams& p, const double* tmpl, int tlen, WfBlock32& B) {
+  for (int i = threadIdx.x; i < tlen; i += blockDim.x) B.tmpl[i] = float(tmpl[i]);
+  if (threadIdx.x == 0) {
+    long long P;
+    B.P_fx = d2fx(p.period, &P) ? P : 0;
+    B.P = float(p.period);
+    B.inv_prec = float(1.0 / p.spe_precision);
+    B.inv_q = float(1.0 / p.spe_ref_charge);
+    B.vthr = float(p.min_voltage);
+    B.sigma = float(p.noise_sigma);
+    B.conv = float(p.adc_conversion);
+    B.off = float(double(p.adc_pedestal) + 0.5);
+    B.nr = reach_samples(p);
+  }
+  __syncthreads();
+}
+
+// Synthesis + zero suppression of the groups whose clusters have at most 16 samples: two groups per warp, a lane per
+// sample, the samples in registers, the neighbours' decisions in ballots.  Sums as k_wf_synth32's for such clusters: every
+// other charge of a chunk in a sum of its own, the two added.  Bound by instructions: about 1,040 a cluster where each has a
+// warp, most of them (noise, decisions, output, the cluster's scalars) on 10 to 14 lanes.  8.9 million clusters of 65,536
+// events, all passes: 11.07 -> 7.97 ms; 280,000 of 2,048 events 417 -> 359 us.  Up to `few` groups (a warp for each on the
+// chip) are left to k_wf_synth32, where two in turn on one warp would only take longer (1,900 groups: 24 against 47 us).
+constexpr int WF16_QS = WF32_QS;  // charges staged per chunk and group: the chunks of k_wf_synth32
+__global__ void __launch_bounds__(256, 4) k_wf_synth16(CrvParams p, WfGroups G, const double* __restrict__ time,
+                                                    const double* __restrict__ charge, const double* __restrict__ tmpl,
+                                                    int tlen, const double* __restrict__ tdc0_rows,
+                                                    const double* __restrict__ g_tdc0,
+                                                    const int32_t* __restrict__ g_maxlen,
+                                                    const int32_t* __restrict__ g_nkept,
+                                                    const WfCluster32* __restrict__ cl, long long few, DigiSlots D,
+                                                    Status* status) {
+  extern __shared__ __align__(16) char smem[];
+  __shared__ WfBlock32 B;
+  const long long ng = *G.n;
+  if (ng <= few) return;                       // a warp for each: left to k_wf_synth32
+  if (tlen > 1024) return;                     // refused by the host; the table must fit the shared copy
+  wf_block32(p, tmpl, tlen, B);
+  const int lane = lane_id(), half = lane >> 4, J = lane & 15, sh = half << 4;
+  // (time from the cluster start, normalised charge) of the half's charges; two are read at a time
+  float2* sq = reinterpret_cast<float2*>(smem) + (size_t(warp_in_block()) * 2 + half) * WF16_QS;
+  const long long P_fx = B.P_fx;
+  const int zs = p.samples_zs;
+  const float ip = B.inv_prec, inv_q = B.inv_q, vthr = B.vthr, sigma = B.sigma;
+  const float JP = __fmul_rn(float(J), B.P);   // rounded before the subtraction, never fused with it
+  const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
+  const int tile = tile_size(ng, warps);
+  for (long long g0 = (blockIdx.x * (long long)(blockDim.x >> 5) + warp_in_block()) * tile; g0 < ng; g0 += warps * tile) {
+   const bool in = lane < tile && g0 + lane < ng;
+   const int mll = in ? g_maxlen[g0 + lane] : 0;
+   unsigned todo = __ballot_sync(0xffffffffu, mll > 0 && mll <= 16);
+   while (todo) {
+    const int b0 = __ffs(todo) - 1;
+    todo &= todo - 1;
+    const int b1 = todo ? __ffs(todo) - 1 : -1;
+    if (todo) todo &= todo - 1;
+    const int bsel = half ? b1 : b0;
+    const bool valid = bsel >= 0;
+    const long long g = g0 + (valid ? bsel : b0);
+    const long long q0 = G.start[g];
+    const double* t = time + q0;
+    const double* qc = charge + q0;
+    const long long lab = G.label[g];
+    const uint32_t run = G.run ? G.run[g] : 0u;
+    const long long evk = lab / 32768;
+    const EvKey ek{uint32_t(evk & 0xFFFFF), uint32_t(evk >> 20), run};
+    const uint32_t chan = uint32_t(lab % 32768);
+    const double tdc0g = g_tdc0[g];
+    const long long slot = D.off[g];
+    const int scap = D.cap[g];
+    const int nk = valid ? g_nkept[g] : 0;
+    int nd = 0;
+#pragma unroll 1
+    for (int kc = 0; __any_sync(0xffffffffu, kc < nk); ++kc) {
+      const bool act = kc < nk;
+      WfCluster32 C{};
+      if (act) C = cl[q0 + kc];
+      const int L = C.L;
+      const long long k0 = C.k0, ts = C.ts_fx;
+      float wave = 0.0f;
+      int left = C.b - C.a, c0 = C.a;
+#pragma unroll 1
+      while (__any_sync(0xffffffffu, left > 0)) {
+        const int nq = min(WF16_QS, max(left, 0));
+        const int most = max(nq, __shfl_xor_sync(0xffffffffu, nq, 16));
+        __syncwarp();
+        for (int i = J; i < most + (most & 1); i += 16) {
+          float2 v = make_float2(3e38f, 0.0f);           // (behind the half's charges: later than every sample)
+          if (i < nq) {
+            long long tf = 0;
+            d2fx(t[c0 + i], &tf);
+            v = make_float2(fx2f(tf - ts), d2f_trunc(qc[c0 + i]) * inv_q);
+          }
+          sq[i] = v;
+        }
+        __syncwarp();
+        float even = 0.0f, odd = 0.0f;
+#pragma unroll 2
+        for (int q = 0; q < most; q += 2) {
+          const float4 v = *reinterpret_cast<const float4*>(sq + q);
+          // nearest integer of st / precision (ties to even) by the 1.5 x 2^23 shift; |st / precision| < 2^22
+          const float se = __fsub_rn(JP, v.x), so = __fsub_rn(JP, v.z);
+          const int te = __float_as_int(fmaf(se, ip, 12582912.0f)) - 0x4B400000;
+          const int to = __float_as_int(fmaf(so, ip, 12582912.0f)) - 0x4B400000;
+          if (se >= 0.0f && te < tlen) even = fmaf(B.tmpl[te], v.y, even);
+          if (so >= 0.0f && to < tlen) odd = fmaf(B.tmpl[to], v.w, odd);
+        }
+        wave = wave + (even + odd);
+        left -= WF16_QS;
+        c0 += WF16_QS;
+      }
+      // keyed electronics noise on every sample
+      if (p.noise_on && J < L) {
+        const long long tk = k0 + J;
+        U4 w = keyed(p.seed, ek, (ST_NOISE << 28) | (chan & 0x7FFFu), uint32_t(tk >> 1));
+        float z0, z1;
+        Math<float>::normal_pair(w, &z0, &z1);
+        wave = wave + sigma * ((tk & 1) ? z1 : z0);
+      }
+      // zero suppression: samples with one above the threshold among their neighbours up to two away, in the window
+      const unsigned over = (__ballot_sync(0xffffffffu, J < L && wave > vthr) >> sh) & 0xFFFFu;
+      const unsigned near = over | over << 1 | over << 2 | over >> 1 | over >> 2;
+      unsigned cand = (__ballot_sync(0xffffffffu, J < L && ((near >> J) & 1u) && J >= C.ilo && J <= C.ihi) >> sh) & 0xFFFFu;
+#pragma unroll 1
+      while (__any_sync(0xffffffffu, cand != 0u)) {
+        const bool on = cand != 0u;
+        const int i0 = on ? __ffs(cand) - 1 : 0;
+        const bool put = on && nd < scap;
+        const long long o = slot + nd;
+        for (int k = J; k - J < zs; k += 16) {
+          const int c = i0 + k;
+          const float x = __shfl_sync(0xffffffffu, wave, sh + (c & 15));
+          const float v = c < L ? x : 0.0f;
+          if (put && k < zs) {
+            if (D.volt) D.volt[o * zs + k] = f2d(v);
+            D.adc[o * zs + k] = adc_of_f(p, v, B.conv, B.off);
+          }
+        }
+        if (put && J == 0) {
+          D.chan[o] = lab;
+          D.start[o] = fx2d(ts + (long long)i0 * P_fx);
+          D.tdc0[o] = tdc0_rows ? tdc0_rows[q0 + C.a] : tdc0g;
+          D.starttdc[o] = k0 + i0;
+        }
+        if (on) {
+          ++nd;
+          cand = i0 + zs < 16 ? cand >> (i0 + zs) << (i0 + zs) : 0u;
+        }
+      }
+    }
+    if (valid && J == 0) {
+      D.n[g] = nd;
+      if (nd > scap) set_flag(status, CRV_ST_CAPACITY);
+    }
+   }
+  }
+}
+
 // Synthesis + zero suppression of the groups whose longest kept cluster is in (lo, cap] (FP32-mixed).
 __global__ void __launch_bounds__(256, 4) k_wf_synth32(CrvParams p, WfGroups G, const double* __restrict__ time,
                                                     const double* __restrict__ charge, const double* __restrict__ tmpl,
@@ -178,41 +344,29 @@ __global__ void __launch_bounds__(256, 4) k_wf_synth32(CrvParams p, WfGroups G, 
                                                     const int32_t* __restrict__ g_maxlen,
                                                     const int32_t* __restrict__ g_nkept,
                                                     const WfCluster32* __restrict__ cl, int lo, int cap,
-                                                    int last_pass, DigiSlots D, Status* status) {
+                                                    int last_pass, long long few, const int* __restrict__ longest,
+                                                    DigiSlots D, Status* status) {
   extern __shared__ __align__(16) char smem[];
-  __shared__ float tmpl_f[1024];
-  __shared__ long long P_fx_s;
+  if (lo >= WF_LONG && *longest <= lo) return;
+  __shared__ WfBlock32 B;
   char* wbase = smem + size_t(warp_in_block()) * wf32_smem_per_warp(cap);
   float* wave = reinterpret_cast<float*>(wbase);
   float2* sq = reinterpret_cast<float2*>(wbase + size_t(cap) * 4);              // (dt, normalised charge)
   int* sj = reinterpret_cast<int*>(wbase + size_t(cap) * 4 + size_t(WF32_QS) * 8);  // first sample reached
-  __shared__ float cf_s[7];
-  __shared__ int nr_s;
   if (tlen > 1024) return;                     // refused by the host; the table must fit the shared copy
-  for (int i = threadIdx.x; i < tlen; i += blockDim.x) tmpl_f[i] = float(tmpl[i]);
-  if (threadIdx.x == 0) {                      // FP64 scalars once per block, in one thread
-    long long P;
-    P_fx_s = d2fx(p.period, &P) ? P : 0;
-    cf_s[0] = float(p.period);
-    cf_s[1] = float(1.0 / p.spe_precision);
-    cf_s[2] = float(1.0 / p.spe_ref_charge);
-    cf_s[3] = float(p.min_voltage);
-    cf_s[4] = float(p.noise_sigma);
-    cf_s[5] = float(p.adc_conversion);
-    cf_s[6] = float(double(p.adc_pedestal) + 0.5);
-    nr_s = reach_samples(p);
-  }
-  __syncthreads();
-  const long long P_fx = P_fx_s;
-  const int nr = nr_s;
+  wf_block32(p, tmpl, tlen, B);
+  const float* const tmpl_f = B.tmpl;
+  const long long P_fx = B.P_fx;
+  const int nr = B.nr;
   const int zs = p.samples_zs;
   const int lane = lane_id();
-  const float Pf = cf_s[0], ip = cf_s[1];
-  const float inv_q = cf_s[2];
-  const float vthr = cf_s[3];
-  const float sigma = cf_s[4];
-  const float conv_f = cf_s[5], off_f = cf_s[6];
+  const float Pf = B.P, ip = B.inv_prec;
+  const float inv_q = B.inv_q;
+  const float vthr = B.vthr;
+  const float sigma = B.sigma;
+  const float conv_f = B.conv, off_f = B.off;
   const long long ng = *G.n;
+  if (ng <= few && lo == 16) lo = 0;           // (k_wf_synth16 leaves them to this kernel)
   const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
   // groups in tiles per warp: one coalesced load of their longest clusters and a ballot pick this pass's groups
   const int tile = tile_size(ng, warps);
