@@ -932,13 +932,15 @@ __device__ __forceinline__ void put_hit(const CrvParams& p, const CoincGeom& G, 
 // Events with at most COINC_HCAP hits, one warp each, everything in shared memory; the others are marked deferred.
 __global__ void __launch_bounds__(32, 16) k_coinc(const __grid_constant__ CrvParams p,
                                                  const __grid_constant__ CoincGeom G, CoincIn I,
-                                                 const __grid_constant__ CoincOut O, int32_t* __restrict__ deferred) {
+                                                 const __grid_constant__ CoincOut O, int32_t* __restrict__ deferred,
+                                                 int* __restrict__ taken) {
   extern __shared__ __align__(16) char smem[];
   constexpr int hcap = COINC_HCAP;
   const CoincShared S = coinc_carve(smem, hcap);
   const CoincWork W = work_carve(smem + coinc_smem_per_warp(hcap), hcap, S);
   const long long nev = bounded_count(I.nev, I.nev_dev);
-  for (long long e = blockIdx.x; e < nev; e += gridDim.x) {
+  // (events differ in their work: each block takes the next one when it is done, taken null when every event has a block)
+  for (long long e = blockIdx.x; e < nev; e = taken ? next_tile(taken, gridDim.x) : nev) {
     const long long r0 = I.ev_start[e];
     const int np_ = I.ev_count[e];
     int H = 0;                                     // hits in pulse order

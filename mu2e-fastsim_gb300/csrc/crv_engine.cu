@@ -92,8 +92,9 @@ __global__ void k_sipm_diag(const long long* __restrict__ nsipm_dev, long long c
 // charge slots per group of photons; *n = ng for the kernels after it; counts cleared (groups without photons keep them)
 __global__ void k_slot_caps(long long ng, const int32_t* __restrict__ gcount, int factor, int32_t* __restrict__ cap,
                             int32_t* __restrict__ nmain, int32_t* __restrict__ nap, int32_t* __restrict__ fired,
-                            long long* __restrict__ n) {
+                            long long* __restrict__ n, int* __restrict__ taken) {
   if (blockIdx.x == 0 && threadIdx.x == 0) *n = ng;
+  if (blockIdx.x == 0 && threadIdx.x < RESP_COUNTS) taken[threadIdx.x] = 0;
   for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < ng; g += (long long)gridDim.x * blockDim.x) {
     cap[g] = gcount[g] > 0 ? factor * gcount[g] + 16 : 0;
     nmain[g] = 0;
@@ -399,9 +400,12 @@ static int response_run(const CrvParams* p, const CrvEvents* ev, int64_t nevents
                                                         w.id_base, w.label, w.run, w.nmain, w.nap, w.fired);
   }
   CK(cudaGetLastError());
-  CK(exclusive_scan(Columns{w.nphot, w.slot_cap, w.ph_off, w.slot_off}, w.nb, &w.totals[0],
-                    ScanEnds{{scan_end(&w.totals[1], photons_dev).check(S, CRV_NEED_PHOTONS_TOTAL, w.pc),
-                              scan_end(&w.totals[2]).check(S, CRV_NEED_SLOTS_TOTAL, w.sc)}}, w.parts, s));
+  ScanEnds sizes{{scan_end(&w.totals[1], photons_dev).check(S, CRV_NEED_PHOTONS_TOTAL, w.pc),
+                  scan_end(&w.totals[2]).check(S, CRV_NEED_SLOTS_TOTAL, w.sc)}};
+  int* const taken = reinterpret_cast<int*>(&w.totals[4]);
+  sizes.e[0].clear = taken;
+  sizes.e[0].nclear = RESP_COUNTS;
+  CK(exclusive_scan(Columns{w.nphot, w.slot_cap, w.ph_off, w.slot_off}, w.nb, &w.totals[0], sizes, w.parts, s));
   // 6. photons of every SiPM (lookup model: each row's photons at the offset of its step in its SiPM)
   if (lk) {
     CK(cudaMemsetAsync(w.lk.row_off, 0xFF, sizeof(long long) * size_t(w.nb), s));
@@ -414,10 +418,12 @@ static int response_run(const CrvParams* p, const CrvEvents* ev, int64_t nevents
     CK(lookup_chain_emit(*lk, w.lk, w.nb, &w.totals[1], w.pc, S, s));
   } else if (p->precision == 1)
     CK(launch_photon_emit<float>(*p, *ev, *st, *bars, w.nb, &w.totals[0], w.s_event, w.s_chan, w.s_seg, w.s_nseg,
-                                 w.step_order, w.count, w.ph_off, (float*)w.ph_t, w.ph_key, &w.totals[1], w.pc, s));
+                                 w.step_order, w.count, w.ph_off, (float*)w.ph_t, w.ph_key, &w.totals[1], w.pc,
+                                 taken + SIPM_PASSES, s));
   else
     CK(launch_photon_emit<double>(*p, *ev, *st, *bars, w.nb, &w.totals[0], w.s_event, w.s_chan, w.s_seg, w.s_nseg,
-                                  w.step_order, w.count, w.ph_off, (double*)w.ph_t, w.ph_key, &w.totals[1], w.pc, s));
+                                  w.step_order, w.count, w.ph_off, (double*)w.ph_t, w.ph_key, &w.totals[1], w.pc,
+                                  taken + SIPM_PASSES, s));
   // 7. SiPM simulation
   SipmGroups G{};
   G.n = &w.totals[0];
@@ -433,6 +439,7 @@ static int response_run(const CrvParams* p, const CrvEvents* ev, int64_t nevents
   G.key64 = nullptr;
   G.photon_id = lk ? reinterpret_cast<const long long*>(w.lk.o_step) : nullptr;
   G.id_base = w.id_base;
+  G.taken = taken;
   G.slot_off = w.slot_off;
   G.slot_cap = w.slot_cap;
   SipmOut O{w.slot_t, w.slot_v, w.slot_id, w.nmain, w.nap, w.fired};
@@ -448,10 +455,10 @@ static int response_run(const CrvParams* p, const CrvEvents* ev, int64_t nevents
                     w.parts, s));
   {
     crv::Mark mark_("k_charge_compact", s);
-    k_charge_compact<<<grid_for(w.nb, 8, 16), 256, 0, s>>>(&w.totals[0], w.label, w.slot_off, w.slot_cap, w.nmain,
+    k_charge_compact<<<grid_for(w.nb, 8, 8), 256, 0, s>>>(&w.totals[0], w.label, w.slot_off, w.slot_cap, w.nmain,
                                                             w.nap, w.out_off, w.slot_t, w.slot_v, w.slot_id,
                                                             p->capacitance, p->overvoltage, p->precision == 1,
-                                                            *out, out_cap);
+                                                            *out, out_cap, G.taken + SIPM_PASSES + 1);
   }
   CK(cudaGetLastError());
   if (sipm_label || sipm_photons || sipm_fired)
@@ -536,7 +543,7 @@ extern "C" int crv_sipm(const CrvParams* p, const CrvPixels* px, int64_t ngroups
   {
     crv::Mark mark_("k_slot_caps", s);
     k_slot_caps<<<grid_for(ngroups, 256, 8), 256, 0, s>>>(ngroups, gcount, factor, w.slot_cap, w.nmain, w.nap, g_fired,
-                                                          &w.totals[0]);
+                                                          &w.totals[0], reinterpret_cast<int*>(&w.totals[4]));
   }
   CK(cudaGetLastError());
   CK(exclusive_scan(column(w.slot_cap, w.slot_off), ngroups, nullptr,
@@ -554,6 +561,7 @@ extern "C" int crv_sipm(const CrvParams* p, const CrvPixels* px, int64_t ngroups
   G.key64 = reinterpret_cast<const long long*>(key);
   G.photon_id = reinterpret_cast<const long long*>(photon);
   G.id_base = nullptr;
+  G.taken = reinterpret_cast<int*>(&w.totals[4]);
   G.slot_off = w.slot_off;
   G.slot_cap = w.slot_cap;
   SipmOut O{w.slot_t, w.slot_v, w.slot_id, w.nmain, w.nap, g_fired};
@@ -565,10 +573,10 @@ extern "C" int crv_sipm(const CrvParams* p, const CrvPixels* px, int64_t ngroups
                     scan_end(&w.totals[3], n_out_dev).check(S, CRV_NEED_CHARGES_OUT, out_cap), w.parts, s));
   {
     crv::Mark mark_("k_charge_compact", s);
-    k_charge_compact<<<grid_for(ngroups, 8, 16), 256, 0, s>>>(&w.totals[0], G.label, w.slot_off, w.slot_cap, w.nmain,
+    k_charge_compact<<<grid_for(ngroups, 8, 8), 256, 0, s>>>(&w.totals[0], G.label, w.slot_off, w.slot_cap, w.nmain,
                                                                w.nap, w.out_off, w.slot_t, w.slot_v, w.slot_id,
                                                                p->capacitance, p->overvoltage, p->precision == 1,
-                                                            *out, out_cap);
+                                                            *out, out_cap, G.taken + SIPM_PASSES + 1);
   }
   CK(cudaGetLastError());
   CK(cudaGetLastError());
@@ -655,7 +663,9 @@ static int digis_run(const CrvParams* p, const CrvChannels* ch, int64_t ncharges
   unsigned gq = grid_for(ncharges, 256, 8);
   int* const longest = reinterpret_cast<int*>(&w.totals[4]);
   ScanEnd groups = scan_end(&w.totals[0]);
-  groups.clear = longest;
+  groups.clear = longest;                   // and the counts of tiles taken (prepass, synthesis passes)
+  groups.nclear = 6;
+  int* const taken = longest + 1;
   CK(exclusive_scan(LabelRuns{lab, w.gstart, w.glabel}, ncharges, nq_dev, groups, w.parts, s));
   {
     crv::Mark mark_("k_group_counts", s);
@@ -666,10 +676,10 @@ static int digis_run(const CrvParams* p, const CrvChannels* ch, int64_t ncharges
   WfGroups G{&w.totals[0], w.gstart, w.gcount, w.glabel, w.grun};
   if (p->precision == 1)
     CK(launch_wf_prepass<float>(*p, *ch, G, ncharges, time, tmpl, tlen, tdc0_rows, w.g_tdc0, w.g_bound,
-                                w.g_maxlen, w.g_nkept, w.dn, longest, w.cl, S, s));
+                                w.g_maxlen, w.g_nkept, w.dn, longest, taken, w.cl, S, s));
   else
     CK(launch_wf_prepass<double>(*p, *ch, G, ncharges, time, tmpl, tlen, tdc0_rows, w.g_tdc0, w.g_bound,
-                                 w.g_maxlen, w.g_nkept, w.dn, longest, w.cl, S, s));
+                                 w.g_maxlen, w.g_nkept, w.dn, longest, taken, w.cl, S, s));
   // synthesis only when the slots fit: it sees no groups otherwise
   CK(exclusive_scan(column(w.g_bound, w.slot_off), ncharges, &w.totals[0],
                     scan_end(&w.totals[1], slots_dev).check(S, CRV_NEED_DIGIS, slot_cap)
@@ -677,10 +687,10 @@ static int digis_run(const CrvParams* p, const CrvChannels* ch, int64_t ncharges
   G.n = &w.totals[2];
   if (p->precision == 1)
     CK(launch_wf_synth<float>(*p, G, ncharges, time, charge, tmpl, tlen, tdc0_rows, w.g_tdc0, w.g_maxlen,
-                              w.g_nkept, longest, w.cl, w.D, S, s));
+                              w.g_nkept, longest, taken, w.cl, w.D, S, s));
   else
     CK(launch_wf_synth<double>(*p, G, ncharges, time, charge, tmpl, tlen, tdc0_rows, w.g_tdc0, w.g_maxlen,
-                               w.g_nkept, longest, w.cl, w.D, S, s));
+                               w.g_nkept, longest, taken, w.cl, w.D, S, s));
   CK(exclusive_scan(column(w.dn, w.out_off), ncharges, &w.totals[2],
                     scan_end(&w.totals[3], n_out_dev).check(S, CRV_NEED_DIGIS_OUT, out_cap).guard(pass_dev, out_cap),
                     w.parts, s));
@@ -1029,8 +1039,10 @@ static int coinc_run(const CrvParams* p, const CrvFinderGeom* g, int64_t nevents
   CK(allow_dynamic_smem(k_coinc));
   {
     const long long maxb = (long long)di.sms * 16;
+    int* const taken = nevents > maxb ? reinterpret_cast<int*>(&w.totals[4]) : nullptr;
+    if (taken) CK(cudaMemsetAsync(taken, 0, sizeof(int), s));
     crv::Mark mark_("k_coinc", s);
-    k_coinc<<<(unsigned)(nevents < maxb ? nevents : maxb), 32, smem, s>>>(*p, G, I, O, w.deferred);
+    k_coinc<<<(unsigned)(nevents < maxb ? nevents : maxb), 32, smem, s>>>(*p, G, I, O, w.deferred, taken);
   }
   CK(cudaGetLastError());
   {

@@ -52,7 +52,8 @@ cudaError_t launch_photon_emit(const CrvParams& p, const CrvEvents& ev, const Cr
                                long long nsipm_bound, const long long* nsipm_dev, const int32_t* s_event,
                                const int32_t* s_chan, const long long* s_seg, const int32_t* s_nseg,
                                const int32_t* step_order, const int32_t* count, const long long* ph_off, R* ph_t,
-                               uint32_t* ph_key, const long long* ph_total, long long ph_cap, cudaStream_t s);
+                               uint32_t* ph_key, const long long* ph_total, long long ph_cap, int* taken,
+                               cudaStream_t s);
 
 template <typename R>
 cudaError_t launch_photon_rows(const CrvParams& p, const CrvEvents& ev, const CrvSteps& st, const CrvBars& bars,
@@ -69,13 +70,13 @@ template <typename R>
 cudaError_t launch_wf_prepass(const CrvParams& p, const CrvChannels& ch, const WfGroups& G, long long ng_bound,
                               const double* time, const double* tmpl, int tlen, const double* tdc0_rows,
                               double* g_tdc0, int32_t* g_bound, int32_t* g_maxlen, int32_t* g_nkept,
-                              int32_t* g_digis, int* longest, WfCluster* cl, Status* status, cudaStream_t s);
+                              int32_t* g_digis, int* longest, int* taken, WfCluster* cl, Status* status, cudaStream_t s);
 
 template <typename R>
 cudaError_t launch_wf_synth(const CrvParams& p, const WfGroups& G, long long ng_bound, const double* time,
                             const double* charge, const double* tmpl, int tlen, const double* tdc0_rows,
                             const double* g_tdc0, const int32_t* g_maxlen, const int32_t* g_nkept,
-                            const int* longest, const WfCluster* cl, const DigiSlots& D, Status* status,
+                            const int* longest, int* taken, const WfCluster* cl, const DigiSlots& D, Status* status,
                             cudaStream_t s);
 
 // The lookup-table photon model inside the resident chain: dense rows (row 4 step + SiPM of the output channel; a

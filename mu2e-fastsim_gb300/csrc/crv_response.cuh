@@ -349,7 +349,9 @@ struct SipmGroups {
   const long long* id_base;
   const long long* slot_off;     // output slot region of the group
   const int32_t* slot_cap;
+  int* taken;                    // counts of tiles taken, one for each pass that hands them out (zeroed before)
 };
+constexpr int SIPM_PASSES = 2, RESP_COUNTS = SIPM_PASSES + 2;   // counts of tiles taken: passes, photons, compaction
 
 struct SipmOut {
   double* t;
@@ -1171,9 +1173,9 @@ __global__ void __launch_bounds__(sipm_block_warps<R>(CAP) * 32, CAP <= 256 ? 2 
   // groups in tiles per warp: one coalesced load of their counts and a ballot pick the groups of this pass (a
   // later pass, which holds few groups, does not walk every group with a dependent load)
   const int tile = tile_size(ngroups, warps);
-  for (long long g0 = (blockIdx.x * (long long)(blockDim.x >> 5) + warp_in_block()) * tile; g0 < ngroups;
-       g0 += warps * tile) {
-   const long long gl = g0 + lane_id();
+  for (long long ti = blockIdx.x * (long long)(blockDim.x >> 5) + warp_in_block(); ti * tile < ngroups;
+       ti = CAP > 1024 ? ti + warps : next_tile(G.taken + (CAP > 256), warps)) {
+   const long long g0 = ti * tile, gl = g0 + lane_id();
    const bool in = lane_id() < tile && gl < ngroups;
    const int cl = in ? G.count[gl] : 0;
    unsigned todo = __ballot_sync(FULL, in && cl > lo);
@@ -1271,17 +1273,18 @@ __global__ void k_charge_compact(const long long* __restrict__ ngroups_dev, cons
                                  const int32_t* __restrict__ nmain, const int32_t* __restrict__ nap,
                                  const long long* __restrict__ out_off, const double* __restrict__ st,
                                  const double* __restrict__ sv, const long long* __restrict__ sid, double capacitance,
-                                 double overvoltage, int fp32, CrvCharges out, long long out_cap) {
+                                 double overvoltage, int fp32, CrvCharges out, long long out_cap,
+                                 int* __restrict__ taken) {
   // out.pe and out.photon may be null (the resident chain reads label, time and charge only): not written
   // FP32-mixed: voltages are FP32 values; charge and PE in FP32 (no FP64 multiply and division per charge)
   const float cap_f = float(capacitance), inv_vov_f = 1.0f / float(overvoltage);
   long long ngroups = *ngroups_dev;
   long long warps = (long long)gridDim.x * (blockDim.x >> 5);
   // groups in tiles per warp: one coalesced load of their sizes and offsets, then the non-empty ones in order
-  const int tile = tile_size(ngroups, warps);
-  for (long long g0 = (blockIdx.x * (long long)(blockDim.x >> 5) + warp_in_block()) * tile; g0 < ngroups;
-       g0 += warps * tile) {
-   const long long gl = g0 + lane_id();
+  const int tile = tile_taken(ngroups, warps);
+  for (long long ti = blockIdx.x * (long long)(blockDim.x >> 5) + warp_in_block(); ti * tile < ngroups;
+       ti = next_tile(taken, warps)) {
+   const long long g0 = ti * tile, gl = g0 + lane_id();
    int nm_l = 0, na_l = 0;
    long long s0_l = 0, o0_l = 0, lab_l = 0;
    bool ok = false;

@@ -92,7 +92,8 @@ struct ScanEnd {
   long long* pass = nullptr;           // set: *pass = the sum (pass_n set: *pass_n), or 0 when the sum is above pass_cap
   const long long* pass_n = nullptr;
   long long pass_cap = 0;
-  int* clear = nullptr;                // set: *clear = 0
+  int* clear = nullptr;                // set: nclear counts from here are zeroed
+  int nclear = 1;
 
   ScanEnd& check(Status* s, int need_slot, long long most) {
     status = s;
@@ -113,7 +114,8 @@ struct ScanEnd {
       set_flag(status, CRV_ST_CAPACITY);
       need_at_least(status, slot, sum);
     }
-    if (clear) *clear = 0;
+    if (clear)
+      for (int k = 0; k < nclear; ++k) clear[k] = 0;
     if (pass) *pass = sum <= pass_cap ? (pass_n ? *pass_n : sum) : 0;
   }
 };

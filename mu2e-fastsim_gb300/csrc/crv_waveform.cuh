@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(256, 3) k_wf_prep(CrvParams p, CrvChannels ch,
                                                  int tlen, const double* __restrict__ tdc0_rows,
                                                  double* __restrict__ g_tdc0, int32_t* __restrict__ g_bound,
                                                  int32_t* __restrict__ g_maxlen, int32_t* __restrict__ g_nkept,
-                                                 int32_t* __restrict__ g_digis, int* __restrict__ longest,
+                                                 int32_t* __restrict__ g_digis, int* __restrict__ longest, int* __restrict__ taken,
                                                  typename Prep::Record* __restrict__ cl, Status* status) {
   __shared__ PrepQueue queue[8];
   __shared__ typename Prep::Consts K_s;
@@ -210,8 +210,10 @@ __global__ void __launch_bounds__(256, 3) k_wf_prep(CrvParams p, CrvChannels ch,
   PrepQueue& Q = queue[warp_in_block()];
   const long long ng = *G.n;
   const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
-  const int tile = tile_size(ng, warps);
-  for (long long g0 = (blockIdx.x * (long long)(blockDim.x >> 5) + warp_in_block()) * tile; g0 < ng; g0 += warps * tile) {
+  const int tile = tile_taken(ng, warps);
+  for (long long ti = blockIdx.x * (long long)(blockDim.x >> 5) + warp_in_block(); ti * tile < ng;
+       ti = next_tile(taken, warps)) {
+    const long long g0 = ti * tile;
     // lane = group of the tile: its rows and its keyed TDC0 (unless the caller gives one per cluster)
     const int ntile = int(min((long long)tile, ng - g0));
     const long long gl = g0 + lane;
@@ -496,7 +498,8 @@ __global__ void __launch_bounds__(256, 3) k_wf_synth(CrvParams p, WfGroups G, co
                                                   const int32_t* __restrict__ g_maxlen,
                                                   const int32_t* __restrict__ g_nkept,
                                                   const WfCluster* __restrict__ cl, int lo, int cap, int last_pass,
-                                                  const int* __restrict__ longest, DigiSlots D, Status* status) {
+                                                  const int* __restrict__ longest, int* __restrict__ taken,
+                                                  DigiSlots D, Status* status) {
   extern __shared__ __align__(16) char smem[];
   if (lo >= WF_LONG && *longest <= lo) return;
   char* wbase = smem + size_t(warp_in_block()) * wf_smem_per_warp(cap);
@@ -518,9 +521,17 @@ __global__ void __launch_bounds__(256, 3) k_wf_synth(CrvParams p, WfGroups G, co
   const int lane = lane_id();
   long long ng = *G.n;
   long long warps = (long long)gridDim.x * (blockDim.x >> 5);
-  for (long long g = blockIdx.x * (long long)(blockDim.x >> 5) + warp_in_block(); g < ng; g += warps) {
-    int ml = g_maxlen[g];
-    if (ml <= lo) continue;
+  // groups in tiles per warp: one coalesced load of their longest clusters and a ballot pick this pass's groups
+  const int tile = tile_taken(ng, warps);
+  for (long long ti = blockIdx.x * (long long)(blockDim.x >> 5) + warp_in_block(); ti * tile < ng;
+       ti = next_tile(taken, warps)) {
+   const int mll = lane < tile && ti * tile + lane < ng ? g_maxlen[ti * tile + lane] : 0;
+   unsigned todo = __ballot_sync(0xffffffffu, mll > lo);
+   while (todo) {
+    const int bsel = __ffs(todo) - 1;
+    todo &= todo - 1;
+    const long long g = ti * tile + bsel;
+    const int ml = __shfl_sync(0xffffffffu, mll, bsel);
     if (ml > cap) {
       if (last_pass && lane == 0) {
         set_flag(status, CRV_ST_CAPACITY);
@@ -671,6 +682,7 @@ __global__ void __launch_bounds__(256, 3) k_wf_synth(CrvParams p, WfGroups G, co
       D.n[g] = nd;
       if (nd > scap) set_flag(status, CRV_ST_CAPACITY);
     }
+   }
   }
 }
 

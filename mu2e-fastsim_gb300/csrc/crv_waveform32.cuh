@@ -208,8 +208,8 @@ __global__ void __launch_bounds__(256, 4) k_wf_synth16(CrvParams p, WfGroups G, 
                                                     const double* __restrict__ g_tdc0,
                                                     const int32_t* __restrict__ g_maxlen,
                                                     const int32_t* __restrict__ g_nkept,
-                                                    const WfCluster32* __restrict__ cl, long long few, DigiSlots D,
-                                                    Status* status) {
+                                                    const WfCluster32* __restrict__ cl, long long few,
+                                                    int* __restrict__ taken, DigiSlots D, Status* status) {
   extern __shared__ __align__(16) char smem[];
   __shared__ WfBlock32 B;
   const long long ng = *G.n;
@@ -224,8 +224,10 @@ __global__ void __launch_bounds__(256, 4) k_wf_synth16(CrvParams p, WfGroups G, 
   const float ip = B.inv_prec, inv_q = B.inv_q, vthr = B.vthr, sigma = B.sigma;
   const float JP = __fmul_rn(float(J), B.P);   // rounded before the subtraction, never fused with it
   const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
-  const int tile = tile_size(ng, warps);
-  for (long long g0 = (blockIdx.x * (long long)(blockDim.x >> 5) + warp_in_block()) * tile; g0 < ng; g0 += warps * tile) {
+  const int tile = tile_taken(ng, warps);
+  for (long long ti = blockIdx.x * (long long)(blockDim.x >> 5) + warp_in_block(); ti * tile < ng;
+       ti = next_tile(taken, warps)) {
+   const long long g0 = ti * tile;
    const bool in = lane < tile && g0 + lane < ng;
    const int mll = in ? g_maxlen[g0 + lane] : 0;
    unsigned todo = __ballot_sync(0xffffffffu, mll > 0 && mll <= 16);
@@ -345,7 +347,7 @@ __global__ void __launch_bounds__(256, 4) k_wf_synth32(CrvParams p, WfGroups G, 
                                                     const int32_t* __restrict__ g_nkept,
                                                     const WfCluster32* __restrict__ cl, int lo, int cap,
                                                     int last_pass, long long few, const int* __restrict__ longest,
-                                                    DigiSlots D, Status* status) {
+                                                    int* __restrict__ taken, DigiSlots D, Status* status) {
   extern __shared__ __align__(16) char smem[];
   if (lo >= WF_LONG && *longest <= lo) return;
   __shared__ WfBlock32 B;
@@ -369,8 +371,10 @@ __global__ void __launch_bounds__(256, 4) k_wf_synth32(CrvParams p, WfGroups G, 
   if (ng <= few && lo == 16) lo = 0;           // (k_wf_synth16 leaves them to this kernel)
   const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
   // groups in tiles per warp: one coalesced load of their longest clusters and a ballot pick this pass's groups
-  const int tile = tile_size(ng, warps);
-  for (long long g0 = (blockIdx.x * (long long)(blockDim.x >> 5) + warp_in_block()) * tile; g0 < ng; g0 += warps * tile) {
+  const int tile = tile_taken(ng, warps);
+  for (long long ti = blockIdx.x * (long long)(blockDim.x >> 5) + warp_in_block(); ti * tile < ng;
+       ti = next_tile(taken, warps)) {
+   const long long g0 = ti * tile;
    const long long gl = g0 + lane;
    const bool in = lane < tile && gl < ng;
    const int mll = in ? g_maxlen[gl] : 0;
