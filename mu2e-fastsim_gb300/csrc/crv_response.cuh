@@ -263,22 +263,15 @@ __global__ void k_sipm_sizes(const long long* __restrict__ nsipm_dev, const int3
 
 #endif  // CRV_ENGINE_TU
 
-// Emission delays, in decay times, of photons c0 + lane of a row of n photons (c0 a multiple of 32; every lane of the
-// warp calls it): the order statistics of n exponential delays by the Renyi representation, S_j = sum_{i <= j} X_i /
-// (n - i) with X_i = -log u_i and u_i photon i's keyed uniform.  The delays have the distribution of n independent
-// exponential delays; photon j (key j) takes the j-th smallest, so every row's photons come out in time order.  Sums:
-// an inclusive Hillis-Steele scan over the chunk's lanes (offsets 1, 2, 4, 8, 16), the earlier chunks' total (*carry,
-// updated) in front; the CPU oracle adds in the same order, so FP64 sums are identical.
+// Emission delays, in decay times, of a row of n photons (every lane of the warp calls it): the order statistics of n
+// exponential delays by the Renyi representation, S_j = sum_{i <= j} X_i / (n - i) with X_i = -log u_i and u_i photon i's
+// keyed uniform.  The delays have the distribution of n independent exponential delays; photon j (key j) takes the j-th
+// smallest, so every row's photons come out in time order.  Sums: over 32 photons at a time an inclusive Hillis-Steele
+// scan (offsets 1, 2, 4, 8, 16), the earlier ones' total in front; the CPU oracle adds in the same order, so FP64 sums are
+// identical.  A Philox block holds two photons' uniforms: a lane draws for two photons where more than 32 are left, and
+// the terms move to the lanes of the scans.  emit(j, S_j) is called by the lane of photon j.
 template <typename R>
-__device__ __forceinline__ R row_delay_chunk(uint32_t seed, const EvKey& ek, uint32_t chan, uint32_t sie, int n, int c0,
-                                             R* carry) {
-  using M = Math<R>;
-  const int j = c0 + lane_id();
-  R v = R(0);
-  if (j < n) {
-    U4 w = keyed(seed, ek, w2_of(ST_PHOTON, 0, 0, 0, chan), (sie << 16) | uint32_t(j >> 1));
-    v = (-M::log(M::uni_open(w, j & 1))) / R(n - j);
-  }
+__device__ __forceinline__ R delay_sums(R v, R* carry) {
 #pragma unroll
   for (int off = 1; off < 32; off <<= 1) {
     const R y = __shfl_up_sync(0xffffffffu, v, off);
@@ -288,42 +281,33 @@ __device__ __forceinline__ R row_delay_chunk(uint32_t seed, const EvKey& ek, uin
   *carry = *carry + __shfl_sync(0xffffffffu, v, 31);
   return S;
 }
-
-// photons of each SiPM, contiguous from ph_off[g]: (time, key = step-in-event << 16 | photon)
-template <typename R>
-__global__ void k_photon_emit(CrvParams p, CrvEvents ev, CrvSteps st, CrvBars bars, long long nsipm,
-                              const int32_t* __restrict__ s_event, const int32_t* __restrict__ s_chan,
-                              const long long* __restrict__ s_seg, const int32_t* __restrict__ s_nseg,
-                              const int32_t* __restrict__ step_order, const int32_t* __restrict__ count,
-                              const long long* __restrict__ ph_off, R* __restrict__ ph_t,
-                              uint32_t* __restrict__ ph_key) {
-  long long warps = (long long)gridDim.x * (blockDim.x >> 5);
-  for (long long g = blockIdx.x * (long long)(blockDim.x >> 5) + warp_in_block(); g < nsipm; g += warps) {
-    int c = s_chan[g], s = c & 3, e = s_event[g];
-    EvKey ek{ev.event[e], ev.subrun[e], ev.run[e]};
-    long long f = ev.first_step[e];
-    long long o = ph_off[g];
-    for (int k = 0; k < s_nseg[g]; ++k) {
-      long long i = step_order[s_seg[g] + k];
-      int n = count[4 * i + s];
-      if (n == 0) continue;
-      uint32_t sie = uint32_t(i - f);
-      int b = st.bar[i];
-      int ax = bars.length_axis[b];
-      double z = step_real(st, ax == 0 ? st.x : (ax == 1 ? st.y : st.z), i) - bars.center_l[b];
-      R d = readout_distance(R(z), R(bars.half_l[b]), s);
-      R t = R(step_real(st, st.t, i));
-      R dt = d / R(p.signal_speed);
-      R carry = R(0);
-      for (int c0 = 0; c0 < n; c0 += 32) {
-        const R S = row_delay_chunk<R>(p.seed, ek, uint32_t(c), sie, n, c0, &carry);
-        const int j = c0 + lane_id();
-        if (j < n) {
-          ph_t[o + j] = t + dt + R(p.decay_time) * S;
-          ph_key[o + j] = (sie << 16) | uint32_t(j);
-        }
-      }
-      o += n;
+template <typename R, typename Emit>
+__device__ __forceinline__ void row_delays(uint32_t seed, const EvKey& ek, uint32_t chan, uint32_t sie, int n, Emit emit) {
+  using M = Math<R>;
+  const int lane = lane_id();
+  const uint32_t w2 = w2_of(ST_PHOTON, 0, 0, 0, chan);
+  R carry = R(0);
+  for (int c0 = 0; c0 < n; c0 += 64) {
+    const bool two = n - c0 > 32;
+    const int j0 = c0 + (two ? 2 * lane : lane);
+    R x0 = R(0), x1 = R(0);
+    if (j0 < n) {
+      const U4 w = keyed(seed, ek, w2, (sie << 16) | uint32_t(j0 >> 1));
+      x0 = (-M::log(M::uni_open(w, two ? 0 : j0 & 1))) / R(n - j0);
+      if (two && j0 + 1 < n) x1 = (-M::log(M::uni_open(w, 1))) / R(n - j0 - 1);
+    }
+    R a = x0, b = R(0);
+    if (two) {
+      const R e0 = __shfl_sync(0xffffffffu, x0, lane >> 1), e1 = __shfl_sync(0xffffffffu, x1, lane >> 1);
+      const R f0 = __shfl_sync(0xffffffffu, x0, 16 + (lane >> 1)), f1 = __shfl_sync(0xffffffffu, x1, 16 + (lane >> 1));
+      a = (lane & 1) ? e1 : e0;
+      b = (lane & 1) ? f1 : f0;
+    }
+    const R S = delay_sums(a, &carry);
+    if (c0 + lane < n) emit(c0 + lane, S);
+    if (two) {
+      const R T = delay_sums(b, &carry);
+      if (c0 + 32 + lane < n) emit(c0 + 32 + lane, T);
     }
   }
 }
