@@ -208,6 +208,9 @@ static RespWs resp_layout(char* base, const CrvParams& p, long long ne, long lon
     w.lk.seed = c.take<uint32_t>(1);
     w.lk.o_step = c.take<int64_t>(photon_cap);
     w.lk.o_time = reinterpret_cast<double*>(w.ph_t);
+    w.lk.kept = reinterpret_cast<uint16_t*>(w.slot_t);
+    const long long room = nr > 0 ? w.sc * (long long)sizeof(double) / (2 * nr) : 0;
+    w.lk.nkept = int((room < 256 ? room : 256) & ~31ll);
   }
   *bytes = c.off + 256;
   return w;

@@ -91,6 +91,8 @@ struct LookupChainWs {
   uint32_t* seed;                // device copy of the parameter block's seed
   int64_t* o_step;               // per photon: the step's row (the photon id)
   double* o_time;                // per photon: arrival time
+  uint16_t* kept;                // arrivals of each row's first nkept substeps (memory of the SiPM stage, which comes later)
+  int nkept;
 };
 cudaError_t lookup_chain_rows(const CrvParams& p, const CrvLookupChain& K, const long long* nsteps_dev,
                               long long step_cap, const LookupChainWs& w, cudaStream_t s);
