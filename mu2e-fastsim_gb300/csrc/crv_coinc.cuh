@@ -17,8 +17,8 @@
 // are formed in list order with ballots (greedy).  Decisions are FP64.
 //
 // Both kernels are bound by the latency of one warp's dependent steps and by instruction fetch, not by bytes.  Measured:
-// 512 full-detector events (9,700 hits each) 44.4 -> 5.7 ms; 65,536 one-module events (142 hits) 8.1 -> 5.7 ms, and
-// 0.64 -> 0.50 ms for the few of them above COINC_HCAP.  Testing the filter's pairs in FP32 first gave nothing (5.8 ms).
+// 512 full-detector events (9,700 hits each) 44.4 -> 5.7 ms; 65,536 one-module events (142 hits) 8.1 -> 5.7 ms
+// (4.2 with events taken as blocks finish), and 0.64 -> 0.50 ms for the few of them above COINC_HCAP.  Testing the filter's pairs in FP32 first gave nothing (5.8 ms).
 #pragma once
 #include "crv_device.cuh"
 

@@ -803,13 +803,13 @@ static PulseWs pulse_layout(char* base, long long nw, long long nsamples, size_t
   w.rec = c.take<PulseRec>(w.rc);
   w.slot_off = c.take<long long>(nw);
   w.out_off = c.take<long long>(nw);
-  w.parts = c.take<long long>(scan_parts_len(nw) + 1);
   w.totals = c.take<long long>(8);
   w.cap = c.take<int32_t>(nw);
   w.count = c.take<int32_t>(nw);
   w.q.st = c.take<PfState>(nw);
   w.q.list[0] = c.take<long long>(nw);
   w.q.list[1] = c.take<long long>(nw);
+  w.parts = w.q.list[0];         // the sums run before and after the rounds (one tile's sum needs none, more fit)
   w.q.counts = c.take<long long>(kPulseRoundsMax + 2);
   w.q.rounds = g_pulse_shape.rounds.load();
   w.q.threads = g_pulse_shape.threads.load();
