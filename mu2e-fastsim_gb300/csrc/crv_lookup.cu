@@ -324,29 +324,16 @@ __device__ __forceinline__ int ceil_uniform(unsigned long long k, int sum) {
   return int(q) + ((lo & ((1ull << 53) - 1ull)) != 0ull);
 }
 
-// arrival time of arrival j at a substep of time t (photons.py:128-137, :214-218)
-__device__ __forceinline__ double arrival_time(const CrvLookup& L, uint32_t seed, long long step, long long chan,
-                                               long long k, int tb, int bin, int j, double t, Status* status) {
+// delay of arrival j at a substep (photons.py:128-137, :214-218), and its number of emissions in a decaying fibre
+__device__ __forceinline__ double arrival_delay(const CrvLookup& L, uint32_t seed, long long step, long long chan,
+                                                long long k, int tb, int bin, int j, int* ne) {
   const CrvLookupTable& T = L.table[tb];
   const U4 w = sub_block(seed, step, chan, tb, SUB_CALL_PHOTON, 0, k, j);
   const int thr = ceil_uniform(bits53(w.x, w.y), T.delay_sum[bin]);
-  double tt = t + i2d((unsigned long long)first_reaching(T.delays, T.nbins, bin, T.ndelay, thr));
-  if (L.fiber_decay_time > 0.0) {
-    const int thr2 = ceil_uniform(bits53(w.z, w.w), T.emis_sum[bin]);
-    const int ne = first_reaching(T.emis, T.nbins, bin, T.nemis, thr2);
-    if (ne > SUB_MAX_EMISSIONS) {
-      set_flag(status, CRV_ST_LIMIT);
-    } else if (ne > 0) {
-      double g = 0.0;
-      for (int i = 0; i < ne; i += 2) {
-        const U4 v = sub_block(seed, step, chan, tb, SUB_CALL_GAMMA, i >> 1, k, j);
-        g = g - dlog(u01_open(v.x, v.y));
-        if (i + 1 < ne) g = g - dlog(u01_open(v.z, v.w));
-      }
-      tt = tt + g * L.fiber_decay_time;
-    }
-  }
-  return tt;
+  const double d = i2d((unsigned long long)first_reaching(T.delays, T.nbins, bin, T.ndelay, thr));
+  if (L.fiber_decay_time > 0.0)
+    *ne = first_reaching(T.emis, T.nbins, bin, T.nemis, ceil_uniform(bits53(w.z, w.w), T.emis_sum[bin]));
+  return d;
 }
 
 // theta bin of a row: from theta, or from cos theta against the cos of the edges
@@ -458,7 +445,7 @@ struct SubQueue {
   uint8_t table[SUB_QUEUE];
 };
 
-// Queue one chunk's arrivals (a[tb] of the lane's substep k) and call emit(slot, lane's output row) for every 32 queued,
+// Queue one chunk's arrivals (a[tb] of the lane's substep k) and call emit(queued, slot, lane's output row) by every lane for every 32 queued,
 // after the row's last chunk for what is left too.  c: queued, o: output row of the queue's front.
 template <typename T, typename Emit>
 __device__ __forceinline__ void queue_chunk(SubQueue<T>& Q, int& c, long long& o, const int a[3], const int bin[3],
@@ -487,7 +474,7 @@ __device__ __forceinline__ void queue_chunk(SubQueue<T>& Q, int& c, long long& o
     int b = 0;
 #pragma unroll 1
     for (; b + 32 <= c || (flush && b < c); b += 32) {
-      if (b + lane < c) emit(b + lane, o + lane);
+      emit(b + lane < c, b + lane, o + lane);
       o += 32;
     }
     __syncwarp();
@@ -506,6 +493,49 @@ __device__ __forceinline__ void queue_chunk(SubQueue<T>& Q, int& c, long long& o
   } while (off < sum);
 }
 
+// The emissions of the warp's arrivals (ne of them each, 0 for none): the sums of their -log u, in order.  The Philox blocks
+// of all arrivals, two emissions each, are dealt out over the lanes, 64 at a time, and each lane adds its own terms: with
+// its own emissions in each lane the warp went on, a logarithm on the FP64 pipe at a time, until the arrival with the most
+// of them was done (20,011 rows of 137 photons: emission 1.81 -> 1.41 ms; in FP32, where a logarithm is cheap, this lost:
+// 3.04 -> 3.40 ms in the lookup chain of 2,048 events).
+struct SubGamma {
+  double x[2][64];
+  int before[33], ne[32];        // blocks before each lane's, emissions
+};
+__device__ __forceinline__ double emission_sum(SubGamma& G, const SubQueue<double>& Q, int b, uint32_t seed, long long step,
+                                          long long chan, int ne) {
+  const int lane = lane_id();
+  int total;
+  const int before = warp_excl((ne + 1) >> 1, &total);
+  G.before[lane] = before;
+  G.ne[lane] = ne;
+  if (lane == 31) G.before[32] = total;
+  __syncwarp();
+  double g = 0.0;
+#pragma unroll 1
+  for (int base = 0; base < total; base += 64) {
+#pragma unroll 1
+    for (int q = base + lane; q < min(base + 64, total); q += 32) {
+      int l = 0;                                   // the last lane whose blocks start at or before q
+#pragma unroll
+      for (int step2 = 16; step2 > 0; step2 >>= 1)
+        if (G.before[l + step2] <= q) l += step2;
+      const int i = q - G.before[l];
+      const uint32_t key = Q.key[b + l];
+      const U4 v = sub_block(seed, step, chan, Q.table[b + l], SUB_CALL_GAMMA, i, (long long)(key >> 12), int(key & 0xFFFu));
+      G.x[0][q - base] = dlog(u01_open(v.x, v.y));
+      if (2 * i + 1 < G.ne[l]) G.x[1][q - base] = dlog(u01_open(v.z, v.w));
+    }
+    __syncwarp();
+    for (int q = max(before, base); q < min(before + ((ne + 1) >> 1), base + 64); ++q) {
+      g = g - G.x[0][q - base];
+      if (2 * (q - before) + 1 < ne) g = g - G.x[1][q - base];
+    }
+    __syncwarp();
+  }
+  return g;
+}
+
 // o_chan may be null (not written); a row whose offset is negative has no place in the output and is skipped
 __global__ void __launch_bounds__(SUB_ROWS_PER_BLOCK * 32) k_substep_emit(CrvLookup L, CrvSubstepRows R, uint32_t seed,
                                                                           long long nrows, RowSel sel,
@@ -516,6 +546,7 @@ __global__ void __launch_bounds__(SUB_ROWS_PER_BLOCK * 32) k_substep_emit(CrvLoo
                                                                           double* __restrict__ o_time,
                                                                           Status* status) {
   __shared__ SubQueue<double> queue[SUB_ROWS_PER_BLOCK];
+  __shared__ SubGamma gamma[SUB_ROWS_PER_BLOCK];
   SubQueue<double>& Q = queue[warp_in_block()];
   if (*total > cap) return;                                    // reported by the capacity check
   seed = sel_seed(sel, seed);
@@ -528,12 +559,24 @@ __global__ void __launch_bounds__(SUB_ROWS_PER_BLOCK * 32) k_substep_emit(CrvLoo
     const long long step = R.step[r], chan = R.chan[r];
     const SubRow w = sub_row(L, R, r, nsub);
     const double t0 = R.t0[r], dt = R.t1[r] - t0;
-    auto emit = [&](int q, long long o) {
-      o_step[o] = step;
-      if (o_chan) o_chan[o] = chan;
-      const uint32_t key = Q.key[q];
-      o_time[o] = arrival_time(L, seed, step, chan, (long long)(key >> 12), Q.table[q], Q.bin[q], int(key & 0xFFFu),
-                               Q.at[q], status);
+    auto emit = [&](bool on, int q, long long o) {
+      double tt = 0.0;
+      int ne = 0;
+      if (on) {
+        o_step[o] = step;
+        if (o_chan) o_chan[o] = chan;
+        const uint32_t key = Q.key[q];
+        tt = Q.at[q] + arrival_delay(L, seed, step, chan, (long long)(key >> 12), Q.table[q], Q.bin[q], int(key & 0xFFFu), &ne);
+        if (ne > SUB_MAX_EMISSIONS) {
+          set_flag(status, CRV_ST_LIMIT);
+          ne = 0;
+        }
+      }
+      if (L.fiber_decay_time > 0.0) {
+        const double g = emission_sum(gamma[warp_in_block()], Q, q - lane_id(), seed, step, chan, ne);
+        if (ne > 0) tt = tt + g * L.fiber_decay_time;
+      }
+      if (on) o_time[o] = tt;
     };
     const uint16_t* const kept = kept_row(sel, r);
     long long o = offset[r];
@@ -834,7 +877,8 @@ __global__ void __launch_bounds__(SUB_ROWS_PER_BLOCK * 32) k_substep_emit_f32(Cr
     long long nsub;
     if (!row_ok(R, r, &nsub, status)) continue;
     const RowF w = load_row_f(R, E, r);
-    auto emit = [&](int q, long long o) {
+    auto emit = [&](bool on, int q, long long o) {
+      if (!on) return;
       o_step[o] = w.step;
       if (o_chan) o_chan[o] = w.chan;
       const uint32_t key = Q.key[q];

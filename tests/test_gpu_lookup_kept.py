@@ -48,3 +48,22 @@ def test_fp32_rows_keep_their_photons(kind):
         s1, c1, t1 = (x.cpu().numpy() for x in eng.run(D, LK.DeviceRows(one), 9, precision="fp32"))
         m = (s == rows["step"][r]) & (c == rows["chan"][r])
         assert np.array_equal(t[m], t1)
+
+
+@pytest.mark.parametrize("columns", (2, 5, 129))
+def test_emissions_dealt_out_equal_the_oracle(columns):
+    """FP64 fibre decay with at most 1, 4 and 128 emissions per arrival (more blocks than are dealt out at a time)."""
+    import copy
+
+    from crvgpu import lookup as LK
+    L, rows = _rows("long")
+    L, rng = copy.deepcopy(L), np.random.default_rng(columns)
+    L.fiber_decay_time = 7.4
+    for t in L.tables.values():
+        t.emis = rng.integers(0, 3, (len(t.prob), columns)).astype(np.uint8)
+        t.emis[:, -1] += 1
+        t.emis_sum = t.emis.sum(1, dtype=np.int32)
+    st, ch, tm = LK.substep_photons(L, rows, 4)
+    ost, och, otm, lim = O.substep_photons(L, rows, 4)
+    assert not lim and len(st) > 1000
+    assert np.array_equal(st, ost) and np.array_equal(ch, och) and np.array_equal(tm, otm)
