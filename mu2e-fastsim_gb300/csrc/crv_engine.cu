@@ -840,19 +840,38 @@ struct PulseCaps {
   }
 };
 
+// Pulse records into the output columns: a tile of 32 waveforms per warp, a lane per pulse, so that a column's stores lie
+// next to each other (a thread per waveform: 65,536 events 0.58 -> 0.53 ms, 262,144 waveforms of five pulses 157 -> 65 us).
 __global__ void k_pulse_compact(long long nw, const long long* __restrict__ nw_dev,
                                 const long long* __restrict__ slot_off, const int32_t* __restrict__ count,
                                 const long long* __restrict__ out_off, const PulseRec* __restrict__ rec,
                                 CrvPulses O, long long out_cap) {
   nw = bounded_count(nw, nw_dev);
-  for (long long w = blockIdx.x * (long long)blockDim.x + threadIdx.x; w < nw; w += (long long)gridDim.x * blockDim.x) {
-    int c = count[w];
-    long long o0 = out_off[w], b0 = slot_off[w];
-    if (o0 + c > out_cap) continue;
-    for (int k = 0; k < c; ++k) {
-      const PulseRec& r = rec[b0 + k];
-      long long o = o0 + k;
-      O.wf[o] = w; O.seq[o] = r.seq;
+  const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
+  for (long long t = blockIdx.x * (long long)(blockDim.x >> 5) + warp_in_block(); 32 * t < nw; t += warps) {
+    const long long wl = 32 * t + lane_id();
+    int c = 0;
+    long long o0 = 0, b0 = 0;
+    if (wl < nw) {
+      c = count[wl];
+      o0 = out_off[wl];
+      b0 = slot_off[wl];
+      if (o0 + c > out_cap) c = 0;
+    }
+    int total;
+    const int before = warp_excl(c, &total);
+    for (int q0 = 0; q0 < total; q0 += 32) {
+      const int q = q0 + lane_id();
+      int l = 0;                                   // the pulse's waveform: the last lane whose pulses start at or before q
+#pragma unroll
+      for (int h = 16; h > 0; h >>= 1)
+        if (__shfl_sync(0xffffffffu, before, l + h) <= q) l += h;
+      const int k = q - __shfl_sync(0xffffffffu, before, l);
+      const long long o = __shfl_sync(0xffffffffu, o0, l) + k;
+      const long long b = __shfl_sync(0xffffffffu, b0, l) + k;
+      if (q >= total) continue;
+      const PulseRec& r = rec[b];
+      O.wf[o] = 32 * t + l; O.seq[o] = r.seq;
       O.pe[o] = r.pe; O.peph[o] = r.peph; O.time[o] = r.time; O.height[o] = r.height; O.beta[o] = r.beta;
       O.chi2[o] = r.chi2; O.letime[o] = r.letime; O.ped[o] = r.ped;
       O.fit_A[o] = r.A; O.fit_mu[o] = r.mu; O.fit_b[o] = r.b;
@@ -902,7 +921,6 @@ static int pulses_run(const CrvParams* p, int64_t nw, const long long* nw_dev, i
   size_t dummy;
   PulseWs w = pulse_layout(base, nw, nsamples, &dummy);
   CK(cudaMemsetAsync(w.q.counts, 0, (kPulseRoundsMax + 2) * sizeof(long long), s));
-  unsigned g = grid_for(nw, 256, 8);
   CK(exclusive_scan(PulseCaps{reinterpret_cast<const long long*>(off), n, nsamples, max_pulses, w.cap, w.slot_off}, nw,
                     nw_dev, scan_end(&w.totals[0]), w.parts, s));
   WaveIn W{nw, nw_dev, reinterpret_cast<const long long*>(off), n, reinterpret_cast<const long long*>(start_tdc), ped_db,
@@ -917,7 +935,7 @@ static int pulses_run(const CrvParams* p, int64_t nw, const long long* nw_dev, i
                     w.parts, s));
   {
     crv::Mark mark_("k_pulse_compact", s);
-    k_pulse_compact<<<g, 256, 0, s>>>(nw, nw_dev, w.slot_off, w.count, w.out_off, w.rec, *out, out_cap);
+    k_pulse_compact<<<grid_for(nw, 256, 8), 256, 0, s>>>(nw, nw_dev, w.slot_off, w.count, w.out_off, w.rec, *out, out_cap);
   }
   CK(cudaGetLastError());
   return CRV_OK;
