@@ -278,8 +278,12 @@ inline long long scan_tiles(long long n) {
   return n > 0 ? (n + t - 1) / t : 1;
 }
 
-// scratch of a sum over up to n items, in 8-byte words
-inline long long scan_parts_len(long long n) { return 2 * scan_tiles(n); }
+// Scratch of a sum over up to n items, in 8-byte words.  A sum over fewer items can have more tiles (of one item per
+// thread), so beyond SCAN_SINGLES it is at least that many items' tiles: one scratch then serves every sum it is sized above.
+inline long long scan_parts_len(long long n) {
+  const long long t = scan_tiles(n), most = scan_tiles(SCAN_SINGLES);
+  return 2 * (n > SCAN_SINGLES && t < most ? most : t);
+}
 
 template <int ITEMS, typename S>
 void scan_launch(const S& src, long long n, const long long* n_dev, const ScanEnds& end, typename S::V* part, long long nb,
