@@ -1102,6 +1102,7 @@ template <typename R>
 __device__ __forceinline__ bool pf_search_warp(const CrvParams& p, const WaveIn& W, const double* yscr, bool want,
                                                long long w, PfState& st) {
   const R thr = R(p.min_adc_difference);
+  __syncwarp();                        // a lane's samples (copied, or less its pulse) are read by the others below
   const long long off = want ? W.off[w] : 0;
   const int n = want ? W.n[w] : 0;
   const R* y = reinterpret_cast<const R*>(yscr) + off;
