@@ -202,6 +202,13 @@ __global__ void __launch_bounds__(256, 3) k_wf_prep(CrvParams p, CrvChannels ch,
   const typename Prep::Consts& K = K_s;
   if (Prep::LIMIT && (!Prep::ok(K) || tlen > 1024)) {
     if (threadIdx.x == 0 && blockIdx.x == 0) set_flag(status, CRV_ST_LIMIT);
+    for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < *G.n; g += (long long)gridDim.x * blockDim.x) {
+      g_bound[g] = 0;              // no group has a cluster or a digi: what follows reads these columns
+      g_maxlen[g] = 0;
+      g_nkept[g] = 0;
+      g_digis[g] = 0;
+      g_tdc0[g] = 0.0;
+    }
     return;
   }
   const int zs = p.samples_zs;
