@@ -140,8 +140,7 @@ struct Prep32 {
                                                        long long tdc0, int tlen) {
     const WfFx& F = K.F;
     long long tf, tl;
-    d2fx(t[a], &tf);
-    d2fx(t[b - 1], &tl);
+    if (!d2fx(t[a], &tf) || !d2fx(t[b - 1], &tl)) return WfCluster32{};      // the group is dropped
     const long long k0 = fx_ceil_div(tf - F.P - tdc0, F.P, F.invP);
     const long long ts = k0 * F.P + tdc0;
     const long long est = fx_floor_div(tl - tf + F.maxt, F.P, F.invP);
