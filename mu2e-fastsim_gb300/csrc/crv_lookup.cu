@@ -298,7 +298,7 @@ __device__ __forceinline__ long long arrivals(const CrvLookup& L, const CrvSubst
     const double mu = R.mu[r];
     if (ord64(mu) != 0) pr = pr * dexp(-mu * z);   // dexp(0) is 1
   }
-  if (!is_nan(pr) && ord64(pr) >= ord64(1.0)) pr = 1.0;
+  if (is_nan(pr) || ord64(pr) >= ord64(1.0)) pr = 1.0;         // (not below 1)
   return binomial(photons_per_substep(R, tb, r), pr, sub_block(seed, step, chan, tb, SUB_CALL_BINOMIAL, 0, k, 0));
 }
 
