@@ -495,17 +495,21 @@ struct SipmK {
 // functions on the IBM RISC System/6000 processor", 1990: two corrections by the exact remainder).  Five instructions;
 // the division's own sequence and slow path are 1.9 KB of code a copy in FP32, a dozen FP64 instructions in FP64.
 // Quotients below the normal range may differ in their last bits and a zero's sign is lost, neither of which an
-// exponential of the result sees.
+// exponential of the result sees.  An infinite or NaN first product (a pixel that fired at -infinity) is the quotient: the
+// remainder of it would be NaN.
 template <typename R>
 __device__ __noinline__ R div_plain(R a, R b) { return a / b; }
 __device__ __forceinline__ float fma_r(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ double fma_r(double a, double b, double c) { return __fma_rn(a, b, c); }
 __device__ __forceinline__ float mul_r(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ double mul_r(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ bool not_finite(float x) { return (__float_as_uint(x) & 0x7F800000u) == 0x7F800000u; }
+__device__ __forceinline__ bool not_finite(double x) { return (__double2hiint(x) & 0x7FF00000) == 0x7FF00000; }
 template <typename R>
 __device__ __forceinline__ R div_const(R a, R b, R y, int plain) {
   if (plain) return div_plain<R>(a, b);
   R q = mul_r(a, y);
+  if (not_finite(q)) return q;
   q = fma_r(fma_r(-q, b, a), y, q);
   return fma_r(fma_r(-q, b, a), y, q);
 }
