@@ -1049,13 +1049,14 @@ __global__ void __launch_bounds__(CO_GWARPS * 32) k_coinc_global(const __grid_co
       int ncl = 0, nmem = 0;
       for (int ti = 0; ti < G.ntypes; ++ti) {
         const int o = toff[ti], c = tcl[ti], m = tmem[ti];
-        if (c && (o != ncl || o != nmem)) {
+        if (c && o != ncl)
           warp_move(reinterpret_cast<uint32_t*>(O.rec + r0 + ncl), reinterpret_cast<const uint32_t*>(O.rec + r0 + o),
                     (long long)c * (sizeof(ClusterRec) / 4));
+        if (c && nmem)                             // (a type counts its members from 0, whether its records moved or not)
           for (int k = lane_id(); k < c; k += 32) O.rec[r0 + ncl + k].mem_begin += nmem;
+        if (c && o != nmem)
           warp_move(reinterpret_cast<uint32_t*>(O.mem_idx + r0 + nmem),
                     reinterpret_cast<const uint32_t*>(O.mem_idx + r0 + o), m);
-        }
         ncl += c;
         nmem += m;
       }
