@@ -908,6 +908,19 @@ __global__ void __launch_bounds__(SUB_ROWS_PER_BLOCK * 32) k_substep_emit_f32(Cr
   }
 }
 
+// FP32 edges of a table in shared memory: up to EDGES_MOST bytes are taken.  The emission holds its queues beside them, and
+// what does not fit the ordinary 48 KB together needs the kernel's opt-in.
+constexpr size_t EDGES_MOST = 48 * 1024;
+static size_t edges_smem(const CrvLookup& L) {
+  int nedge = 0;
+  for (int i = 0; i < 7; ++i) nedge += L.nedges[i];
+  return sizeof(float) * size_t(nedge + L.nedges[5] + L.nedges[4]);
+}
+static cudaError_t allow_edges(size_t bytes) {
+  if (bytes + sizeof(SubQueue<float>) * SUB_ROWS_PER_BLOCK <= 48 * 1024) return cudaSuccess;
+  return allow_dynamic_smem(k_substep_emit_f32);
+}
+
 struct SubWs {
   long long *count, *offset, *parts, *total;
   uint16_t* kept;
@@ -979,10 +992,9 @@ extern "C" int crv_substep_photons(const CrvLookup* L, uint32_t seed, const CrvS
   const unsigned grid = (unsigned)(blocks < maxb ? blocks : maxb);
   const bool f32 = L->precision == 1;
   const RowSel sel{nullptr, nullptr, nullptr, 0, w.kept, SUB_KEPT};
-  int nedge = 0;
-  for (int i = 0; i < 7; ++i) nedge += L->nedges[i];
-  const size_t esm = sizeof(float) * size_t(nedge + L->nedges[5] + L->nedges[4]);
-  if (f32 && esm > 48 * 1024) return CRV_ERR_ARG;
+  const size_t esm = edges_smem(*L);
+  if (f32 && esm > EDGES_MOST) return CRV_ERR_ARG;
+  if (f32 && allow_edges(esm) != cudaSuccess) return CRV_ERR_CUDA;
   if (f32) {
     crv::Mark mark_("k_substep_count", s);
     k_substep_count_f32<<<grid, SUB_ROWS_PER_BLOCK * 32, esm, s>>>(*L, *rows, seed, nrows, sel, w.count, S);
@@ -1293,12 +1305,6 @@ static CrvSubstepRows rows_in(const CrvSubstepRowsOut& o) {
   return r;
 }
 
-static size_t edges_smem(const CrvLookup& L) {
-  int nedge = 0;
-  for (int i = 0; i < 7; ++i) nedge += L.nedges[i];
-  return sizeof(float) * size_t(nedge + L.nedges[5] + L.nedges[4]);
-}
-
 static unsigned step_grid(long long n) {
   const long long blocks = (n + 255) / 256;
   const long long maxb = (long long)device_info().sms * 8;
@@ -1328,7 +1334,7 @@ cudaError_t lookup_chain_count(const CrvLookupChain& K, const LookupChainWs& w, 
   const unsigned grid = row_grid(row_cap);
   for (int k = 0; k < K.ngroups; ++k) {
     const CrvLookup& L = K.table[k];
-    if (L.precision == 1 && edges_smem(L) > 48 * 1024) return cudaErrorInvalidValue;
+    if (L.precision == 1 && edges_smem(L) > EDGES_MOST) return cudaErrorInvalidValue;
     const RowSel sel{w.nrows, w.row_group, w.seed, k, w.kept, w.nkept};
     crv::Mark mark_("k_substep_count", s);
     if (L.precision == 1)
@@ -1351,6 +1357,10 @@ cudaError_t lookup_chain_emit(const CrvLookupChain& K, const LookupChainWs& w, l
   for (int k = 0; k < K.ngroups; ++k) {
     const CrvLookup& L = K.table[k];
     const RowSel sel{w.nrows, w.row_group, w.seed, k, w.kept, w.nkept};
+    if (L.precision == 1) {
+      const cudaError_t e = allow_edges(edges_smem(L));
+      if (e != cudaSuccess) return e;
+    }
     crv::Mark mark_("k_substep_emit", s);
     if (L.precision == 1)
       k_substep_emit_f32<<<grid, SUB_ROWS_PER_BLOCK * 32, edges_smem(L), s>>>(L, R, 0u, row_cap, sel, w.row_off,
