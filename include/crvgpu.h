@@ -540,6 +540,8 @@ int crv_lookup_rows(const CrvLookupGroup *G, uint32_t seed, const CrvLookupSteps
                     CrvSubstepRowsOut *out, int64_t cap, int64_t *n_rows_dev, void *workspace, int64_t workspace_bytes,
                     void *stream, CrvStatus *status_dev);
 
+/* 512 of its bytes per row keep arrival counts between the two passes; down to that much less is accepted too, the counts
+ * without room are drawn twice (the same photons, FP32-mixed emission about a fifth slower). */
 int64_t crv_substeps_workspace(int64_t nrows);
 /* Photons of every row, in (row, substep, table, arrival) order: step index, channel, arrival time (capacity cap;
  * *n_out_dev receives the count). */

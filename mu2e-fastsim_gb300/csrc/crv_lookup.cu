@@ -926,7 +926,8 @@ struct SubWs {
   uint16_t* kept;
 };
 
-static SubWs sub_layout(char* base, long long n, size_t* bytes) {
+// least: the bytes without the kept counts, which come last
+static SubWs sub_layout(char* base, long long n, size_t* bytes, size_t* least) {
   size_t off = 0;
   auto take = [&](long long cnt) {
     off = (off + 255) & ~size_t(255);
@@ -939,6 +940,7 @@ static SubWs sub_layout(char* base, long long n, size_t* bytes) {
   w.offset = take(n);
   w.parts = take(scan_parts_len(n) + 1);
   w.total = take(1);
+  *least = ((off + 255) & ~size_t(255)) + 256;
   w.kept = reinterpret_cast<uint16_t*>(take(n * (SUB_KEPT / 4)));
   *bytes = off + 256;
   return w;
@@ -950,8 +952,8 @@ using namespace crv;
 
 extern "C" int64_t crv_substeps_workspace(int64_t nrows) {
   if (nrows < 0) return -1;
-  size_t b = 0;
-  sub_layout(nullptr, nrows, &b);
+  size_t b = 0, least = 0;
+  sub_layout(nullptr, nrows, &b, &least);
   return (int64_t)b;
 }
 
@@ -980,18 +982,20 @@ extern "C" int crv_substep_photons(const CrvLookup* L, uint32_t seed, const CrvS
       !rows->chan || !rows->n_scint || !rows->n_ck_s || !rows->n_ck_f)
     return CRV_ERR_ARG;
   if (!rows->theta && (!rows->cos_theta || !L->cos_theta_edges)) return CRV_ERR_ARG;
-  size_t need = 0;
-  sub_layout(nullptr, nrows, &need);
-  if (!workspace || (long long)need > workspace_bytes) return CRV_ERR_ARG;
+  size_t whole = 0, least = 0;
+  sub_layout(nullptr, nrows, &whole, &least);
+  if (!workspace || (long long)least > workspace_bytes) return CRV_ERR_ARG;
+  // counts kept for as many substeps of each row as there is room for (the others are drawn again)
+  const long long room = (workspace_bytes - (long long)least) / (2 * nrows);
+  const int nkept = int(room < SUB_KEPT ? room : SUB_KEPT) & ~31;
   char* base = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(workspace) + 255) & ~uintptr_t(255));
-  size_t dummy;
-  SubWs w = sub_layout(base, nrows, &dummy);
+  SubWs w = sub_layout(base, nrows, &whole, &least);
   Status* S = reinterpret_cast<Status*>(status_dev);
   const long long blocks = (nrows + SUB_ROWS_PER_BLOCK - 1) / SUB_ROWS_PER_BLOCK;
   const long long maxb = (long long)device_info().sms * 8;
   const unsigned grid = (unsigned)(blocks < maxb ? blocks : maxb);
   const bool f32 = L->precision == 1;
-  const RowSel sel{nullptr, nullptr, nullptr, 0, w.kept, SUB_KEPT};
+  const RowSel sel{nullptr, nullptr, nullptr, 0, w.kept, nkept};
   const size_t esm = edges_smem(*L);
   if (f32 && esm > EDGES_MOST) return CRV_ERR_ARG;
   if (f32 && allow_edges(esm) != cudaSuccess) return CRV_ERR_CUDA;
