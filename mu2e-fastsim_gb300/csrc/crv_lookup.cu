@@ -654,7 +654,10 @@ __device__ __forceinline__ int find_bin_cos_f(const float* ce, int ne, float c) 
   return lo - 1;
 }
 
-// 32-bit counts throughout: conversions between 64-bit integers and floats run on the FP64 pipe
+// 32-bit counts throughout: conversions between 64-bit integers and floats run on the FP64 pipe.  Where the inversion's first
+// term is below FP32's normal range (means from 88 on, from 63 at q = 1/2, up to 256; as 0 it would never let a draw end
+// before n) FP64 draws from the same words: with WIDE; else -1 is returned.
+template <bool WIDE>
 __device__ __forceinline__ int binomial_f(int n, float p, const U4& w) {
   if (n <= 0 || !(p > 0.f)) return 0;
   if (p >= 1.f) return n;
@@ -672,6 +675,10 @@ __device__ __forceinline__ int binomial_f(int n, float p, const U4& w) {
     const float s = q / (1.f - q);
     const float a = float(n + 1) * s;
     float r = __expf(float(n) * log1pf(-q));
+    if (r < 1.17549435e-38f) {
+      if constexpr (WIDE) return int(binomial_64(n, f2d(p), w));
+      else return -1;
+    }
     k = 0;
     while (u > r && k < n) {
       u = u - r;
@@ -780,12 +787,13 @@ __device__ __forceinline__ void substep_bins_f(const GeoF& g, const EdgesF& E, c
   *frac_out = frac;
 }
 
+template <bool WIDE>
 __device__ __forceinline__ int arrivals_f(const CrvLookup& L, const CrvSubstepRows& R, const RowF& w, uint32_t seed,
                                           int k, int tb, int bin, float z) {
   float pr = L.table[tb].prob[bin] * w.dev;
   if (R.mu) pr = pr * __expf(-w.mu * z);
   pr = fminf(pr, 1.f);
-  return binomial_f(w.n[tb], pr, sub_block(seed, w.step, w.chan, tb, SUB_CALL_BINOMIAL, 0, k, 0));
+  return binomial_f<WIDE>(w.n[tb], pr, sub_block(seed, w.step, w.chan, tb, SUB_CALL_BINOMIAL, 0, k, 0));
 }
 
 // offset of arrival j from the row start time (FP32: substep time, delay, fibre decay)
@@ -812,6 +820,38 @@ __device__ __forceinline__ float arrival_offset_f(const CrvLookup& L, float deca
   return off;
 }
 
+// arrivals of row r, by the warp; -1 when one of its draws needs FP64 (not with WIDE)
+template <bool WIDE>
+__device__ __forceinline__ long long count_row_f(const CrvLookup& L, const CrvSubstepRows& R, const EdgesF& E, const GeoF& g,
+                                                 uint32_t seed, const RowSel& sel, long long r, Status* status) {
+  long long nsub;
+  long long tot = 0;
+  int low = 0;
+  if (row_ok(R, r, &nsub, status)) {
+    const RowF w = load_row_f(R, E, r);
+    uint16_t* const kept = kept_row(sel, r);
+    int sum = 0;
+    for (int k = lane_id(); k < w.nsub; k += 32) {
+      int bin[3];
+      float z, frac;
+      substep_bins_f(g, E, w, k, bin, &z, &frac);
+      int in_or_fibre = 0, ck = 0;
+      for (int tb = 0; tb < 3; ++tb)
+        if (bin[tb] >= 0) {
+          int a = arrivals_f<WIDE>(L, R, w, seed, k, tb, bin[tb], z);
+          if (!WIDE) low = min(low, a);
+          if (a >= SUB_MAX_ARRIVALS) { set_flag(status, CRV_ST_LIMIT); a = 0; }
+          sum += a;
+          if (tb == 1) ck = a; else in_or_fibre = a;
+        }
+      keep_counts(kept, sel.nkept, k, in_or_fibre, ck);
+    }
+    tot = sum;
+  }
+  tot = warp_sum(tot);
+  return !WIDE && __any_sync(0xffffffffu, low < 0) ? -1 : tot;
+}
+
 __global__ void __launch_bounds__(SUB_ROWS_PER_BLOCK * 32) k_substep_count_f32(CrvLookup L, CrvSubstepRows R,
                                                                                uint32_t seed, long long nrows,
                                                                                RowSel sel,
@@ -825,30 +865,35 @@ __global__ void __launch_bounds__(SUB_ROWS_PER_BLOCK * 32) k_substep_count_f32(C
   const long long warps = (long long)gridDim.x * SUB_ROWS_PER_BLOCK;
   for (long long r = (long long)blockIdx.x * SUB_ROWS_PER_BLOCK + warp_in_block(); r < nrows; r += warps) {
     if (!sel_row(sel, r)) continue;                          // warp-uniform
-    long long nsub;
-    long long tot = 0;
-    if (row_ok(R, r, &nsub, status)) {
-      const RowF w = load_row_f(R, E, r);
-      uint16_t* const kept = kept_row(sel, r);
-      int sum = 0;
-      for (int k = lane_id(); k < w.nsub; k += 32) {
-        int bin[3];
-        float z, frac;
-        substep_bins_f(g, E, w, k, bin, &z, &frac);
-        int in_or_fibre = 0, ck = 0;
-        for (int tb = 0; tb < 3; ++tb)
-          if (bin[tb] >= 0) {
-            int a = arrivals_f(L, R, w, seed, k, tb, bin[tb], z);
-            if (a >= SUB_MAX_ARRIVALS) { set_flag(status, CRV_ST_LIMIT); a = 0; }
-            sum += a;
-            if (tb == 1) ck = a; else in_or_fibre = a;
-          }
-        keep_counts(kept, sel.nkept, k, in_or_fibre, ck);
-      }
-      tot = sum;
-    }
-    tot = warp_sum(tot);
+    const long long tot = count_row_f<false>(L, R, E, g, seed, sel, r, status);
     if (lane_id() == 0) count[r] = tot;
+  }
+}
+
+// The rows that k_substep_count_f32 left at -1, counted with FP64 draws where they are needed.  Ordinary tables have none
+// (means below 5), and the FP64 draw among the others takes registers from every warp: 200,000 rows 1.21 -> 1.34 ms, as a
+// call for a whole row 1.29; marked rows and this launch, a lane per row until one is found, 1.21 -> 1.23 + 0.01 ms.
+__global__ void __launch_bounds__(SUB_ROWS_PER_BLOCK * 32) k_substep_count_wide(CrvLookup L, CrvSubstepRows R,
+                                                                                uint32_t seed, long long nrows,
+                                                                                RowSel sel,
+                                                                                long long* __restrict__ count,
+                                                                                Status* status) {
+  extern __shared__ float edges_sm[];
+  seed = sel_seed(sel, seed);
+  nrows = sel_nrows(sel, nrows);
+  const long long tiles = (nrows + blockDim.x - 1) / blockDim.x;
+  for (long long t = blockIdx.x; t < tiles; t += gridDim.x) {
+    const long long r0 = t * blockDim.x + threadIdx.x;
+    const bool mine = r0 < nrows && sel_row(sel, r0) && count[r0] < 0;
+    if (!__syncthreads_or(mine)) continue;
+    const EdgesF E = stage_edges_f(L, edges_sm);
+    const GeoF g = geo_f(L);
+    for (unsigned m = __ballot_sync(0xffffffffu, mine); m; m &= m - 1u) {
+      const long long r = r0 - lane_id() + __ffs(m) - 1;
+      const long long tot = count_row_f<true>(L, R, E, g, seed, sel, r, status);
+      if (lane_id() == 0) count[r] = tot;
+    }
+    __syncthreads();
   }
 }
 
@@ -899,7 +944,7 @@ __global__ void __launch_bounds__(SUB_ROWS_PER_BLOCK * 32) k_substep_emit_f32(Cr
 #pragma unroll
         for (int tb = 0; tb < 3; ++tb)
           if (!drawn && bin[tb] >= 0) {
-            a[tb] = arrivals_f(L, R, w, seed, k, tb, bin[tb], z);
+            a[tb] = arrivals_f<true>(L, R, w, seed, k, tb, bin[tb], z);
             if (a[tb] >= SUB_MAX_ARRIVALS) a[tb] = 0;
           }
       }
@@ -919,6 +964,19 @@ static size_t edges_smem(const CrvLookup& L) {
 static cudaError_t allow_edges(size_t bytes) {
   if (bytes + sizeof(SubQueue<float>) * SUB_ROWS_PER_BLOCK <= 48 * 1024) return cudaSuccess;
   return allow_dynamic_smem(k_substep_emit_f32);
+}
+
+static void launch_count_f32(const CrvLookup& L, const CrvSubstepRows& R, uint32_t seed, long long nrows, const RowSel& sel,
+                             long long* count, Status* status, unsigned grid, cudaStream_t s) {
+  constexpr int TH = SUB_ROWS_PER_BLOCK * 32;
+  {
+    crv::Mark mark_("k_substep_count", s);
+    k_substep_count_f32<<<grid, TH, edges_smem(L), s>>>(L, R, seed, nrows, sel, count, status);
+  }
+  const long long blocks = (nrows + TH - 1) / TH;
+  crv::Mark mark_("k_substep_count_wide", s);
+  k_substep_count_wide<<<(unsigned)(blocks < (long long)grid ? blocks : (long long)grid), TH, edges_smem(L), s>>>(
+      L, R, seed, nrows, sel, count, status);
 }
 
 struct SubWs {
@@ -1000,8 +1058,7 @@ extern "C" int crv_substep_photons(const CrvLookup* L, uint32_t seed, const CrvS
   if (f32 && esm > EDGES_MOST) return CRV_ERR_ARG;
   if (f32 && allow_edges(esm) != cudaSuccess) return CRV_ERR_CUDA;
   if (f32) {
-    crv::Mark mark_("k_substep_count", s);
-    k_substep_count_f32<<<grid, SUB_ROWS_PER_BLOCK * 32, esm, s>>>(*L, *rows, seed, nrows, sel, w.count, S);
+    launch_count_f32(*L, *rows, seed, nrows, sel, w.count, S, grid, s);
   } else {
     crv::Mark mark_("k_substep_count", s);
     k_substep_count<<<grid, SUB_ROWS_PER_BLOCK * 32, 0, s>>>(*L, *rows, seed, nrows, sel, w.count, S);
@@ -1340,12 +1397,12 @@ cudaError_t lookup_chain_count(const CrvLookupChain& K, const LookupChainWs& w, 
     const CrvLookup& L = K.table[k];
     if (L.precision == 1 && edges_smem(L) > EDGES_MOST) return cudaErrorInvalidValue;
     const RowSel sel{w.nrows, w.row_group, w.seed, k, w.kept, w.nkept};
-    crv::Mark mark_("k_substep_count", s);
-    if (L.precision == 1)
-      k_substep_count_f32<<<grid, SUB_ROWS_PER_BLOCK * 32, edges_smem(L), s>>>(L, R, 0u, row_cap, sel, w.count,
-                                                                              status);
-    else
+    if (L.precision == 1) {
+      launch_count_f32(L, R, 0u, row_cap, sel, w.count, status, grid, s);
+    } else {
+      crv::Mark mark_("k_substep_count", s);
       k_substep_count<<<grid, SUB_ROWS_PER_BLOCK * 32, 0, s>>>(L, R, 0u, row_cap, sel, w.count, status);
+    }
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
