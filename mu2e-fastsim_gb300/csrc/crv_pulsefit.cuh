@@ -328,34 +328,21 @@ __device__ __forceinline__ float round_half_away_f(float x) {
 }
 
 // subtract round(fit) from the samples it reaches: walk out from the mode while the rounded value can be non-zero
-template <typename R>
-__device__ __forceinline__ void subtract_lane(const CrvParams& p, R* y, int n, long long st_tdc, double A,
+__device__ __forceinline__ void subtract_lane(const CrvParams& p, double* y, int n, long long st_tdc, double A,
                                               double mu, double b, int* lo_o, int* hi_o) {
   long long im = (long long)floor(mu / p.period) - st_tdc;
   if (im < 0) im = 0;
   if (im > n - 1) im = n - 1;
   int lo = int(im), hi = int(im);
-  // FP32: sample times relative to the mode's sample (exact small multiples of the period)
-  const float mu_rel = float(mu - double(st_tdc + im) * p.period);
-  const float inv_b = 1.0f / float(b), Af = float(A), Pf = float(p.period);
   for (int dir = -1; dir <= 1; dir += 2) {
     for (int i = int(im) + (dir > 0 ? 1 : 0); i >= 0 && i < n; i += dir) {
-      if (sizeof(R) == 8) {
-        double t = double(st_tdc + i) * p.period;
-        double z = (t - mu) / b;
-        double gv = A * exp(-z - exp(-z));
-        y[i] -= R(round_half_away(gv));
-        if (dir < 0) lo = i; else hi = i;
-        // unimodal: past the mode the value only shrinks; stop well below the rounding threshold
-        if (fabs(gv) < 0.25 && ((dir < 0 && t < mu) || (dir > 0 && t > mu))) break;
-      } else {
-        float tr = float(i - int(im)) * Pf;
-        float z = (tr - mu_rel) * inv_b;
-        float gv = Af * __expf(-z - __expf(-z));
-        y[i] -= R(round_half_away_f(gv));
-        if (dir < 0) lo = i; else hi = i;
-        if (fabsf(gv) < 0.25f && ((dir < 0 && tr < mu_rel) || (dir > 0 && tr > mu_rel))) break;
-      }
+      double t = double(st_tdc + i) * p.period;
+      double z = (t - mu) / b;
+      double gv = A * exp(-z - exp(-z));
+      y[i] -= round_half_away(gv);
+      if (dir < 0) lo = i; else hi = i;
+      // unimodal: past the mode the value only shrinks; stop well below the rounding threshold
+      if (fabs(gv) < 0.25 && ((dir < 0 && t < mu) || (dir > 0 && t > mu))) break;
     }
   }
   *lo_o = lo;
@@ -1075,7 +1062,7 @@ __device__ __forceinline__ bool pf_close(const CrvParams& p, const WaveIn& W, do
   st.cnt = seq + 1;
   st.fb = fseq;
   int lo, hi;
-  subtract_lane<double>(p, y, n, st_tdc, A, mu, b, &lo, &hi);
+  subtract_lane(p, y, n, st_tdc, A, mu, b, &lo, &hi);
   st.near = st.near || near_lane<double>(y, n, lo - 1, hi + 1, p.min_adc_difference, p.knife_edge_adc);
   st.start = fe;
   return st.cnt < max_pulses;
