@@ -50,3 +50,18 @@ def test_fp32_draws_of_large_means_equal_the_oracles(p, n):
     assert not want[3] and abs(len(want[0]) / (300 * 20 * n * p) - 1) < 0.01
     st, _, _ = LK.substep_photons(L, rows, 9, precision="fp32")
     assert np.array_equal(np.bincount(st, minlength=300), np.bincount(want[0], minlength=300))
+
+
+@pytest.mark.parametrize("p,n", [(2.0 ** -11, 500), (0.0015, 486), (0.01, 60), (0.03, 900), (0.2, 3), (0.2, 500), (0.48, 40),
+                                 (0.489, 170), (0.49, 40), (0.3, 420), (1e-5, 900000), (1.3e-4, 980000), (0.999, 30)])
+def test_fp64_draws_decided_in_fp32_equal_the_oracles(p, n):
+    """30,000 to 300,000 draws of each (probability, photons), from means of 0.24 to 127 at the ends of what FP32 decides: a
+    comparison trusted wrongly moves a count or the photons behind it.  Bit for bit."""
+    from crvgpu import lookup as LK
+    nsub = 1000 if n * p < 20 else 100
+    L, rows = _case(p, n, rows=300, nsub=nsub)
+    want = O.substep_photons(L, rows, 21)
+    assert not want[3] and len(want[0]) > 10000
+    got = LK.substep_photons(L, rows, 21)
+    for a, b in zip(got, want):
+        assert np.array_equal(a, b)
