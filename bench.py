@@ -955,10 +955,10 @@ def main():
     top_group = max(by_group.items(), key=lambda kv: kv[1])[0]
 
     # DRAM bytes (read + write) over algorithmic bytes of one 16,384-event chain batch, from single-kernel ncu captures
-    # of every launch of the stage in that batch (k_sipm_sim, 3 launches: 3.419 GB over 2.978 GB; k_wf_synth32,
-    # 3 launches: 1.823 GB over 1.405 GB; k_pf_persist, 1 launch: 0.757 GB over 0.396 GB); the traffic of a stage grows
-    # with the events processed, so the ratio scales it to this run's batch
-    traffic_ratio = {"k_sipm_sim": 1.148, "k_wf_synth": 1.298, "pulse fit": 1.910}
+    # of every launch of the stage in that batch (k_sipm_sim, 3 launches: 3.441 GB over 2.984 GB; k_wf_synth16 and
+    # k_wf_synth32, 4 launches: 1.646 GB over 1.407 GB; k_pf_persist, 1 launch: 0.495 GB over 0.397 GB); the traffic of a
+    # stage grows with the events processed, so the ratio scales it to this run's batch
+    traffic_ratio = {"k_sipm_sim": 1.153, "k_wf_synth": 1.170, "pulse fit": 1.247}
 
     def roofline_of(group):
         ks = groups.get(group, (group,))

@@ -8,7 +8,7 @@
 // everything that need not be FP64 arithmetic is integer or certain FP32 work: bins and box tests compare ordered bits,
 // the binomial draws are decided in FP32 where that is certain, uniforms become integer thresholds (20,011 rows of 137
 // photons: count 2.9 -> 0.33 ms, emit 8.1 -> 1.9 ms, of which the fibre-decay logarithms are most).  FP32-mixed:
-// instruction issue (200,000 rows: count 1.33 -> 1.16 ms, emit 6.8 -> 2.7 ms).
+// instruction issue (200,000 rows: count 1.33 -> 1.23 ms, emit 6.8 -> 2.25 ms).
 //
 // Layout: a warp per row, lanes over its substeps (a 20 mm crossing has 200).  Pass 1 counts the arrivals of every
 // row, an exclusive scan turns the counts into output offsets, pass 2 repeats the draws (keyed: the same numbers) and

@@ -503,9 +503,10 @@ __device__ __forceinline__ bool same3(const float a[3], const float b[3]) {
 // the state stays in registers (addresses of it are never taken).
 //
 // What bounds it.  FP32: issue slots, half of them in lanes that differ (fits take 5 to 40 evaluations, 19 on average;
-// 20 of 32 lanes take part in an evaluation).  Lanes that are done were served and refilled while others still fitted,
-// from a third or a half of the lanes on: 9.1 -> 13 and 12 ms at 65,536 events (a service costs as much as 4 to 9
-// evaluations whoever takes part), so a warp serves when all its fits are done.  FP64: the FP64 pipe, which takes 64 cycles
+// 21 of 32 lanes active per instruction on the workload's fits, 11 on uneven waveforms).  Lanes that are done were served
+// and refilled while others still fitted, from a third or a half of the lanes on: 9.1 -> 13 and 12 ms at 65,536 events (a
+// service costs as much as 4 to 9 evaluations whoever takes part), so a warp serves when all its fits are done.  FP64: the
+// FP64 pipe, which takes 64 cycles
 // of a scheduler (19 of an SM with four warps busy) per warp instruction whatever the number of its active lanes; most of
 // an evaluation is exponentials.  Hence divisions from a reciprocal, derivatives only for accepted steps, comparisons on
 // integers, the points dealt out (pf_eval_warp), small batches spread over every scheduler.

@@ -93,7 +93,7 @@ __device__ __forceinline__ int tmpl_index_f(int J, float dt, float P, float inv_
   return ti < float(tlen) ? int(ti) : -1;
 }
 
-// A kept cluster, computed once per cluster by the prepass (one thread per SiPM): t_start = k0 P + TDC0, charge rows
+// A kept cluster, computed once per cluster by the prepass (a lane per cluster): t_start = k0 P + TDC0, charge rows
 // [a, b) relative to the group start, length in samples, and the samples whose start lies in the window [ilo, ihi]
 // (valid while the length fits a synthesis pass, at most 16,384 samples).
 struct WfCluster {
